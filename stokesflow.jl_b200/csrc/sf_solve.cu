@@ -3,7 +3,10 @@
 //
 // The reference runs, per PT iteration, compute_P_tau! -> compute_dV! ->
 // compute_V! -> four BC kernels (:48-57), with tau, divV, dtau* stored as full
-// arrays.  Here one fused kernel does the whole iteration:
+// arrays.  Here sf_march.cu runs two or three whole iterations per launch, and
+// k_pt_iter (this file) runs one: the iterations whose tau and divV the
+// residual check needs, and those of a decomposed solve, which exchanges halos
+// after each:
 //
 //   * the domain is cut into BX x BY tiles of points (i, j), 0 <= i < Nx-1,
 //     0 <= j < Ny-1 (the pressure index space, which contains the dVx and dVy
@@ -23,12 +26,14 @@
 //     fourth CTA per SM);
 //   * the free-slip ghost rows / columns of the new velocities are written by
 //     the CTAs on the domain edge, in the reference's BC order (:53-56);
-//   * V and P are double-buffered (the iteration is Jacobi-like: every read is
-//     an old value), dV is updated in place.
+//   * V, P and dV are double-buffered (the iteration is Jacobi-like: every
+//     read is an old value).
 //
-// HBM bytes per iteration: read Vx, Vy, P, dVx, dVy, rho, mu_b, mu_p and write
-// Vx, Vy, P, dVx, dVy -- 13 arrays, ~104 * Nx * Ny bytes, which is all the
-// kernel reads and writes.
+// HBM bytes per iteration of k_pt_iter: read Vx, Vy, P, dVx, dVy, rho, mu_b,
+// mu_p and write Vx, Vy, P, dVx, dVy -- 13 arrays, ~104 * Nx * Ny bytes, which
+// is all the kernel reads and writes.  The march reads three arrays more
+// (dtauP, dtauVx, dtauVy) and shares its 128 bytes among the iterations of a
+// launch.
 //
 // Fields live in a padded internal layout (one leading dimension LD, a
 // multiple of 32 doubles, for every field) packed from / unpacked to the
@@ -48,19 +53,23 @@
 #include <vector>
 
 #include "sf_internal.cuh"
+#include "sf_march.cuh"
 #include "sf_tma.cuh"
 
 namespace sf {
 
+// The slabs of the march's two tensor copies first, in its order (sf_march.cuh); mu_p and what the checks write
+// behind them.  DT*: the pseudo-time steps of compute_timesteps! (:128-133); MUP2: 2 mu_p; MUB: 2.0 * mu_b * 0.5.
 enum {
-    F_VXA, F_VXB, F_VYA, F_VYB, F_PA, F_PB, F_DVX, F_DVY, F_RHO, F_MUB, F_MUP,
-    F_TXX, F_TYY, F_TXY, F_DIV, F_RX, F_RY, F_NUM
+    F_VXA, F_VYA, F_PA, F_DVXA, F_DVYA, F_VXB, F_VYB, F_PB, F_DVXB, F_DVYB, F_RHO, F_MUB, F_MUP2, F_DTP, F_DTX, F_DTY,
+    F_MUP, F_TXX, F_TYY, F_TXY, F_DIV, F_RX, F_RY, F_NUM
 };
+static_assert(F_VXB == MARCH_Z_B && F_RHO == MARCH_Z_MAT && F_MUP == MARCH_NZ, "slab order");
 
 struct Layout {
-    int64_t Nx, Ny, LD, rows, fstride;
+    int64_t Nx, Ny, LD, rows, fstride;   // rows of a field; the slabs are two rows longer (skew)
     double* base;
-    double* f(int k) const { return base + (int64_t)k * fstride; }
+    double* f(int k) const { return base + (int64_t)k * fstride + (k < MARCH_NZ ? MARCH_SKEW[k] * LD : 0); }
 };
 
 struct PTParams {
@@ -231,7 +240,7 @@ __global__ void __launch_bounds__(PT_THREADS, PT_MIN_BLOCKS) k_pt_iter(const __g
                     double vy0 = sVy[b][a], vy1 = sVy[b][a + 1];
                     double dVx_dy = (vx1 - vx0) * _dy;
                     double dVy_dx = (vy1 - vy0) * _dx;
-                    double tv = 2.0 * sMub[b][a] * 0.5 * (dVx_dy + dVy_dx);
+                    double tv = sMub[b][a] * (dVx_dy + dVy_dx);   // 2.0 * mu_b * 0.5 (k_pack_mub)
                     sTxy[b][a] = tv;
                     if (STORE && (a < BX || i == Nx - 1) && (b < BY || j == Ny - 1)) p.txy[i + (int64_t)j * LD] = tv;
                 }
@@ -498,6 +507,16 @@ __global__ void k_copy2d(double* __restrict__ dst, int64_t ld_dst, const double*
     }
 }
 
+// the factor of tau_xy, 2.0 * mu_b * 0.5 (:166): mu_b itself unless the doubling overflows
+__global__ void k_pack_mub(double* __restrict__ dst, int64_t ld_dst, const double* __restrict__ src, int64_t nx,
+                           int64_t ny) {
+    int64_t n = nx * ny;
+    for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < n; k += (int64_t)gridDim.x * blockDim.x) {
+        int64_t i = k % nx, j = k / nx;
+        dst[i + j * ld_dst] = 2.0 * src[k] * 0.5;
+    }
+}
+
 // Vx_pad[2:end-1, :] = Vx_s; Vx_pad[1,:] = -Vx_pad[3,:]; Vx_pad[end,:] = -Vx_pad[end-2,:] (:89-92, :278-282)
 __global__ void k_pad_vx(double* __restrict__ pad, const double* __restrict__ Vx, int64_t LD, int Nx, int Ny) {
     int64_t W = Nx + 2, n = W * (Ny + 1);
@@ -525,10 +544,11 @@ __global__ void k_pad_vy(double* __restrict__ pad, const double* __restrict__ Vy
 }
 
 // compute_timesteps! (:128-133): dtVx (Nx-2,Ny-1), dtVy (Nx-1,Ny-2), dtPt (Nx-1,Ny-1) with leading
-// dimensions ld_x, ld_y, ld_p (the caller's dense arrays, or the padded internal ones); NULL skips one
+// dimensions ld_x, ld_y, ld_p (the caller's dense arrays, or the padded internal ones); mup2 = 2 mu_p in the padded
+// layout; NULL skips one
 __global__ void k_timesteps(const double* __restrict__ mup, int64_t LD, int Nx, int Ny, double c_vsc, double c_ptsc,
                             double max_nxy, double* __restrict__ dtVx, int64_t ld_x, double* __restrict__ dtVy,
-                            int64_t ld_y, double* __restrict__ dtPt, int64_t ld_p) {
+                            int64_t ld_y, double* __restrict__ dtPt, int64_t ld_p, double* __restrict__ mup2) {
     int64_t W = Nx - 1, n = W * (Ny - 1);
     for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < n; k += (int64_t)gridDim.x * blockDim.x) {
         int i = (int)(k % W), j = (int)(k / W);
@@ -536,6 +556,7 @@ __global__ void k_timesteps(const double* __restrict__ mup, int64_t LD, int Nx, 
         if (dtVx && i < Nx - 2) dtVx[i + (int64_t)j * ld_x] = c_vsc / ((mup[o] + mup[o + 1]) * 0.5) / 4.1;
         if (dtVy && j < Ny - 2) dtVy[i + (int64_t)j * ld_y] = c_vsc / ((mup[o] + mup[o + LD]) * 0.5) / 4.1;
         if (dtPt) dtPt[i + (int64_t)j * ld_p] = c_ptsc * mup[o] / max_nxy;
+        if (mup2) mup2[o] = 2.0 * mup[o];
     }
 }
 
@@ -597,16 +618,16 @@ static int get_encoder(PFN_encodeTiled* out) {
     return SF_OK;
 }
 
-// rank 2 (a field of rows x ld elements) or rank 3 (nfields such fields, fstride elements apart); box depth 1
+// rank 2 (a field of rows x ld elements) or rank 3 (nfields such fields, fstride elements apart)
 static int encode_tiled(CUtensorMap* map, CUtensorMapDataType dtype, int esize, const void* base, int64_t ld,
-                        int64_t rows, int64_t nfields, int64_t fstride, int box_w, int box_h) {
+                        int64_t rows, int64_t nfields, int64_t fstride, int box_w, int box_h, int box_d = 1) {
     PFN_encodeTiled fn = nullptr;
     int rc = get_encoder(&fn);
     if (rc) return rc;
     const cuuint32_t rank = nfields > 0 ? 3 : 2;
     cuuint64_t dims[3] = {(cuuint64_t)ld, (cuuint64_t)rows, (cuuint64_t)(nfields > 0 ? nfields : 1)};
     cuuint64_t strides[2] = {(cuuint64_t)ld * (cuuint64_t)esize, (cuuint64_t)fstride * (cuuint64_t)esize};
-    cuuint32_t box[3] = {(cuuint32_t)box_w, (cuuint32_t)box_h, 1};
+    cuuint32_t box[3] = {(cuuint32_t)box_w, (cuuint32_t)box_h, (cuuint32_t)box_d};
     cuuint32_t estr[3] = {1, 1, 1};
     CUresult r = fn(map, dtype, rank, (void*)base, dims, strides, box, estr,
                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -631,8 +652,10 @@ struct Solver {
     Layout L;
     PTParams pt;
     ResParams rp;
+    MarchMaps march_maps;
+    MarchParams mp[MARCH_MAX_T + 1];  // [T]: plan and parameters of T iterations per launch
     TmaMaps maps[2];  // [cur]: inputs read from the A (cur = 0) or B (cur = 1) buffers
-    int cur = 0;      // 0: current V/P in A buffers, 1: in B buffers
+    int cur = 0;      // 0: the current state in the A buffers, 1: in the B buffers
     int res_blocks = 0;
     int maxv_blocks = 0;
     int pt_blocks = 0;
@@ -646,10 +669,17 @@ struct Solver {
                 int rc = encode_tmap_f64(&maps[c].f[k], L.f(fields[k]), LD, R, TW, TH);
                 if (rc) return rc;
             }
-            int rc = encode_tmap_f64(&maps[c].dvx, L.f(F_DVX), LD, R, BX, BY);
-            if (!rc) rc = encode_tmap_f64(&maps[c].dvy, L.f(F_DVY), LD, R, BX, BY);
+            int rc = encode_tmap_f64(&maps[c].dvx, L.f(c ? F_DVXB : F_DVXA), LD, R, BX, BY);
+            if (!rc) rc = encode_tmap_f64(&maps[c].dvy, L.f(c ? F_DVYB : F_DVYA), LD, R, BX, BY);
             if (rc) return rc;
         }
+        // all slabs as one 3-D tensor (the slab is z)
+        int rc3 = encode_tiled(&march_maps.state, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 8, L.base, LD, R + 2, MARCH_NZ,
+                               L.fstride, MARCH_CW, 1, MARCH_Z_B - MARCH_Z_A);
+        if (!rc3)
+            rc3 = encode_tiled(&march_maps.mat, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 8, L.base, LD, R + 2, MARCH_NZ,
+                               L.fstride, MARCH_CW, 1, MARCH_NZ - MARCH_Z_MAT);
+        if (rc3) return rc3;
         static bool attr_set = false;
         if (!attr_set) {
             SF_CUDA(cudaFuncSetAttribute(k_pt_iter<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
@@ -671,16 +701,34 @@ struct Solver {
         pt.Vx_out = L.f(cur ? F_VXA : F_VXB);
         pt.Vy_out = L.f(cur ? F_VYA : F_VYB);
         pt.P_out = L.f(cur ? F_PA : F_PB);
+        pt.dVx = L.f(cur ? F_DVXA : F_DVXB);
+        pt.dVy = L.f(cur ? F_DVYA : F_DVYB);
+        const TmaMaps& m = maps[cur];
         dim3 block(BX, TY);
         if (store)
-            k_pt_iter<true><<<pt_blocks, block, SMEM_BYTES, s>>>(maps[cur], pt);
+            k_pt_iter<true><<<pt_blocks, block, SMEM_BYTES, s>>>(m, pt);
         else
-            k_pt_iter<false><<<pt_blocks, block, SMEM_BYTES, s>>>(maps[cur], pt);
+            k_pt_iter<false><<<pt_blocks, block, SMEM_BYTES, s>>>(m, pt);
         SF_LAUNCHED(ctx);
         cur ^= 1;
         return SF_OK;
     }
 
+    // T iterations in one launch
+    int launch_march(int T) {
+        MarchParams& m = mp[T];
+        m.z_in = cur ? MARCH_Z_B : MARCH_Z_A;
+        cur ^= 1;
+        m.Vx_out = const_cast<double*>(Vx_cur());
+        m.Vy_out = const_cast<double*>(Vy_cur());
+        m.P_out = const_cast<double*>(P_cur());
+        m.dVx_out = dVx_cur();
+        m.dVy_out = dVy_cur();
+        return march_launch(ctx, march_maps, m, T, s);
+    }
+
+    double* dVx_cur() const { return L.f(cur ? F_DVXB : F_DVXA); }
+    double* dVy_cur() const { return L.f(cur ? F_DVYB : F_DVYA); }
     const double* Vx_cur() const { return L.f(cur ? F_VXB : F_VXA); }
     const double* Vy_cur() const { return L.f(cur ? F_VYB : F_VYA); }
     const double* P_cur() const { return L.f(cur ? F_PB : F_PA); }
@@ -721,7 +769,7 @@ struct SolveArgs {
 // ones on a single domain.
 static int solver_prepare(Solver& S, sf_ctx* ctx, cudaStream_t s, const SolveArgs& A, int64_t Nx, int64_t Ny,
                           double g_y, double dx, double dy, double dt, double maxdisp, int use_stab, int64_t nx_g,
-                          int64_t ny_g) {
+                          int64_t ny_g, bool march) {
     int rc;
     S.ctx = ctx;
     S.s = s;
@@ -729,7 +777,7 @@ static int solver_prepare(Solver& S, sf_ctx* ctx, cudaStream_t s, const SolveArg
     S.L.Ny = Ny;
     S.L.LD = round_up(Nx + 2, 32);
     S.L.rows = Ny + 3;
-    S.L.fstride = S.L.LD * S.L.rows;
+    S.L.fstride = S.L.LD * (S.L.rows + 2);
     size_t fbytes = (size_t)S.L.fstride * 8 * F_NUM;
     bool fresh = fbytes > ctx->fields.bytes;
     if ((rc = ensure(ctx, ctx->fields, fbytes))) return rc;
@@ -755,27 +803,33 @@ static int solver_prepare(Solver& S, sf_ctx* ctx, cudaStream_t s, const SolveArg
     const int64_t LD = S.L.LD;
     struct Pk { int f; const double* src; int64_t nx, ny; } packs[] = {
         {F_VXA, A.Vx_s, Nx, Ny + 1}, {F_VYA, A.Vy_s, Nx + 1, Ny}, {F_PA, A.P, Nx - 1, Ny - 1},
-        {F_DVX, A.dVxdt, Nx - 2, Ny - 1}, {F_DVY, A.dVydt, Nx - 1, Ny - 2}, {F_RHO, A.rho_vy, Nx + 1, Ny},
-        {F_MUB, A.mu_b, Nx, Ny}, {F_MUP, A.mu_p, Nx - 1, Ny - 1}};
+        {F_DVXA, A.dVxdt, Nx - 2, Ny - 1}, {F_DVYA, A.dVydt, Nx - 1, Ny - 2}, {F_RHO, A.rho_vy, Nx + 1, Ny},
+        {F_MUP, A.mu_p, Nx - 1, Ny - 1}};
     for (const Pk& k : packs) {
         k_copy2d<<<copy_blocks(ctx, k.nx * k.ny), 256, 0, s>>>(S.L.f(k.f), LD, k.src, k.nx, k.nx, k.ny);
         SF_LAUNCHED(ctx);
     }
+    k_pack_mub<<<copy_blocks(ctx, Nx * Ny), 256, 0, s>>>(S.L.f(F_MUB), LD, A.mu_b, Nx, Ny);
+    SF_LAUNCHED(ctx);
     k_set_scalar<<<1, 1, 0, s>>>(ctx->d_scalars + SC_DT, dt);
     SF_LAUNCHED(ctx);
-    // compute_timesteps! (:34) into the caller's work arrays, if given; the fused kernel computes the same
+    if (march) {   // the march streams the pseudo-time steps and 2 mu_p
+        k_timesteps<<<copy_blocks(ctx, (Nx - 1) * (Ny - 1)), 256, 0, s>>>(
+            S.L.f(F_MUP), LD, (int)Nx, (int)Ny, Vsc * min_dxy2, Ptsc * 4.1, max_nxy, S.L.f(F_DTX), LD, S.L.f(F_DTY),
+            LD, S.L.f(F_DTP), LD, S.L.f(F_MUP2));
+        SF_LAUNCHED(ctx);
+    }
+    // compute_timesteps! (:34) into the caller's work arrays, if given; k_pt_iter computes the same
     // pseudo-time steps from the staged mu_p as it needs them
     if (A.dtVx || A.dtVy || A.dtPt) {
         k_timesteps<<<copy_blocks(ctx, (Nx - 1) * (Ny - 1)), 256, 0, s>>>(S.L.f(F_MUP), LD, (int)Nx, (int)Ny,
                                                                          Vsc * min_dxy2, Ptsc * 4.1, max_nxy,
                                                                          A.dtVx, Nx - 2, A.dtVy, Nx - 1, A.dtPt,
-                                                                         Nx - 1);
+                                                                         Nx - 1, nullptr);
         SF_LAUNCHED(ctx);
     }
 
     PTParams& pt = S.pt;
-    pt.dVx = S.L.f(F_DVX);
-    pt.dVy = S.L.f(F_DVY);
     pt.rho = S.L.f(F_RHO);
     pt.mub = S.L.f(F_MUB);
     pt.mup = S.L.f(F_MUP);
@@ -804,6 +858,21 @@ static int solver_prepare(Solver& S, sf_ctx* ctx, cudaStream_t s, const SolveArg
     pt.err_flag = ctx->d_flags;
     SF_CUDA(cudaMemsetAsync(ctx->d_flags, 0, sizeof(int), s));
     if ((rc = S.setup_maps())) return rc;
+    for (int T = 1; march && T <= MARCH_MAX_T; ++T) {
+        MarchParams& m = S.mp[T];
+        m = MarchParams{};
+        m.dt_ptr = pt.dt_ptr;
+        m.Nx = pt.Nx;
+        m.Ny = pt.Ny;
+        m.LD = LD;
+        m._dx = pt._dx;
+        m._dy = pt._dy;
+        m.g_y = g_y;
+        m.dampX = dampX;
+        m.dampY = dampY;
+        m.err_flag = pt.err_flag;
+        march_plan(m, T, ctx->num_sms);
+    }
     ResParams& rp = S.rp;
     rp.txx = S.L.f(F_TXX);
     rp.tyy = S.L.f(F_TYY);
@@ -830,7 +899,7 @@ static int solver_unpack(Solver& S, const SolveArgs& A, int64_t niter, int64_t n
     const int64_t Nx = S.L.Nx, Ny = S.L.Ny, LD = S.L.LD;
     struct Uk { double* dst; const double* src; int64_t nx, ny; } unpacks[] = {
         {A.Vx_s, S.Vx_cur(), Nx, Ny + 1}, {A.Vy_s, S.Vy_cur(), Nx + 1, Ny}, {A.P, S.P_cur(), Nx - 1, Ny - 1},
-        {A.dVxdt, S.L.f(F_DVX), Nx - 2, Ny - 1}, {A.dVydt, S.L.f(F_DVY), Nx - 1, Ny - 2},
+        {A.dVxdt, S.dVx_cur(), Nx - 2, Ny - 1}, {A.dVydt, S.dVy_cur(), Nx - 1, Ny - 2},
         {A.txx, S.L.f(F_TXX), Nx - 1, Ny - 1}, {A.tyy, S.L.f(F_TYY), Nx - 1, Ny - 1}, {A.txy, S.L.f(F_TXY), Nx, Ny},
         {A.divV, S.L.f(F_DIV), Nx - 1, Ny - 1},
         {nchecks ? A.Rx : nullptr, S.L.f(F_RX), Nx - 2, Ny - 1}, {nchecks ? A.Ry : nullptr, S.L.f(F_RY), Nx - 1, Ny - 2}};
@@ -1059,7 +1128,8 @@ int sf_solve_stokes(sf_ctx* ctx, double* P, double* Vx_pad, double* Vy_pad, cons
     Solver S;
     const SolveArgs A{P, Vx_pad, Vy_pad, rho_vy, mu_b, mu_p, txx, tyy, txy, divV, dtPt, Rx, Ry, dVxdt, dVydt,
                       dtVx, dtVy, Vx_s, Vy_s};
-    if ((rc = solver_prepare(S, ctx, s, A, Nx, Ny, g_y, dx, dy, dt, maxdisp, use_stab, Nx, Ny))) return rc;
+    if ((rc = solver_prepare(S, ctx, s, A, Nx, Ny, g_y, dx, dy, dt, maxdisp, use_stab, Nx, Ny, true)))
+        return rc;
     const int64_t mnxy = std::min(Nx, Ny);
     const int64_t ncheck = std::min<int64_t>(5 * mnxy, 2000);  // :35
     const int64_t ndtupdate = 10 * mnxy;                       // :36
@@ -1068,6 +1138,7 @@ int sf_solve_stokes(sf_ctx* ctx, double* P, double* Vx_pad, double* Vy_pad, cons
     double err = 2.0 * eps;
     int64_t iter = 1, niter = 0, nchecks = 0;
     const int64_t itert1 = 11;
+    const int march_t = march_iterations(Nx, Ny);
     bool have_t1 = false;
     int64_t fused = 0;
     SF_CUDA(cudaEventRecord(ctx->ev_c, s));
@@ -1080,8 +1151,18 @@ int sf_solve_stokes(sf_ctx* ctx, double* P, double* Vx_pad, double* Vy_pad, cons
                 SF_CUDA(cudaEventRecord(ctx->ev_a, s));
                 have_t1 = true;
             }
-            bool store = (it % ncheck == 0) || (it == iter_max);
-            if ((rc = S.launch_iter(store))) return rc;
+            // the last iteration before the residual check (or the end) stores tau and divV; the ones before it
+            // run several to a launch, up to the next dt update and to where the timing starts
+            int64_t stop = last - 1;
+            if (use_stab) stop = std::min(stop, ((it - 1) / ndtupdate + 1) * ndtupdate);
+            if (it < itert1) stop = std::min(stop, itert1 - 1);
+            if (it <= stop) {
+                const int T = (int)std::min<int64_t>(march_t, stop - it + 1);
+                if ((rc = S.launch_march(T))) return rc;
+                it += T - 1;
+            } else if ((rc = S.launch_iter(true))) {
+                return rc;
+            }
             ++fused;
             bool dt_up = use_stab && (it % ndtupdate == 0);
             bool check = (it % ncheck == 0);
@@ -1193,7 +1274,8 @@ int sf_solve_stokes_decomposed(sf_domain* domains, int32_t dims_x, int32_t dims_
         k.up = nb(d.coord_x, d.coord_y + 1);
         k.A = SolveArgs{d.P, d.Vx_pad, d.Vy_pad, d.rho_vy, d.mu_b, d.mu_p, nullptr, nullptr, nullptr, nullptr, nullptr,
                         nullptr, nullptr, d.dVxdt, d.dVydt, nullptr, nullptr, d.Vx_s, d.Vy_s};
-        if ((rc = solver_prepare(k.S, k.ctx, k.s, k.A, Nx, Ny, g_y, dx, dy, dt, maxdisp, use_stab, nx_g, ny_g)))
+        if ((rc = solver_prepare(k.S, k.ctx, k.s, k.A, Nx, Ny, g_y, dx, dy, dt, maxdisp, use_stab, nx_g, ny_g,
+                                 false)))
             return rc;
         SF_CUDA(cudaEventRecord(k.ev, k.s));
     }
