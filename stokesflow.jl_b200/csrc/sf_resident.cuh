@@ -1,0 +1,57 @@
+// sf_resident.cuh -- many pseudo-transient iterations of a small grid in one launch
+// (sf_resident.cu): the kernel's parameters, its plan and its host-side launcher.
+#pragma once
+
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+#include "sf_internal.cuh"
+
+namespace sf {
+
+constexpr int RESIDENT_MIN_ITERS = 4;       // fewer are faster by the march
+constexpr int RESIDENT_MAX_ITERS = 20000;   // of one launch
+
+struct ResidentParams {
+    // the state that is read, the state that is written (other buffers) and the parameters, all in the padded layout
+    const double *Vx_in, *Vy_in, *P_in, *dVx_in, *dVy_in;
+    double *Vx_out, *Vy_out, *P_out, *dVx_out, *dVy_out;
+    const double *rho, *mub, *mup2, *dtp, *dtx, *dty;   // mub = 2.0 mu_b 0.5, mup2 = 2 mu_p
+    const double* dt_ptr;
+    int Nx, Ny;
+    int64_t LD;
+    double _dx, _dy, g_y, dampX, dampY;
+    int ntx, nty, W, H;          // tiles, and the points of one
+    int iters;
+    uint32_t tag0;               // iteration k (0-based) publishes with tag tag0 + k
+    ulonglong2* comm;            // received halo entries, [parity][tile][slot]
+    int* err_flag;
+};
+
+struct ResidentPlan {
+    bool fits = false;           // the grid is small enough for one tile per SM
+    int ntx = 0, nty = 0, W = 0, H = 0, k = 0, threads = 0, smem = 0;
+    int share = 0;               // quarters of an SM that a tile takes: 1, 2 or 4
+};
+
+// Room on a device for the tiles of a plan, held while a solve uses it.  The tiles of a launch wait for one another, so
+// all must become resident whatever else runs: concurrent solves (other threads, streams and contexts) hold at most
+// four quarters of every SM together.  Then a tile of one quarter always finds a place (an SM without one holds four
+// quarters already, and not all SMs can); its launch ends; and what is left of two and four quarters finds its place
+// in turn.  A solve that gets no room marches instead (same results).
+class ResidentRoom {
+   public:
+    ~ResidentRoom() { release(); }
+    bool acquire(int device, int num_sms, const ResidentPlan& plan, cudaStream_t s);
+    void release();
+
+   private:
+    int device_ = -1, held_ = 0;
+    cudaStream_t stream_ = nullptr;
+};
+
+ResidentPlan resident_plan(int64_t Nx, int64_t Ny, int num_sms);
+// `iters` iterations (p.iters); p.tag0 and p.comm are set here
+int resident_launch(sf_ctx* ctx, ResidentParams& p, const ResidentPlan& plan, cudaStream_t s);
+
+}  // namespace sf

@@ -54,6 +54,7 @@
 
 #include "sf_internal.cuh"
 #include "sf_march.cuh"
+#include "sf_resident.cuh"
 #include "sf_tma.cuh"
 
 namespace sf {
@@ -654,6 +655,8 @@ struct Solver {
     ResParams rp;
     MarchMaps march_maps;
     MarchParams mp[MARCH_MAX_T + 1];  // [T]: plan and parameters of T iterations per launch
+    ResidentPlan plan;
+    ResidentParams res;
     TmaMaps maps[2];  // [cur]: inputs read from the A (cur = 0) or B (cur = 1) buffers
     int cur = 0;      // 0: the current state in the A buffers, 1: in the B buffers
     int res_blocks = 0;
@@ -725,6 +728,24 @@ struct Solver {
         m.dVx_out = dVx_cur();
         m.dVy_out = dVy_cur();
         return march_launch(ctx, march_maps, m, T, s);
+    }
+
+    // n iterations of a small grid in one launch
+    int launch_resident(int n) {
+        ResidentParams& r = res;
+        r.Vx_in = Vx_cur();
+        r.Vy_in = Vy_cur();
+        r.P_in = P_cur();
+        r.dVx_in = dVx_cur();
+        r.dVy_in = dVy_cur();
+        cur ^= 1;
+        r.Vx_out = const_cast<double*>(Vx_cur());
+        r.Vy_out = const_cast<double*>(Vy_cur());
+        r.P_out = const_cast<double*>(P_cur());
+        r.dVx_out = dVx_cur();
+        r.dVy_out = dVy_cur();
+        r.iters = n;
+        return resident_launch(ctx, r, plan, s);
     }
 
     double* dVx_cur() const { return L.f(cur ? F_DVXB : F_DVXA); }
@@ -872,6 +893,27 @@ static int solver_prepare(Solver& S, sf_ctx* ctx, cudaStream_t s, const SolveArg
         m.dampY = dampY;
         m.err_flag = pt.err_flag;
         march_plan(m, T, ctx->num_sms);
+    }
+    if (march) {
+        ResidentParams& r = S.res;
+        r = ResidentParams{};
+        r.rho = pt.rho;
+        r.mub = pt.mub;
+        r.mup2 = S.L.f(F_MUP2);
+        r.dtp = S.L.f(F_DTP);
+        r.dtx = S.L.f(F_DTX);
+        r.dty = S.L.f(F_DTY);
+        r.dt_ptr = pt.dt_ptr;
+        r.Nx = pt.Nx;
+        r.Ny = pt.Ny;
+        r.LD = LD;
+        r._dx = pt._dx;
+        r._dy = pt._dy;
+        r.g_y = g_y;
+        r.dampX = dampX;
+        r.dampY = dampY;
+        r.err_flag = pt.err_flag;
+        S.plan = resident_plan(Nx, Ny, ctx->num_sms);
     }
     ResParams& rp = S.rp;
     rp.txx = S.L.f(F_TXX);
@@ -1135,6 +1177,8 @@ int sf_solve_stokes(sf_ctx* ctx, double* P, double* Vx_pad, double* Vy_pad, cons
     const int64_t ndtupdate = 10 * mnxy;                       // :36
 
     // ---- PT loop (:43-77) ----
+    ResidentRoom room;
+    const bool resident = iter_max >= RESIDENT_MIN_ITERS && room.acquire(ctx->device, ctx->num_sms, S.plan, s);
     double err = 2.0 * eps;
     int64_t iter = 1, niter = 0, nchecks = 0;
     const int64_t itert1 = 11;
@@ -1156,7 +1200,11 @@ int sf_solve_stokes(sf_ctx* ctx, double* P, double* Vx_pad, double* Vy_pad, cons
             int64_t stop = last - 1;
             if (use_stab) stop = std::min(stop, ((it - 1) / ndtupdate + 1) * ndtupdate);
             if (it < itert1) stop = std::min(stop, itert1 - 1);
-            if (it <= stop) {
+            if (it <= stop && resident && stop - it + 1 >= RESIDENT_MIN_ITERS) {
+                const int64_t n = std::min<int64_t>(stop - it + 1, RESIDENT_MAX_ITERS);
+                if ((rc = S.launch_resident((int)n))) return rc;
+                it += n - 1;
+            } else if (it <= stop) {
                 const int T = (int)std::min<int64_t>(march_t, stop - it + 1);
                 if ((rc = S.launch_march(T))) return rc;
                 it += T - 1;

@@ -1,20 +1,28 @@
-"""Several PT iterations per launch (sf_march.cu) against the oracle, bit for bit, at the sizes where its split into
-strips of columns and segments of rows changes: the smallest grids, the widest grid of one strip (59 points) and its
-neighbours, odd strip widths, several strips, segments of two rows and of many, and iteration counts that leave one
-and two iterations over.  No tolerance: every expression is evaluated in the reference's order."""
+"""Several PT iterations per launch against the oracle, bit for bit.  No tolerance: every expression is evaluated in
+the reference's order.
+
+* resident iterations (sf_resident.cu): the smallest grids, both sides of the one-tile limit (800 points), ragged last
+  tiles, one to four points per thread, thin tiles with more halo slots than threads, the largest grid;
+* the march (sf_march.cu), on grids beyond that, at the sizes where its split into strips of columns and segments of rows
+  changes: the narrowest grids (one strip), odd strip widths, short and long segments, and iteration counts that leave one
+  and two iterations over (the first ten and chunks of up to three iterations run on every grid)."""
 import numpy as np
 import pytest
 
 from fields import random_fields
-from test_gpu_parity import NAMES, gpu_solve
+from test_gpu_parity import NAMES, dev, gpu_solve, host
 
 pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("Nx,Ny,iters,stab", [
-    (4, 4, 60, True), (5, 9, 61, True), (9, 5, 62, False), (58, 21, 230, True), (59, 22, 231, True), (60, 23, 232, True),
-    (61, 4, 61, True), (113, 30, 320, True), (114, 31, 321, True), (171, 7, 150, True), (20, 700, 260, True),
-    (233, 129, 700, True), (300, 301, 500, False), (700, 61, 700, True), (801, 903, 94, True)])
+    # resident
+    (4, 4, 60, True), (5, 9, 61, True), (9, 5, 62, False), (27, 31, 300, True), (28, 31, 301, True), (59, 22, 231, True),
+    (61, 4, 61, True), (114, 31, 321, True), (20, 700, 260, True), (3000, 20, 230, True), (233, 129, 700, True),
+    (300, 301, 500, False), (511, 385, 94, True), (550, 552, 61, True),
+    # march
+    (552, 551, 62, True), (58, 5400, 63, True), (59, 5400, 64, True), (60, 5300, 65, True), (5400, 60, 66, True),
+    (20000, 17, 187, True), (801, 903, 94, False), (1023, 1101, 41, True)])
 def test_march_bitexact(sf, oracle_lib, Nx, Ny, iters, stab):
     O = oracle_lib
     dx, dy = 1.0 / (Nx - 1), 1.2 / (Ny - 1)
@@ -30,3 +38,38 @@ def test_march_bitexact(sf, oracle_lib, Nx, Ny, iters, stab):
     assert info["dt"] == r.dt
     for k in NAMES:
         assert np.array_equal(b[k], a[k], equal_nan=True), f"{k} differs from the oracle"
+
+
+def test_concurrent_solves_bitexact(sf, oracle_lib):
+    """Solves of several threads at once, contexts and streams of their own, more of them than the device has room for
+    resident tiles (the rest marches): each equals the oracle."""
+    import threading
+
+    import torch
+
+    O = oracle_lib
+    Nx, Ny, iters, n = 300, 260, 150, 6
+    dx, dy = 1.0 / (Nx - 1), 1.0 / (Ny - 1)
+    want, got = [], [None] * n
+    for k in range(n):
+        a = O.stokes_arrays(Nx, Ny)
+        a["rho_vy"][:], a["mu_b"][:], a["mu_p"][:] = random_fields(Nx, Ny, seed=k, contrast=5.0)
+        want.append(a)
+
+    def one(k, a):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            t = {q: dev(v) for q, v in a.items()}
+            sf.solve_stokes_info(*[t[q] for q in NAMES], 9.81, dx, dy, Nx, Ny, 1e-3, 0.5, eps=1e-300, iter_max=iters,
+                                 ctx=sf.Context(0))
+            got[k] = {q: host(v) for q, v in t.items()}
+
+    threads = [threading.Thread(target=one, args=(k, {q: v.copy(order="F") for q, v in a.items()}))
+               for k, a in enumerate(want)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for k, a in enumerate(want):
+        O.solve_stokes(a, 9.81, dx, dy, Nx, Ny, 1e-3, 0.5, True, 1e-300, iters)
+        for q in NAMES:
+            assert np.array_equal(got[k][q], a[q]), f"solve {k}: {q} differs from the oracle"
