@@ -352,7 +352,9 @@ typedef struct {
                                   fastest per point is then used and recorded in the context, so later
                                   rounds and solves of that class take it at once.  Every shape and
                                   schedule computes the same bits, so the choice changes the speed
-                                  only (0)                                                            */
+                                  only.  A batched solve (not an engine) whose sweeps' second rate
+                                  buffers fit the device runs three sweeps per launch instead, in rounds
+                                  after its class is recorded; the same bits again (0)                 */
     int32_t tile_schedule;     /* with tile_rows set: 1 strided (CTA b of G takes tiles b, b+G, ...),
                                   2 chunked (CTA b takes one contiguous run of tiles); 0 = 1.  With
                                   tile_rows 0 it must be 0 (0)                                        */

@@ -25,7 +25,8 @@
 // checks are replayed from captured CUDA graphs.  The tile rows (8, 16, 32),
 // the order in which the CTAs take the tiles and whether consecutive sweeps
 // overlap their launches are chosen per workload class by timing them (the
-// tuner); every choice computes the same bits.  Instances move between phases
+// tuner); every choice computes the same bits.  A batched solve's sweeps run
+// three to a launch instead (sf_mixed_march.cuh).  Instances move between phases
 // independently, which is what lets a serving loop add and retire instances
 // while others run.
 //
@@ -74,13 +75,16 @@ struct Shape {
 constexpr uint64_t WAIT_BUDGET_NS = 2000000000ull;
 
 // FP32 fields of an instance (each LD32 x rows floats)
-enum { G_VXA, G_VXB, G_VYA, G_VYB, G_PA, G_PB, G_RVX, G_RVY, G_MUB, G_MUP, G_RHO, G_RX, G_RY, G_RDIV, G_NUM };
+// FP32 fields in the order of the march's copies (sf_mixed_march.cuh); the last two, the rates' second buffers, only
+// where the engine lays them out (Inst::rates_b)
+enum { G_VXA, G_VYA, G_PA, G_VXB, G_VYB, G_PB, G_RVX, G_RVY, G_RHO, G_MUB, G_MUP, G_RDIV, G_RX, G_RY, G_NUM,
+       G_RVXB = G_NUM, G_RVYB, G_NUM_B };
 // FP64 fields of an instance (each LD64 x rows doubles)
 enum { D_VX, D_VY, D_P, D_RHO, D_MUB, D_MUP, D_NUM };
-// tensor maps per instance, in the order a stage is filled
-// tensor maps per instance and shape: all G_NUM FP32 fields as one 3-D tensor (the field index is z), read
-// through a halo box and through a tile box
+// tensor maps per instance and shape: all FP32 fields as one 3-D tensor (the field index is z), read through a halo box
+// and through a tile box; the march's, read through boxes of one row of one, two and three fields, in a set of their own
 enum { M_HALO, M_TILE, M_NUM };
+enum { M_ROW1, M_ROW2, M_ROW3, M_NUM_MARCH };
 
 struct Inst {  // device-side description of one instance
     int Nx, Ny;
@@ -100,6 +104,8 @@ struct Inst {  // device-side description of one instance
     double dx, dy, _dx, _dy, g_y, dt, dt_cfl, dt_in, maxdisp;
     int use_stab;
     int dtau_max;           // pseudo-time step from the stencil's largest viscosity
+    int rates_b;            // the rates have second buffers
+    int pad2_;
 };
 
 // Per-instance control word, written by host copies between rounds only (never by a kernel):
@@ -107,8 +113,9 @@ struct Inst {  // device-side description of one instance
 //   budget  sweeps the instance runs in this round: it sweeps in launches 0 .. budget-1 of the round and
 //           sits out the rest, so that every round ends exactly where the reference's loop has an event
 //           (a dt update every ndtupdate iterations, a residual check every ncheck, iterMax);
-//   flags   the events at the end of that round (CTL_DT, CTL_CHECK), read by the FP64 kernels of the next.
-struct Ctl { int parity, budget, flags, pad_; };
+//   flags   the events at the end of that round (CTL_DT, CTL_CHECK), read by the FP64 kernels of the next;
+//   rparity likewise which rate buffer holds the current rates (k_pt32 updates them in place).
+struct Ctl { int parity, budget, flags, rparity; };
 enum { CTL_DT = 1, CTL_CHECK = 2 };
 
 __device__ __forceinline__ float* gf(const Inst& I, int k) { return I.f32 + (int64_t)k * I.fstride32; }
@@ -202,8 +209,9 @@ __global__ void __launch_bounds__(NT, MINB) k_pt32(const CUtensorMap* __restrict
         tma_load_3d(st + 5 * HALO_BYTES, H, &bar[s], i0, j0, G_RHO);
         tma_load_3d(st + 6 * HALO_BYTES, H, &bar[s], i0, j0, G_RDIV);
         unsigned char* tb = st + NHALO * HALO_BYTES;
-        tma_load_3d(tb + 0 * TILE_BYTES, T, &bar[s], i0, j0, G_RVX);
-        tma_load_3d(tb + 1 * TILE_BYTES, T, &bar[s], i0, j0, G_RVY);
+        const int zr = ctl[td.x].rparity & 1 ? G_RVXB : G_RVX;
+        tma_load_3d(tb + 0 * TILE_BYTES, T, &bar[s], i0, j0, zr);
+        tma_load_3d(tb + 1 * TILE_BYTES, T, &bar[s], i0, j0, zr + 1);
         tma_load_3d(tb + 2 * TILE_BYTES, T, &bar[s], i0, j0, G_RX);
         tma_load_3d(tb + 3 * TILE_BYTES, T, &bar[s], i0, j0, G_RY);
     };
@@ -253,8 +261,8 @@ __global__ void __launch_bounds__(NT, MINB) k_pt32(const CUtensorMap* __restrict
         float* Vx_out = gf(I, in ? G_VXA : G_VXB) + tbase;
         float* Vy_out = gf(I, in ? G_VYA : G_VYB) + tbase;
         float* P_out = gf(I, in ? G_PA : G_PB) + tbase;
-        float* Rvx = gf(I, G_RVX) + tbase;
-        float* Rvy = gf(I, G_RVY) + tbase;
+        float* Rvx = gf(I, ctl[td.x].rparity & 1 ? G_RVXB : G_RVX) + tbase;
+        float* Rvy = Rvx + I.fstride32;
         const float c_pt = I.c_ptscf, cdampX = I.cdampXf, cdampY = I.cdampYf, g_dt = I.g_dtf;
         const float h_dx = 0.5f * _dx, h_dy = 0.5f * _dy;
         // pseudo-time step c_vsc / mu_av = (2 c_vsc) / (mu_0 + mu_1) (the reference's average, :129-130), or
@@ -372,6 +380,14 @@ __global__ void __launch_bounds__(NT, MINB) k_pt32(const CUtensorMap* __restrict
         s = (s + 1 == NST) ? 0 : s + 1;
     }
 }
+
+}  // namespace mx
+}  // namespace sf
+
+#include "sf_mixed_march.cuh"
+
+namespace sf {
+namespace mx {
 
 // ---------------------------------------------------------------------------
 // FP64 kernels over tile lists (one CTA per tile)
@@ -783,6 +799,9 @@ static_assert(NCAND == 12, "sf_engine_stats.tune_ns has one entry per candidate"
 constexpr int cand_of(int k, int c, int o) { return (k * NSCHED + c) * NLAUNCH + o; }
 constexpr int DEFAULT_SHAPE = 1;                      // 32 x 16 rows ...
 constexpr int DEFAULT_CAND = cand_of(DEFAULT_SHAPE, 1, 0);  // ... chunked, serialised, until measured
+// the march (sf_mixed_march.cuh): sweeps per launch, warps (blocks) per SM, and the rows of a segment where there are
+// more strips than warps
+constexpr int MARCH_T = 3, MARCH_WARPS = 8, MARCH_ROWS = 96;
 constexpr int TUNE_PASSES = 2;                        // timed pieces per candidate; the fastest counts
 
 static int shape_of_rows(int rows) {
@@ -810,11 +829,11 @@ static int shape_per_sm(int device, int k, int* out) {
 // arena bytes of one instance: FP32 fields, then FP64 fields, each 256-byte aligned
 struct Layout {
     int64_t LD, rows, fstride, bytes32, bytes64;
-    Layout(int64_t Nx, int64_t Ny) {
+    Layout(int64_t Nx, int64_t Ny, bool rates_b) {
         LD = round_up(Nx + 4, 32);
         rows = Ny + 3;
         fstride = LD * rows;
-        bytes32 = round_up((int64_t)G_NUM * fstride * 4, 256);
+        bytes32 = round_up((int64_t)(rates_b ? G_NUM_B : G_NUM) * fstride * 4, 256);
         bytes64 = round_up((int64_t)D_NUM * fstride * 8, 256);
     }
     int64_t bytes() const { return bytes32 + bytes64; }
@@ -876,6 +895,8 @@ struct Slot {  // an admitted instance
     bool active = false;
     bool swept = false;        // ran sweeps since its last fold
     int budget = 0;            // sweeps of its last round
+    int flips = 0, rflips = 0; // how often that round changed the correction's buffers, and the rates'
+    int ns = 0, w = 0;         // the march's strips and their columns
     int64_t ncheck = 0, ndtupdate = 0;   // the reference's event periods for this grid (:35-36)
     int64_t base = 0;          // inner_total when the current attempt started (a retry starts a new schedule)
     int64_t inner_total = 0, outer = 0;
@@ -946,6 +967,17 @@ struct sf_engine {
     cudaGraphExec_t gexec[NCAND] = {};
     int graph_k[NCAND] = {};
     int blocks = 0;                      // persistent CTAs of the current shape
+    // the march: what the batched solve's sweeps run once their workload class is measured
+    bool rates_b = false;                // instances have second rate buffers
+    CUtensorMap* d_march_maps = nullptr; // [slot][M_NUM_MARCH]
+    MItem* d_items = nullptr;
+    int64_t item_cap = 0;
+    std::vector<MItem> h_items;
+    int* d_nitems = nullptr;
+    int h_nitems = 0;
+    cudaGraph_t march_graph = nullptr;
+    cudaGraphExec_t march_gexec = nullptr;
+    int march_graph_k = 0;
     cudaEvent_t ev_in = nullptr, ev_out = nullptr;
     // the sweep candidate in use (shape, schedule, launch mode) and its tuner: the first round of a workload
     // class the context has not seen starts with short timed pieces of every candidate on the engine stream; the
@@ -978,8 +1010,16 @@ void drop_graph(sf_engine* e, int c) {
     e->graph[c] = nullptr;
 }
 
+void drop_march_graph(sf_engine* e) {
+    if (e->march_gexec) cudaGraphExecDestroy(e->march_gexec);
+    if (e->march_graph) cudaGraphDestroy(e->march_graph);
+    e->march_gexec = nullptr;
+    e->march_graph = nullptr;
+}
+
 void drop_graph(sf_engine* e) {
     for (int c = 0; c < NCAND; ++c) drop_graph(e, c);
+    drop_march_graph(e);
 }
 
 void engine_free(sf_engine* e) {
@@ -991,6 +1031,7 @@ void engine_free(sf_engine* e) {
         if (t) cudaFree(t);
     if (e->d_tiles64) cudaFree(e->d_tiles64);
     if (e->d_part) cudaFree(e->d_part);
+    if (e->d_items) cudaFree(e->d_items);
     if (e->h_out) cudaFreeHost(e->h_out);
     if (e->arena_owned && e->arena) cudaFree(e->arena);
     if (e->ev_in) cudaEventDestroy(e->ev_in);
@@ -1013,7 +1054,8 @@ int engine_init(sf_engine* e, sf_ctx* ctx, int slot_cap, const sf_mixed_options*
     const size_t n = (size_t)slot_cap;
     const size_t o_ins = 0, o_ctl = round_up(o_ins + n * sizeof(Inst), 256);
     const size_t o_map = round_up(o_ctl + n * sizeof(Ctl), 256);
-    const size_t o_seg = round_up(o_map + (size_t)NSHAPES * n * M_NUM * sizeof(CUtensorMap), 256);
+    const size_t o_mm = round_up(o_map + (size_t)NSHAPES * n * M_NUM * sizeof(CUtensorMap), 256);
+    const size_t o_seg = round_up(o_mm + n * M_NUM_MARCH * sizeof(CUtensorMap), 256);
     const size_t o_out = round_up(o_seg + n * sizeof(Seg), 256);
     const size_t o_scl = round_up(o_out + n * 4 * 8, 256);
     const size_t o_lst = round_up(o_scl + n * 8, 256);
@@ -1028,11 +1070,13 @@ int engine_init(sf_engine* e, sf_ctx* ctx, int slot_cap, const sf_mixed_options*
     e->d_insts = (Inst*)(b + o_ins);
     e->d_ctl = (Ctl*)(b + o_ctl);
     e->d_maps = (CUtensorMap*)(b + o_map);
+    e->d_march_maps = (CUtensorMap*)(b + o_mm);
     e->d_segs = (Seg*)(b + o_seg);
     e->d_out = (double*)(b + o_out);
     e->d_scale = (double*)(b + o_scl);
     e->d_list = (int*)(b + o_lst);
     e->d_ntiles = (int*)(b + o_nt);
+    e->d_nitems = e->d_ntiles + 16;      // (the tile counts take NSHAPES of the 32 words)
     e->d_flag = (int*)(b + o_flg);
     SF_CUDA(cudaMemsetAsync(e->tables, 0, total, e->s));
     SF_CUDA(cudaMallocHost(&e->h_out, n * 4 * 8 + 64));  // 4 results per slot (k_inst_err), then the flag word
@@ -1112,12 +1156,73 @@ int encode_maps(sf_engine* e, int q) {
     for (int k = 0; k < NSHAPES; ++k) {
         const int rows = kShapes[k].rows;
         h.ntiles[k] = (int64_t)I.ntx * ceil_div(I.Ny - 1, rows);
-        int rc = encode_tmap_f32_fields(&maps[M_HALO], I.f32, I.LD32, I.rows, G_NUM, I.fstride32, TW, rows + 2);
-        if (rc || (rc = encode_tmap_f32_fields(&maps[M_TILE], I.f32, I.LD32, I.rows, G_NUM, I.fstride32, BX, rows)))
+        const int nf = I.rates_b ? G_NUM_B : G_NUM;
+        int rc = encode_tmap_f32_fields(&maps[M_HALO], I.f32, I.LD32, I.rows, nf, I.fstride32, TW, rows + 2, 1);
+        if (rc || (rc = encode_tmap_f32_fields(&maps[M_TILE], I.f32, I.LD32, I.rows, nf, I.fstride32, BX, rows, 1)))
             return rc;
         // pageable source: staged before the call returns, so `maps` is free again
         SF_CUDA(cudaMemcpyAsync(maps_of(e, k) + (size_t)q * M_NUM, maps, sizeof(maps), cudaMemcpyHostToDevice, e->s));
     }
+    if (e->rates_b) {
+        CUtensorMap mm[M_NUM_MARCH];
+        for (int d = 0; d < M_NUM_MARCH; ++d) {
+            int rc = encode_tmap_f32_fields(&mm[d], I.f32, I.LD32, I.rows, G_NUM_B, I.fstride32, MRing::MC,
+                                            2, d + 1);
+            if (rc) return rc;
+        }
+        SF_CUDA(cudaMemcpyAsync(e->d_march_maps + (size_t)q * M_NUM_MARCH, mm, sizeof(mm), cudaMemcpyHostToDevice, e->s));
+        // 4 columns of halo to the left; to the right T + 1 at least (the last column misses its neighbour)
+        const int cols = I.Nx - 1, most = MRing::MC - 8;
+        h.ns = ML + cols <= MRing::MC - 2 ? 1 : (int)ceil_div(cols, most);
+        h.w = (int)round_up(ceil_div(cols, h.ns), 4);
+        h.ns = (int)ceil_div(cols, h.w);
+    }
+    return SF_OK;
+}
+
+// The march's items for the slots in `ids`: segments of rows as long as they can be while every warp of the launch has
+// one (short segments compute more halo rows); of MARCH_ROWS where even whole strips are more than that.
+int upload_march_list(sf_engine* e, const std::vector<int>& ids) {
+    const int64_t warps = (int64_t)e->ctx->num_sms * MARCH_WARPS;
+    auto count = [&](int rows) {
+        int64_t n = 0;
+        for (int q : ids) n += e->slots[q].ns * ceil_div(e->slots[q].d.Ny - 1, rows);
+        return n;
+    };
+    int most = 1;
+    for (int q : ids) most = std::max(most, e->slots[q].d.Ny - 1);
+    int rows = MARCH_ROWS;
+    if (count(most) <= warps) {
+        int lo = 2, hi = most;          // the smallest count of rows with at most `warps` items
+        while (lo < hi) {
+            const int mid = (lo + hi) / 2;
+            if (count(mid) <= warps) hi = mid; else lo = mid + 1;
+        }
+        rows = lo;
+    }
+    const int64_t n = count(rows);
+    if (n > e->item_cap) {
+        SF_CUDA(cudaStreamSynchronize(e->s));  // the old list may still be read by queued kernels
+        drop_march_graph(e);
+        if (e->d_items) cudaFree(e->d_items);
+        e->d_items = nullptr;
+        e->item_cap = 0;
+        const int64_t cap = std::max<int64_t>(n, 4096);
+        if (cudaMalloc(&e->d_items, (size_t)cap * sizeof(MItem)) != cudaSuccess) {
+            cudaGetLastError();
+            return fail(SF_ERR_OOM, "sf_engine: item list");
+        }
+        e->item_cap = cap;
+    }
+    e->h_items.clear();
+    for (int q : ids) {
+        const Slot& h = e->slots[q];
+        for (int r = 1; r < h.d.Ny; r += rows)
+            for (int k = 0; k < h.ns; ++k) e->h_items.push_back(MItem{q, k * h.w, r, h.w | rows << 8});
+    }
+    SF_CUDA(cudaMemcpyAsync(e->d_items, e->h_items.data(), e->h_items.size() * sizeof(MItem), cudaMemcpyHostToDevice, e->s));
+    e->h_nitems = (int)n;
+    SF_CUDA(cudaMemcpyAsync(e->d_nitems, &e->h_nitems, sizeof(int), cudaMemcpyHostToDevice, e->s));
     return SF_OK;
 }
 
@@ -1239,10 +1344,60 @@ int launch_trials(sf_engine* e, const std::vector<int>& ids, double points) {
     return SF_OK;
 }
 
+// one fold's worth of sweeps over the sweep set `ids`, marching
+int launch_march32(sf_engine* e, const std::vector<int>& ids) {
+    const int K = e->opt.fold_every, T = MARCH_T;
+    constexpr int smem = MRing::BYTES;
+    const auto kern = k_march32<MARCH_T, MARCH_WARPS>;
+    int rc = upload_march_list(e, ids);
+    if (rc) return rc;
+    static bool ready[64] = {};
+    if (!ready[e->ctx->device & 63]) {
+        SF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        ready[e->ctx->device & 63] = true;
+    }
+    for (int q : ids) {
+        Slot& h = e->slots[q];
+        h.flips = march_launches(T, h.budget, (e->h_ctl[q].flags & CTL_CHECK) != 0);
+        h.rflips = h.flips;
+    }
+    const int n = march_launches(T, K, true);   // enough for every instance, with a check at its end or without
+    auto direct = [&]() -> int {
+        for (int l = 0; l < n; ++l)
+            SF_CUDA(launch_overlapped(true, kern, dim3((unsigned)(e->ctx->num_sms * MARCH_WARPS)), dim3(32),
+                                      (size_t)smem, e->s, (const CUtensorMap*)e->d_march_maps, (const Inst*)e->d_insts,
+                                      (const Ctl*)e->d_ctl, (const MItem*)e->d_items, (const int*)e->d_nitems, l,
+                                      e->d_flag));
+        return SF_OK;
+    };
+    if (!e->opt.use_graphs) {
+        if ((rc = direct())) return rc;
+    } else {
+        if (e->march_gexec && e->march_graph_k != K) drop_march_graph(e);
+        if (!e->march_gexec) {
+            SF_CUDA(cudaStreamBeginCapture(e->s, cudaStreamCaptureModeThreadLocal));
+            const int lrc = direct();
+            const cudaError_t ce = cudaStreamEndCapture(e->s, &e->march_graph);
+            if (lrc) return lrc;
+            SF_CUDA(ce);
+            SF_CUDA(cudaGraphInstantiate(&e->march_gexec, e->march_graph, 0));
+            e->march_graph_k = K;
+        }
+        SF_CUDA(cudaGraphLaunch(e->march_gexec, e->s));
+    }
+    e->ctx->launches += n;
+    e->sweeps += K;
+    return SF_OK;
+}
+
 // one fold's worth of sweeps over the sweep set `ids`, in the shape the tuner (or the caller) chose
 int launch_sweeps(sf_engine* e, const std::vector<int>& ids) {
     const int K = e->opt.fold_every;
     int rc;
+    for (int q : ids) {   // k_pt32: the buffers change with every sweep, the rates stay where they are
+        e->slots[q].flips = e->slots[q].budget;
+        e->slots[q].rflips = 0;
+    }
     if (e->tune_state != SF_TUNE_FIXED) {
         // the workload class of this round's sweep set; a new class takes the context's recorded choice, or
         // is measured now (a batch that drains and a serving mix move through classes)
@@ -1267,6 +1422,7 @@ int launch_sweeps(sf_engine* e, const std::vector<int>& ids) {
             e->sweeps += K;
             return SF_OK;
         }
+        if (e->rates_b) return launch_march32(e, ids);
     }
     if ((rc = upload_sweep_list(e, ids, e->shape))) return rc;
     if (e->opt.use_graphs) {
@@ -1302,7 +1458,8 @@ int admit(sf_engine* e, int q, sf_batch_instance& u, int dtau_max) {
     Slot& h = e->slots[q];
     Inst& I = h.d;
     memset(&I, 0, sizeof(I));
-    const Layout L(u.Nx, u.Ny);
+    const Layout L(u.Nx, u.Ny, e->rates_b);
+    I.rates_b = e->rates_b ? 1 : 0;
     I.Nx = (int)u.Nx;
     I.Ny = (int)u.Ny;
     I.ntx = (int)ceil_div(u.Nx - 1, BX);
@@ -1390,8 +1547,9 @@ int write_back(sf_engine* e, int q, double dt_cfl) {
         k_copy64<<<grid1(k.nx * k.ny, 256), 256, 0, s>>>(k.dst, k.nx, I.f64 + (int64_t)k.f * I.fstride64, LD, k.nx, k.ny);
         SF_LAUNCHED(ctx);
     }
-    struct Rt { double* dst; int g; int64_t nx, ny; } rts[] = {{u.dVxdt, G_RVX, Nx - 2, Ny - 1},
-                                                               {u.dVydt, G_RVY, Nx - 1, Ny - 2}};
+    const int zr = e->h_ctl[q].rparity & 1 ? G_RVXB : G_RVX;
+    struct Rt { double* dst; int g; int64_t nx, ny; } rts[] = {{u.dVxdt, zr, Nx - 2, Ny - 1},
+                                                               {u.dVydt, zr + 1, Nx - 1, Ny - 2}};
     for (const Rt& r : rts) {
         if (!r.dst) continue;
         k_f32_to_f64<<<grid1(r.nx * r.ny, 256), 256, 0, s>>>(r.dst, r.nx, I.f32 + (int64_t)r.g * I.fstride32, LD, r.nx,
@@ -1425,7 +1583,7 @@ int validate(const sf_batch_instance& u, const char* who) {
 int engine_submit(sf_engine* e, sf_batch_instance* u, cudaStream_t caller, int64_t* ticket) {
     int rc = validate(*u, "sf_engine_submit");
     if (rc) return rc;
-    const int64_t bytes = Layout(u->Nx, u->Ny).bytes();
+    const int64_t bytes = Layout(u->Nx, u->Ny, e->rates_b).bytes();
     if (bytes > e->alloc.cap())
         return fail(SF_ERR_TOO_LARGE, "sf_engine_submit: the instance needs " + std::to_string(bytes) +
                                           " arena bytes, more than the engine has");
@@ -1473,8 +1631,9 @@ int engine_round(sf_engine* e, cudaStream_t caller) {
             Slot& h = e->slots[q];
             if (h.swept) {
                 swept.push_back(q);
-                // an odd budget leaves the current correction in the other buffer
-                if (h.budget & 1) e->h_ctl[q].parity ^= 1;
+                // an odd number of changes leaves the current correction in the other buffer
+                e->h_ctl[q].parity ^= h.flips & 1;
+                e->h_ctl[q].rparity ^= h.rflips & 1;
                 any_check = any_check || (e->h_ctl[q].flags & CTL_CHECK);
             }
         }
@@ -1610,7 +1769,7 @@ void sf::mixed_engine_release(sf_ctx* ctx) {
 // ---------------------------------------------------------------------------
 extern "C" int sf_engine_instance_bytes(int64_t Nx, int64_t Ny, int64_t* bytes) {
     SF_REQUIRE(bytes && Nx >= 4 && Ny >= 4 && Nx < (1 << 20) && Ny < (1 << 20), "sf_engine_instance_bytes: bad arguments");
-    *bytes = Layout(Nx, Ny).bytes();
+    *bytes = Layout(Nx, Ny, false).bytes();
     return SF_OK;
 }
 
@@ -1702,10 +1861,10 @@ extern "C" int sf_solve_stokes_batch_mixed(sf_ctx* ctx, sf_batch_instance* inst,
     SF_REQUIRE(ctx && inst && n >= 1, "sf_solve_stokes_batch_mixed: bad arguments");
     int rc = set_device(ctx);
     if (rc) return rc;
-    int64_t total = 0;
+    int64_t total[2] = {0, 0};   // without and with second rate buffers
     for (int b = 0; b < n; ++b) {
         if ((rc = validate(inst[b], "sf_solve_stokes_batch_mixed"))) return rc;
-        total += Layout(inst[b].Nx, inst[b].Ny).bytes();
+        for (int k = 0; k < 2; ++k) total[k] += Layout(inst[b].Nx, inst[b].Ny, k == 1).bytes();
     }
     // the context keeps one engine for this call (tables, graph); its arena is the context's scratch,
     // sized to the batch, so every instance is admitted at once
@@ -1724,9 +1883,11 @@ extern "C" int sf_solve_stokes_batch_mixed(sf_ctx* ctx, sf_batch_instance* inst,
     }
     e->opt = normalized(o);
     if ((rc = configure_tuner(e))) return rc;
-    if ((rc = ensure(ctx, ctx->mixed, (size_t)total))) return rc;
+    // where the device has no room for the rates' second buffers, the sweeps do without (one per launch)
+    e->rates_b = e->opt.tile_rows == 0 && ensure(ctx, ctx->mixed, (size_t)total[1]) == SF_OK;
+    if (!e->rates_b && (rc = ensure(ctx, ctx->mixed, (size_t)total[0]))) return rc;
     e->arena = (unsigned char*)ctx->mixed.ptr;
-    e->alloc.reset(total);
+    e->alloc.reset(total[e->rates_b ? 1 : 0]);
     auto run = [&]() -> int {
         int r;
         cudaStream_t caller = as_stream(stream);

@@ -643,8 +643,8 @@ static int encode_tmap(CUtensorMap* map, CUtensorMapDataType dtype, int esize, c
 }
 
 int encode_tmap_f32_fields(CUtensorMap* map, const float* base, int64_t ld, int64_t rows, int64_t nfields,
-                           int64_t fstride, int box_w, int box_h) {
-    return encode_tiled(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, base, ld, rows, nfields, fstride, box_w, box_h);
+                           int64_t fstride, int box_w, int box_h, int box_d) {
+    return encode_tiled(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, base, ld, rows, nfields, fstride, box_w, box_h, box_d);
 }
 
 struct Solver {

@@ -96,8 +96,8 @@ __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, u
 int encode_tmap_f64(CUtensorMap* map, const double* base, int64_t ld, int64_t rows, int box_w, int box_h);
 int encode_tmap_f32(CUtensorMap* map, const float* base, int64_t ld, int64_t rows, int box_w, int box_h);
 // host: a 3-D FP32 tensor map over nfields such buffers, fstride elements apart (the field is the z
-// coordinate), box = box_w x box_h x 1
+// coordinate), box = box_w x box_h x box_d
 int encode_tmap_f32_fields(CUtensorMap* map, const float* base, int64_t ld, int64_t rows, int64_t nfields,
-                           int64_t fstride, int box_w, int box_h);
+                           int64_t fstride, int box_w, int box_h, int box_d);
 
 }  // namespace sf
