@@ -1,4 +1,4 @@
-// sf_core.cu -- context, errors, scratch, prefix scan, warning counters and
+// sf_core.cu -- context, errors, scratch, warning counters and
 // marker initialisation (scripts/common.jl:40-110) for libstokesflow_b200.so.
 #include <algorithm>
 #include <cstdio>
@@ -114,123 +114,6 @@ int ensure(sf_ctx* ctx, Scratch& s, size_t bytes) {
         return cuda_fail(e, "cudaMalloc(scratch)", __FILE__, __LINE__);
     }
     s.bytes = want;
-    return SF_OK;
-}
-
-// --------------------------------------------------------------------------
-// exclusive scan of int32 (3 passes: tile sums, scan of tile sums, tile scan)
-// --------------------------------------------------------------------------
-constexpr int SCAN_THREADS = 1024;
-constexpr int SCAN_ITEMS = 8;
-constexpr int SCAN_TILE = SCAN_THREADS * SCAN_ITEMS;
-
-__device__ __forceinline__ int32_t block_exclusive_scan(int32_t v, int32_t* warp_sums, int32_t* total) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int32_t x = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        int32_t y = __shfl_up_sync(0xffffffffu, x, o);
-        if (lane >= o) x += y;
-    }
-    if (lane == 31) warp_sums[warp] = x;
-    __syncthreads();
-    if (warp == 0) {
-        int32_t w = (lane < (int)(blockDim.x >> 5)) ? warp_sums[lane] : 0;
-        int32_t s = w;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            int32_t y = __shfl_up_sync(0xffffffffu, s, o);
-            if (lane >= o) s += y;
-        }
-        warp_sums[lane] = s - w;  // exclusive warp offsets
-        if (lane == 31) *total = s;
-    }
-    __syncthreads();
-    int32_t r = warp_sums[warp] + x - v;
-    __syncthreads();
-    return r;
-}
-
-__global__ void k_scan_tile_sums(const int32_t* __restrict__ in, int64_t n, int32_t* __restrict__ tile_sums) {
-    __shared__ int32_t warp_sums[32];
-    __shared__ int32_t total;
-    int64_t base = (int64_t)blockIdx.x * SCAN_TILE + (int64_t)threadIdx.x * SCAN_ITEMS;
-    int32_t s = 0;
-#pragma unroll
-    for (int k = 0; k < SCAN_ITEMS; ++k)
-        if (base + k < n) s += in[base + k];
-    block_exclusive_scan(s, warp_sums, &total);
-    if (threadIdx.x == 0) tile_sums[blockIdx.x] = total;
-}
-
-// single block: exclusive scan of the tile sums in place, grand total -> *d_total
-__global__ void k_scan_tile_offsets(int32_t* __restrict__ tile_sums, int64_t ntiles, int32_t* __restrict__ d_total) {
-    __shared__ int32_t warp_sums[32];
-    __shared__ int32_t total;
-    int32_t carry = 0;
-    for (int64_t b0 = 0; b0 < ntiles; b0 += SCAN_THREADS) {
-        int64_t i = b0 + threadIdx.x;
-        int32_t v = (i < ntiles) ? tile_sums[i] : 0;
-        int32_t e = block_exclusive_scan(v, warp_sums, &total);
-        if (i < ntiles) tile_sums[i] = carry + e;
-        carry += total;
-        __syncthreads();
-    }
-    if (threadIdx.x == 0 && d_total) *d_total = carry;
-}
-
-__global__ void k_scan_tiles(const int32_t* in, int32_t* out, int64_t n, const int32_t* __restrict__ tile_offsets) {
-    __shared__ int32_t warp_sums[32];
-    __shared__ int32_t total;
-    int64_t base = (int64_t)blockIdx.x * SCAN_TILE + (int64_t)threadIdx.x * SCAN_ITEMS;
-    int32_t v[SCAN_ITEMS];
-    int32_t s = 0;
-#pragma unroll
-    for (int k = 0; k < SCAN_ITEMS; ++k) {
-        v[k] = (base + k < n) ? in[base + k] : 0;
-        s += v[k];
-    }
-    int32_t e = block_exclusive_scan(s, warp_sums, &total) + tile_offsets[blockIdx.x];
-#pragma unroll
-    for (int k = 0; k < SCAN_ITEMS; ++k) {
-        if (base + k < n) out[base + k] = e;
-        e += v[k];
-    }
-}
-
-int exclusive_scan_i32(sf_ctx* ctx, const int32_t* in, int32_t* out, int64_t n, int32_t* d_total,
-                       cudaStream_t stream) {
-    int64_t ntiles = ceil_div(n, SCAN_TILE);
-    if (ntiles == 0) {
-        if (d_total) SF_CUDA(cudaMemsetAsync(d_total, 0, sizeof(int32_t), stream));
-        return SF_OK;
-    }
-    int rc = ensure(ctx, ctx->scan_tmp, (size_t)ntiles * sizeof(int32_t));
-    if (rc) return rc;
-    int32_t* tiles = (int32_t*)ctx->scan_tmp.ptr;
-    k_scan_tile_sums<<<(unsigned)ntiles, SCAN_THREADS, 0, stream>>>(in, n, tiles);
-    SF_LAUNCHED(ctx);
-    k_scan_tile_offsets<<<1, SCAN_THREADS, 0, stream>>>(tiles, ntiles, d_total);
-    SF_LAUNCHED(ctx);
-    k_scan_tiles<<<(unsigned)ntiles, SCAN_THREADS, 0, stream>>>(in, out, n, tiles);
-    SF_LAUNCHED(ctx);
-    return SF_OK;
-}
-
-// Same scan with the caller's tile buffer (ceil(n / 8192) ints); allocates nothing.
-int exclusive_scan_i32_into(const int32_t* in, int32_t* out, int64_t n, int32_t* d_total, int32_t* tiles,
-                            cudaStream_t stream) {
-    int64_t ntiles = ceil_div(n, SCAN_TILE);
-    if (ntiles == 0) {
-        if (d_total) SF_CUDA(cudaMemsetAsync(d_total, 0, sizeof(int32_t), stream));
-        return SF_OK;
-    }
-    k_scan_tile_sums<<<(unsigned)ntiles, SCAN_THREADS, 0, stream>>>(in, n, tiles);
-    SF_CHECK_LAUNCH();
-    k_scan_tile_offsets<<<1, SCAN_THREADS, 0, stream>>>(tiles, ntiles, d_total);
-    SF_CHECK_LAUNCH();
-    k_scan_tiles<<<(unsigned)ntiles, SCAN_THREADS, 0, stream>>>(in, out, n, tiles);
-    SF_CHECK_LAUNCH();
     return SF_OK;
 }
 
@@ -401,7 +284,7 @@ int sf_ctx_destroy(sf_ctx* c) {
     cudaSetDevice(c->device);
     cudaDeviceSynchronize();
     mixed_engine_release(c);
-    Scratch* all[] = {&c->keys,     &c->counts, &c->offsets,  &c->cursor, &c->perm,  &c->payload, &c->longs,
+    Scratch* all[] = {&c->keys,     &c->counts, &c->offsets,  &c->perm,  &c->payload, &c->longs,
                       &c->scan_tmp, &c->fields, &c->partials, &c->mixed,  &c->exch, &c->halo};
     for (Scratch* s : all)
         if (s->ptr) cudaFree(s->ptr);
@@ -419,7 +302,7 @@ int sf_ctx_destroy(sf_ctx* c) {
 
 int sf_ctx_scratch_bytes(sf_ctx* c, int64_t* bytes) {
     if (!c || !bytes) return fail(SF_ERR_INVALID_ARG, "sf_ctx_scratch_bytes: NULL argument");
-    const Scratch* all[] = {&c->keys,     &c->counts, &c->offsets,  &c->cursor, &c->perm,  &c->payload, &c->longs,
+    const Scratch* all[] = {&c->keys,     &c->counts, &c->offsets,  &c->perm,  &c->payload, &c->longs,
                             &c->scan_tmp, &c->fields, &c->partials, &c->mixed,  &c->exch, &c->halo};
     int64_t b = 0;
     for (const Scratch* s : all) b += (int64_t)s->bytes;

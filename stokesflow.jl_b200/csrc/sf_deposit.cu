@@ -4,16 +4,17 @@
 // Design: the reference scatters 8 floating-point adds per marker (serial on
 // the CPU, CUDA.@atomic on the GPU, MarkerToGrid.jl:58-155).  Here the adds
 // become a gather with no floating-point atomics:
-//   1. k_cell_keys     cell (ix, iy) of every marker for this grid, exactly
+//   1. k_cell_keys     cell (ix, iy) of every marker for each grid, exactly
 //                      topleftIndexRelDist (common.jl:22-33); per-cell counts
 //                      with warp-aggregated integer atomics.
-//   2. exclusive scan  counts -> cell offsets.
+//   2. k_scan_*        exclusive scan of the counts -> cell offsets (and the
+//                      list of long cells).
 //   3. k_scatter       marker indices into their cell's segment (in no
 //                      particular order inside it).
 //   4. segment sort    every segment ascending by marker index, which makes
 //                      the whole a stable counting sort:
-//                      k_long_cells + k_sort_long sort the cells holding more
-//                      than SORT_LONG markers in place (a block-wide LSD radix
+//                      k_sort_long sorts the cells holding more than
+//                      SORT_LONG markers in place (a block-wide LSD radix
 //                      sort per cell, stable, linear in the cell's count, so a
 //                      cell where markers pile up costs no more than its
 //                      size); k_sort_cells sorts the others in shared memory,
@@ -29,6 +30,9 @@
 // the gather streams contiguous records of neighbouring cells instead of
 // chasing marker indices into x, y and val.  Steps 1-4 with the permutation as
 // output are the rebin (sf_rebin_markers).
+//
+// The grids of a timestep go through each kernel together (8 launches instead of
+// 32): small deposits were bound by their launches.
 #include <algorithm>
 
 #include "sf_internal.cuh"
@@ -40,6 +44,10 @@ constexpr int SORT_THREADS = 256;
 constexpr int SORT_CPB = 256;     // cells per block of k_sort_cells
 constexpr int SORT_CAP = 4096;    // entries of a k_sort_cells window in shared memory
 constexpr int SORT_LONG = 64;     // cells with more markers are sorted by k_sort_long
+// markers up to which the grids of a deposit go through each kernel in one launch, every grid in scratch of its own (40
+// bytes per marker and grid).  145 k markers: 228 -> 84 us; 1.4 M: 443 -> 315; 4.2 M: 920 -> 714.  Beyond, launches
+// no longer count (26 M markers: 4.10 ms either way) and one grid's scratch serves all.
+constexpr int64_t DEPOSIT_TOGETHER = 1 << 22;
 
 // A sorted deposit entry: the marker's relative position in its cell (topleftIndexRelDist's dxij, dyij), its
 // value and its index.  32 bytes: one sector.
@@ -48,49 +56,35 @@ struct __align__(32) Payload {
     int32_t m, pad_;
 };
 
-// 1. cell key of every marker; counts[key]++ (warp-aggregated).
-__global__ void k_cell_keys(const double* __restrict__ x, const double* __restrict__ y, int64_t nm, double xmin,
-                            double ymin, double dx, double dy, int64_t nx, int64_t ny, int32_t* __restrict__ keys,
-                            int32_t* __restrict__ counts, unsigned long long* __restrict__ bad_counter) {
-    const int lane = threadIdx.x & 31;
-    int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t base = (int64_t)blockIdx.x * blockDim.x; base < nm; base += stride) {
-        int64_t m = base + threadIdx.x;
-        int32_t key = -1;
-        if (m < nm) {
-            TopLeft t = topleft(xmin, ymin, x[m], y[m], dx, dy);
-            // MarkerToGrid.jl:66: accept iff 0 <= ix <= Nx && 0 <= iy <= Ny (ix = qx + 1)
-            if (t.qx >= -1.0 && t.qx <= (double)(nx - 1) && t.qy >= -1.0 && t.qy <= (double)(ny - 1))
-                key = (int32_t)((int64_t)t.qx + 1 + ((int64_t)t.qy + 1) * (nx + 1));
-            keys[m] = key;
-        }
-        unsigned active = __ballot_sync(0xffffffffu, m < nm);
-        if (m < nm) {
-            unsigned peers = __match_any_sync(active, key);
-            int leader = __ffs(peers) - 1;
-            if (lane == leader) {
-                int n = __popc(peers);
-                if (key >= 0)
-                    atomicAdd(&counts[key], n);
-                else if (bad_counter)
-                    atomicAdd(bad_counter, (unsigned long long)n);
-            }
-        }
-    }
-}
-
-// 1 for several grids over the same markers (the three deposits of a timestep): each marker's position is read
-// once, and every grid gets its own keys and counts, exactly as k_cell_keys computes them.
-struct GridKeys {
-    double xmin[SF_MAX_GRIDS], ymin[SF_MAX_GRIDS];
-    int64_t nx[SF_MAX_GRIDS], ny[SF_MAX_GRIDS];
-    int32_t* keys[SF_MAX_GRIDS];
-    int32_t* counts[SF_MAX_GRIDS];
+// One grid of a sort: what its kernels read and write.  Several grids over the same markers (the deposits of a timestep)
+// go through each kernel together, blockIdx.y choosing the grid.
+struct SortGrid {
+    double xmin, ymin;
+    int64_t nx, ny, ncells;    // nodes, cells (nx + 1) * (ny + 1)
+    int32_t* keys;             // cell of each marker (-1: none); spent after the scatter, then the radix sort's buffer
+    int32_t* counts;           // markers of each cell
+    int32_t* offsets;          // [ncells + 1]
+    int32_t* cursor;           // next place in each cell's segment (scatter)
+    int32_t* tiles;            // sums of the scan's tiles
+    int32_t* n_list;           // the cells holding more than SORT_LONG markers: their number ...
+    int32_t* list;             // ... and the cells
+    int32_t* perm;
+    Payload* payload;          // (deposit)
+    const double* val;
+    double *val_grid, *val_wt_sum, *wt_sum;
+    int64_t ld_sum;
+};
+struct SortGrids {
+    SortGrid g[SF_MAX_GRIDS];
     int n;
 };
 
-__global__ void k_cell_keys_grids(const double* __restrict__ x, const double* __restrict__ y, int64_t nm, double dx,
-                                  double dy, const GridKeys g, unsigned long long* __restrict__ bad_counter) {
+// 1. cell key of every marker for every grid (positions are read once); counts[key]++ (warp-aggregated).  (Keeping the
+// counters' old values as the markers' places, so that the scatter needs no atomics, costs more here, 87 us per grid and
+// 26 M markers, than the 25 us it saves there.)
+template <int MOST>   // grids at most
+__global__ void k_cell_keys(const double* __restrict__ x, const double* __restrict__ y, int64_t nm, double dx, double dy,
+                            const __grid_constant__ SortGrids s, unsigned long long* __restrict__ bad_counter) {
     const int lane = threadIdx.x & 31;
     int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t base = (int64_t)blockIdx.x * blockDim.x; base < nm; base += stride) {
@@ -99,20 +93,21 @@ __global__ void k_cell_keys_grids(const double* __restrict__ x, const double* __
         const double xm = live ? x[m] : 0.0, ym = live ? y[m] : 0.0;
         const unsigned active = __ballot_sync(0xffffffffu, live);
 #pragma unroll
-        for (int k = 0; k < SF_MAX_GRIDS; ++k) {
-            if (k >= g.n) break;
+        for (int k = 0; k < MOST; ++k) {
+            if (MOST > 1 && k >= s.n) break;
             if (!live) continue;
+            const SortGrid& g = s.g[k];
             int32_t key = -1;
-            const TopLeft t = topleft(g.xmin[k], g.ymin[k], xm, ym, dx, dy);
+            const TopLeft t = topleft(g.xmin, g.ymin, xm, ym, dx, dy);
             // MarkerToGrid.jl:66: accept iff 0 <= ix <= Nx && 0 <= iy <= Ny (ix = qx + 1)
-            if (t.qx >= -1.0 && t.qx <= (double)(g.nx[k] - 1) && t.qy >= -1.0 && t.qy <= (double)(g.ny[k] - 1))
-                key = (int32_t)((int64_t)t.qx + 1 + ((int64_t)t.qy + 1) * (g.nx[k] + 1));
-            g.keys[k][m] = key;
+            if (t.qx >= -1.0 && t.qx <= (double)(g.nx - 1) && t.qy >= -1.0 && t.qy <= (double)(g.ny - 1))
+                key = (int32_t)((int64_t)t.qx + 1 + ((int64_t)t.qy + 1) * (g.nx + 1));
+            g.keys[m] = key;
             const unsigned peers = __match_any_sync(active, key);
             if (lane == __ffs(peers) - 1) {
                 const int n = __popc(peers);
                 if (key >= 0)
-                    atomicAdd(&g.counts[k][key], n);
+                    atomicAdd(&g.counts[key], n);
                 else if (bad_counter)
                     atomicAdd(bad_counter, (unsigned long long)n);
             }
@@ -120,23 +115,117 @@ __global__ void k_cell_keys_grids(const double* __restrict__ x, const double* __
     }
 }
 
+// 2. exclusive scan of the counts -> offsets, in tiles of SCAN_TILE cells: the tiles' sums, then every tile with the sum
+// of the tiles before it, which a block adds up itself (or, of more than SCAN_DIRECT tiles, finds scanned already).
+// The second pass also lists the long cells.
+constexpr int SCAN_THREADS = 1024, SCAN_ITEMS = 8, SCAN_TILE = SCAN_THREADS * SCAN_ITEMS, SCAN_DIRECT = 2048;
+
+__device__ __forceinline__ int32_t block_exclusive_scan(int32_t v, int32_t* warp_sums, int32_t* total) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int32_t x = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        int32_t y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+    }
+    if (lane == 31) warp_sums[warp] = x;
+    __syncthreads();
+    if (warp == 0) {
+        int32_t w = (lane < (int)(blockDim.x >> 5)) ? warp_sums[lane] : 0;
+        int32_t s = w;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            int32_t y = __shfl_up_sync(0xffffffffu, s, o);
+            if (lane >= o) s += y;
+        }
+        warp_sums[lane] = s - w;  // exclusive warp offsets
+        if (lane == 31) *total = s;
+    }
+    __syncthreads();
+    int32_t r = warp_sums[warp] + x - v;
+    __syncthreads();
+    return r;
+}
+
+__global__ void __launch_bounds__(SCAN_THREADS) k_scan_tile_sums(const __grid_constant__ SortGrids s) {
+    __shared__ int32_t warp_sums[32];
+    __shared__ int32_t total;
+    const SortGrid& g = s.g[blockIdx.y];
+    if ((int64_t)blockIdx.x * SCAN_TILE >= g.ncells) return;
+    const int64_t base = (int64_t)blockIdx.x * SCAN_TILE + (int64_t)threadIdx.x * SCAN_ITEMS;
+    int32_t sum = 0;
+#pragma unroll
+    for (int k = 0; k < SCAN_ITEMS; ++k)
+        if (base + k < g.ncells) sum += g.counts[base + k];
+    block_exclusive_scan(sum, warp_sums, &total);
+    if (threadIdx.x == 0) g.tiles[blockIdx.x] = total;
+}
+
+// single block per grid: exclusive scan of the tile sums in place
+__global__ void __launch_bounds__(SCAN_THREADS) k_scan_tile_offsets(const __grid_constant__ SortGrids s) {
+    __shared__ int32_t warp_sums[32];
+    __shared__ int32_t total;
+    const SortGrid& g = s.g[blockIdx.y];
+    const int64_t ntiles = (g.ncells + SCAN_TILE - 1) / SCAN_TILE;
+    int32_t carry = 0;
+    for (int64_t b0 = 0; b0 < ntiles; b0 += SCAN_THREADS) {
+        int64_t i = b0 + threadIdx.x;
+        int32_t v = (i < ntiles) ? g.tiles[i] : 0;
+        int32_t e = block_exclusive_scan(v, warp_sums, &total);
+        if (i < ntiles) g.tiles[i] = carry + e;
+        carry += total;
+        __syncthreads();
+    }
+}
+
+__global__ void __launch_bounds__(SCAN_THREADS) k_scan_tiles(const __grid_constant__ SortGrids s, int scanned) {
+    __shared__ int32_t warp_sums[32];
+    __shared__ int32_t total;
+    const SortGrid& g = s.g[blockIdx.y];
+    if ((int64_t)blockIdx.x * SCAN_TILE >= g.ncells) return;
+    int32_t before = 0;
+    if (scanned) {
+        before = g.tiles[blockIdx.x];
+    } else {
+        for (int t = threadIdx.x; t < (int)blockIdx.x; t += SCAN_THREADS) before += g.tiles[t];
+        block_exclusive_scan(before, warp_sums, &total);
+        before = total;
+        __syncthreads();
+    }
+    const int64_t base = (int64_t)blockIdx.x * SCAN_TILE + (int64_t)threadIdx.x * SCAN_ITEMS;
+    int32_t v[SCAN_ITEMS];
+    int32_t sum = 0;
+#pragma unroll
+    for (int k = 0; k < SCAN_ITEMS; ++k) {
+        v[k] = (base + k < g.ncells) ? g.counts[base + k] : 0;
+        sum += v[k];
+    }
+    int32_t e = block_exclusive_scan(sum, warp_sums, &total) + before;
+#pragma unroll
+    for (int k = 0; k < SCAN_ITEMS; ++k) {
+        if (base + k < g.ncells) g.offsets[base + k] = g.cursor[base + k] = e;
+        e += v[k];
+        if (base + k == g.ncells - 1) g.offsets[g.ncells] = e;
+        if (v[k] > SORT_LONG) g.list[atomicAdd(g.n_list, 1)] = (int32_t)(base + k);
+    }
+}
+
 // 3. scatter marker indices into their cells (order within a cell arbitrary).
-__global__ void k_scatter(const int32_t* __restrict__ keys, int64_t nm, const int32_t* __restrict__ offsets,
-                          int32_t* __restrict__ cursor, int32_t* __restrict__ perm) {
+__global__ void k_scatter(const __grid_constant__ SortGrids s, int64_t nm) {
+    const SortGrid& g = s.g[blockIdx.y];
     const int lane = threadIdx.x & 31;
     int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t base = (int64_t)blockIdx.x * blockDim.x; base < nm; base += stride) {
         int64_t m = base + threadIdx.x;
-        int32_t key = (m < nm) ? keys[m] : -1;
+        int32_t key = (m < nm) ? g.keys[m] : -1;
         unsigned active = __ballot_sync(0xffffffffu, key >= 0);
         if (key >= 0) {
             unsigned peers = __match_any_sync(active, key);
             int leader = __ffs(peers) - 1;
             int32_t pos0 = 0;
-            if (lane == leader) pos0 = atomicAdd(&cursor[key], __popc(peers));
+            if (lane == leader) pos0 = atomicAdd(&g.cursor[key], __popc(peers));
             pos0 = __shfl_sync(peers, pos0, leader);
-            int rank = __popc(peers & ((1u << lane) - 1u));
-            perm[offsets[key] + pos0 + rank] = (int32_t)m;
+            g.perm[pos0 + __popc(peers & ((1u << lane) - 1u))] = (int32_t)m;
         }
     }
 }
@@ -160,30 +249,23 @@ __global__ void k_sort_segments(const int32_t* __restrict__ offsets, int64_t nce
     }
 }
 
-// 4a. the cells holding more than SORT_LONG markers -> list[0 .. *n_list)
-__global__ void k_long_cells(const int32_t* __restrict__ offsets, int64_t ncells, int32_t* __restrict__ list,
-                             int32_t* __restrict__ n_list) {
-    for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < ncells; c += (int64_t)gridDim.x * blockDim.x)
-        if (offsets[c + 1] - offsets[c] > SORT_LONG) list[atomicAdd(n_list, 1)] = (int32_t)c;
-}
-
-// 4b. each long cell's segment sorted ascending in place by a block-wide LSD radix sort on 8-bit digits of the
+// 4a. each long cell's segment sorted ascending in place by a block-wide LSD radix sort on 8-bit digits of the
 // marker index (indices are non-negative 31-bit values: 4 digits), stable, through `tmp` at the same offsets.
 // A digit on which the whole segment agrees moves nothing and is skipped.  Tiles of SORT_THREADS entries are
 // ranked in order: lanes within a warp by __match_any_sync, warps by their per-digit counts.
-__global__ void __launch_bounds__(SORT_THREADS) k_sort_long(const int32_t* __restrict__ offsets,
-                                                            const int32_t* __restrict__ list,
-                                                            const int32_t* __restrict__ n_list, int32_t* perm,
-                                                            int32_t* tmp) {
+__global__ void __launch_bounds__(SORT_THREADS) k_sort_long(const __grid_constant__ SortGrids s) {
     constexpr int NW = SORT_THREADS / 32;
     __shared__ int hist[256];
     __shared__ int base[256];
     __shared__ int wcnt[NW][256];
     __shared__ int skip;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int n_long = *n_list;
+    const SortGrid& g = s.g[blockIdx.y];
+    const int32_t* offsets = g.offsets;
+    int32_t *perm = g.perm, *tmp = g.keys;
+    const int n_long = *g.n_list;
     for (int li = blockIdx.x; li < n_long; li += gridDim.x) {
-        const int c = list[li];
+        const int c = g.list[li];
         const int32_t b = offsets[c], n = offsets[c + 1] - b;
         int32_t* src = perm + b;
         int32_t* dst = tmp + b;
@@ -239,20 +321,25 @@ __global__ void __launch_bounds__(SORT_THREADS) k_sort_long(const int32_t* __res
     }
 }
 
-// 4c. every short segment sorted ascending; long segments (sorted by k_sort_long) pass through in order.  A
+// 4b. every short segment sorted ascending; long segments (sorted by k_sort_long) pass through in order.  A
 // block takes SORT_CPB consecutive cells and works through them in windows of consecutive cells holding at most
 // SORT_CAP entries: it loads a window's marker indices into shared memory, ranks each entry within its cell by
 // counting the smaller indices there, and writes it to its sorted place -- back into perm (the rebin), or as a
 // payload record (the deposit: topleftIndexRelDist of the marker and its value, once per marker).
 template <bool PAYLOAD>
-__global__ void __launch_bounds__(SORT_THREADS) k_sort_cells(const int32_t* __restrict__ offsets, int64_t ncells,
-                                                             int32_t* perm, Payload* __restrict__ out,
+__global__ void __launch_bounds__(SORT_THREADS) k_sort_cells(const __grid_constant__ SortGrids s,
                                                              const double* __restrict__ x, const double* __restrict__ y,
-                                                             const double* __restrict__ val, double xmin, double ymin,
                                                              double dx, double dy) {
     __shared__ int32_t soff[SORT_CPB + 1];
     __shared__ int32_t sm[SORT_CAP];
     const int tid = threadIdx.x;
+    const SortGrid& g = s.g[blockIdx.y];
+    const int64_t ncells = g.ncells;
+    const int32_t* __restrict__ offsets = g.offsets;
+    int32_t* perm = g.perm;
+    Payload* __restrict__ out = g.payload;
+    const double* __restrict__ val = g.val;
+    const double xmin = g.xmin, ymin = g.ymin;
     const int64_t c0 = (int64_t)blockIdx.x * SORT_CPB;
     if (c0 >= ncells) return;
     const int nc = (int)min((int64_t)SORT_CPB, ncells - c0);
@@ -327,12 +414,12 @@ constexpr int GT_NONE = 0x7fffffff;   // head of an exhausted list
 constexpr int GT_X = 32, GT_Y = 4;    // nodes of a block: one warp per node row, 4 rows that share cell rows
 // (launched 8 blocks per SM: 64 registers, more warps in flight than a spill-free 68)
 
-__global__ void __launch_bounds__(GT_X * GT_Y, 8) k_gather_sorted(const Payload* __restrict__ pl,
-                                                               const int32_t* __restrict__ offsets, int64_t nx,
-                                                               int64_t ny, double* __restrict__ val_grid,
-                                                               double* __restrict__ val_wt_sum,
-                                                               double* __restrict__ wt_sum, int64_t ld_sum,
+__global__ void __launch_bounds__(GT_X * GT_Y, 8) k_gather_sorted(const __grid_constant__ SortGrids s,
                                                                unsigned long long* __restrict__ empty_counter) {
+    const SortGrid& g = s.g[blockIdx.y];
+    const Payload* __restrict__ pl = g.payload;
+    const int32_t* __restrict__ offsets = g.offsets;
+    const int64_t nx = g.nx, ny = g.ny;
     const int64_t ntx = (nx + GT_X - 1) / GT_X;
     const int64_t I = (int64_t)(blockIdx.x % ntx) * GT_X + (threadIdx.x % GT_X) + 1;
     const int64_t J = (int64_t)(blockIdx.x / ntx) * GT_Y + (threadIdx.x / GT_X) + 1;
@@ -410,12 +497,12 @@ __global__ void __launch_bounds__(GT_X * GT_Y, 8) k_gather_sorted(const Payload*
                 hv[k] = v;
             }
     }
-    if (wt_sum) {
-        wt_sum[(I - 1) + (J - 1) * ld_sum] = ws;
-        val_wt_sum[(I - 1) + (J - 1) * ld_sum] = vs;
+    if (g.wt_sum) {
+        g.wt_sum[(I - 1) + (J - 1) * g.ld_sum] = ws;
+        g.val_wt_sum[(I - 1) + (J - 1) * g.ld_sum] = vs;
     }
     if (ws != 0.0)
-        val_grid[(I - 1) + (J - 1) * nx] = vs / ws;   // safeDivision (MarkerToGrid.jl:164-172)
+        g.val_grid[(I - 1) + (J - 1) * nx] = vs / ws;   // safeDivision (MarkerToGrid.jl:164-172)
     else if (empty_counter)
         atomicAdd(empty_counter, 1ull);
 }
@@ -480,70 +567,149 @@ static unsigned grid_for(sf_ctx* ctx, int64_t n, int threads) {
     return (unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div(n, threads), (int64_t)ctx->num_sms * 32));
 }
 
-// Steps 2-4 from cell keys and per-cell counts already computed (step 1): the stable counting sort of markers by
-// cell -> ctx->offsets, and either the cell-ordered permutation in ctx->perm or (with val) the cell-ordered
-// payload records in ctx->payload.  keys is spent afterwards: it is the radix sort's second buffer.
-static int sort_from_keys(sf_ctx* ctx, int32_t* keys, const int32_t* counts, const double* x, const double* y,
-                          const double* val, int64_t nm, double xmin, double ymin, double dx, double dy, int64_t nx,
-                          int64_t ny, cudaStream_t s) {
-    int64_t ncells = (nx + 1) * (ny + 1);
+// Step 1 for all grids of s
+static int launch_keys(sf_ctx* ctx, const SortGrids& s, const double* x, const double* y, int64_t nm, double dx, double dy,
+                       unsigned long long* bad_counter, cudaStream_t st) {
+    if (nm == 0) return SF_OK;
+    if (s.n == 1)
+        k_cell_keys<1><<<grid_for(ctx, nm, DEP_THREADS), DEP_THREADS, 0, st>>>(x, y, nm, dx, dy, s, bad_counter);
+    else
+        k_cell_keys<SF_MAX_GRIDS><<<grid_for(ctx, nm, DEP_THREADS), DEP_THREADS, 0, st>>>(x, y, nm, dx, dy, s, bad_counter);
+    SF_LAUNCHED(ctx);
+    return SF_OK;
+}
+
+// Step 2 for the grids of s, blockIdx.y each; no context (the allocation-free deposit), *launches: kernels launched
+static int launch_scan(const SortGrids& s, cudaStream_t st, int* launches) {
+    int64_t tiles = 0;
+    for (int k = 0; k < s.n; ++k) tiles = std::max(tiles, ceil_div(s.g[k].ncells, SCAN_TILE));
+    const dim3 grid((unsigned)tiles, (unsigned)s.n);
+    const int scanned = tiles > SCAN_DIRECT;
+    k_scan_tile_sums<<<grid, SCAN_THREADS, 0, st>>>(s);
+    SF_CHECK_LAUNCH();
+    if (scanned) {
+        k_scan_tile_offsets<<<dim3(1, (unsigned)s.n), SCAN_THREADS, 0, st>>>(s);
+        SF_CHECK_LAUNCH();
+    }
+    k_scan_tiles<<<grid, SCAN_THREADS, 0, st>>>(s, scanned);
+    SF_CHECK_LAUNCH();
+    *launches = 2 + scanned;
+    return SF_OK;
+}
+
+// Steps 2-4 for the grids of s: the stable counting sort of the markers by cell -> offsets, and either the cell-ordered
+// permutation (rebin) or the cell-ordered payload records (deposit).
+static int launch_sort(sf_ctx* ctx, const SortGrids& s, const double* x, const double* y, int64_t nm, double dx, double dy,
+                       bool payload, cudaStream_t st) {
+    int n = 0;
+    int rc = launch_scan(s, st, &n);
+    ctx->launches += n;
+    if (rc || nm == 0) return rc;
+    int64_t cells = 0;
+    for (int k = 0; k < s.n; ++k) cells = std::max(cells, s.g[k].ncells);
+    k_scatter<<<dim3(grid_for(ctx, nm, DEP_THREADS), (unsigned)s.n), DEP_THREADS, 0, st>>>(s, nm);
+    SF_LAUNCHED(ctx);
+    k_sort_long<<<dim3((unsigned)ctx->num_sms * 2, (unsigned)s.n), SORT_THREADS, 0, st>>>(s);
+    SF_LAUNCHED(ctx);
+    const dim3 blocks((unsigned)ceil_div(cells, SORT_CPB), (unsigned)s.n);
+    if (payload)
+        k_sort_cells<true><<<blocks, SORT_THREADS, 0, st>>>(s, x, y, dx, dy);
+    else
+        k_sort_cells<false><<<blocks, SORT_THREADS, 0, st>>>(s, x, y, dx, dy);
+    SF_LAUNCHED(ctx);
+    return SF_OK;
+}
+
+// Scratch of a sort over the grids of s (xmin .. ncells set): what all grids need at once (keys and counts come from one
+// pass over the markers) and, `together`, offsets, cursors, permutation and payload of each grid, else those of one.
+// The counts and list lengths are one block, zeroed here.
+static int sort_scratch(sf_ctx* ctx, SortGrids& s, int64_t nm, bool together, bool payload, cudaStream_t st) {
+    const int64_t nmk = std::max<int64_t>(nm, 1), per = round_up(nmk, 64), nlist = nm / (SORT_LONG + 1) + 1;
+    int64_t cells = 0, most = 0, tiles = 0;
+    for (int k = 0; k < s.n; ++k) {
+        cells += s.g[k].ncells + 1;
+        most = std::max(most, s.g[k].ncells + 1);
+        tiles += ceil_div(s.g[k].ncells, SCAN_TILE);
+    }
+    const int n = together ? s.n : 1;
     int rc;
-    if ((rc = ensure(ctx, ctx->perm, (size_t)std::max<int64_t>(nm, 1) * 4))) return rc;
-    if ((rc = ensure(ctx, ctx->offsets, (size_t)(ncells + 1) * 4))) return rc;
-    if ((rc = ensure(ctx, ctx->cursor, (size_t)(ncells + 1) * 4))) return rc;
-    if ((rc = ensure(ctx, ctx->longs, (size_t)(ncells + 1) * 4))) return rc;
-    if (val && (rc = ensure(ctx, ctx->payload, (size_t)std::max<int64_t>(nm, 1) * sizeof(Payload)))) return rc;
-    int32_t* offsets = (int32_t*)ctx->offsets.ptr;
-    int32_t* cursor = (int32_t*)ctx->cursor.ptr;
-    int32_t* perm = (int32_t*)ctx->perm.ptr;
-    int32_t* n_long = (int32_t*)ctx->longs.ptr;   // the count, then the list
-    SF_CUDA(cudaMemsetAsync(cursor, 0, (size_t)(ncells + 1) * 4, s));
-    SF_CUDA(cudaMemsetAsync(n_long, 0, 4, s));
-    if ((rc = exclusive_scan_i32(ctx, counts, offsets, ncells, offsets + ncells, s))) return rc;
-    if (nm > 0) {
-        k_scatter<<<grid_for(ctx, nm, DEP_THREADS), DEP_THREADS, 0, s>>>(keys, nm, offsets, cursor, perm);
-        SF_LAUNCHED(ctx);
-        k_long_cells<<<grid_for(ctx, ncells, DEP_THREADS), DEP_THREADS, 0, s>>>(offsets, ncells, n_long + 1, n_long);
-        SF_LAUNCHED(ctx);
-        // the keys are spent: they are the radix sort's second buffer
-        k_sort_long<<<(unsigned)ctx->num_sms * 2, SORT_THREADS, 0, s>>>(offsets, n_long + 1, n_long, perm, keys);
-        SF_LAUNCHED(ctx);
-        const unsigned blocks = (unsigned)ceil_div(ncells, SORT_CPB);
-        if (val)
-            k_sort_cells<true><<<blocks, SORT_THREADS, 0, s>>>(offsets, ncells, perm, (Payload*)ctx->payload.ptr, x, y,
-                                                               val, xmin, ymin, dx, dy);
-        else
-            k_sort_cells<false><<<blocks, SORT_THREADS, 0, s>>>(offsets, ncells, perm, nullptr, x, y, val, xmin, ymin,
-                                                                dx, dy);
-        SF_LAUNCHED(ctx);
+    if ((rc = ensure(ctx, ctx->keys, (size_t)(s.n * per) * 4))) return rc;
+    if ((rc = ensure(ctx, ctx->counts, (size_t)(cells + s.n) * 4))) return rc;    // counts, list lengths
+    if ((rc = ensure(ctx, ctx->offsets, (size_t)(2 * n * most) * 4))) return rc;  // offsets, cursors
+    if ((rc = ensure(ctx, ctx->scan_tmp, (size_t)tiles * 4))) return rc;
+    if ((rc = ensure(ctx, ctx->longs, (size_t)(n * nlist) * 4))) return rc;
+    if ((rc = ensure(ctx, ctx->perm, (size_t)(n * per) * 4))) return rc;
+    if (payload && (rc = ensure(ctx, ctx->payload, (size_t)(n * nmk) * sizeof(Payload)))) return rc;
+    SF_CUDA(cudaMemsetAsync(ctx->counts.ptr, 0, (size_t)(cells + s.n) * 4, st));
+    int32_t* counts = (int32_t*)ctx->counts.ptr;
+    int32_t* tile = (int32_t*)ctx->scan_tmp.ptr;
+    int64_t at = 0;
+    for (int k = 0; k < s.n; ++k) {
+        SortGrid& g = s.g[k];
+        const int64_t q = together ? k : 0;
+        g.keys = (int32_t*)ctx->keys.ptr + k * per;
+        g.counts = counts + at;
+        g.n_list = counts + cells + k;
+        g.offsets = (int32_t*)ctx->offsets.ptr + 2 * q * most;
+        g.cursor = g.offsets + most;
+        g.tiles = tile;
+        g.list = (int32_t*)ctx->longs.ptr + q * nlist;
+        g.perm = (int32_t*)ctx->perm.ptr + q * per;
+        g.payload = payload ? (Payload*)ctx->payload.ptr + q * nmk : nullptr;
+        at += g.ncells + 1;
+        tile += ceil_div(g.ncells, SCAN_TILE);
     }
     return SF_OK;
 }
 
-// Steps 1-4 for one grid: cell keys and counts into ctx->keys / ctx->counts, then the sort.
-static int sort_by_cell(sf_ctx* ctx, const double* x, const double* y, const double* val, int64_t nm, double xmin,
-                        double ymin, double dx, double dy, int64_t nx, int64_t ny, unsigned long long* bad_counter,
-                        cudaStream_t s) {
-    int64_t ncells = (nx + 1) * (ny + 1);
-    int rc;
-    if ((rc = ensure(ctx, ctx->keys, (size_t)std::max<int64_t>(nm, 1) * 4))) return rc;
-    if ((rc = ensure(ctx, ctx->counts, (size_t)(ncells + 1) * 4))) return rc;
-    int32_t* keys = (int32_t*)ctx->keys.ptr;
-    int32_t* counts = (int32_t*)ctx->counts.ptr;
-    SF_CUDA(cudaMemsetAsync(counts, 0, (size_t)(ncells + 1) * 4, s));
-    if (nm > 0) {
-        k_cell_keys<<<grid_for(ctx, nm, DEP_THREADS), DEP_THREADS, 0, s>>>(x, y, nm, xmin, ymin, dx, dy, nx, ny, keys,
-                                                                             counts, bad_counter);
-        SF_LAUNCHED(ctx);
-    }
-    return sort_from_keys(ctx, keys, counts, x, y, val, nm, xmin, ymin, dx, dy, nx, ny, s);
+static int launch_gather(sf_ctx* ctx, const SortGrids& s, cudaStream_t st) {
+    int64_t blocks = 0;
+    for (int k = 0; k < s.n; ++k) blocks = std::max(blocks, ceil_div(s.g[k].nx, GT_X) * ceil_div(s.g[k].ny, GT_Y));
+    k_gather_sorted<<<dim3((unsigned)blocks, (unsigned)s.n), GT_X * GT_Y, 0, st>>>(s, ctx->d_counters + CNT_EMPTY_NODES);
+    SF_LAUNCHED(ctx);
+    return SF_OK;
 }
 
-static void launch_gather(sf_ctx* ctx, int64_t nx, int64_t ny, double* val_grid, double* val_wt_sum, double* wt_sum,
-                          int64_t ld_sum, cudaStream_t s) {
-    k_gather_sorted<<<(unsigned)(ceil_div(nx, GT_X) * ceil_div(ny, GT_Y)), GT_X * GT_Y, 0, s>>>(
-        (const Payload*)ctx->payload.ptr, (const int32_t*)ctx->offsets.ptr, nx, ny, val_grid, val_wt_sum, wt_sum,
-        ld_sum, ctx->d_counters + CNT_EMPTY_NODES);
+// whether two of the arrays that the deposits of s write overlap
+static bool outputs_overlap(const SortGrids& s, int64_t n_sum) {
+    struct Range { const double *b, *e; } r[SF_MAX_GRIDS + 2];
+    int n = 0;
+    for (int k = 0; k < s.n; ++k) {
+        r[n++] = Range{s.g[k].val_grid, s.g[k].val_grid + s.g[k].nx * s.g[k].ny};
+        if (s.g[k].wt_sum) {
+            r[n++] = Range{s.g[k].wt_sum, s.g[k].wt_sum + n_sum};
+            r[n++] = Range{s.g[k].val_wt_sum, s.g[k].val_wt_sum + n_sum};
+        }
+    }
+    for (int i = 0; i < n; ++i)
+        for (int j = i + 1; j < n; ++j)
+            if (r[i].b < r[j].e && r[j].b < r[i].e) return true;
+    return false;
+}
+
+// The deposits of s's grids over the same markers (only the last one's sums are kept).  Up to DEPOSIT_TOGETHER markers
+// all grids go through each kernel in one launch; beyond, or where they write the same places, one grid after the other,
+// in the scratch of one.
+static int deposit(sf_ctx* ctx, SortGrids& s, const double* x, const double* y, int64_t nm, double dx, double dy,
+                   int64_t n_sum, cudaStream_t st) {
+    const bool together = s.n > 1 && nm <= DEPOSIT_TOGETHER && !outputs_overlap(s, n_sum);
+    int rc;
+    if ((rc = sort_scratch(ctx, s, nm, together, true, st))) return rc;
+    if ((rc = launch_keys(ctx, s, x, y, nm, dx, dy, ctx->d_counters + CNT_BAD_MARKERS, st))) return rc;
+    const SortGrid& last = s.g[s.n - 1];
+    for (int k = 0; k < (together ? 1 : s.n); ++k) {
+        SortGrids one{};
+        one.g[0] = s.g[k];
+        one.n = 1;
+        const SortGrids& pass = together ? s : one;
+        if ((rc = launch_sort(ctx, pass, x, y, nm, dx, dy, true, st))) return rc;
+        if (last.wt_sum && (together || k == s.n - 1)) {
+            SF_CUDA(cudaMemsetAsync(last.wt_sum, 0, (size_t)n_sum * 8, st));
+            SF_CUDA(cudaMemsetAsync(last.val_wt_sum, 0, (size_t)n_sum * 8, st));
+        }
+        if ((rc = launch_gather(ctx, pass, st))) return rc;
+    }
+    return SF_OK;
 }
 
 }  // namespace sf
@@ -567,16 +733,20 @@ int sf_bilinear_marker_to_grid(sf_ctx* ctx, double x_grid_min, double y_grid_min
     int rc = set_device(ctx);
     if (rc) return rc;
     cudaStream_t s = as_stream(stream);
-    if ((rc = sort_by_cell(ctx, x_m, y_m, val_m, nm, x_grid_min, y_grid_min, dx, dy, nx, ny,
-                           ctx->d_counters + CNT_BAD_MARKERS, s)))
-        return rc;
-    if (wt_sum) {
-        SF_CUDA(cudaMemsetAsync(wt_sum, 0, (size_t)n_sum * 8, s));
-        SF_CUDA(cudaMemsetAsync(val_wt_sum, 0, (size_t)n_sum * 8, s));
-    }
-    launch_gather(ctx, nx, ny, val_grid, val_wt_sum, wt_sum, ld_sum, s);
-    SF_LAUNCHED(ctx);
-    return SF_OK;
+    SortGrids sg{};
+    sg.n = 1;
+    SortGrid& g = sg.g[0];
+    g.xmin = x_grid_min;
+    g.ymin = y_grid_min;
+    g.nx = nx;
+    g.ny = ny;
+    g.ncells = (nx + 1) * (ny + 1);
+    g.val = val_m;
+    g.val_grid = val_grid;
+    g.val_wt_sum = val_wt_sum;
+    g.wt_sum = wt_sum;
+    g.ld_sum = ld_sum;
+    return deposit(ctx, sg, x_m, y_m, nm, dx, dy, n_sum, s);
 }
 
 int sf_bilinear_marker_to_grids(sf_ctx* ctx, const sf_deposit_grid* grids, int n_grids, const double* x_m,
@@ -602,44 +772,24 @@ int sf_bilinear_marker_to_grids(sf_ctx* ctx, const sf_deposit_grid* grids, int n
     int rc = set_device(ctx);
     if (rc) return rc;
     cudaStream_t s = as_stream(stream);
-    const int64_t nmk = std::max<int64_t>(nm, 1);
-    if ((rc = ensure(ctx, ctx->keys, (size_t)(n_grids * nmk) * 4))) return rc;
-    if ((rc = ensure(ctx, ctx->counts, (size_t)total_cells * 4))) return rc;
-    int32_t* keys = (int32_t*)ctx->keys.ptr;
-    int32_t* counts = (int32_t*)ctx->counts.ptr;
-    SF_CUDA(cudaMemsetAsync(counts, 0, (size_t)total_cells * 4, s));
-    GridKeys gk{};
-    gk.n = n_grids;
-    int64_t off = 0;
-    for (int g = 0; g < n_grids; ++g) {
-        gk.xmin[g] = grids[g].x_grid_min;
-        gk.ymin[g] = grids[g].y_grid_min;
-        gk.nx[g] = grids[g].nx;
-        gk.ny[g] = grids[g].ny;
-        gk.keys[g] = keys + g * nmk;
-        gk.counts[g] = counts + off;
-        off += (grids[g].nx + 1) * (grids[g].ny + 1) + 1;
-    }
-    if (nm > 0) {
-        k_cell_keys_grids<<<grid_for(ctx, nm, DEP_THREADS), DEP_THREADS, 0, s>>>(x_m, y_m, nm, dx, dy, gk,
-                                                                                   ctx->d_counters + CNT_BAD_MARKERS);
-        SF_LAUNCHED(ctx);
-    }
-    for (int g = 0; g < n_grids; ++g) {
-        const sf_deposit_grid& d = grids[g];
-        if ((rc = sort_from_keys(ctx, gk.keys[g], gk.counts[g], x_m, y_m, d.val_m, nm, d.x_grid_min, d.y_grid_min, dx,
-                                 dy, d.nx, d.ny, s)))
-            return rc;
+    SortGrids sg{};
+    sg.n = n_grids;
+    for (int k = 0; k < n_grids; ++k) {
+        const sf_deposit_grid& d = grids[k];
+        SortGrid& g = sg.g[k];
+        g.xmin = d.x_grid_min;
+        g.ymin = d.y_grid_min;
+        g.nx = d.nx;
+        g.ny = d.ny;
+        g.ncells = (d.nx + 1) * (d.ny + 1);
+        g.val = d.val_m;
+        g.val_grid = d.val_grid;
         // as after one call per grid in order: the sum arrays hold the last grid's sums
-        const bool last = g == n_grids - 1;
-        if (wt_sum && last) {
-            SF_CUDA(cudaMemsetAsync(wt_sum, 0, (size_t)n_sum * 8, s));
-            SF_CUDA(cudaMemsetAsync(val_wt_sum, 0, (size_t)n_sum * 8, s));
-        }
-        launch_gather(ctx, d.nx, d.ny, d.val_grid, last ? val_wt_sum : nullptr, last ? wt_sum : nullptr, ld_sum, s);
-        SF_LAUNCHED(ctx);
+        g.val_wt_sum = k == n_grids - 1 ? val_wt_sum : nullptr;
+        g.wt_sum = k == n_grids - 1 ? wt_sum : nullptr;
+        g.ld_sum = ld_sum;
     }
-    return SF_OK;
+    return deposit(ctx, sg, x_m, y_m, nm, dx, dy, n_sum, s);
 }
 
 int sf_rebin_markers(sf_ctx* ctx, const double* x_m, const double* y_m, int64_t nm, double x_grid_min,
@@ -652,14 +802,24 @@ int sf_rebin_markers(sf_ctx* ctx, const double* x_m, const double* y_m, int64_t 
     int rc = set_device(ctx);
     if (rc) return rc;
     cudaStream_t s = as_stream(stream);
-    if ((rc = sort_by_cell(ctx, x_m, y_m, nullptr, nm, x_grid_min, y_grid_min, dx, dy, nx, ny,
-                           ctx->d_counters + CNT_OUTSIDE, s)))
-        return rc;
-    int64_t ncells = (nx + 1) * (ny + 1);
-    if (counts) SF_CUDA(cudaMemcpyAsync(counts, ctx->counts.ptr, (size_t)ncells * 4, cudaMemcpyDeviceToDevice, s));
-    if (offsets) SF_CUDA(cudaMemcpyAsync(offsets, ctx->offsets.ptr, (size_t)(ncells + 1) * 4, cudaMemcpyDeviceToDevice, s));
-    if (perm && nm > 0) SF_CUDA(cudaMemcpyAsync(perm, ctx->perm.ptr, (size_t)nm * 4, cudaMemcpyDeviceToDevice, s));
-    return SF_OK;
+    SortGrids sg{};
+    sg.n = 1;
+    SortGrid& g = sg.g[0];
+    g.xmin = x_grid_min;
+    g.ymin = y_grid_min;
+    g.nx = nx;
+    g.ny = ny;
+    g.ncells = (nx + 1) * (ny + 1);
+    if ((rc = sort_scratch(ctx, sg, nm, false, false, s))) return rc;
+    // the caller's arrays, where given, are the sort's own
+    if (counts) {
+        SF_CUDA(cudaMemsetAsync(counts, 0, (size_t)g.ncells * 4, s));
+        g.counts = counts;
+    }
+    if (offsets) g.offsets = offsets;
+    if (perm && nm > 0) g.perm = perm;
+    if ((rc = launch_keys(ctx, sg, x_m, y_m, nm, dx, dy, ctx->d_counters + CNT_OUTSIDE, s))) return rc;
+    return launch_sort(ctx, sg, x_m, y_m, nm, dx, dy, false, s);
 }
 
 }  // extern "C"
@@ -683,14 +843,15 @@ namespace sf {
 constexpr int64_t NA_MAX_MARKERS = SF_NOALLOC_MAX_MARKERS;
 constexpr int64_t NA_MAX_CELLS = SF_NOALLOC_MAX_CELLS;          // (nx + 1) * (ny + 1)
 constexpr int64_t NA_SCAN_TILES = (NA_MAX_CELLS + 1 + 8191) / 8192;
-// layout (bytes): keys | perm | counts | offsets | cursor | scan tiles | counters
+// layout (bytes): keys | perm | offsets | counts | cursors | scan tiles | long cells | counters
 constexpr size_t NA_OFF_KEYS = 0;
 constexpr size_t NA_OFF_PERM = NA_OFF_KEYS + 4 * NA_MAX_MARKERS;
-constexpr size_t NA_OFF_COUNTS = NA_OFF_PERM + 4 * NA_MAX_MARKERS;
-constexpr size_t NA_OFF_OFFSETS = NA_OFF_COUNTS + 4 * (NA_MAX_CELLS + 64);
-constexpr size_t NA_OFF_CURSOR = NA_OFF_OFFSETS + 4 * (NA_MAX_CELLS + 64);
+constexpr size_t NA_OFF_OFFSETS = NA_OFF_PERM + 4 * NA_MAX_MARKERS;
+constexpr size_t NA_OFF_COUNTS = NA_OFF_OFFSETS + 4 * (NA_MAX_CELLS + 64);
+constexpr size_t NA_OFF_CURSOR = NA_OFF_COUNTS + 4 * (NA_MAX_CELLS + 64);
 constexpr size_t NA_OFF_TILES = NA_OFF_CURSOR + 4 * (NA_MAX_CELLS + 64);
-constexpr size_t NA_OFF_COUNTERS = NA_OFF_TILES + 4 * ((NA_SCAN_TILES + 63) / 64 * 64);
+constexpr size_t NA_OFF_LIST = NA_OFF_TILES + 4 * ((NA_SCAN_TILES + 63) / 64 * 64);
+constexpr size_t NA_OFF_COUNTERS = NA_OFF_LIST + 4 * ((NA_MAX_MARKERS / (SORT_LONG + 1) + 64) / 64 * 64);
 constexpr size_t NA_BYTES = NA_OFF_COUNTERS + 4 * sizeof(unsigned long long);   // 2 counters, the long-cell count
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[NA_BYTES];
@@ -748,36 +909,42 @@ extern "C" int sf_bilinear_marker_to_grid_noalloc(double x_grid_min, double y_gr
     int rc = noalloc_scratch(&base, &num_sms);
     if (rc) return rc;
     cudaStream_t s = as_stream(stream);
-    int32_t* keys = (int32_t*)(base + NA_OFF_KEYS);
-    int32_t* perm = (int32_t*)(base + NA_OFF_PERM);
-    int32_t* counts = (int32_t*)(base + NA_OFF_COUNTS);
-    int32_t* offsets = (int32_t*)(base + NA_OFF_OFFSETS);
-    int32_t* cursor = (int32_t*)(base + NA_OFF_CURSOR);
-    int32_t* tiles = (int32_t*)(base + NA_OFF_TILES);
     unsigned long long* counters = (unsigned long long*)(base + NA_OFF_COUNTERS);
     const int64_t ncells = (nx + 1) * (ny + 1);
-    int32_t* n_long = (int32_t*)(counters + 2);
+    SortGrids sg{};
+    sg.n = 1;
+    SortGrid& g = sg.g[0];
+    g.xmin = x_grid_min;
+    g.ymin = y_grid_min;
+    g.nx = nx;
+    g.ny = ny;
+    g.ncells = ncells;
+    g.keys = (int32_t*)(base + NA_OFF_KEYS);
+    g.perm = (int32_t*)(base + NA_OFF_PERM);
+    g.offsets = (int32_t*)(base + NA_OFF_OFFSETS);
+    g.counts = (int32_t*)(base + NA_OFF_COUNTS);
+    g.cursor = (int32_t*)(base + NA_OFF_CURSOR);
+    g.tiles = (int32_t*)(base + NA_OFF_TILES);
+    g.list = (int32_t*)(base + NA_OFF_LIST);
+    g.n_list = (int32_t*)(counters + 2);
+    int32_t *offsets = g.offsets, *perm = g.perm;
     // the array keeps the previous call's contents: clear what must start at zero
-    SF_CUDA(cudaMemsetAsync(counts, 0, (size_t)(ncells + 1) * 4, s));
-    SF_CUDA(cudaMemsetAsync(cursor, 0, (size_t)(ncells + 1) * 4, s));
+    SF_CUDA(cudaMemsetAsync(g.counts, 0, (size_t)ncells * 4, s));
     SF_CUDA(cudaMemsetAsync(counters, 0, 4 * sizeof(unsigned long long), s));
     // grid-stride marker kernels: up to 32 blocks per SM of this device
     const unsigned blocks =
         (unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div(nm, DEP_THREADS), (int64_t)num_sms * 32));
     if (nm > 0) {
-        k_cell_keys<<<blocks, DEP_THREADS, 0, s>>>(x_m, y_m, nm, x_grid_min, y_grid_min, dx, dy, nx, ny, keys, counts,
-                                                   counters + 0);
+        k_cell_keys<1><<<blocks, DEP_THREADS, 0, s>>>(x_m, y_m, nm, dx, dy, sg, counters + 0);
         SF_CHECK_LAUNCH();
     }
-    if ((rc = exclusive_scan_i32_into(counts, offsets, ncells, offsets + ncells, tiles, s))) return rc;
+    int n = 0;
+    if ((rc = launch_scan(sg, s, &n))) return rc;
     if (nm > 0) {
-        k_scatter<<<blocks, DEP_THREADS, 0, s>>>(keys, nm, offsets, cursor, perm);
+        k_scatter<<<blocks, DEP_THREADS, 0, s>>>(sg, nm);
         SF_CHECK_LAUNCH();
-        // long segments by the radix sort (the spent cursors hold their list, the spent keys are its buffer),
-        // the others one thread per cell
-        k_long_cells<<<blocks, DEP_THREADS, 0, s>>>(offsets, ncells, cursor, n_long);
-        SF_CHECK_LAUNCH();
-        k_sort_long<<<(unsigned)num_sms * 2, SORT_THREADS, 0, s>>>(offsets, cursor, n_long, perm, keys);
+        // long segments by the radix sort (the spent keys are its buffer), the others one thread per cell
+        k_sort_long<<<(unsigned)num_sms * 2, SORT_THREADS, 0, s>>>(sg);
         SF_CHECK_LAUNCH();
     }
     k_sort_segments<<<(unsigned)ceil_div(ncells, 128), 128, 0, s>>>(offsets, ncells, perm);

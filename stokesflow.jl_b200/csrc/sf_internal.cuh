@@ -65,9 +65,9 @@ enum { SC_DT = 0, SC_DT_CHECK = 1, SC_ERR = 2, SC_SUM_RX = 3, SC_SUM_RY = 4, SC_
 struct sf_ctx {
     int device = 0;
     int num_sms = 148;
-    // deposit / rebin scratch: cell keys, counts, offsets, scatter cursors, the cell-ordered permutation, scan
-    // tiles, the deposit's sorted payload records and the list of long cells
-    sf::Scratch keys, counts, offsets, cursor, perm, scan_tmp, payload, longs;
+    // deposit / rebin scratch: cell keys and ranks, counts, offsets, the cell-ordered permutation, scan tiles, the
+    // deposit's sorted payload records and the lists of long cells
+    sf::Scratch keys, counts, offsets, perm, scan_tmp, payload, longs;
     // PT solve: padded internal fields, reduction partials; mixed/batched engine arena
     sf::Scratch fields, partials, mixed;
     // decomposed timestep: marker-exchange and overlap-sum staging
@@ -136,13 +136,6 @@ cudaError_t launch_overlapped(bool overlap, void (*kern)(Params...), dim3 grid, 
 
 inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 inline int64_t round_up(int64_t a, int64_t b) { return ceil_div(a, b) * b; }
-
-// exclusive scan of n int32 values (in may alias out); total -> *d_total (device)
-int exclusive_scan_i32(sf_ctx* ctx, const int32_t* in, int32_t* out, int64_t n, int32_t* d_total,
-                       cudaStream_t stream);
-// the same with a caller-provided tile buffer of ceil(n / 8192) ints; allocates nothing
-int exclusive_scan_i32_into(const int32_t* in, int32_t* out, int64_t n, int32_t* d_total, int32_t* tiles,
-                            cudaStream_t stream);
 
 // --------------------------------------------------------------------------
 // device helpers
