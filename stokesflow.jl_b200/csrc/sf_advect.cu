@@ -3,6 +3,14 @@
 // expression keeps the reference's order and the file is compiled with
 // -fmad=false, so positions are bit-identical to the reference's.
 //
+// Markers whose four stages stay inside the grid, away from the reference's
+// index failsafes -- all but a few -- take interpolate_fast: 32-bit indices,
+// one range test instead of the failsafes, and the divisions by dx and dy as
+// divisions by a constant (div_const).  The others take the general code.
+// FP64 bounds it: 61% of the pipe, 1005 warp instructions per 32 markers (1885
+// with the failsafes and divisions of the general code for all).  26 M markers
+// 1.72 -> 1.13 ms, 67 M 4.45 -> 2.89.
+//
 // The padded velocity arrays (2 x (N+2)(N+1) doubles, 67 MB at N = 2048) sit
 // in the 126 MB L2, so the 4 x 12 gathers per marker are L2 hits; HBM traffic
 // is the marker read/write (32 B per marker) plus one pass over V.
@@ -18,6 +26,8 @@ struct AdvectArgs {
     int64_t vx_nx, vx_ny, vy_nx, vy_ny;
     double x_vx_min, y_vx_min, x_vy_min, y_vy_min;
     double dx, dy;
+    double rdx, rdy;     // RN(1 / dx), RN(1 / dy)
+    int fast;            // interpolate_fast may be used: arrays of less than 2^31 entries, dx and dy of ordinary size
 };
 
 // MoveMarkers.jl:181-187 bilinearInterp
@@ -33,9 +43,78 @@ __device__ __forceinline__ double bilinear_interp(double v1, double v2, double v
 #define VXA(i, j) __ldg(&a.Vx[((i) - 1) + ((j) - 1) * a.vx_nx])
 #define VYA(i, j) __ldg(&a.Vy[((i) - 1) + ((j) - 1) * a.vy_nx])
 
+// a / b correctly rounded, from y = RN(1 / b): q = RN(a y) is within 1.5 ulp of a / b; one correction by its remainder
+// brings it within 1 ulp, and then the remainder a - b q is exact and RN(q + r y) = RN(a / b) (Markstein, "Computation of
+// elementary functions on the IBM RISC System/6000 processor", 1990: the theorem on a faithful quotient and a correctly
+// rounded reciprocal).  Needs |a| of 2^-960 .. 2^960 (or 0) and b of 2^-60 .. 2^60, so that nothing is lost below the
+// exponent range.  Five FP64 operations; the division is about twice that.
+__device__ __forceinline__ double div_const(double a, double b, double y) {
+    double q = a * y;
+    q = __fma_rn(__fma_rn(-b, q, a), y, q);
+    return __fma_rn(__fma_rn(-b, q, a), y, q);
+}
+
+// topleftIndexRelDist (common.jl:22-33) along one axis: the 0-based index floor((x - xmin) / dx) and the relative distance.
+// False where div_const's range, or an int, does not hold them: NaN, infinities, distances below 2^-895.
+__device__ __forceinline__ bool axis_fast(double x, double xmin, double dx, double rdx, int& i, double& d) {
+    i = __double2int_rd(div_const(x - xmin, dx, rdx));
+    const double rel = x - (xmin + (double)i * dx);
+    d = div_const(rel, dx, rdx);
+    const unsigned hi = (unsigned)__double2hiint(rel) & 0x7fffffffu;
+    return hi - 0x08000000u < 0x70000000u || (hi | (unsigned)__double2loint(rel)) == 0u;
+}
+
+// interpolate_v where no failsafe applies; false (and nothing of use) elsewhere.
+__device__ __forceinline__ bool interpolate_fast(const AdvectArgs& a, double x, double y, double& vx, double& vy) {
+    bool ok;
+    {
+        int i, j;
+        double dx, dy;
+        ok = axis_fast(x, a.x_vx_min, a.dx, a.rdx, i, dx) & axis_fast(y, a.y_vx_min, a.dy, a.rdy, j, dy);
+        const int nx = (int)a.vx_nx, ny = (int)a.vx_ny;
+        // 2 <= ix <= nx - 2, 1 <= iy <= ny - 1 (1-based)
+        ok = ok && (unsigned)(i - 1) < (unsigned)(nx - 3) && (unsigned)j < (unsigned)(ny - 1);
+        if (!ok) return false;
+        const double* __restrict__ p = a.Vx + (i + j * nx);
+        const double* __restrict__ q = p + nx;
+        const double v1 = __ldg(p), v2 = __ldg(p + 1), v3 = __ldg(q), v4 = __ldg(q + 1);
+        const double v = bilinear_interp(v1, v2, v3, v4, dx, dy);
+        const bool far = dx >= 0.5;
+        const int e = far ? 2 : -1;
+        const double v5 = __ldg(p + e), v6 = __ldg(q + e);
+        const double h = dx - 0.5;
+        // far: v1 - 2 v2 + v5, else v5 - 2 v1 + v2 (and likewise one row up)
+        const double l = (far ? v1 : v5) - 2.0 * (far ? v2 : v1) + (far ? v5 : v2);
+        const double u = (far ? v3 : v6) - 2.0 * (far ? v4 : v3) + (far ? v6 : v4);
+        vx = v + 0.5 * (h * h) * ((1.0 - dy) * l + dy * u);
+    }
+    {
+        int i, j;
+        double dx, dy;
+        ok = axis_fast(x, a.x_vy_min, a.dx, a.rdx, i, dx) & axis_fast(y, a.y_vy_min, a.dy, a.rdy, j, dy);
+        const int nx = (int)a.vy_nx, ny = (int)a.vy_ny;
+        // 1 <= ix <= nx - 1, 2 <= iy <= ny - 2
+        ok = ok && (unsigned)i < (unsigned)(nx - 1) && (unsigned)(j - 1) < (unsigned)(ny - 3);
+        if (!ok) return false;
+        const double* __restrict__ p = a.Vy + (i + j * nx);
+        const double* __restrict__ q = p + nx;
+        const double v1 = __ldg(p), v2 = __ldg(p + 1), v3 = __ldg(q), v4 = __ldg(q + 1);
+        const double v = bilinear_interp(v1, v2, v3, v4, dx, dy);
+        const bool far = dy >= 0.5;
+        const int e = far ? 2 * nx : -nx;
+        const double v5 = __ldg(p + e), v6 = __ldg(p + e + 1);
+        const double h = dy - 0.5;
+        const double l = (far ? v1 : v5) - 2.0 * (far ? v3 : v1) + (far ? v5 : v3);
+        const double u = (far ? v2 : v6) - 2.0 * (far ? v4 : v2) + (far ? v6 : v4);
+        vy = v + 0.5 * (h * h) * ((1.0 - dx) * l + dx * u);
+    }
+    return true;
+}
+
 // MoveMarkers.jl:76-174 interpolateV.  ix, iy are 1-based as in the reference.
-__device__ __forceinline__ void interpolate_v(const AdvectArgs& a, double x, double y, double& vx_out, double& vy_out,
-                                              int& nfail) {
+struct Velocity { double vx, vy; int nfail; };
+__device__ __noinline__ Velocity interpolate_v(const AdvectArgs& a, double x, double y) {
+    int nfail = 0;
     // ---- Vx ----
     TopLeft t = topleft(a.x_vx_min, a.y_vx_min, x, y, a.dx, a.dy);
     double dxij = t.dxij, dyij = t.dyij;
@@ -88,12 +167,11 @@ __device__ __forceinline__ void interpolate_v(const AdvectArgs& a, double x, dou
         correction = 0.5 * (h * h) * ((1.0 - dxij) * (v5 - 2.0 * v1 + v3) + dxij * (v6 - 2.0 * v2 + v4));
     }
     vy = vy + correction;
-    vx_out = vx;
-    vy_out = vy;
+    return Velocity{vx, vy, nfail};
 }
 
 // MoveMarkers.jl:30-69 moveMarkersRK4_Kernel!
-__global__ void __launch_bounds__(256) k_move_markers_rk4(AdvectArgs a, double* __restrict__ x_m,
+__global__ void __launch_bounds__(256) k_move_markers_rk4(const __grid_constant__ AdvectArgs a, double* __restrict__ x_m,
                                                          double* __restrict__ y_m, int64_t nm, double dt, double lx,
                                                          double ly, unsigned long long* __restrict__ fail_counter) {
     const double rk4_dt[4] = {0.0, 0.5 * dt, 0.5 * dt, dt};
@@ -106,7 +184,12 @@ __global__ void __launch_bounds__(256) k_move_markers_rk4(AdvectArgs a, double* 
         for (int it = 0; it < 4; ++it) {
             double x_rk = x_old + rk4_dt[it] * vx_rk;
             double y_rk = y_old + rk4_dt[it] * vy_rk;
-            interpolate_v(a, x_rk, y_rk, vx_rk, vy_rk, nfail);
+            if (!(a.fast && interpolate_fast(a, x_rk, y_rk, vx_rk, vy_rk))) {
+                const Velocity w = interpolate_v(a, x_rk, y_rk);
+                vx_rk = w.vx;
+                vy_rk = w.vy;
+                nfail += w.nfail;
+            }
             vx_eff = vx_eff + rk4_wt[it] * vx_rk;
             vy_eff = vy_eff + rk4_wt[it] * vy_rk;
         }
@@ -139,7 +222,9 @@ int sf_move_markers_rk4(sf_ctx* ctx, double* x_m, double* y_m, int64_t nm, const
     if (nm == 0) return SF_OK;
     int rc = set_device(ctx);
     if (rc) return rc;
-    AdvectArgs a{Vx, Vy, vx_nx, vx_ny, vy_nx, vy_ny, x_vx_min, y_vx_min, x_vy_min, y_vy_min, dx, dy};
+    AdvectArgs a{Vx, Vy, vx_nx, vx_ny, vy_nx, vy_ny, x_vx_min, y_vx_min, x_vy_min, y_vy_min, dx, dy, 1.0 / dx, 1.0 / dy, 0};
+    auto ordinary = [](double v) { return v > 0x1p-60 && v < 0x1p60; };
+    a.fast = ordinary(dx) && ordinary(dy) && vx_nx < INT32_MAX / 4 / vx_ny && vy_nx < INT32_MAX / 4 / vy_ny;
     unsigned blocks = (unsigned)std::min<int64_t>(ceil_div(nm, 256), (int64_t)ctx->num_sms * 16);
     k_move_markers_rk4<<<blocks, 256, 0, as_stream(stream)>>>(a, x_m, y_m, nm, dt, lx, ly,
                                                               ctx->d_counters + CNT_INTERP_FAILSAFE);
