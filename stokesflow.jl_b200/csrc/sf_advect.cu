@@ -43,25 +43,13 @@ __device__ __forceinline__ double bilinear_interp(double v1, double v2, double v
 #define VXA(i, j) __ldg(&a.Vx[((i) - 1) + ((j) - 1) * a.vx_nx])
 #define VYA(i, j) __ldg(&a.Vy[((i) - 1) + ((j) - 1) * a.vy_nx])
 
-// a / b correctly rounded, from y = RN(1 / b): q = RN(a y) is within 1.5 ulp of a / b; one correction by its remainder
-// brings it within 1 ulp, and then the remainder a - b q is exact and RN(q + r y) = RN(a / b) (Markstein, "Computation of
-// elementary functions on the IBM RISC System/6000 processor", 1990: the theorem on a faithful quotient and a correctly
-// rounded reciprocal).  Needs |a| of 2^-960 .. 2^960 (or 0) and b of 2^-60 .. 2^60, so that nothing is lost below the
-// exponent range.  Five FP64 operations; the division is about twice that.
-__device__ __forceinline__ double div_const(double a, double b, double y) {
-    double q = a * y;
-    q = __fma_rn(__fma_rn(-b, q, a), y, q);
-    return __fma_rn(__fma_rn(-b, q, a), y, q);
-}
-
 // topleftIndexRelDist (common.jl:22-33) along one axis: the 0-based index floor((x - xmin) / dx) and the relative distance.
 // False where div_const's range, or an int, does not hold them: NaN, infinities, distances below 2^-895.
 __device__ __forceinline__ bool axis_fast(double x, double xmin, double dx, double rdx, int& i, double& d) {
     i = __double2int_rd(div_const(x - xmin, dx, rdx));
     const double rel = x - (xmin + (double)i * dx);
     d = div_const(rel, dx, rdx);
-    const unsigned hi = (unsigned)__double2hiint(rel) & 0x7fffffffu;
-    return hi - 0x08000000u < 0x70000000u || (hi | (unsigned)__double2loint(rel)) == 0u;
+    return div_const_takes_a(rel);
 }
 
 // interpolate_v where no failsafe applies; false (and nothing of use) elsewhere.
@@ -223,8 +211,7 @@ int sf_move_markers_rk4(sf_ctx* ctx, double* x_m, double* y_m, int64_t nm, const
     int rc = set_device(ctx);
     if (rc) return rc;
     AdvectArgs a{Vx, Vy, vx_nx, vx_ny, vy_nx, vy_ny, x_vx_min, y_vx_min, x_vy_min, y_vy_min, dx, dy, 1.0 / dx, 1.0 / dy, 0};
-    auto ordinary = [](double v) { return v > 0x1p-60 && v < 0x1p60; };
-    a.fast = ordinary(dx) && ordinary(dy) && vx_nx < INT32_MAX / 4 / vx_ny && vy_nx < INT32_MAX / 4 / vy_ny;
+    a.fast = div_const_takes(dx) && div_const_takes(dy) && vx_nx < INT32_MAX / 4 / vx_ny && vy_nx < INT32_MAX / 4 / vy_ny;
     unsigned blocks = (unsigned)std::min<int64_t>(ceil_div(nm, 256), (int64_t)ctx->num_sms * 16);
     k_move_markers_rk4<<<blocks, 256, 0, as_stream(stream)>>>(a, x_m, y_m, nm, dt, lx, ly,
                                                               ctx->d_counters + CNT_INTERP_FAILSAFE);

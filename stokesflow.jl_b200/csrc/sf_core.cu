@@ -284,7 +284,7 @@ int sf_ctx_destroy(sf_ctx* c) {
     cudaSetDevice(c->device);
     cudaDeviceSynchronize();
     mixed_engine_release(c);
-    Scratch* all[] = {&c->keys,     &c->counts, &c->offsets,  &c->perm,  &c->payload, &c->longs,
+    Scratch* all[] = {&c->keys,     &c->counts, &c->offsets,  &c->perm,  &c->records, &c->longs,
                       &c->scan_tmp, &c->fields, &c->partials, &c->mixed,  &c->exch, &c->halo};
     for (Scratch* s : all)
         if (s->ptr) cudaFree(s->ptr);
@@ -302,7 +302,7 @@ int sf_ctx_destroy(sf_ctx* c) {
 
 int sf_ctx_scratch_bytes(sf_ctx* c, int64_t* bytes) {
     if (!c || !bytes) return fail(SF_ERR_INVALID_ARG, "sf_ctx_scratch_bytes: NULL argument");
-    const Scratch* all[] = {&c->keys,     &c->counts, &c->offsets,  &c->perm,  &c->payload, &c->longs,
+    const Scratch* all[] = {&c->keys,     &c->counts, &c->offsets,  &c->perm,  &c->records, &c->longs,
                             &c->scan_tmp, &c->fields, &c->partials, &c->mixed,  &c->exch, &c->halo};
     int64_t b = 0;
     for (const Scratch* s : all) b += (int64_t)s->bytes;

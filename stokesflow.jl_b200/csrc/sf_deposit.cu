@@ -3,33 +3,35 @@
 //
 // Design: the reference scatters 8 floating-point adds per marker (serial on
 // the CPU, CUDA.@atomic on the GPU, MarkerToGrid.jl:58-155).  Here the adds
-// become a gather with no floating-point atomics:
-//   1. k_cell_keys     cell (ix, iy) of every marker for each grid, exactly
-//                      topleftIndexRelDist (common.jl:22-33); per-cell counts
-//                      with warp-aggregated integer atomics.
+// become a gather with no floating-point atomics: a node visits the markers of
+// its four adjacent cells in ascending marker index, the reference CPU loop's
+// order, so its sums are bit-identical to it.  Markers keep much of their
+// initial lattice order, so a cell's markers are a few runs of consecutive
+// indices; the deposit sorts runs, not markers:
+//   1. k_cell_runs     cell (ix, iy) of every marker for each grid, exactly
+//                      topleftIndexRelDist (common.jl:22-33); runs of
+//                      consecutive markers of one cell (within a warp's 32),
+//                      counted per cell, their last markers as a bit mask; and
+//                      the markers' x, y and values as records of 32 bytes.
 //   2. k_scan_*        exclusive scan of the counts -> cell offsets (and the
 //                      list of long cells).
-//   3. k_scatter       marker indices into their cell's segment (in no
-//                      particular order inside it).
-//   4. segment sort    every segment ascending by marker index, which makes
-//                      the whole a stable counting sort:
-//                      k_sort_long sorts the cells holding more than
-//                      SORT_LONG markers in place (a block-wide LSD radix
-//                      sort per cell, stable, linear in the cell's count, so a
-//                      cell where markers pile up costs no more than its
-//                      size); k_sort_cells sorts the others in shared memory,
-//                      a window of consecutive cells at a time.
-//   5. k_gather_sorted one thread per node merges the four adjacent cells'
-//                      segments by marker index and accumulates w and w*val in
-//                      ascending marker order -- the reference CPU loop's
-//                      order, so each node's sums are bit-identical to it --
-//                      then divides (safeDivision, :164-172).
-// For the deposit, step 4 writes each sorted entry as a payload record
-// {dxij, dyij, val, m} (the marker's relative position in its cell, computed
-// once with topleftIndexRelDist's IEEE divisions, its value and its index), so
-// the gather streams contiguous records of neighbouring cells instead of
-// chasing marker indices into x, y and val.  Steps 1-4 with the permutation as
-// output are the rebin (sf_rebin_markers).
+//   3. k_scatter_runs  the runs' first markers into their cell's segment (in
+//                      no particular order inside it).
+//   4. segment sort    every segment ascending: k_sort_long sorts the cells
+//                      holding more than SORT_LONG entries in place (a
+//                      block-wide LSD radix sort per cell, stable, linear in
+//                      the cell's count, so a cell where markers pile up costs
+//                      no more than its size); k_sort_cells sorts the others
+//                      in shared memory, a window of consecutive cells at a
+//                      time.
+//   5. k_gather_runs   one thread per node merges the four adjacent cells'
+//                      runs (they are disjoint intervals, so a run is taken
+//                      whole, its records loaded several at a time),
+//                      accumulates w and w*val, and divides (safeDivision,
+//                      :164-172).
+// The rebin (sf_rebin_markers) sorts markers the same way: k_cell_keys,
+// k_scan_*, k_scatter, segment sort; the allocation-free deposit gathers from
+// that.
 //
 // The grids of a timestep go through each kernel together (8 launches instead of
 // 32): small deposits were bound by their launches.
@@ -44,16 +46,14 @@ constexpr int SORT_THREADS = 256;
 constexpr int SORT_CPB = 256;     // cells per block of k_sort_cells
 constexpr int SORT_CAP = 4096;    // entries of a k_sort_cells window in shared memory
 constexpr int SORT_LONG = 64;     // cells with more markers are sorted by k_sort_long
-// markers up to which the grids of a deposit go through each kernel in one launch, every grid in scratch of its own (40
-// bytes per marker and grid).  145 k markers: 228 -> 84 us; 1.4 M: 443 -> 315; 4.2 M: 920 -> 714.  Beyond, launches
-// no longer count (26 M markers: 4.10 ms either way) and one grid's scratch serves all.
+// markers up to which the grids of a deposit go through each kernel in one launch, every grid in scratch of its own (4
+// bytes per marker and grid).  Against one grid after the other, 145 k markers: 228 -> 84 us; 1.4 M: 443 -> 315; 4.2 M:
+// 920 -> 714.  Beyond, launches no longer count (26 M markers: 4.10 ms either way) and one grid's scratch serves all.
 constexpr int64_t DEPOSIT_TOGETHER = 1 << 22;
 
-// A sorted deposit entry: the marker's relative position in its cell (topleftIndexRelDist's dxij, dyij), its
-// value and its index.  32 bytes: one sector.
-struct __align__(32) Payload {
-    double dxij, dyij, val;
-    int32_t m, pad_;
+// What the gather reads of a marker: its position and its values in up to two arrays.  32 bytes: one sector.
+struct __align__(32) Record {
+    double x, y, v0, v1;
 };
 
 // One grid of a sort: what its kernels read and write.  Several grids over the same markers (the deposits of a timestep)
@@ -68,8 +68,10 @@ struct SortGrid {
     int32_t* tiles;            // sums of the scan's tiles
     int32_t* n_list;           // the cells holding more than SORT_LONG markers: their number ...
     int32_t* list;             // ... and the cells
-    int32_t* perm;
-    Payload* payload;          // (deposit)
+    int32_t* perm;             // sorted markers, or (deposit) first markers of runs
+    uint32_t* ends;            // (deposit) bit m & 31 of word m / 32: marker m is the last of its run
+    int32_t* general;          // (deposit) not 0: some distance is out of div_const's range
+    int second;                // (deposit) the grid's values are the records' v1
     const double* val;
     double *val_grid, *val_wt_sum, *wt_sum;
     int64_t ld_sum;
@@ -77,39 +79,84 @@ struct SortGrid {
 struct SortGrids {
     SortGrid g[SF_MAX_GRIDS];
     int n;
+    const double *val0, *val1; // (deposit) the records' values
+    Record* rec;
 };
 
-// 1. cell key of every marker for every grid (positions are read once); counts[key]++ (warp-aggregated).  (Keeping the
+// 1 for the rebin and the allocation-free deposit: cell key of every marker; counts[key]++ (warp-aggregated).  (Keeping the
 // counters' old values as the markers' places, so that the scatter needs no atomics, costs more here, 87 us per grid and
 // 26 M markers, than the 25 us it saves there.)
-template <int MOST>   // grids at most
 __global__ void k_cell_keys(const double* __restrict__ x, const double* __restrict__ y, int64_t nm, double dx, double dy,
                             const __grid_constant__ SortGrids s, unsigned long long* __restrict__ bad_counter) {
+    const SortGrid& g = s.g[0];
     const int lane = threadIdx.x & 31;
     int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t base = (int64_t)blockIdx.x * blockDim.x; base < nm; base += stride) {
+        int64_t m = base + threadIdx.x;
+        int32_t key = -1;
+        if (m < nm) {
+            TopLeft t = topleft(g.xmin, g.ymin, x[m], y[m], dx, dy);
+            // MarkerToGrid.jl:66: accept iff 0 <= ix <= Nx && 0 <= iy <= Ny (ix = qx + 1)
+            if (t.qx >= -1.0 && t.qx <= (double)(g.nx - 1) && t.qy >= -1.0 && t.qy <= (double)(g.ny - 1))
+                key = (int32_t)((int64_t)t.qx + 1 + ((int64_t)t.qy + 1) * (g.nx + 1));
+            g.keys[m] = key;
+        }
+        unsigned active = __ballot_sync(0xffffffffu, m < nm);
+        if (m < nm) {
+            unsigned peers = __match_any_sync(active, key);
+            if (lane == __ffs(peers) - 1) {
+                int n = __popc(peers);
+                if (key >= 0)
+                    atomicAdd(&g.counts[key], n);
+                else if (bad_counter)
+                    atomicAdd(bad_counter, (unsigned long long)n);
+            }
+        }
+    }
+}
+
+// 1 for a deposit: the runs of consecutive markers that share a cell, and the records.
+template <int MOST>
+__global__ void k_cell_runs(const double* __restrict__ x, const double* __restrict__ y, int64_t nm, double dx, double dy,
+                            const __grid_constant__ SortGrids s, unsigned long long* __restrict__ bad_counter) {
+    const int lane = threadIdx.x & 31;
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t base = (int64_t)blockIdx.x * blockDim.x; base < nm; base += stride) {
         const int64_t m = base + threadIdx.x;
         const bool live = m < nm;
         const double xm = live ? x[m] : 0.0, ym = live ? y[m] : 0.0;
-        const unsigned active = __ballot_sync(0xffffffffu, live);
+        if (live) {
+            Record r;
+            r.x = xm;
+            r.y = ym;
+            r.v0 = s.val0[m];
+            r.v1 = s.val1 ? s.val1[m] : 0.0;
+            s.rec[m] = r;
+        }
 #pragma unroll
         for (int k = 0; k < MOST; ++k) {
             if (MOST > 1 && k >= s.n) break;
-            if (!live) continue;
             const SortGrid& g = s.g[k];
             int32_t key = -1;
             const TopLeft t = topleft(g.xmin, g.ymin, xm, ym, dx, dy);
             // MarkerToGrid.jl:66: accept iff 0 <= ix <= Nx && 0 <= iy <= Ny (ix = qx + 1)
             if (t.qx >= -1.0 && t.qx <= (double)(g.nx - 1) && t.qy >= -1.0 && t.qy <= (double)(g.ny - 1))
                 key = (int32_t)((int64_t)t.qx + 1 + ((int64_t)t.qy + 1) * (g.nx + 1));
-            g.keys[m] = key;
-            const unsigned peers = __match_any_sync(active, key);
-            if (lane == __ffs(peers) - 1) {
-                const int n = __popc(peers);
-                if (key >= 0)
-                    atomicAdd(&g.counts[key], n);
-                else if (bad_counter)
-                    atomicAdd(bad_counter, (unsigned long long)n);
+            const int32_t prev = __shfl_up_sync(0xffffffffu, key, 1);
+            const bool start = !live || lane == 0 || prev != key;
+            const unsigned starts = __ballot_sync(0xffffffffu, start);
+            const unsigned bad = __ballot_sync(0xffffffffu, live && key < 0);
+            if (live) {
+                g.keys[m] = key;
+                if (start && key >= 0) atomicAdd(&g.counts[key], 1);
+            }
+            // the gather divides these by dx, dy (topleft's dxij, dyij)
+            const bool odd = live && key >= 0 &&
+                             !(div_const_takes_a(xm - (g.xmin + t.qx * dx)) && div_const_takes_a(ym - (g.ymin + t.qy * dy)));
+            if (__any_sync(0xffffffffu, odd) && lane == 0) *g.general = 1;
+            if (lane == 0 && live) {
+                g.ends[m >> 5] = starts >> 1 | 0x80000000u;
+                if (bad && bad_counter) atomicAdd(bad_counter, (unsigned long long)__popc(bad));
             }
         }
     }
@@ -230,6 +277,17 @@ __global__ void k_scatter(const __grid_constant__ SortGrids s, int64_t nm) {
     }
 }
 
+// 3 for a deposit: the runs' first markers.
+__global__ void k_scatter_runs(const __grid_constant__ SortGrids s, int64_t nm) {
+    const SortGrid& g = s.g[blockIdx.y];
+    for (int64_t m = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; m < nm; m += (int64_t)gridDim.x * blockDim.x) {
+        const int q = (int)(m & 31);
+        if (q != 0 && !(g.ends[m >> 5] >> (q - 1) & 1u)) continue;
+        const int32_t key = g.keys[m];
+        if (key >= 0) g.perm[atomicAdd(&g.cursor[key], 1)] = (int32_t)m;
+    }
+}
+
 // The allocation-free deposit's per-cell sort of short segments (one thread per cell; its long segments are
 // sorted by k_sort_long first, and are skipped here).
 __global__ void k_sort_segments(const int32_t* __restrict__ offsets, int64_t ncells, int32_t* __restrict__ perm) {
@@ -321,15 +379,11 @@ __global__ void __launch_bounds__(SORT_THREADS) k_sort_long(const __grid_constan
     }
 }
 
-// 4b. every short segment sorted ascending; long segments (sorted by k_sort_long) pass through in order.  A
-// block takes SORT_CPB consecutive cells and works through them in windows of consecutive cells holding at most
-// SORT_CAP entries: it loads a window's marker indices into shared memory, ranks each entry within its cell by
-// counting the smaller indices there, and writes it to its sorted place -- back into perm (the rebin), or as a
-// payload record (the deposit: topleftIndexRelDist of the marker and its value, once per marker).
-template <bool PAYLOAD>
-__global__ void __launch_bounds__(SORT_THREADS) k_sort_cells(const __grid_constant__ SortGrids s,
-                                                             const double* __restrict__ x, const double* __restrict__ y,
-                                                             double dx, double dy) {
+// 4b. every short segment sorted ascending, in place; long segments are sorted already (k_sort_long).  A block takes
+// SORT_CPB consecutive cells and works through them in windows of consecutive cells holding at most SORT_CAP entries:
+// it loads a window's entries into shared memory, ranks each within its cell by counting the smaller ones there, and
+// writes it to its sorted place.
+__global__ void __launch_bounds__(SORT_THREADS) k_sort_cells(const __grid_constant__ SortGrids s) {
     __shared__ int32_t soff[SORT_CPB + 1];
     __shared__ int32_t sm[SORT_CAP];
     const int tid = threadIdx.x;
@@ -337,24 +391,11 @@ __global__ void __launch_bounds__(SORT_THREADS) k_sort_cells(const __grid_consta
     const int64_t ncells = g.ncells;
     const int32_t* __restrict__ offsets = g.offsets;
     int32_t* perm = g.perm;
-    Payload* __restrict__ out = g.payload;
-    const double* __restrict__ val = g.val;
-    const double xmin = g.xmin, ymin = g.ymin;
     const int64_t c0 = (int64_t)blockIdx.x * SORT_CPB;
     if (c0 >= ncells) return;
     const int nc = (int)min((int64_t)SORT_CPB, ncells - c0);
     for (int i = tid; i <= nc; i += SORT_THREADS) soff[i] = offsets[c0 + i];
     __syncthreads();
-    auto record = [&](int32_t m) {
-        const TopLeft t = topleft(xmin, ymin, x[m], y[m], dx, dy);
-        Payload p;
-        p.dxij = t.dxij;
-        p.dyij = t.dyij;
-        p.val = val[m];
-        p.m = m;
-        p.pad_ = 0;
-        return p;
-    };
     int w0 = 0;
     while (w0 < nc) {
         // the largest w1 with soff[w1] - soff[w0] <= SORT_CAP (w1 == w0: cell w0 alone holds more)
@@ -364,9 +405,7 @@ __global__ void __launch_bounds__(SORT_THREADS) k_sort_cells(const __grid_consta
             if (soff[mid] - soff[w0] <= SORT_CAP) lo = mid; else hi = mid - 1;
         }
         const int w1 = lo;
-        if (w1 == w0) {  // a long cell, sorted already: pass it through
-            if (PAYLOAD)
-                for (int32_t pos = soff[w0] + tid; pos < soff[w0 + 1]; pos += SORT_THREADS) out[pos] = record(perm[pos]);
+        if (w1 == w0) {  // a long cell
             ++w0;
             continue;
         }
@@ -375,11 +414,6 @@ __global__ void __launch_bounds__(SORT_THREADS) k_sort_cells(const __grid_consta
         for (int i = tid; i < ne; i += SORT_THREADS) sm[i] = perm[e0 + i];
         __syncthreads();
         for (int i = tid; i < ne; i += SORT_THREADS) {
-            // the record's scattered loads come first: the search and the count below hide them (3.16 -> 3.03 ms per
-            // grid of 67 M markers)
-            const int32_t v = sm[i];
-            Payload p{};
-            if (PAYLOAD) p = record(v);
             // the entry's cell k: the last one in [w0, w1) starting at or before it
             int a = w0, z = w1 - 1;
             while (a < z) {
@@ -387,118 +421,100 @@ __global__ void __launch_bounds__(SORT_THREADS) k_sort_cells(const __grid_consta
                 if (soff[mid] - e0 <= i) a = mid; else z = mid - 1;
             }
             const int cb = soff[a] - e0, ce = soff[a + 1] - e0;
-            int rank = i - cb;
             if (ce - cb <= SORT_LONG) {
-                rank = 0;
+                const int32_t v = sm[i];
+                int rank = 0;
                 for (int j = cb; j < ce; ++j) rank += (sm[j] < v) ? 1 : 0;
-            }
-            if (PAYLOAD)
-                out[e0 + cb + rank] = p;
-            else
                 perm[e0 + cb + rank] = v;
+            }
         }
         __syncthreads();
         w0 = w1;
     }
 }
 
-// 5. per-node gather over the sorted payload.  Node (I, J), 1-based.  A marker in cell (ix, iy) contributes to
+// 5. per-node gather over the sorted runs.  Node (I, J), 1-based.  A marker in cell (ix, iy) contributes to
 // node (ix, iy) with (1-dx)(1-dy), (ix+1, iy) with dx(1-dy), (ix, iy+1) with (1-dx)dy and (ix+1, iy+1) with dx*dy
-// (MarkerToGrid.jl:124-151), so node (I, J) merges the cells (I,J), (I-1,J), (I,J-1), (I-1,J-1), whose records
-// are sorted by marker index: taking the smallest head each time visits the node's markers in ascending
-// index order, the reference's serial order.
+// (MarkerToGrid.jl:124-151), so node (I, J) merges the cells (I,J), (I-1,J), (I,J-1), (I-1,J-1), whose runs are sorted by
+// marker index: taking the run with the smallest first marker each time visits the node's markers in ascending index
+// order, the reference's serial order.  The next run's start is loaded while the taken run's records are, GT_AHEAD of
+// them at once, so a node waits for memory once per run, not once per marker.
 //
-// Each list's head record is held in registers, so a visit reads its record once, with one 32-byte load (the
-// four threads that use a record read it from L2).  The merge gallops: once the smallest head is chosen, the
-// records of its list that stay below the other lists' smallest head are the merge's next picks, in order,
-// and are taken in an inner loop without comparing the four heads again.  Markers keep much of their initial
-// lattice order, so these runs are several records long.
-constexpr int GT_NONE = 0x7fffffff;   // head of an exhausted list
+// What bounds it: the latency of those loads (27 warps per SM) and half the L1 rate: each of 32 lanes reads a line of its
+// own.  Three grids over 67 M markers: 9.07 -> 7.73 ms against sorting the markers themselves into 32-byte records per
+// grid (sort 0.95, gather 1.14 ms per grid); 26 M with 25 per cell 3.9 -> 3.03 ms; the same in random order 10.3 -> 6.1.
+// Four records ahead with 5 blocks per SM: 9.5 ms, one ahead 10.4; three 7.9 - 8.1; 10 blocks 8.7; dividing with a range
+// test per record instead of once per deposit (SortGrid::general) 8.5.
+constexpr int GT_NONE = 0x7fffffff;   // start of an exhausted list
 constexpr int GT_X = 32, GT_Y = 4;    // nodes of a block: one warp per node row, 4 rows that share cell rows
-// (launched 8 blocks per SM: 64 registers, more warps in flight than a spill-free 68)
+constexpr int GT_AHEAD = 2;           // records of a run loaded at once
+constexpr int GT_BLOCKS = 8;          // blocks per SM (64 registers)
 
-__global__ void __launch_bounds__(GT_X * GT_Y, 8) k_gather_sorted(const __grid_constant__ SortGrids s,
-                                                               unsigned long long* __restrict__ empty_counter) {
-    const SortGrid& g = s.g[blockIdx.y];
-    const Payload* __restrict__ pl = g.payload;
+// FAST: every marker's distances from its cell's corner are within div_const's range (and dx, dy too).
+template <bool FAST>
+__device__ __forceinline__ void gather_node(const SortGrids& s, const SortGrid& g, double dx, double dy, double rdx,
+                                            double rdy, unsigned long long* __restrict__ empty_counter) {
+    const Record* __restrict__ rec = s.rec;
     const int32_t* __restrict__ offsets = g.offsets;
+    const int32_t* __restrict__ runs = g.perm;
+    const uint32_t* __restrict__ ends = g.ends;
     const int64_t nx = g.nx, ny = g.ny;
     const int64_t ntx = (nx + GT_X - 1) / GT_X;
     const int64_t I = (int64_t)(blockIdx.x % ntx) * GT_X + (threadIdx.x % GT_X) + 1;
     const int64_t J = (int64_t)(blockIdx.x / ntx) * GT_Y + (threadIdx.x / GT_X) + 1;
     if (I > nx || J > ny) return;
     const int64_t ldc = nx + 1;
+    const bool second = g.second != 0;
     // corner k: 0 = marker's top-left node (cell I,J), 1 = top-right (cell I-1,J),
     //           2 = bottom-left (cell I,J-1), 3 = bottom-right (cell I-1,J-1)
     int32_t cur[4], end[4], hm[4];
-    double hdx[4], hdy[4], hv[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
         const int64_t key = (I - (k & 1)) + (J - (k >> 1)) * ldc;
         cur[k] = offsets[key];
         end[k] = offsets[key + 1];
-        hdx[k] = hdy[k] = hv[k] = 0.0;
-        hm[k] = GT_NONE;
-        if (cur[k] < end[k]) {
-            const Payload p = pl[cur[k]];
-            hdx[k] = p.dxij;
-            hdy[k] = p.dyij;
-            hv[k] = p.val;
-            hm[k] = p.m;
-        }
+        hm[k] = cur[k] < end[k] ? runs[cur[k]] : GT_NONE;
     }
+    // topleftIndexRelDist's node coordinate x_grid_min + (ix - 1) * dx of the cells ix = I and I - 1 (likewise y)
+    const double xr = g.xmin + (double)(I - 1) * dx, xl = g.xmin + (double)(I - 2) * dx;
+    const double yr = g.ymin + (double)(J - 1) * dy, yl = g.ymin + (double)(J - 2) * dy;
     double ws = 0.0, vs = 0.0;
     while (true) {
         int kb = 0;
-        int32_t best = hm[0];
+        int32_t m = hm[0];
 #pragma unroll
         for (int k = 1; k < 4; ++k)
-            if (hm[k] < best) {
-                best = hm[k];
+            if (hm[k] < m) {
+                m = hm[k];
                 kb = k;
             }
-        if (best == GT_NONE) break;
-        int32_t t = GT_NONE;   // the smallest head of the other lists
-        int32_t c = 0, e = 0;
-        double dx = 0.0, dy = 0.0, v = 0.0;
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            if (k != kb && hm[k] < t) t = hm[k];
-            if (k == kb) {
-                c = cur[k];
-                e = end[k];
-                dx = hdx[k];
-                dy = hdy[k];
-                v = hv[k];
-            }
-        }
-        const bool fx = kb & 1, fy = kb >> 1;
-        int32_t h;
-        do {   // list kb's run below t
-            const double wx = fx ? dx : (1.0 - dx);
-            const double wy = fy ? dy : (1.0 - dy);
-            const double w = wx * wy;
-            ws = ws + w;
-            vs = vs + w * v;
-            ++c;
-            h = GT_NONE;
-            if (c < e) {
-                const Payload p = pl[c];
-                dx = p.dxij;
-                dy = p.dyij;
-                v = p.val;
-                h = p.m;
-            }
-        } while (h < t);
+        if (m == GT_NONE) break;
+        const int stop = m + __ffs(ends[m >> 5] >> (m & 31));
 #pragma unroll
         for (int k = 0; k < 4; ++k)
             if (k == kb) {
-                cur[k] = c;
-                hm[k] = h;
-                hdx[k] = dx;
-                hdy[k] = dy;
-                hv[k] = v;
+                ++cur[k];
+                hm[k] = cur[k] < end[k] ? runs[cur[k]] : GT_NONE;
             }
+        const bool fx = kb & 1, fy = kb >> 1;
+        const double xc = fx ? xl : xr, yc = fy ? yl : yr;
+        for (; m < stop; m += GT_AHEAD) {
+            Record r[GT_AHEAD];
+#pragma unroll
+            for (int q = 0; q < GT_AHEAD; ++q)
+                if (m + q < stop) r[q] = rec[m + q];
+#pragma unroll
+            for (int q = 0; q < GT_AHEAD; ++q)
+                if (m + q < stop) {
+                    const double rx = r[q].x - xc, ry = r[q].y - yc;
+                    const double px = FAST ? div_const(rx, dx, rdx) : rx / dx, py = FAST ? div_const(ry, dy, rdy) : ry / dy;
+                    const double wx = fx ? px : (1.0 - px);
+                    const double wy = fy ? py : (1.0 - py);
+                    const double w = wx * wy;
+                    ws = ws + w;
+                    vs = vs + w * (second ? r[q].v1 : r[q].v0);
+                }
+        }
     }
     if (g.wt_sum) {
         g.wt_sum[(I - 1) + (J - 1) * g.ld_sum] = ws;
@@ -508,6 +524,16 @@ __global__ void __launch_bounds__(GT_X * GT_Y, 8) k_gather_sorted(const __grid_c
         g.val_grid[(I - 1) + (J - 1) * nx] = vs / ws;   // safeDivision (MarkerToGrid.jl:164-172)
     else if (empty_counter)
         atomicAdd(empty_counter, 1ull);
+}
+
+__global__ void __launch_bounds__(GT_X * GT_Y, GT_BLOCKS) k_gather_runs(const __grid_constant__ SortGrids s, double dx,
+                                                                      double dy, double rdx, double rdy,
+                                                                      unsigned long long* __restrict__ empty_counter) {
+    const SortGrid& g = s.g[blockIdx.y];
+    if (*g.general == 0)
+        gather_node<true>(s, g, dx, dy, rdx, rdy, empty_counter);
+    else
+        gather_node<false>(s, g, dx, dy, rdx, rdy, empty_counter);
 }
 
 // The allocation-free deposit's gather (its scratch holds no payload): the same merge of node (I, J)'s cells
@@ -570,14 +596,17 @@ static unsigned grid_for(sf_ctx* ctx, int64_t n, int threads) {
     return (unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div(n, threads), (int64_t)ctx->num_sms * 32));
 }
 
-// Step 1 for all grids of s
+// Step 1 for all grids of s: markers, or (records) runs
 static int launch_keys(sf_ctx* ctx, const SortGrids& s, const double* x, const double* y, int64_t nm, double dx, double dy,
                        unsigned long long* bad_counter, cudaStream_t st) {
     if (nm == 0) return SF_OK;
-    if (s.n == 1)
-        k_cell_keys<1><<<grid_for(ctx, nm, DEP_THREADS), DEP_THREADS, 0, st>>>(x, y, nm, dx, dy, s, bad_counter);
+    const unsigned blocks = grid_for(ctx, nm, DEP_THREADS);
+    if (!s.rec)
+        k_cell_keys<<<blocks, DEP_THREADS, 0, st>>>(x, y, nm, dx, dy, s, bad_counter);
+    else if (s.n == 1)
+        k_cell_runs<1><<<blocks, DEP_THREADS, 0, st>>>(x, y, nm, dx, dy, s, bad_counter);
     else
-        k_cell_keys<SF_MAX_GRIDS><<<grid_for(ctx, nm, DEP_THREADS), DEP_THREADS, 0, st>>>(x, y, nm, dx, dy, s, bad_counter);
+        k_cell_runs<SF_MAX_GRIDS><<<blocks, DEP_THREADS, 0, st>>>(x, y, nm, dx, dy, s, bad_counter);
     SF_LAUNCHED(ctx);
     return SF_OK;
 }
@@ -600,33 +629,32 @@ static int launch_scan(const SortGrids& s, cudaStream_t st, int* launches) {
     return SF_OK;
 }
 
-// Steps 2-4 for the grids of s: the stable counting sort of the markers by cell -> offsets, and either the cell-ordered
-// permutation (rebin) or the cell-ordered payload records (deposit).
-static int launch_sort(sf_ctx* ctx, const SortGrids& s, const double* x, const double* y, int64_t nm, double dx, double dy,
-                       bool payload, cudaStream_t st) {
+// Steps 2-4 for the grids of s: the markers (or the first markers of the runs) in cell order, ascending in each cell,
+// that is a stable counting sort.
+static int launch_sort(sf_ctx* ctx, const SortGrids& s, int64_t nm, cudaStream_t st) {
     int n = 0;
     int rc = launch_scan(s, st, &n);
     ctx->launches += n;
     if (rc || nm == 0) return rc;
     int64_t cells = 0;
     for (int k = 0; k < s.n; ++k) cells = std::max(cells, s.g[k].ncells);
-    k_scatter<<<dim3(grid_for(ctx, nm, DEP_THREADS), (unsigned)s.n), DEP_THREADS, 0, st>>>(s, nm);
+    const dim3 blocks(grid_for(ctx, nm, DEP_THREADS), (unsigned)s.n);
+    if (s.rec)
+        k_scatter_runs<<<blocks, DEP_THREADS, 0, st>>>(s, nm);
+    else
+        k_scatter<<<blocks, DEP_THREADS, 0, st>>>(s, nm);
     SF_LAUNCHED(ctx);
     k_sort_long<<<dim3((unsigned)ctx->num_sms * 2, (unsigned)s.n), SORT_THREADS, 0, st>>>(s);
     SF_LAUNCHED(ctx);
-    const dim3 blocks((unsigned)ceil_div(cells, SORT_CPB), (unsigned)s.n);
-    if (payload)
-        k_sort_cells<true><<<blocks, SORT_THREADS, 0, st>>>(s, x, y, dx, dy);
-    else
-        k_sort_cells<false><<<blocks, SORT_THREADS, 0, st>>>(s, x, y, dx, dy);
+    k_sort_cells<<<dim3((unsigned)ceil_div(cells, SORT_CPB), (unsigned)s.n), SORT_THREADS, 0, st>>>(s);
     SF_LAUNCHED(ctx);
     return SF_OK;
 }
 
-// Scratch of a sort over the grids of s (xmin .. ncells set): what all grids need at once (keys and counts come from one
-// pass over the markers) and, `together`, offsets, cursors, permutation and payload of each grid, else those of one.
-// The counts and list lengths are one block, zeroed here.
-static int sort_scratch(sf_ctx* ctx, SortGrids& s, int64_t nm, bool together, bool payload, cudaStream_t st) {
+// Scratch of a sort over the grids of s (xmin .. ncells set): what all grids need at once (records, keys, run ends and
+// counts come from one pass over the markers) and, `together`, offsets, cursors and permutation of each grid, else those
+// of one.  The counts and list lengths are one block, zeroed here.
+static int sort_scratch(sf_ctx* ctx, SortGrids& s, int64_t nm, bool together, bool records, cudaStream_t st) {
     const int64_t nmk = std::max<int64_t>(nm, 1), per = round_up(nmk, 64), nlist = nm / (SORT_LONG + 1) + 1;
     int64_t cells = 0, most = 0, tiles = 0;
     for (int k = 0; k < s.n; ++k) {
@@ -636,14 +664,15 @@ static int sort_scratch(sf_ctx* ctx, SortGrids& s, int64_t nm, bool together, bo
     }
     const int n = together ? s.n : 1;
     int rc;
-    if ((rc = ensure(ctx, ctx->keys, (size_t)(s.n * per) * 4))) return rc;
-    if ((rc = ensure(ctx, ctx->counts, (size_t)(cells + s.n) * 4))) return rc;    // counts, list lengths
-    if ((rc = ensure(ctx, ctx->offsets, (size_t)(2 * n * most) * 4))) return rc;  // offsets, cursors
+    if ((rc = ensure(ctx, ctx->keys, (size_t)(s.n * (per + per / 32)) * 4))) return rc;   // keys, run ends
+    if ((rc = ensure(ctx, ctx->counts, (size_t)(cells + 2 * s.n) * 4))) return rc;        // counts, list lengths, general
+    if ((rc = ensure(ctx, ctx->offsets, (size_t)(2 * n * most) * 4))) return rc;          // offsets, cursors
     if ((rc = ensure(ctx, ctx->scan_tmp, (size_t)tiles * 4))) return rc;
     if ((rc = ensure(ctx, ctx->longs, (size_t)(n * nlist) * 4))) return rc;
     if ((rc = ensure(ctx, ctx->perm, (size_t)(n * per) * 4))) return rc;
-    if (payload && (rc = ensure(ctx, ctx->payload, (size_t)(n * nmk) * sizeof(Payload)))) return rc;
-    SF_CUDA(cudaMemsetAsync(ctx->counts.ptr, 0, (size_t)(cells + s.n) * 4, st));
+    if (records && (rc = ensure(ctx, ctx->records, (size_t)nmk * sizeof(Record)))) return rc;
+    SF_CUDA(cudaMemsetAsync(ctx->counts.ptr, 0, (size_t)(cells + 2 * s.n) * 4, st));
+    s.rec = records ? (Record*)ctx->records.ptr : nullptr;
     int32_t* counts = (int32_t*)ctx->counts.ptr;
     int32_t* tile = (int32_t*)ctx->scan_tmp.ptr;
     int64_t at = 0;
@@ -651,24 +680,26 @@ static int sort_scratch(sf_ctx* ctx, SortGrids& s, int64_t nm, bool together, bo
         SortGrid& g = s.g[k];
         const int64_t q = together ? k : 0;
         g.keys = (int32_t*)ctx->keys.ptr + k * per;
+        g.ends = (uint32_t*)ctx->keys.ptr + s.n * per + k * (per / 32);
         g.counts = counts + at;
         g.n_list = counts + cells + k;
+        g.general = counts + cells + s.n + k;
         g.offsets = (int32_t*)ctx->offsets.ptr + 2 * q * most;
         g.cursor = g.offsets + most;
         g.tiles = tile;
         g.list = (int32_t*)ctx->longs.ptr + q * nlist;
         g.perm = (int32_t*)ctx->perm.ptr + q * per;
-        g.payload = payload ? (Payload*)ctx->payload.ptr + q * nmk : nullptr;
         at += g.ncells + 1;
         tile += ceil_div(g.ncells, SCAN_TILE);
     }
     return SF_OK;
 }
 
-static int launch_gather(sf_ctx* ctx, const SortGrids& s, cudaStream_t st) {
+static int launch_gather(sf_ctx* ctx, const SortGrids& s, double dx, double dy, cudaStream_t st) {
     int64_t blocks = 0;
     for (int k = 0; k < s.n; ++k) blocks = std::max(blocks, ceil_div(s.g[k].nx, GT_X) * ceil_div(s.g[k].ny, GT_Y));
-    k_gather_sorted<<<dim3((unsigned)blocks, (unsigned)s.n), GT_X * GT_Y, 0, st>>>(s, ctx->d_counters + CNT_EMPTY_NODES);
+    k_gather_runs<<<dim3((unsigned)blocks, (unsigned)s.n), GT_X * GT_Y, 0, st>>>(
+        s, dx, dy, 1.0 / dx, 1.0 / dy, ctx->d_counters + CNT_EMPTY_NODES);
     SF_LAUNCHED(ctx);
     return SF_OK;
 }
@@ -690,27 +721,55 @@ static bool outputs_overlap(const SortGrids& s, int64_t n_sum) {
     return false;
 }
 
-// The deposits of s's grids over the same markers (only the last one's sums are kept).  Up to DEPOSIT_TOGETHER markers
-// all grids go through each kernel in one launch; beyond, or where they write the same places, one grid after the other,
-// in the scratch of one.
-static int deposit(sf_ctx* ctx, SortGrids& s, const double* x, const double* y, int64_t nm, double dx, double dy,
-                   int64_t n_sum, cudaStream_t st) {
+// The deposits of s's grids over the same markers (only the last one's sums are kept), whose values come from at most
+// two arrays.  Up to DEPOSIT_TOGETHER markers all grids go through each kernel in one launch; beyond, or where they
+// write the same places, one grid after the other, in the scratch of one.
+static int deposit_group(sf_ctx* ctx, SortGrids& s, const double* x, const double* y, int64_t nm, double dx, double dy,
+                         int64_t n_sum, cudaStream_t st) {
     const bool together = s.n > 1 && nm <= DEPOSIT_TOGETHER && !outputs_overlap(s, n_sum);
     int rc;
     if ((rc = sort_scratch(ctx, s, nm, together, true, st))) return rc;
+    s.val0 = s.g[0].val;
+    s.val1 = nullptr;
+    for (int k = 0; k < s.n; ++k) {
+        s.g[k].second = s.g[k].val != s.val0;
+        if (s.g[k].second) s.val1 = s.g[k].val;
+    }
+    if (!(div_const_takes(dx) && div_const_takes(dy)))
+        SF_CUDA(cudaMemsetAsync(s.g[0].general, 1, (size_t)s.n * 4, st));
     if ((rc = launch_keys(ctx, s, x, y, nm, dx, dy, ctx->d_counters + CNT_BAD_MARKERS, st))) return rc;
     const SortGrid& last = s.g[s.n - 1];
     for (int k = 0; k < (together ? 1 : s.n); ++k) {
-        SortGrids one{};
+        SortGrids one = s;
         one.g[0] = s.g[k];
         one.n = 1;
         const SortGrids& pass = together ? s : one;
-        if ((rc = launch_sort(ctx, pass, x, y, nm, dx, dy, true, st))) return rc;
+        if ((rc = launch_sort(ctx, pass, nm, st))) return rc;
         if (last.wt_sum && (together || k == s.n - 1)) {
             SF_CUDA(cudaMemsetAsync(last.wt_sum, 0, (size_t)n_sum * 8, st));
             SF_CUDA(cudaMemsetAsync(last.val_wt_sum, 0, (size_t)n_sum * 8, st));
         }
-        if ((rc = launch_gather(ctx, pass, st))) return rc;
+        if ((rc = launch_gather(ctx, pass, dx, dy, st))) return rc;
+    }
+    return SF_OK;
+}
+
+// any grids: in order, in groups whose values come from at most two arrays
+static int deposit(sf_ctx* ctx, const SortGrids& all, const double* x, const double* y, int64_t nm, double dx, double dy,
+                   int64_t n_sum, cudaStream_t st) {
+    for (int k = 0; k < all.n;) {
+        SortGrids s{};
+        const double* second = nullptr;
+        for (; k < all.n; ++k) {
+            const double* v = all.g[k].val;
+            if (s.n > 0 && v != s.g[0].val) {
+                if (second && v != second) break;
+                second = v;
+            }
+            s.g[s.n++] = all.g[k];
+        }
+        const int rc = deposit_group(ctx, s, x, y, nm, dx, dy, n_sum, st);
+        if (rc) return rc;
     }
     return SF_OK;
 }
@@ -822,7 +881,7 @@ int sf_rebin_markers(sf_ctx* ctx, const double* x_m, const double* y_m, int64_t 
     if (offsets) g.offsets = offsets;
     if (perm && nm > 0) g.perm = perm;
     if ((rc = launch_keys(ctx, sg, x_m, y_m, nm, dx, dy, ctx->d_counters + CNT_OUTSIDE, s))) return rc;
-    return launch_sort(ctx, sg, x_m, y_m, nm, dx, dy, false, s);
+    return launch_sort(ctx, sg, nm, s);
 }
 
 }  // extern "C"
@@ -938,7 +997,7 @@ extern "C" int sf_bilinear_marker_to_grid_noalloc(double x_grid_min, double y_gr
     const unsigned blocks =
         (unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div(nm, DEP_THREADS), (int64_t)num_sms * 32));
     if (nm > 0) {
-        k_cell_keys<1><<<blocks, DEP_THREADS, 0, s>>>(x_m, y_m, nm, dx, dy, sg, counters + 0);
+        k_cell_keys<<<blocks, DEP_THREADS, 0, s>>>(x_m, y_m, nm, dx, dy, sg, counters + 0);
         SF_CHECK_LAUNCH();
     }
     int n = 0;

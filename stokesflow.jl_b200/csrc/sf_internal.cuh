@@ -65,9 +65,9 @@ enum { SC_DT = 0, SC_DT_CHECK = 1, SC_ERR = 2, SC_SUM_RX = 3, SC_SUM_RY = 4, SC_
 struct sf_ctx {
     int device = 0;
     int num_sms = 148;
-    // deposit / rebin scratch: cell keys and ranks, counts, offsets, the cell-ordered permutation, scan tiles, the
-    // deposit's sorted payload records and the lists of long cells
-    sf::Scratch keys, counts, offsets, perm, scan_tmp, payload, longs;
+    // deposit / rebin scratch: cell keys and run ends, counts, offsets, the cell-ordered permutation, scan tiles, the
+    // deposit's marker records and the lists of long cells
+    sf::Scratch keys, counts, offsets, perm, scan_tmp, records, longs;
     // PT solve: padded internal fields, reduction partials; mixed/batched engine arena
     sf::Scratch fields, partials, mixed;
     // decomposed timestep: marker-exchange and overlap-sum staging
@@ -160,6 +160,23 @@ __device__ __forceinline__ TopLeft topleft(double xmin, double ymin, double x, d
     t.dyij = (y - y_iy) / dy;
     return t;
 }
+
+// a / b correctly rounded, from y = RN(1 / b): q = RN(a y) is within 1.5 ulp of a / b; one correction by its remainder
+// brings it within 1 ulp, and then the remainder a - b q is exact and RN(q + r y) = RN(a / b) (Markstein, "Computation of
+// elementary functions on the IBM RISC System/6000 processor", 1990: the theorem on a faithful quotient and a correctly
+// rounded reciprocal).  Needs |a| of 2^-960 .. 2^960 (or 0) and b of 2^-60 .. 2^60, so that nothing is lost below the
+// exponent range.  Five FP64 operations; the division is about twice that.
+__device__ __forceinline__ double div_const(double a, double b, double y) {
+    double q = a * y;
+    q = __fma_rn(__fma_rn(-b, q, a), y, q);
+    return __fma_rn(__fma_rn(-b, q, a), y, q);
+}
+
+__device__ __forceinline__ bool div_const_takes_a(double a) {   // false for NaN and infinities
+    const unsigned hi = (unsigned)__double2hiint(a) & 0x7fffffffu;
+    return hi - 0x08000000u < 0x70000000u || (hi | (unsigned)__double2loint(a)) == 0u;
+}
+inline bool div_const_takes(double b) { return b > 0x1p-60 && b < 0x1p60; }
 
 // SplitMix64 finaliser; sf_uniform(seed, k) = top 53 bits of
 // mix(mix(seed) ^ k*C) / 2^53.
