@@ -21,13 +21,15 @@
 // reference's order of operations (and the file is compiled without contraction): bit-identical to T single
 // iterations.
 //
-// What bounds it: at 2048^2 a launch of three iterations moves 558 MB (128 B per point and the halos) at 5.3 TB/s and
-// keeps the FP64 pipe 59% busy; 46.5 M warp instructions, against 3 x 50.6 M of k_pt_iter.  85 -> 37.3 us per
-// iteration at 2048^2, 241 -> 115 at 4001 x 3003, 24.6 -> 12.7 at 1024^2, 8.4 -> 5.5 at 511 x 385 (there the halo rows
-// and the launches bound it).  One warp per block, 240 registers, 8 blocks per SM: two columns to a lane halve the
-// shuffles, and 32 doubles in flight per lane hide the latencies that few warps would not.  The first form of this
-// kernel loaded each field's row by its own copy, divided by max(Nx, Ny) and tested the edges in every strip: 79 M
-// instructions, 50.6 us.
+// What bounds it: at 2048^2 a launch of three iterations moves 558 MB (128 B per point and the halos) in 100 us, 5.5 TB/s,
+// with the FP64 pipe some 60% busy; on smaller grids the halo rows of short segments.  85 -> 33.5 us per iteration at
+// 2048^2, 241 -> 97 at 4001 x 3003, 24.6 -> 11.9 at 1024^2; in runs of seconds, which draw the 1000 W limit and settle at
+// 1.69 GHz, 89.9 -> 37.5, 258 -> 105 and (1.86 GHz) 24.6 -> 12.4.  One warp per block, 234 registers, 8 blocks per SM (two warps
+// per scheduler): two columns to a lane halve the shuffles, and 32 doubles in flight per lane hide the latencies that few
+// warps would not (four per SM: 56 us at 2048^2; twelve with T = 2: 68; T = 4 spills: 63).  Every item runs the same code,
+// the boundary entries as selects: with a leaner body for the items inside, the two bodies shared the instruction cache
+// and the others finished late (37 us at 2048^2, 113 at 4001 x 3003); branches around the boundary entries cost as much.
+// The first form of this kernel loaded each field's row by its own copy and divided by max(Nx, Ny): 50.6 us.
 #include <algorithm>
 
 #include "sf_march.cuh"
@@ -143,10 +145,11 @@ __device__ __forceinline__ void march_step(Level& L, const MarchParams& k, doubl
     L.Yr = Yr;
 }
 
-// A strip's segment.  EDGE: its columns or rows (halo included) see a side of the domain.
-template <int T, int NSS, bool EDGE>
+// A strip's segment; edge: its columns or rows (halo included) see a side of the domain, so that its stores are not whole
+// pairs of columns.
+template <int T, int NSS>
 __device__ __forceinline__ void march_segment(const MarchMaps& maps, const MarchParams& p, unsigned char* smem,
-                                              int strip, int seg) {
+                                              int strip, int seg, const bool edge) {
     using R = Ring<T, NSS>;
     constexpr int NSM = R::NSM;
     unsigned char* const mats = smem + NSS * STATE_ROW;
@@ -219,7 +222,7 @@ __device__ __forceinline__ void march_segment(const MarchMaps& maps, const March
             const double Pold[2] = {L[l].Pn[0], L[l].Pn[1]};   // new P of row r - 2: the next level's input
             double Xn[2], Yn[2], dvx[2], dvy[2];
             march_step(L[l], p, dt, mo[l], X, Y, Xl, Yr, P0, dvx0, dvy0, Xn, Yn, dvx, dvy);
-            if (EDGE) {   // bc_x_zero! on Vx, bc_x_noflux! on Vy
+            {   // bc_x_zero! on Vx, bc_x_noflux! on Vy (selects, in strips inside too)
                 const double y_right = from_right(Yn[0]), y_left = from_left(Yn[1]);
                 if (c + 1 == -1) Yn[1] = y_right;
                 if (c + 1 == Nx - 1) Yn[1] = Yn[0];
@@ -240,7 +243,7 @@ __device__ __forceinline__ void march_segment(const MarchMaps& maps, const March
                     pdx[l][h] = dvx[h];
                     pdy[l][h] = dvy[h];
                 }
-                if (EDGE) {   // bc_y_noflux! on Vx, bc_y_zero! on Vy
+                {   // bc_y_noflux! on Vx, bc_y_zero! on Vy
                     Level& N = L[(l + 1 < T) ? l + 1 : l];
                     const int rn = r - 1;
                     if (rn == 1) {
@@ -259,7 +262,7 @@ __device__ __forceinline__ void march_segment(const MarchMaps& maps, const March
                 }
                 Xl = from_left(X[1]);
                 Yr = from_right(Y[0]);
-            } else if (!EDGE) {
+            } else if (!edge) {
                 // the row r - 1 leaves, with P and the rates of pressure row r - 2; {c, c + 1} of Vx is an aligned pair
                 const double x_left = from_left(Xn[1]), y_left = from_left(Yn[1]);
                 if (own && r > ra && r <= rb) {
@@ -338,10 +341,7 @@ __global__ void __launch_bounds__(32, WPS) k_pt_march(const __grid_constant__ Ma
     }
     __syncwarp();
     const bool edge = ca == 0 || ca + p.w + T >= p.Nx - 1 || ra - T <= 1 || ra + p.rows + T >= p.Ny - 1;
-    if (edge)
-        march_segment<T, NSS, true>(maps, p, smem, strip, seg);
-    else
-        march_segment<T, NSS, false>(maps, p, smem, strip, seg);
+    march_segment<T, NSS>(maps, p, smem, strip, seg, edge);
 }
 
 template <int T, int NSS, int WPS>
@@ -363,7 +363,8 @@ constexpr int WARPS_PER_SM = 8;
 
 // A warp of a grid of some 600 points per side or less has few rows of its own, and the rows above and below that it
 // computes for T = 3 outweigh what a third iteration saves: 5.5 us per iteration with T = 2 against 6.4 at 511 x 385
-// points, but 13.9 against 12.7 at 1024^2 and 54.4 against 37.3 at 2048^2 (T = 1: 8.4, 24.7, 101.5).
+// points (where no resident tiles are to be had), but 13.9 against 12.7 at 1024^2 and 54.4 against 37.3 at 2048^2 (T = 1:
+// 8.4, 24.7, 101.5), timed before the items' code was made one.
 int march_iterations(int64_t Nx, int64_t Ny) { return Nx * Ny < 600 * 600 ? 2 : 3; }
 
 void march_plan(MarchParams& p, int T, int num_sms) {

@@ -11,10 +11,11 @@
 // has not.
 //
 // What bounds it: issue slots (57% active at 1024^2) and, on small sets, the halo rows of short segments and a launch's
-// start.  One 1024^2 instance 17.5 -> 9.4 us per sweep (T = 3; one launch 28 us), 2048^2 59 -> 26.5, 16 instances of
-// 128 .. 512 points per side 27.2 -> 15.9, 100^2 4.5 -> 2.7.  496 warp instructions per row step of 64 columns and three
-// sweeps.  Two warps per scheduler (8 per SM): ten leave the schedulers uneven (11.4 us at 1024^2), twelve shorten the
-// segments (11.0); four columns per lane need fewer instructions, but their code misses the instruction cache (2.6 of 5
+// start.  One 1024^2 instance 17.5 -> 8.5 us per sweep (T = 3; one launch 25 us), 2048^2 59 -> 25.5, 16 instances of
+// 128 .. 512 points per side 27.2 -> 15.6, 100^2 4.5 -> 2.8.  Some 500 warp instructions per row step of 64 columns and
+// three sweeps, the same for every item (a leaner body for items inside the domain: 9.4 us at 1024^2).  With that leaner
+// body: two warps per scheduler (8 per SM) 9.4 us, ten leave the schedulers uneven (11.4), twelve shorten the segments
+// (11.0); four columns per lane need fewer instructions, but their code misses the instruction cache (2.6 of 5
 // stall cycles; 11.3 - 14.6 us); T = 2 with 12 warps 11.8.  One sweep per launch is no faster than k_pt32.
 #pragma once
 
@@ -136,11 +137,11 @@ __device__ __forceinline__ void mstep(MLevel& L, const MConst& k, const unsigned
 // position in the rings; carried from item to item (in_: lane 0's, of the next copies)
 struct MPos { int b, m, in_b, in_m; uint32_t phase; };
 
-// One item: T levels.  EDGE: its columns or rows (halo included) see a side of the domain; DMAX: the stencil-maximum
+// One item: T levels.  edge: its columns or rows (halo included) see a side of the domain; DMAX: the stencil-maximum
 // pseudo-step.  false: a copy never came.
-template <int T, bool EDGE, bool DMAX>
-__device__ __forceinline__ bool mitem(const CUtensorMap* __restrict__ maps, const Inst& I, const MItem& w, int in, int rin,
-                                      unsigned char* smem, MPos& pos) {
+template <int T, bool DMAX>
+__device__ __forceinline__ bool mitem(const CUtensorMap* __restrict__ maps, const Inst& I, const MItem& w, bool edge,
+                                      int in, int rin, unsigned char* smem, MPos& pos) {
     using R = MRing;
     unsigned char* const mats = smem + MPAIRS * R::STATE;
     uint64_t* const bar = reinterpret_cast<uint64_t*>(smem + R::BAR);
@@ -237,7 +238,7 @@ __device__ __forceinline__ bool mitem(const CUtensorMap* __restrict__ maps, cons
 #pragma unroll
                 for (int h = 0; h < NC; ++h) Pold[h] = L[l].P[h];
                 mstep<DMAX>(L[l], k, m, X, Y, Xl, Yr, P0, rx0, ry0, Xn, Yn, rxn, ryn);
-                if (EDGE) {
+                {   // (as in sf_march.cu: every item, so that all take the same time)
                     const float y_right = fr_right(Yn[0]), y_left = fr_left(Yn[NC - 1]);
                     if (c + NC - 1 == -1) Yn[NC - 1] = y_right;
 #pragma unroll
@@ -257,7 +258,7 @@ __device__ __forceinline__ bool mitem(const CUtensorMap* __restrict__ maps, cons
                         prx[l][h] = rxn[h];
                         pry[l][h] = ryn[h];
                     }
-                    if (EDGE) {
+                    {
                         MLevel& N = L[(l + 1 < T) ? l + 1 : l];
                         const int rn = r - 1;
                         if (rn == 1) {
@@ -279,7 +280,7 @@ __device__ __forceinline__ bool mitem(const CUtensorMap* __restrict__ maps, cons
                     }
                     Xl = fr_left(X[NC - 1]);
                     Yr = fr_right(Y[0]);
-                } else if (!EDGE) {
+                } else if (!edge) {
                     float xs[NC], ys[NC];    // {Vx(c), ..}: the column to the left, then this lane's but its last
                     xs[0] = fr_left(Xn[NC - 1]);
                     ys[0] = fr_left(Yn[NC - 1]);
@@ -384,16 +385,13 @@ __global__ void __launch_bounds__(32, WPS) k_march32(const CUtensorMap* __restri
         const bool edge = w.ca == 0 || w.ca + cols + T >= I.Nx - 1 || w.ra - T <= 1 || w.ra + rows + T >= I.Ny - 1;
         bool ok;
         if (I.dtau_max)
-            ok = n == T ? mitem<T, true, true>(m, I, w, in, rin, smem, pos)
-                 : n == 2 ? mitem<2, true, true>(m, I, w, in, rin, smem, pos)
-                                    : mitem<1, true, true>(m, I, w, in, rin, smem, pos);
-        else if (n == T)
-            ok = edge ? mitem<T, true, false>(m, I, w, in, rin, smem, pos)
-                      : mitem<T, false, false>(m, I, w, in, rin, smem, pos);
-        else if (n == 2)
-            ok = mitem<2, true, false>(m, I, w, in, rin, smem, pos);
+            ok = n == T ? mitem<T, true>(m, I, w, edge, in, rin, smem, pos)
+                 : n == 2 ? mitem<2, true>(m, I, w, edge, in, rin, smem, pos)
+                          : mitem<1, true>(m, I, w, edge, in, rin, smem, pos);
         else
-            ok = mitem<1, true, false>(m, I, w, in, rin, smem, pos);
+            ok = n == T ? mitem<T, false>(m, I, w, edge, in, rin, smem, pos)
+                 : n == 2 ? mitem<2, false>(m, I, w, edge, in, rin, smem, pos)
+                          : mitem<1, false>(m, I, w, edge, in, rin, smem, pos);
         if (!ok) {
             // flag it, give the copies in flight a bounded chance to land, leave
             if (threadIdx.x == 0) atomicExch(err_flag, 1);
