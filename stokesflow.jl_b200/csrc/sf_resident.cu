@@ -5,21 +5,25 @@
 //
 //   * the grid is cut into at most one tile per SM; a thread owns the same points in every iteration and keeps their
 //     P, rates and parameters in registers.  Vx, Vy and the stage-1 results of a tile (P, tau_xx, tau_yy, tau_xy) are in
-//     shared memory.  An iteration is the two stages of k_pt_iter, a block barrier after each, and the exchange;
-//   * the tiles exchange the velocities of their borders through L2: every value travels in a 16-byte slot as two
-//     8-byte words {half, tag}, the tag being the iteration's number, so that a reader that sees its tag has the
-//     value: one store and one load instead of data, fence and flag.  Slots are double-buffered by parity; a tile
-//     cannot be two iterations ahead of one that it exchanges with, so a slot is never overwritten unread;
-//   * the launch is cooperative (all tiles resident), and every wait has a wall-clock budget.
+//     shared memory.  An iteration is the two stages of k_pt_iter, a barrier after each, and the exchange of the
+//     velocities on the tiles' borders, one of:
+//   * the tiles are the blocks of one cluster (up to 16): a thread stores a border point's velocities also into the
+//     neighbours' shared memory, and the second barrier is the cluster's.  The velocities are double-buffered: a
+//     neighbour's border may come in while the old ones are still read;
+//   * through L2: every value travels in a 16-byte slot as two 8-byte words {half, tag}, the tag being the iteration's
+//     number, so that a reader that sees its tag has the value: one store and one load instead of data, fence and flag.
+//     Slots are double-buffered by parity; a tile cannot be two iterations ahead of one that it exchanges with, so a
+//     slot is never overwritten unread.  The launch is cooperative (all tiles resident), and every wait has a
+//     wall-clock budget.
 //
 // A tile's halo column and row of P and tau are computed by both neighbours from the same values.  Every expression
 // keeps the reference's order of operations (compiled without contraction): bit-identical to single iterations.
 //
-// What bounds it: latency.  At 128^2 (110 tiles of 150 points, 8 warps) an iteration takes 1.5 us, about half of it the
-// exchange (a store to L2 and a load from it, two barriers) and half the two stages' dependent FP64 chains; at 511 x 385
-// (1450 points per SM) 2.8 us, there mostly issue slots.  5.2 -> 1.65 us per iteration at 128^2 (k_pt_iter: one launch
-// each), 8.3 -> 2.8 at 511 x 385, 4.5 -> 1.4 at 20 x 26, checks included.  Testing every point's flags and sending
-// borders from the update itself took 905 instructions per warp and iteration at 511 x 385 and 4.2 us.
+// What bounds it: latency.  A cluster's iteration takes 0.62 us at 20 x 26 and about 0.8 at 64^2, the two stages'
+// dependent FP64 chains and the barriers; with the checks 1.1 and 1.1 us (k_pt_iter, one launch each: 4.5 and 4.4).
+// Through L2, 128^2 (110 tiles of 150 points, 8 warps) takes 1.5 us, about half of it the exchange, against 5.2; at
+// 511 x 385 (1450 points per SM) 2.8 us, there mostly issue slots, against 8.3.  Testing every point's flags and
+// sending borders to L2 from the update itself took 905 instructions per warp and iteration at 511 x 385 and 4.2 us.
 #include <algorithm>
 #include <mutex>
 
@@ -51,20 +55,38 @@ __device__ __forceinline__ bool get(const ulonglong2* slot, uint32_t tag, double
     return true;
 }
 
+// the address of this block's shared-memory entry p in the block of the given rank of the cluster
+__device__ __forceinline__ uint32_t in_block(const void* p, uint32_t rank) {
+    uint32_t a;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
+    return a;
+}
+__device__ __forceinline__ void put_in_block(uint32_t addr, double v) {
+    asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(addr), "d"(v) : "memory");
+}
+// every thread of the cluster: earlier shared-memory writes, remote ones too, are seen by all afterwards
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
 // what a thread's point is: one whose Vx / Vy it updates (the others' are boundary entries, zero), one of the tile (not
 // of its halo column or row), and the sides of the domain that it lies on
-enum { PT_X = 1, PT_Y = 2, PT_OWN = 4, PT_I0 = 8, PT_I1 = 16, PT_J0 = 32, PT_J1 = 64,
+enum { PT_X = 1, PT_Y = 2, PT_OWN = 4, PT_I0 = 8, PT_I1 = 16, PT_J0 = 32, PT_J1 = 64, PT_DX = 128,
        PT_BOUND = PT_I0 | PT_I1 | PT_J0 | PT_J1 };
 
-// K points per thread
-template <int K>
-__global__ void __launch_bounds__(K == 1 ? 1024 : 512, 1) k_pt_resident(const __grid_constant__ ResidentParams p) {
+// K points per thread.  CLUSTER: the tiles are the blocks of one cluster (or there is one tile)
+template <int K, bool CLUSTER>
+__global__ void __launch_bounds__(512, 1) k_pt_resident(const __grid_constant__ ResidentParams p) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ int gave_up;
     const int W = p.W, H = p.H, pitch = W + 2;
-    double* const sVx = reinterpret_cast<double*>(smem_raw);      // (H + 2) x (W + 2): entry (0, 0) is Vx(i0, j0)
-    double* const sVy = sVx + (H + 2) * pitch;
-    double* const sTxx = sVy + (H + 2) * pitch;                   // (H + 1) rows of the same pitch
+    const int comp1 = (H + 2) * pitch;                            // from an entry of Vx to that of Vy
+    double* sVx = reinterpret_cast<double*>(smem_raw);            // (H + 2) x (W + 2): entry (0, 0) is Vx(i0, j0)
+    double* sVy = sVx + comp1;
+    // CLUSTER: a second pair, written while the first is read (a neighbour's border may come in at any time)
+    double* sVx_n = CLUSTER ? sVy + comp1 : sVx;
+    double* sVy_n = sVx_n + comp1;
+    double* const sTxx = sVy_n + comp1;                           // (H + 1) rows of the same pitch
     double* const sTyy = sTxx + (H + 1) * pitch;
     double* const sPn = sTyy + (H + 1) * pitch;
     double* const sTxy = sPn + (H + 1) * pitch;
@@ -83,6 +105,7 @@ __global__ void __launch_bounds__(K == 1 ? 1024 : 512, 1) k_pt_resident(const __
         const int64_t o = i0 + a + (int64_t)(j0 + b) * LD;
         sVx[n] = in ? p.Vx_in[o] : 0.0;
         sVy[n] = in ? p.Vy_in[o] : 0.0;
+        if (CLUSTER) sVx_n[n] = sVy_n[n] = 0.0;
     }
     double P[K], dvx[K], dvy[K], tp[K], mu2[K], mb[K], tx[K], ty[K], rho[K], gx[K], gy[K];
     int off[K];      // b * pitch + a of the thread's points (a <= W, b <= H: the tile and one more column and row)
@@ -127,7 +150,7 @@ __global__ void __launch_bounds__(K == 1 ? 1024 : 512, 1) k_pt_resident(const __
     // right][from below][from above][Vx of the upper left tile, Vy of the lower right one].  The last tiles of a row or
     // column may hold fewer points than W x H.
     const int nslots = slots_of(W, H), tiles = p.ntx * p.nty;
-    const int hv = min(H, Ny - 1 - j0), wv = min(W, Nx - 1 - i0), comp1 = (H + 2) * pitch;
+    const int hv = min(H, Ny - 1 - j0), wv = min(W, Nx - 1 - i0);
     // slot n: where its value goes in this tile (an offset from sVx), which entry of this tile fills the slot of the
     // same kind of the neighbour on the other side, and that neighbour (as a difference of tile numbers); -1: nobody's
     auto halo = [&](int n, int& to, int& from, int& peer) {
@@ -153,10 +176,33 @@ __global__ void __launch_bounds__(K == 1 ? 1024 : 512, 1) k_pt_resident(const __
             peer = p.ntx - 1;
         }
     };
-    int to0, from0, peer0;
-    halo(tid, to0, from0, peer0);
-    if (tid == 0) gave_up = 0;
-    __syncthreads();
+    int to0 = -1, from0 = -1, peer0 = 0;
+    // CLUSTER: where a border point's Vx goes in the neighbour to its left or right, in the one below or above, and (a
+    // corner's Vx or Vy) in the diagonal one; 0: nowhere.  Vy lies behind Vx, the other pair of buffers `other` further
+    uint32_t at_x[K], at_y[K], at_d[K];
+    uint32_t other = (uint32_t)(2 * comp1 * 8);
+    if (CLUSTER) {
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            at_x[k] = at_y[k] = at_d[k] = 0;
+            if (!(kind[k] & PT_OWN)) continue;
+            const int b = off[k] / pitch, a = off[k] - b * pitch, t = blockIdx.x;
+            if (a == 0 && has_l) at_x[k] = in_block(sVx_n + (b + 1) * pitch + W + 1, t - 1);
+            if (a == W - 1 && has_r) at_x[k] = in_block(sVx_n + (b + 1) * pitch, t + 1);
+            if (b == 0 && has_b) at_y[k] = in_block(sVx_n + (H + 1) * pitch + a + 1, t - p.ntx);
+            if (b == H - 1 && has_t) at_y[k] = in_block(sVx_n + a + 1, t + p.ntx);
+            if (a == W - 1 && b == 0 && has_r && has_b) {
+                at_d[k] = in_block(sVx_n + (H + 1) * pitch, t + 1 - p.ntx);
+                kind[k] |= PT_DX;
+            }
+            if (a == 0 && b == H - 1 && has_l && has_t) at_d[k] = in_block(sVy_n + W + 1, t - 1 + p.ntx);
+        }
+        cluster_sync();
+    } else {
+        halo(tid, to0, from0, peer0);
+        if (tid == 0) gave_up = 0;
+        __syncthreads();
+    }
 
     for (int it = 0; it < p.iters; ++it) {
         // ---- stage 1: compute_P_tau! (:140-169) on the tile and one more column and row.  Evaluated at every point
@@ -202,24 +248,58 @@ __global__ void __launch_bounds__(K == 1 ? 1024 : 512, 1) k_pt_resident(const __
             const double xn = (kind[k] & PT_X) ? sVx[o + pitch + 1] + tx[k] * dvx[k] : 0.0;
             const double yn = (kind[k] & PT_Y) ? sVy[o + pitch + 1] + ty[k] * dvy[k] : 0.0;
             if (kind[k] & PT_OWN) {
-                sVx[o + pitch + 1] = xn;
-                sVy[o + pitch + 1] = yn;
+                sVx_n[o + pitch + 1] = xn;
+                sVy_n[o + pitch + 1] = yn;
             }
             if (kind[k] & PT_BOUND) {
                 if (kind[k] & PT_I0) {
-                    sVx[o + pitch] = 0.0;
-                    sVy[o + pitch] = yn;
+                    sVx_n[o + pitch] = 0.0;
+                    sVy_n[o + pitch] = yn;
                 }
-                if (kind[k] & PT_I1) sVy[o + pitch + 2] = yn;
+                if (kind[k] & PT_I1) sVy_n[o + pitch + 2] = yn;
                 if (kind[k] & PT_J0) {
-                    sVx[o + 1] = xn;
-                    sVy[o + 1] = 0.0;
+                    sVx_n[o + 1] = xn;
+                    sVy_n[o + 1] = 0.0;
                 }
-                if (kind[k] & PT_J1) sVx[o + 2 * pitch + 1] = xn;
+                if (kind[k] & PT_J1) sVx_n[o + 2 * pitch + 1] = xn;
+            }
+            if (CLUSTER && it + 1 < p.iters) {
+                if (at_x[k]) {
+                    put_in_block(at_x[k], xn);
+                    put_in_block(at_x[k] + comp1 * 8, yn);
+                }
+                if (at_y[k]) {
+                    put_in_block(at_y[k], xn);
+                    put_in_block(at_y[k] + comp1 * 8, yn);
+                }
+                if (at_d[k]) put_in_block(at_d[k], (kind[k] & PT_DX) ? xn : yn);
+                at_x[k] = at_x[k] ? at_x[k] - other : 0;
+                at_y[k] = at_y[k] ? at_y[k] - other : 0;
+                at_d[k] = at_d[k] ? at_d[k] - other : 0;
             }
         }
+        if (CLUSTER) {
+            // corners whose owner is a boundary entry of a neighbour's column or row: zero from the first iteration on
+            // (the second pair of buffers is zero there from the start)
+            if (it == 1 && tid == 0) {
+                if (!has_l && has_t) sVx_n[(H + 1) * pitch] = 0.0;
+                if (!has_b && has_r) sVy_n[W + 1] = 0.0;
+            }
+            other = 0u - other;
+            double* t = sVx;
+            sVx = sVx_n;
+            sVx_n = t;
+            t = sVy;
+            sVy = sVy_n;
+            sVy_n = t;
+            if (tiles == 1)
+                __syncthreads();
+            else
+                cluster_sync();
+            continue;
+        }
         __syncthreads();
-        if (tiles == 1 || it + 1 == p.iters) continue;
+        if (it + 1 == p.iters) continue;
         // ---- this tile's borders to the neighbours, theirs into the halo ----
         const uint32_t tag = p.tag0 + (uint32_t)it;
         ulonglong2* const mine = p.comm + ((int64_t)(it & 1) * tiles + blockIdx.x) * nslots;
@@ -286,51 +366,116 @@ __global__ void __launch_bounds__(K == 1 ? 1024 : 512, 1) k_pt_resident(const __
 }
 
 typedef void (*ResKernel)(const ResidentParams);
-const ResKernel kKernels[RES_MAX_K + 1] = {nullptr, k_pt_resident<1>, k_pt_resident<2>, k_pt_resident<3>,
-                                           k_pt_resident<4>};
+const ResKernel kKernels[RES_MAX_K + 1] = {k_pt_resident<1, true>, k_pt_resident<1, false>, k_pt_resident<2, false>,
+                                           k_pt_resident<3, false>, k_pt_resident<4, false>};
+const ResKernel kCluster = kKernels[0];
+constexpr int CLUSTER_MAX = 16;
+constexpr int CLUSTER_PTS = 512;     // of a tile with its halo column and row: a thread each
+constexpr int RES_SMEM = 200 * 1024;
 
 // the last array is one row longer: stage 2 reads a row above its points, those of the halo row too
-int smem_of(int W, int H) { return (2 * (H + 2) + 4 * (H + 1) + 1) * (W + 2) * 8; }
+int smem_of(int W, int H, bool cluster) { return ((cluster ? 4 : 2) * (H + 2) + 4 * (H + 1) + 1) * (W + 2) * 8; }
+
+// threads and points per thread for n points of a tile; false if they do not fit
+bool threads_for(int64_t n, ResidentPlan& p) {
+    for (p.k = 1; p.k <= RES_MAX_K; ++p.k) {
+        p.threads = (int)round_up(ceil_div(n, p.k), 32);
+        if (p.threads <= 512) return true;
+    }
+    return false;
+}
+
+void set_tiles(ResidentPlan& p, int64_t cols, int64_t rows, int64_t W, int64_t H) {
+    p.fits = true;
+    p.ntx = (int)ceil_div(cols, W);
+    p.nty = (int)ceil_div(rows, H);
+    p.W = (int)W;
+    p.H = (int)H;
+    p.smem = smem_of(p.W, p.H, p.cluster);
+}
+
+// the largest cluster that the device places at all (one in a partition of the device may have fewer SMs together)
+int cluster_limit(int device) {
+    static std::mutex m;
+    static int limit[64] = {};
+    std::lock_guard<std::mutex> lock(m);
+    int& have = limit[device & 63];
+    if (have) return have;
+    have = 1;
+    if (cudaFuncSetAttribute((const void*)kCluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+        cudaGetLastError();
+        return have;
+    }
+    for (int c = CLUSTER_MAX; c > 1 && have == 1; c /= 2) {
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = (unsigned)c;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)c);
+        cfg.blockDim = dim3(CLUSTER_PTS);
+        cfg.dynamicSmemBytes = 48 * 1024;   // more than any tile of CLUSTER_PTS points takes
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        int n = 0;
+        if (cudaOccupancyMaxActiveClusters(&n, kCluster, &cfg) == cudaSuccess && n > 0)
+            have = c;
+        else
+            cudaGetLastError();
+    }
+    return have;
+}
 
 }  // namespace
 
-// Which grids, and how many tiles.  Up to 512 x 4 points per SM (registers: 22 per point) the state fits, and is faster
-// than the march wherever it does (3.5 against 5.8 us per iteration at 512^2, 1.65 against 4.3 at 128^2).  One tile up
-// to 800 points: it needs no exchange (27^2: 1.66 us against 1.70 with five tiles, 33^2: 2.04 against 1.62, residual
-// checks included).  Above, one per 150 points: the exchange costs the same whatever the tiles' size, and smaller ones
+// The tiles as one cluster, for grids of which 16 tiles hold at most 512 points each, halo column and row included (up to
+// about 84^2).  Writing a border into the neighbour's shared memory and one cluster barrier take less than the exchange
+// through L2 and its two block barriers; beyond, 16 SMs compute for longer than that gains.  Microseconds per iteration,
+// checks included, against the exchange through L2: 20 x 26 1.12 : 1.60 (with one tile that needs no exchange 1.40),
+// 40^2 0.98 : 1.61, 64^2 1.09 : 1.52, 84^2 1.25 : 1.58, 114 x 31 1.09 : 1.65, 170 x 40 1.53 : 1.70; 100^2 with two
+// points per thread or 832 threads 1.68 : 1.63.  Tiles of 32 points (a warp or two): the barrier costs the same for 2
+// and 16 blocks, and a block's barrier less with fewer warps (20 x 26, kernel alone: 0.90 us with one block, 0.78 with
+// two, 0.70 with four, 0.64 with eight, 0.61 with sixteen).
+ResidentPlan cluster_plan(int64_t Nx, int64_t Ny, int device) {
+    ResidentPlan best;
+    const int64_t cols = Nx - 1, rows = Ny - 1, pts = cols * rows;
+    const int most = cluster_limit(device);
+    int tiles = 1;
+    while (tiles < most && pts > (int64_t)tiles * 32) tiles *= 2;
+    int64_t best_pts = CLUSTER_PTS + 1;
+    for (; tiles >= 1 && !best.fits; tiles /= 2)   // (fewer only where a thin grid does not split so far)
+        for (int ntx = 1; ntx <= tiles; ntx *= 2) {
+            const int64_t W = ceil_div(cols, ntx), H = ceil_div(rows, tiles / ntx), n = (W + 1) * (H + 1);
+            if (W < 2 || H < 2 || ceil_div(cols, W) != ntx || ceil_div(rows, H) != tiles / ntx || n >= best_pts) continue;
+            best.cluster = true;
+            best.k = 1;
+            best.threads = (int)round_up(n, 32);
+            set_tiles(best, cols, rows, W, H);
+            best_pts = n;
+        }
+    return best;
+}
+
+// The exchange through L2: which grids, and how many tiles.  Up to 512 x 4 points per SM (registers: 22 per point) the
+// state fits, and is faster than the march wherever it does (3.5 against 5.8 us per iteration at 512^2, 1.65 against 4.3
+// at 128^2).  One tile per 150 points: the exchange costs the same whatever the tiles' size, and smaller ones
 // compute faster until they no longer do (128^2: 1.67 us, with 450 points 2.02, with 100 1.70); a small grid still
 // leaves SMs to solves on other streams.
 ResidentPlan resident_plan(int64_t Nx, int64_t Ny, int num_sms) {
     ResidentPlan best;
     const int64_t cols = Nx - 1, rows = Ny - 1, pts = cols * rows;
-    if (pts > (int64_t)num_sms * 512 * RES_MAX_K) return best;
-    int tiles = 1;
-    if (pts > 800) tiles = (int)std::min<int64_t>(num_sms, ceil_div(pts, 150));
     int64_t best_pts = 0;
+    if (pts > (int64_t)num_sms * 512 * RES_MAX_K) return best;
+    const int tiles = (int)std::min<int64_t>(num_sms, ceil_div(pts, 150));
     for (int ntx = 1; ntx <= tiles && ntx <= cols; ++ntx) {
         const int nty = (int)std::min<int64_t>(tiles / ntx, rows);
-        const int64_t W = ceil_div(cols, ntx), H = ceil_div(rows, nty);
-        const int64_t n = (W + 1) * (H + 1);
-        if (W < 2 || H < 2 || (best.fits && n >= best_pts)) continue;
-        const int64_t nx = ceil_div(cols, W), ny = ceil_div(rows, H);
-        int k = 0, threads = 0;
-        for (k = 1; k <= RES_MAX_K; ++k) {
-            threads = (int)round_up(ceil_div(n, k), 32);
-            if (threads <= (k == 1 ? 1024 : 512)) break;
-        }
-        if (k > RES_MAX_K) continue;
-        best.fits = true;
-        best.ntx = (int)nx;
-        best.nty = (int)ny;
-        best.W = (int)W;
-        best.H = (int)H;
-        best.k = k;
-        best.threads = threads;
-        best.smem = smem_of((int)W, (int)H);
-        // registers: 64 per thread with one point (the launch bound), else up to 128
-        const int regs = threads * (k == 1 ? 64 : 128);
-        best.share = regs <= 65536 / 4 && best.smem <= 50 * 1024 ? 1
-                     : regs <= 65536 / 2 && best.smem <= 100 * 1024 ? 2 : 4;
+        const int64_t W = ceil_div(cols, ntx), H = ceil_div(rows, nty), n = (W + 1) * (H + 1);
+        ResidentPlan p;
+        if (W < 2 || H < 2 || (best.fits && n >= best_pts) || !threads_for(n, p)) continue;
+        set_tiles(p, cols, rows, W, H);
+        const int regs = p.threads * 128;   // the launch bound
+        p.share = regs <= 65536 / 4 && p.smem <= 50 * 1024 ? 1 : regs <= 65536 / 2 && p.smem <= 100 * 1024 ? 2 : 4;
+        best = p;
         best_pts = n;
     }
     return best;
@@ -338,17 +483,24 @@ ResidentPlan resident_plan(int64_t Nx, int64_t Ny, int num_sms) {
 
 namespace {
 std::mutex g_room_mutex;
-int g_room_used[64] = {};   // quarters of SMs held, by device
+int g_room_used[64] = {};       // quarters of SMs held by solves that exchange through L2, by device
+int g_room_clusters[64] = {};   // solves that use a cluster, by device
 }
 
 bool ResidentRoom::acquire(int device, int num_sms, const ResidentPlan& plan, cudaStream_t s) {
-    if (!plan.fits || device < 0 || device >= 64) return false;
-    const int need = plan.ntx * plan.nty * plan.share;
+    if (!plan.fits || device < 0 || device >= 64 || device_ >= 0) return false;
+    const int need = plan.cluster ? 0 : plan.ntx * plan.nty * plan.share;
     std::lock_guard<std::mutex> lock(g_room_mutex);
-    if (g_room_used[device] + need > 4 * num_sms) return false;
-    g_room_used[device] += need;
+    if (plan.cluster) {
+        if (g_room_used[device]) return false;
+        ++g_room_clusters[device];
+    } else {
+        if (g_room_clusters[device] || g_room_used[device] + need > 4 * num_sms) return false;
+        g_room_used[device] += need;
+    }
     device_ = device;
     held_ = need;
+    cluster_ = plan.cluster;
     stream_ = s;
     return true;
 }
@@ -358,35 +510,53 @@ void ResidentRoom::release() {
     cudaStreamSynchronize(stream_);   // nothing of the solve runs any more
     std::lock_guard<std::mutex> lock(g_room_mutex);
     g_room_used[device_] -= held_;
+    g_room_clusters[device_] -= cluster_;
     device_ = -1;
 }
 
 int resident_launch(sf_ctx* ctx, ResidentParams& p, const ResidentPlan& plan, cudaStream_t s) {
     const int tiles = plan.ntx * plan.nty;
-    const size_t bytes = (size_t)2 * tiles * slots_of(plan.W, plan.H) * sizeof(ulonglong2);
-    // tags of earlier launches stay in the slots: new memory, and a wrap of the counter, start from zeroed slots
-    const bool fresh = bytes > ctx->halo.bytes, wrap = ctx->halo_tag > 0xffffffffu - (uint32_t)p.iters - 1u;
-    int rc = ensure(ctx, ctx->halo, bytes);
-    if (rc) return rc;
-    if (fresh || wrap) {
-        SF_CUDA(cudaMemsetAsync(ctx->halo.ptr, 0, ctx->halo.bytes, s));
-        ctx->halo_tag = 1;
+    if (!plan.cluster) {
+        const size_t bytes = (size_t)2 * tiles * slots_of(plan.W, plan.H) * sizeof(ulonglong2);
+        // tags of earlier launches stay in the slots: new memory, and a wrap of the counter, start from zeroed slots
+        const bool fresh = bytes > ctx->halo.bytes, wrap = ctx->halo_tag > 0xffffffffu - (uint32_t)p.iters - 1u;
+        int rc = ensure(ctx, ctx->halo, bytes);
+        if (rc) return rc;
+        if (fresh || wrap) {
+            SF_CUDA(cudaMemsetAsync(ctx->halo.ptr, 0, ctx->halo.bytes, s));
+            ctx->halo_tag = 1;
+        }
+        p.comm = (ulonglong2*)ctx->halo.ptr;
+        p.tag0 = ctx->halo_tag;
+        ctx->halo_tag += (uint32_t)p.iters;
     }
     p.ntx = plan.ntx;
     p.nty = plan.nty;
     p.W = plan.W;
     p.H = plan.H;
-    p.comm = (ulonglong2*)ctx->halo.ptr;
-    p.tag0 = ctx->halo_tag;
-    ctx->halo_tag += (uint32_t)p.iters;
+    const int which = plan.cluster ? 0 : plan.k;
     static bool ready[64][RES_MAX_K + 1] = {};
-    if (!ready[ctx->device & 63][plan.k]) {
-        SF_CUDA(cudaFuncSetAttribute((const void*)kKernels[plan.k], cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-        ready[ctx->device & 63][plan.k] = true;
+    if (!ready[ctx->device & 63][which]) {
+        SF_CUDA(cudaFuncSetAttribute((const void*)kKernels[which], cudaFuncAttributeMaxDynamicSharedMemorySize, RES_SMEM));
+        ready[ctx->device & 63][which] = true;
     }
-    void* args[] = {&p};
-    SF_CUDA(cudaLaunchCooperativeKernel((const void*)kKernels[plan.k], dim3((unsigned)tiles), dim3((unsigned)plan.threads),
-                                        args, (size_t)plan.smem, s));
+    cudaLaunchAttribute attr[1];
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)tiles);
+    cfg.blockDim = dim3((unsigned)plan.threads);
+    cfg.dynamicSmemBytes = (size_t)plan.smem;
+    cfg.stream = s;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    if (plan.cluster) {
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = (unsigned)tiles;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    } else {
+        attr[0].id = cudaLaunchAttributeCooperative;
+        attr[0].val.cooperative = 1;
+    }
+    SF_CUDA(cudaLaunchKernelEx(&cfg, kKernels[which], (const ResidentParams)p));
     SF_LAUNCHED(ctx);
     return SF_OK;
 }

@@ -29,7 +29,8 @@ struct ResidentParams {
 };
 
 struct ResidentPlan {
-    bool fits = false;           // the grid is small enough for one tile per SM
+    bool fits = false;           // the grid is small enough
+    bool cluster = false;        // the tiles are one thread-block cluster
     int ntx = 0, nty = 0, W = 0, H = 0, k = 0, threads = 0, smem = 0;
     int share = 0;               // quarters of an SM that a tile takes: 1, 2 or 4
 };
@@ -38,7 +39,9 @@ struct ResidentPlan {
 // all must become resident whatever else runs: concurrent solves (other threads, streams and contexts) hold at most
 // four quarters of every SM together.  Then a tile of one quarter always finds a place (an SM without one holds four
 // quarters already, and not all SMs can); its launch ends; and what is left of two and four quarters finds its place
-// in turn.  A solve that gets no room marches instead (same results).
+// in turn.  A cluster is placed whole or not at all and needs no such room, but one that waits for a free group of SMs
+// could stand before tiles that others wait for: clusters and tiles that exchange through L2 do not run together.
+// A solve that gets no room marches instead (same results).
 class ResidentRoom {
    public:
     ~ResidentRoom() { release(); }
@@ -47,11 +50,13 @@ class ResidentRoom {
 
    private:
     int device_ = -1, held_ = 0;
+    bool cluster_ = false;
     cudaStream_t stream_ = nullptr;
 };
 
+ResidentPlan cluster_plan(int64_t Nx, int64_t Ny, int device);
 ResidentPlan resident_plan(int64_t Nx, int64_t Ny, int num_sms);
-// `iters` iterations (p.iters); p.tag0 and p.comm are set here
+// p.iters iterations; the tiles and the exchange's slots of p are set here
 int resident_launch(sf_ctx* ctx, ResidentParams& p, const ResidentPlan& plan, cudaStream_t s);
 
 }  // namespace sf

@@ -913,7 +913,6 @@ static int solver_prepare(Solver& S, sf_ctx* ctx, cudaStream_t s, const SolveArg
         r.dampX = dampX;
         r.dampY = dampY;
         r.err_flag = pt.err_flag;
-        S.plan = resident_plan(Nx, Ny, ctx->num_sms);
     }
     ResParams& rp = S.rp;
     rp.txx = S.L.f(F_TXX);
@@ -1178,7 +1177,14 @@ int sf_solve_stokes(sf_ctx* ctx, double* P, double* Vx_pad, double* Vy_pad, cons
 
     // ---- PT loop (:43-77) ----
     ResidentRoom room;
-    const bool resident = iter_max >= RESIDENT_MIN_ITERS && room.acquire(ctx->device, ctx->num_sms, S.plan, s);
+    bool resident = false;
+    if (iter_max >= RESIDENT_MIN_ITERS) {
+        S.plan = cluster_plan(Nx, Ny, ctx->device);
+        if (!(resident = room.acquire(ctx->device, ctx->num_sms, S.plan, s))) {
+            S.plan = resident_plan(Nx, Ny, ctx->num_sms);
+            resident = room.acquire(ctx->device, ctx->num_sms, S.plan, s);
+        }
+    }
     double err = 2.0 * eps;
     int64_t iter = 1, niter = 0, nchecks = 0;
     const int64_t itert1 = 11;

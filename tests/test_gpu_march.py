@@ -1,8 +1,9 @@
 """Several PT iterations per launch against the oracle, bit for bit.  No tolerance: every expression is evaluated in
 the reference's order.
 
-* resident iterations (sf_resident.cu): the smallest grids, both sides of the one-tile limit (800 points), ragged last
-  tiles, one to four points per thread, thin tiles with more halo slots than threads, the largest grid;
+* resident iterations (sf_resident.cu): the smallest grids, clusters of 1 to 16 tiles in rows, columns and blocks, both
+  sides of the cluster's limit, ragged last tiles; the exchange through L2 with one to four points per thread, thin tiles
+  with more halo slots than threads, the largest grid;
 * the march (sf_march.cu), on grids beyond that, at the sizes where its split into strips of columns and segments of rows
   changes: the narrowest grids (one strip), odd strip widths, short and long segments, and iteration counts that leave one
   and two iterations over (the first ten and chunks of up to three iterations run on every grid)."""
@@ -17,6 +18,8 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("Nx,Ny,iters,stab", [
     # resident
+    (7, 6, 61, True), (10, 9, 93, False), (4, 61, 61, True), (18, 33, 185, True), (85, 85, 851, True), (86, 86, 861, True),
+    (170, 40, 403, True), (6, 900, 62, False), (70, 5, 104, True), (1000, 5, 51, True), (1400, 4, 61, True),
     (4, 4, 60, True), (5, 9, 61, True), (9, 5, 62, False), (27, 31, 300, True), (28, 31, 301, True), (59, 22, 231, True),
     (61, 4, 61, True), (114, 31, 321, True), (20, 700, 260, True), (3000, 20, 230, True), (233, 129, 700, True),
     (300, 301, 500, False), (511, 385, 94, True), (550, 552, 61, True),
@@ -42,21 +45,24 @@ def test_march_bitexact(sf, oracle_lib, Nx, Ny, iters, stab):
 
 def test_concurrent_solves_bitexact(sf, oracle_lib):
     """Solves of several threads at once, contexts and streams of their own, more of them than the device has room for
-    resident tiles (the rest marches): each equals the oracle."""
+    resident tiles (the rest marches), some of them small enough for a cluster: each equals the oracle."""
     import threading
 
     import torch
 
     O = oracle_lib
-    Nx, Ny, iters, n = 300, 260, 150, 6
-    dx, dy = 1.0 / (Nx - 1), 1.0 / (Ny - 1)
+    n = 8
+    shape = lambda k: (61, 47, 600) if k % 3 == 1 else (300, 260, 150)
     want, got = [], [None] * n
     for k in range(n):
+        Nx, Ny, iters = shape(k)
         a = O.stokes_arrays(Nx, Ny)
         a["rho_vy"][:], a["mu_b"][:], a["mu_p"][:] = random_fields(Nx, Ny, seed=k, contrast=5.0)
         want.append(a)
 
     def one(k, a):
+        Nx, Ny, iters = shape(k)
+        dx, dy = 1.0 / (Nx - 1), 1.0 / (Ny - 1)
         with torch.cuda.stream(torch.cuda.Stream()):
             t = {q: dev(v) for q, v in a.items()}
             sf.solve_stokes_info(*[t[q] for q in NAMES], 9.81, dx, dy, Nx, Ny, 1e-3, 0.5, eps=1e-300, iter_max=iters,
@@ -70,6 +76,8 @@ def test_concurrent_solves_bitexact(sf, oracle_lib):
     for t in threads:
         t.join()
     for k, a in enumerate(want):
+        Nx, Ny, iters = shape(k)
+        dx, dy = 1.0 / (Nx - 1), 1.0 / (Ny - 1)
         O.solve_stokes(a, 9.81, dx, dy, Nx, Ny, 1e-3, 0.5, True, 1e-300, iters)
         for q in NAMES:
             assert np.array_equal(got[k][q], a[q]), f"solve {k}: {q} differs from the oracle"
