@@ -56,9 +56,10 @@ enum { CNT_BAD_MARKERS = 0, CNT_EMPTY_NODES = 1, CNT_INTERP_FAILSAFE = 2, CNT_OU
 // device scalars used by the PT solve
 // SC_DT: dt used by the stabilisation term; SC_DT_CHECK: dt of the residual
 // check; SC_DT_OUT: dt returned by the solve; SC_MAXBITS (2 slots): max|Vx|,
-// max|Vy| as ordered bit patterns during a reduction.
+// max|Vy| as ordered bit patterns during a reduction, zero between reductions;
+// SC_TICKET: blocks of k_residuals that are done, zero between launches.
 enum { SC_DT = 0, SC_DT_CHECK = 1, SC_ERR = 2, SC_SUM_RX = 3, SC_SUM_RY = 4, SC_SUM_DIV = 5,
-       SC_MAX_VX = 6, SC_MAX_VY = 7, SC_SCALE = 8, SC_DT_OUT = 9, SC_MAXBITS = 12, SC_N = 16 };
+       SC_MAX_VX = 6, SC_MAX_VY = 7, SC_SCALE = 8, SC_DT_OUT = 9, SC_MAXBITS = 12, SC_TICKET = 14, SC_N = 16 };
 
 }  // namespace sf
 

@@ -79,6 +79,7 @@ template <int K, bool CLUSTER>
 __global__ void __launch_bounds__(512, 1) k_pt_resident(const __grid_constant__ ResidentParams p) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ int gave_up;
+    __shared__ unsigned long long max_v[2];
     const int W = p.W, H = p.H, pitch = W + 2;
     const int comp1 = (H + 2) * pitch;                            // from an entry of Vx to that of Vy
     double* sVx = reinterpret_cast<double*>(smem_raw);            // (H + 2) x (W + 2): entry (0, 0) is Vx(i0, j0)
@@ -101,12 +102,15 @@ __global__ void __launch_bounds__(512, 1) k_pt_resident(const __grid_constant__ 
     // ---- state and parameters onto the chip ----
     for (int n = tid; n < (H + 2) * pitch; n += NT) {
         const int b = n / pitch, a = n - b * pitch;
-        const bool in = i0 + a <= Nx && j0 + b <= Ny;
-        const int64_t o = i0 + a + (int64_t)(j0 + b) * LD;
+        // (the domain's corners are read by nothing but the last iteration's tau_xy, which finds them zero)
+        const int i = i0 + a, j = j0 + b;
+        const bool in = i <= Nx && j <= Ny && !(i == 0 && (j == 0 || j == Ny)) && !(i == Nx && j == 0);
+        const int64_t o = i + (int64_t)j * LD;
         sVx[n] = in ? p.Vx_in[o] : 0.0;
         sVy[n] = in ? p.Vy_in[o] : 0.0;
         if (CLUSTER) sVx_n[n] = sVy_n[n] = 0.0;
     }
+    if (tid < 2) max_v[tid] = 0;   // (barriers follow)
     double P[K], dvx[K], dvy[K], tp[K], mu2[K], mb[K], tx[K], ty[K], rho[K], gx[K], gy[K];
     int off[K];      // b * pitch + a of the thread's points (a <= W, b <= H: the tile and one more column and row)
     int kind[K];
@@ -221,6 +225,10 @@ __global__ void __launch_bounds__(512, 1) k_pt_resident(const __grid_constant__ 
             const double dVy_dy = (vy11 - vy01) * _dy;
             const double div = dVx_dx + dVy_dy;
             P[k] = P[k] - tp[k] * div;
+            if (p.divV && it + 1 == p.iters && (kind[k] & PT_OWN)) {
+                const int b = o / pitch;
+                p.divV[i0 + o - b * pitch + (int64_t)(j0 + b) * LD] = div;
+            }
             const double third = 1.0 / 3.0 * div;
             const double txx = mu2[k] * (dVx_dx - third), tyy = mu2[k] * (dVy_dy - third);
             // the gravity term of compute_ResY (:189-202), from the old velocities
@@ -334,6 +342,42 @@ __global__ void __launch_bounds__(512, 1) k_pt_resident(const __grid_constant__ 
         }
     }
 
+    // ---- tau, stage 1 of the last iteration.  tau_xy: the tile's points as new velocities see them, one further in x and
+    // y, and the domain's first column and row ----
+    if (p.txx) {
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            const int o = off[k], b = o / pitch, a = o - b * pitch;
+            const int i = i0 + a, j = j0 + b;
+            const int64_t q = i + (int64_t)j * LD;
+            if (kind[k] & PT_OWN) {
+                p.txx[q] = sTxx[o];
+                p.tyy[q] = sTyy[o];
+            }
+            if (tid + k * NT < (W + 1) * (H + 1) && i < Nx && j < Ny && (a || !has_l) && (b || !has_b)) p.txy[q] = sTxy[o];
+        }
+    }
+    if (p.max_bits) {   // max|V| over the tile; the boundary entries are copies or zero
+        unsigned long long mx = 0, my = 0;
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            if (!(kind[k] & PT_OWN)) continue;
+            const int o = off[k] + pitch + 1;
+            mx = max(mx, (unsigned long long)__double_as_longlong(fabs(sVx[o])));
+            my = max(my, (unsigned long long)__double_as_longlong(fabs(sVy[o])));
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+            my = max(my, __shfl_xor_sync(0xffffffffu, my, o));
+        }
+        if ((tid & 31) == 0) {
+            atomicMax(&max_v[0], mx);
+            atomicMax(&max_v[1], my);
+        }
+        __syncthreads();
+        if (tid < 2) atomicMax(&p.max_bits[tid], max_v[tid]);
+    }
     // ---- the state back, with the boundary entries ----
 #pragma unroll
     for (int k = 0; k < K; ++k) {
@@ -414,7 +458,7 @@ int cluster_limit(int device) {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3((unsigned)c);
         cfg.blockDim = dim3(CLUSTER_PTS);
-        cfg.dynamicSmemBytes = 48 * 1024;   // more than any tile of CLUSTER_PTS points takes
+        cfg.dynamicSmemBytes = 44 * 1024;   // more than any tile of CLUSTER_PTS points takes
         cfg.attrs = attr;
         cfg.numAttrs = 1;
         int n = 0;

@@ -26,6 +26,10 @@ struct ResidentParams {
     uint32_t tag0;               // iteration k (0-based) publishes with tag tag0 + k
     ulonglong2* comm;            // received halo entries, [parity][tile][slot]
     int* err_flag;
+    // of the last iteration, where wanted: tau and divV (NULL: not), and max|Vx|, max|Vy| as bit patterns, accumulated
+    // onto what is there (NULL: not)
+    double *txx, *tyy, *txy, *divV;
+    unsigned long long* max_bits;
 };
 
 struct ResidentPlan {

@@ -373,20 +373,48 @@ struct ResParams {
     const double* __restrict__ Vx;
     const double* __restrict__ Vy;
     const double* __restrict__ divV;
-    const double* __restrict__ dt_ptr;
+    // the stabilisation's dt: from *dt_ptr (0 where NULL), or, where max_bits is given, from the maxima there, which are
+    // then zeroed; written to *dt_out where that is given, too
+    const double* dt_ptr;
+    unsigned long long* max_bits;
+    double* dt_out;
+    double maxdisp, dx, dy;
     double* __restrict__ Rx;
     double* __restrict__ Ry;
-    double* __restrict__ partials;  // [gridDim.x][3]
+    double* partials;  // [gridDim.x][3]
     int Nx, Ny;
     int64_t LD;
     double _dx, _dy, g_y;
+    double* scalars;
+    double* host_err;  // pinned host memory
 };
 
-__global__ void __launch_bounds__(RES_THREADS) k_residuals(ResParams p) {
+// dt = maxdisp * min(dx / max|Vx|, dy / max|Vy|) (:118-121)
+__device__ __forceinline__ double dt_of(double mvx, double mvy, double maxdisp, double dx, double dy) {
+    double a = dx / mvx, b = dy / mvy;
+    double m = (b < a) ? b : a;
+    if (a != a) m = a;
+    if (b != b) m = b;
+    return maxdisp * m;
+}
+
+// The block that finishes last sums all blocks' partials in a fixed order: err = max of the three means.  One launch per
+// check, and with the dt and the copy of err to the host in it two after the iterations of a resident grid (its last
+// iteration leaves tau, divV and max|V|) instead of eight: 112 -> 100 us per 100 iterations with a check at 20 x 26.
+__global__ void __launch_bounds__(RES_THREADS) k_residuals(const ResParams p) {
     __shared__ double sh[32];
+    __shared__ bool last;
     const int Nx = p.Nx, Ny = p.Ny;
     const int64_t LD = p.LD, W = Nx - 1, npts = (int64_t)(Nx - 1) * (Ny - 1);
-    const double dt = *p.dt_ptr, _dx = p._dx, _dy = p._dy;
+    const double _dx = p._dx, _dy = p._dy;
+    double dt = 0.0;
+    if (p.max_bits) {
+        dt = dt_of(__longlong_as_double((long long)p.max_bits[0]), __longlong_as_double((long long)p.max_bits[1]),
+                   p.maxdisp, p.dx, p.dy);
+        if (p.dt_out && blockIdx.x == 0 && threadIdx.x == 0) *p.dt_out = dt;
+    } else if (p.dt_ptr) {
+        dt = *p.dt_ptr;
+    }
     double srx = 0.0, sry = 0.0, sdv = 0.0;
     for (int64_t n = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; n < npts; n += (int64_t)gridDim.x * blockDim.x) {
         int i = (int)(n % W), j = (int)(n / W);
@@ -414,28 +442,43 @@ __global__ void __launch_bounds__(RES_THREADS) k_residuals(ResParams p) {
         p.partials[blockIdx.x * 3 + 0] = a;
         p.partials[blockIdx.x * 3 + 1] = b;
         p.partials[blockIdx.x * 3 + 2] = c;
+        __threadfence();
+        // (wraps to zero with the last block)
+        last = atomicInc(reinterpret_cast<unsigned*>(p.scalars + SC_TICKET), gridDim.x - 1) == gridDim.x - 1;
     }
-}
-
-// single block: sum partials in a fixed order; err = max of the three means
-__global__ void k_err_finalize(const double* __restrict__ partials, int nblocks, int64_t nrx, int64_t nry,
-                               int64_t ndv, double* __restrict__ scalars) {
-    __shared__ double sh[32];
-    double s[3] = {0.0, 0.0, 0.0};
-    for (int b = threadIdx.x; b < nblocks; b += blockDim.x)
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    // the partials in 1024 strided sums, their warps' trees, and the tree of those 32
+    double t[3];
 #pragma unroll
-        for (int k = 0; k < 3; ++k) s[k] += partials[b * 3 + k];
-    double t0 = block_sum(s[0], sh), t1 = block_sum(s[1], sh), t2 = block_sum(s[2], sh);
+    for (int k = 0; k < 3; ++k) {
+#pragma unroll
+        for (int q = 0; q < 1024 / RES_THREADS; ++q) {
+            double v = 0.0;
+            for (int n = q * RES_THREADS + threadIdx.x; n < (int)gridDim.x; n += 1024) v += __ldcg(p.partials + n * 3 + k);
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+            if ((threadIdx.x & 31) == 0) sh[(q * RES_THREADS + threadIdx.x) >> 5] = v;
+        }
+        __syncthreads();
+        t[k] = sh[threadIdx.x & 31];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) t[k] += __shfl_down_sync(0xffffffffu, t[k], o);
+        __syncthreads();
+    }
     if (threadIdx.x == 0) {
-        double a = t0 / (double)nrx, b = t1 / (double)nry, c = t2 / (double)ndv;
+        double a = t[0] / (double)((int64_t)(Nx - 2) * (Ny - 1)), b = t[1] / (double)((int64_t)(Nx - 1) * (Ny - 2)),
+               c = t[2] / (double)npts;
         double m = a;
         if (b > m || b != b) m = b;
         if (c > m || c != c) m = c;
         if (a != a) m = a;
-        scalars[SC_SUM_RX] = t0;
-        scalars[SC_SUM_RY] = t1;
-        scalars[SC_SUM_DIV] = t2;
-        scalars[SC_ERR] = m;
+        p.scalars[SC_SUM_RX] = t[0];
+        p.scalars[SC_SUM_RY] = t[1];
+        p.scalars[SC_SUM_DIV] = t[2];
+        *p.host_err = m;
+        if (p.max_bits) p.max_bits[0] = p.max_bits[1] = 0;
     }
 }
 
@@ -478,20 +521,14 @@ __global__ void k_maxabs_v(const double* __restrict__ Vx, const double* __restri
     }
 }
 
-// dt = maxdisp * min(dx / max|Vx|, dy / max|Vy|); written to every slot in mask
-__global__ void k_dt_finalize(const unsigned long long* __restrict__ maxbits, double maxdisp, double dx, double dy,
-                              double* __restrict__ scalars, int slot_a, int slot_b) {
+__global__ void k_dt_finalize(unsigned long long* __restrict__ maxbits, double maxdisp, double dx, double dy,
+                              double* __restrict__ scalars, int slot) {
     double mvx = __longlong_as_double((long long)maxbits[0]);
     double mvy = __longlong_as_double((long long)maxbits[1]);
-    double a = dx / mvx, b = dy / mvy;
-    double m = (b < a) ? b : a;
-    if (a != a) m = a;
-    if (b != b) m = b;
-    double dt = maxdisp * m;
+    maxbits[0] = maxbits[1] = 0;
     scalars[SC_MAX_VX] = mvx;
     scalars[SC_MAX_VY] = mvy;
-    if (slot_a >= 0) scalars[slot_a] = dt;
-    if (slot_b >= 0) scalars[slot_b] = dt;
+    if (slot >= 0) scalars[slot] = dt_of(mvx, mvy, maxdisp, dx, dy);
 }
 
 __global__ void k_set_scalar(double* __restrict__ p, double v) { *p = v; }
@@ -730,8 +767,8 @@ struct Solver {
         return march_launch(ctx, march_maps, m, T, s);
     }
 
-    // n iterations of a small grid in one launch
-    int launch_resident(int n) {
+    // n iterations of a small grid in one launch; the last one stores tau and divV, and max|V|, where wanted
+    int launch_resident(int n, bool store, bool maxima) {
         ResidentParams& r = res;
         r.Vx_in = Vx_cur();
         r.Vy_in = Vy_cur();
@@ -745,6 +782,11 @@ struct Solver {
         r.dVx_out = dVx_cur();
         r.dVy_out = dVy_cur();
         r.iters = n;
+        r.txx = store ? L.f(F_TXX) : nullptr;
+        r.tyy = store ? L.f(F_TYY) : nullptr;
+        r.txy = store ? L.f(F_TXY) : nullptr;
+        r.divV = store ? L.f(F_DIV) : nullptr;
+        r.max_bits = maxima ? max_bits() : nullptr;
         return resident_launch(ctx, r, plan, s);
     }
 
@@ -754,25 +796,31 @@ struct Solver {
     const double* Vy_cur() const { return L.f(cur ? F_VYB : F_VYA); }
     const double* P_cur() const { return L.f(cur ? F_PB : F_PA); }
 
-    int compute_dt(int slot_a, int slot_b) {
-        unsigned long long* bits = (unsigned long long*)(ctx->d_scalars + SC_MAXBITS);
-        SF_CUDA(cudaMemsetAsync(bits, 0, 2 * sizeof(unsigned long long), s));
-        k_maxabs_v<<<maxv_blocks, 256, 0, s>>>(Vx_cur(), Vy_cur(), (int)L.Nx, (int)L.Ny, L.LD, bits);
-        SF_LAUNCHED(ctx);
-        k_dt_finalize<<<1, 1, 0, s>>>(bits, maxdisp, dx, dy, ctx->d_scalars, slot_a, slot_b);
+    unsigned long long* max_bits() const { return (unsigned long long*)(ctx->d_scalars + SC_MAXBITS); }
+
+    int max_v() {
+        k_maxabs_v<<<maxv_blocks, 256, 0, s>>>(Vx_cur(), Vy_cur(), (int)L.Nx, (int)L.Ny, L.LD, max_bits());
         SF_LAUNCHED(ctx);
         return SF_OK;
     }
 
-    int residuals() {
+    int compute_dt(int slot) {
+        int rc = max_v();
+        if (rc) return rc;
+        k_dt_finalize<<<1, 1, 0, s>>>(max_bits(), maxdisp, dx, dy, ctx->d_scalars, slot);
+        SF_LAUNCHED(ctx);
+        return SF_OK;
+    }
+
+    // the residuals and their sums; dt: see ResParams.  err is in h_scalars[SC_ERR] once the stream is done
+    int residuals(const double* dt_ptr, bool dt_from_max, double* dt_out) {
         rp.P = P_cur();
         rp.Vx = Vx_cur();
         rp.Vy = Vy_cur();
+        rp.dt_ptr = dt_ptr;
+        rp.max_bits = dt_from_max ? max_bits() : nullptr;
+        rp.dt_out = dt_out;
         k_residuals<<<res_blocks, RES_THREADS, 0, s>>>(rp);
-        SF_LAUNCHED(ctx);
-        int64_t Nx = L.Nx, Ny = L.Ny;
-        k_err_finalize<<<1, 1024, 0, s>>>(rp.partials, res_blocks, (Nx - 2) * (Ny - 1), (Nx - 1) * (Ny - 2),
-                                          (Nx - 1) * (Ny - 1), ctx->d_scalars);
         SF_LAUNCHED(ctx);
         return SF_OK;
     }
@@ -807,6 +855,7 @@ static int solver_prepare(Solver& S, sf_ctx* ctx, cudaStream_t s, const SolveArg
     S.res_blocks = (int)std::min<int64_t>(ceil_div((Nx - 1) * (Ny - 1), RES_THREADS), (int64_t)ctx->num_sms * 8);
     S.maxv_blocks = (int)std::min<int64_t>(ceil_div(Nx * (Ny + 1), 256), (int64_t)ctx->num_sms * 8);
     if ((rc = ensure(ctx, ctx->partials, (size_t)S.res_blocks * 3 * 8))) return rc;
+    SF_CUDA(cudaMemsetAsync(S.max_bits(), 0, (SC_N - SC_MAXBITS) * sizeof(double), s));   // maxima and ticket
     S.maxdisp = maxdisp;
     S.dx = dx;
     S.dy = dy;
@@ -920,7 +969,11 @@ static int solver_prepare(Solver& S, sf_ctx* ctx, cudaStream_t s, const SolveArg
     rp.txy = S.L.f(F_TXY);
     rp.rho = S.L.f(F_RHO);
     rp.divV = S.L.f(F_DIV);
-    rp.dt_ptr = ctx->d_scalars + SC_DT_CHECK;
+    rp.maxdisp = maxdisp;
+    rp.dx = dx;
+    rp.dy = dy;
+    rp.scalars = ctx->d_scalars;
+    rp.host_err = ctx->h_scalars + SC_ERR;
     rp.Rx = S.L.f(F_RX);
     rp.Ry = S.L.f(F_RY);
     rp.partials = (double*)ctx->partials.ptr;
@@ -1042,7 +1095,7 @@ static std::vector<HaloArray> state_halos(std::vector<Rank>& R) {
 static int global_dt(std::vector<Rank>& R, double maxdisp, double dx, double dy, double* dt) {
     for (Rank& k : R) {
         SF_CUDA(cudaSetDevice(k.ctx->device));
-        int rc = k.S.compute_dt(-1, -1);
+        int rc = k.S.compute_dt(-1);
         if (rc) return rc;
         SF_CUDA(cudaMemcpyAsync(k.ctx->h_scalars + SC_MAX_VX, k.ctx->d_scalars + SC_MAX_VX, 2 * 8,
                                 cudaMemcpyDeviceToHost, k.s));
@@ -1201,39 +1254,38 @@ int sf_solve_stokes(sf_ctx* ctx, double* P, double* Vx_pad, double* Vy_pad, cons
                 SF_CUDA(cudaEventRecord(ctx->ev_a, s));
                 have_t1 = true;
             }
-            // the last iteration before the residual check (or the end) stores tau and divV; the ones before it
-            // run several to a launch, up to the next dt update and to where the timing starts
-            int64_t stop = last - 1;
+            // the last iteration before the residual check (or the end) stores tau and divV.  Several iterations run
+            // per launch, up to the next dt update and to where the timing starts; with the resident kernel up to and
+            // including the last one, with the march up to the one before
+            int64_t stop = last;
+            bool maxima = false;   // of the velocities, by the launch
             if (use_stab) stop = std::min(stop, ((it - 1) / ndtupdate + 1) * ndtupdate);
             if (it < itert1) stop = std::min(stop, itert1 - 1);
-            if (it <= stop && resident && stop - it + 1 >= RESIDENT_MIN_ITERS) {
+            if (resident && stop - it + 1 >= RESIDENT_MIN_ITERS) {
                 const int64_t n = std::min<int64_t>(stop - it + 1, RESIDENT_MAX_ITERS);
-                if ((rc = S.launch_resident((int)n))) return rc;
                 it += n - 1;
-            } else if (it <= stop) {
-                const int T = (int)std::min<int64_t>(march_t, stop - it + 1);
+                maxima = use_stab && it == last && it % ncheck == 0;
+                if ((rc = S.launch_resident((int)n, it == last, maxima))) return rc;
+            } else if (it < last) {
+                const int T = (int)std::min<int64_t>(march_t, std::min(stop, last - 1) - it + 1);
                 if ((rc = S.launch_march(T))) return rc;
                 it += T - 1;
             } else if ((rc = S.launch_iter(true))) {
                 return rc;
             }
             ++fused;
-            bool dt_up = use_stab && (it % ndtupdate == 0);
-            bool check = (it % ncheck == 0);
-            if (dt_up || (check && use_stab)) {
-                if ((rc = S.compute_dt(dt_up ? SC_DT : -1, check ? SC_DT_CHECK : -1))) return rc;
-            }
-            if (check && !use_stab) {
-                k_set_scalar<<<1, 1, 0, s>>>(ctx->d_scalars + SC_DT_CHECK, 0.0);
-                SF_LAUNCHED(ctx);
+            const bool dt_up = use_stab && (it % ndtupdate == 0);
+            if (it % ncheck == 0) {
+                if (use_stab && !maxima && (rc = S.max_v())) return rc;
+                if ((rc = S.residuals(nullptr, use_stab, dt_up ? ctx->d_scalars + SC_DT : nullptr))) return rc;
+            } else if (dt_up && (rc = S.compute_dt(SC_DT))) {
+                return rc;
             }
         }
         niter += last - iter + 1;
         iter = last + 1;
         if (last % ncheck == 0) {
-            if ((rc = S.residuals())) return rc;
             ++nchecks;
-            SF_CUDA(cudaMemcpyAsync(ctx->h_scalars + SC_ERR, ctx->d_scalars + SC_ERR, 8, cudaMemcpyDeviceToHost, s));
             SF_CUDA(cudaStreamSynchronize(s));
             err = ctx->h_scalars[SC_ERR];
             if (!(err == err) || std::isinf(err)) break;
@@ -1243,7 +1295,7 @@ int sf_solve_stokes(sf_ctx* ctx, double* P, double* Vx_pad, double* Vy_pad, cons
 
     // ---- unpack (:89-95) ----
     if ((rc = solver_unpack(S, A, niter, nchecks))) return rc;
-    if ((rc = S.compute_dt(SC_DT_OUT, -1))) return rc;  // returned dt (:95)
+    if ((rc = S.compute_dt(SC_DT_OUT))) return rc;  // returned dt (:95)
     SF_CUDA(cudaMemcpyAsync(ctx->h_scalars, ctx->d_scalars, SC_N * 8, cudaMemcpyDeviceToHost, s));
     SF_CUDA(cudaStreamSynchronize(s));
     double dt_out = ctx->h_scalars[SC_DT_OUT];
@@ -1427,7 +1479,7 @@ int sf_solve_stokes_decomposed(sf_domain* domains, int32_t dims_x, int32_t dims_
         if (check) {  // :69-70, compute_err with the SUM Allreduce of the local means (:103-109)
             for (Rank& k : R) {
                 SF_CUDA(cudaSetDevice(k.ctx->device));
-                if ((rc = k.S.residuals())) return rc;
+                if ((rc = k.S.residuals(k.ctx->d_scalars + SC_DT_CHECK, false, nullptr))) return rc;
                 SF_CUDA(cudaMemcpyAsync(k.ctx->h_scalars + SC_SUM_RX, k.ctx->d_scalars + SC_SUM_RX, 3 * 8,
                                         cudaMemcpyDeviceToHost, k.s));
             }
