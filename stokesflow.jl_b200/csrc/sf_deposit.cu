@@ -446,7 +446,11 @@ __global__ void __launch_bounds__(SORT_THREADS) k_sort_cells(const __grid_consta
 // Four records ahead with 5 blocks per SM: 9.5 ms, one ahead 10.4; three 7.9 - 8.1; 10 blocks 8.7; dividing with a range
 // test per record instead of once per deposit (SortGrid::general) 8.5.
 constexpr int GT_NONE = 0x7fffffff;   // start of an exhausted list
-constexpr int GT_X = 32, GT_Y = 4;    // nodes of a block: one warp per node row, 4 rows that share cell rows
+// nodes of a block, and of a warp along x.  Neighbours read the same records, in both directions: compact warps and blocks
+// find more of them in L1 (33% of the sectors before) and L2.  Against rows of 32 nodes in blocks of 4, 67 M markers: 7.73
+// -> 7.48 ms; 26 M 3.04 -> 2.92, after a strong swirl 5.03 -> 4.62, shuffled in their cells 4.16 -> 4.10, sorted by cell
+// 3.30 -> 3.31, in rows along x 2.79 -> 2.83.  Warps of 4 x 8 nodes: 7.51, of 1 x 32 7.71 and 5.37 after the swirl.
+constexpr int GT_X = 16, GT_Y = 8, GT_LX = 8, GT_LY = 32 / GT_LX;
 constexpr int GT_AHEAD = 2;           // records of a run loaded at once
 constexpr int GT_BLOCKS = 8;          // blocks per SM (64 registers)
 
@@ -460,8 +464,9 @@ __device__ __forceinline__ void gather_node(const SortGrids& s, const SortGrid& 
     const uint32_t* __restrict__ ends = g.ends;
     const int64_t nx = g.nx, ny = g.ny;
     const int64_t ntx = (nx + GT_X - 1) / GT_X;
-    const int64_t I = (int64_t)(blockIdx.x % ntx) * GT_X + (threadIdx.x % GT_X) + 1;
-    const int64_t J = (int64_t)(blockIdx.x / ntx) * GT_Y + (threadIdx.x / GT_X) + 1;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t I = (int64_t)(blockIdx.x % ntx) * GT_X + (warp % (GT_X / GT_LX)) * GT_LX + lane % GT_LX + 1;
+    const int64_t J = (int64_t)(blockIdx.x / ntx) * GT_Y + (warp / (GT_X / GT_LX)) * GT_LY + lane / GT_LX + 1;
     if (I > nx || J > ny) return;
     const int64_t ldc = nx + 1;
     const bool second = g.second != 0;
