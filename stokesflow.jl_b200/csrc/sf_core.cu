@@ -265,7 +265,9 @@ int sf_ctx_create(int device, sf_ctx** out) {
         cudaMalloc(&c->d_flags, sizeof(int) * 4) != cudaSuccess ||
         cudaMallocHost(&c->h_scalars, sizeof(double) * SC_N) != cudaSuccess ||
         cudaEventCreate(&c->ev_a) != cudaSuccess || cudaEventCreate(&c->ev_b) != cudaSuccess ||
-        cudaEventCreate(&c->ev_c) != cudaSuccess || cudaEventCreate(&c->ev_d) != cudaSuccess ||
+        cudaEventCreate(&c->ev_c) != cudaSuccess ||
+        cudaEventCreateWithFlags(&c->ev_check[0], cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&c->ev_check[1], cudaEventDisableTiming) != cudaSuccess ||
         cudaStreamCreateWithFlags(&c->work, cudaStreamNonBlocking) != cudaSuccess) {
         cudaError_t le = cudaGetLastError();
         sf_ctx_destroy(c);
@@ -293,7 +295,7 @@ int sf_ctx_destroy(sf_ctx* c) {
     if (c->d_flags) cudaFree(c->d_flags);
     if (c->work) cudaStreamDestroy(c->work);
     if (c->h_scalars) cudaFreeHost(c->h_scalars);
-    cudaEvent_t evs[] = {c->ev_a, c->ev_b, c->ev_c, c->ev_d};
+    cudaEvent_t evs[] = {c->ev_a, c->ev_b, c->ev_c, c->ev_check[0], c->ev_check[1]};
     for (cudaEvent_t ev : evs)
         if (ev) cudaEventDestroy(ev);
     delete c;

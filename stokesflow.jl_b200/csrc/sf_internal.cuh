@@ -59,7 +59,8 @@ enum { CNT_BAD_MARKERS = 0, CNT_EMPTY_NODES = 1, CNT_INTERP_FAILSAFE = 2, CNT_OU
 // max|Vy| as ordered bit patterns during a reduction, zero between reductions;
 // SC_TICKET: blocks of k_residuals that are done, zero between launches.
 enum { SC_DT = 0, SC_DT_CHECK = 1, SC_ERR = 2, SC_SUM_RX = 3, SC_SUM_RY = 4, SC_SUM_DIV = 5,
-       SC_MAX_VX = 6, SC_MAX_VY = 7, SC_SCALE = 8, SC_DT_OUT = 9, SC_MAXBITS = 12, SC_TICKET = 14, SC_N = 16 };
+       SC_MAX_VX = 6, SC_MAX_VY = 7, SC_SCALE = 8, SC_DT_OUT = 9,
+       SC_ERR2 = 10 /* host: every other check's err */, SC_MAXBITS = 12, SC_TICKET = 14, SC_N = 16 };
 
 }  // namespace sf
 
@@ -82,7 +83,8 @@ struct sf_ctx {
     double* d_scalars = nullptr;
     double* h_scalars = nullptr;  // pinned mirror
     int* d_flags = nullptr;       // device error flags (int[4]); [0]: a bounded wait timed out
-    cudaEvent_t ev_a = nullptr, ev_b = nullptr, ev_c = nullptr, ev_d = nullptr;
+    cudaEvent_t ev_a = nullptr, ev_b = nullptr, ev_c = nullptr;
+    cudaEvent_t ev_check[2] = {};  // the PT loop's residual checks
     int64_t launches = 0;         // kernels launched through this context
     sf_engine* batch_engine = nullptr;  // the engine sf_solve_stokes_batch_mixed reuses across calls
     // sweep shapes the engines' autotuner measured best, by workload class (sf_mixed.cu)

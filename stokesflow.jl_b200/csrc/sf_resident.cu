@@ -80,6 +80,7 @@ __global__ void __launch_bounds__(512, 1) k_pt_resident(const __grid_constant__ 
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ int gave_up;
     __shared__ unsigned long long max_v[2];
+    if (p.err && !goes_on(p.err, p.eps)) return;   // (all blocks)
     const int W = p.W, H = p.H, pitch = W + 2;
     const int comp1 = (H + 2) * pitch;                            // from an entry of Vx to that of Vy
     double* sVx = reinterpret_cast<double*>(smem_raw);            // (H + 2) x (W + 2): entry (0, 0) is Vx(i0, j0)

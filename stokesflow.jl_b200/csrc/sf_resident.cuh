@@ -30,7 +30,12 @@ struct ResidentParams {
     // onto what is there (NULL: not)
     double *txx, *tyy, *txy, *divV;
     unsigned long long* max_bits;
+    const double* err;           // where given, nothing is done unless eps < *err < infinity
+    double eps;
 };
+
+// whether the loop goes on after a check (StokesSolver_multixpu.jl:43, :75): for kernels launched behind the check
+__device__ __forceinline__ bool goes_on(const double* err, double eps) { return *err > eps && !isinf(*err); }
 
 struct ResidentPlan {
     bool fits = false;           // the grid is small enough

@@ -387,6 +387,8 @@ struct ResParams {
     double _dx, _dy, g_y;
     double* scalars;
     double* host_err;  // pinned host memory
+    const double* err; // where given, nothing is done unless eps < *err < infinity
+    double eps;
 };
 
 // dt = maxdisp * min(dx / max|Vx|, dy / max|Vy|) (:118-121)
@@ -404,6 +406,7 @@ __device__ __forceinline__ double dt_of(double mvx, double mvy, double maxdisp, 
 __global__ void __launch_bounds__(RES_THREADS) k_residuals(const ResParams p) {
     __shared__ double sh[32];
     __shared__ bool last;
+    if (p.err && !goes_on(p.err, p.eps)) return;   // (all blocks: *err is written below, when all are here)
     const int Nx = p.Nx, Ny = p.Ny;
     const int64_t LD = p.LD, W = Nx - 1, npts = (int64_t)(Nx - 1) * (Ny - 1);
     const double _dx = p._dx, _dy = p._dy;
@@ -477,6 +480,7 @@ __global__ void __launch_bounds__(RES_THREADS) k_residuals(const ResParams p) {
         p.scalars[SC_SUM_RX] = t[0];
         p.scalars[SC_SUM_RY] = t[1];
         p.scalars[SC_SUM_DIV] = t[2];
+        p.scalars[SC_ERR] = m;
         *p.host_err = m;
         if (p.max_bits) p.max_bits[0] = p.max_bits[1] = 0;
     }
@@ -768,7 +772,7 @@ struct Solver {
     }
 
     // n iterations of a small grid in one launch; the last one stores tau and divV, and max|V|, where wanted
-    int launch_resident(int n, bool store, bool maxima) {
+    int launch_resident(int n, bool store, bool maxima, const double* err, double eps) {
         ResidentParams& r = res;
         r.Vx_in = Vx_cur();
         r.Vy_in = Vy_cur();
@@ -787,6 +791,8 @@ struct Solver {
         r.txy = store ? L.f(F_TXY) : nullptr;
         r.divV = store ? L.f(F_DIV) : nullptr;
         r.max_bits = maxima ? max_bits() : nullptr;
+        r.err = err;
+        r.eps = eps;
         return resident_launch(ctx, r, plan, s);
     }
 
@@ -812,14 +818,18 @@ struct Solver {
         return SF_OK;
     }
 
-    // the residuals and their sums; dt: see ResParams.  err is in h_scalars[SC_ERR] once the stream is done
-    int residuals(const double* dt_ptr, bool dt_from_max, double* dt_out) {
+    // the residuals and their sums; dt and the condition: see ResParams.  err is in host_err once the stream is done
+    int residuals(const double* dt_ptr, bool dt_from_max, double* dt_out, double* host_err, const double* err = nullptr,
+                  double eps = 0.0) {
         rp.P = P_cur();
         rp.Vx = Vx_cur();
         rp.Vy = Vy_cur();
         rp.dt_ptr = dt_ptr;
         rp.max_bits = dt_from_max ? max_bits() : nullptr;
         rp.dt_out = dt_out;
+        rp.host_err = host_err;
+        rp.err = err;
+        rp.eps = eps;
         k_residuals<<<res_blocks, RES_THREADS, 0, s>>>(rp);
         SF_LAUNCHED(ctx);
         return SF_OK;
@@ -973,7 +983,6 @@ static int solver_prepare(Solver& S, sf_ctx* ctx, cudaStream_t s, const SolveArg
     rp.dx = dx;
     rp.dy = dy;
     rp.scalars = ctx->d_scalars;
-    rp.host_err = ctx->h_scalars + SC_ERR;
     rp.Rx = S.L.f(F_RX);
     rp.Ry = S.L.f(F_RY);
     rp.partials = (double*)ctx->partials.ptr;
@@ -1245,11 +1254,11 @@ int sf_solve_stokes(sf_ctx* ctx, double* P, double* Vx_pad, double* Vy_pad, cons
     bool have_t1 = false;
     int64_t fused = 0;
     SF_CUDA(cudaEventRecord(ctx->ev_c, s));
-    while (err > eps && iter <= iter_max) {
-        // iterations up to and including the next check (or iter_max)
-        int64_t next_check = ((iter - 1) / ncheck + 1) * ncheck;
-        int64_t last = std::min(next_check, iter_max);
-        for (int64_t it = iter; it <= last; ++it) {
+    // launches the iterations from `it` to `last`, the next check or iter_max, and the check; all of it on the condition
+    // that the loop goes on after the check before, if cond
+    auto iterations = [&](int64_t it, int64_t last, bool cond) {
+        const double* const cond_err = cond ? ctx->d_scalars + SC_ERR : nullptr;
+        for (; it <= last; ++it) {
             if (it == itert1) {
                 SF_CUDA(cudaEventRecord(ctx->ev_a, s));
                 have_t1 = true;
@@ -1265,7 +1274,7 @@ int sf_solve_stokes(sf_ctx* ctx, double* P, double* Vx_pad, double* Vy_pad, cons
                 const int64_t n = std::min<int64_t>(stop - it + 1, RESIDENT_MAX_ITERS);
                 it += n - 1;
                 maxima = use_stab && it == last && it % ncheck == 0;
-                if ((rc = S.launch_resident((int)n, it == last, maxima))) return rc;
+                if ((rc = S.launch_resident((int)n, it == last, maxima, cond_err, eps))) return rc;
             } else if (it < last) {
                 const int T = (int)std::min<int64_t>(march_t, std::min(stop, last - 1) - it + 1);
                 if ((rc = S.launch_march(T))) return rc;
@@ -1276,20 +1285,51 @@ int sf_solve_stokes(sf_ctx* ctx, double* P, double* Vx_pad, double* Vy_pad, cons
             ++fused;
             const bool dt_up = use_stab && (it % ndtupdate == 0);
             if (it % ncheck == 0) {
+                const int odd = (int)(it / ncheck & 1);
                 if (use_stab && !maxima && (rc = S.max_v())) return rc;
-                if ((rc = S.residuals(nullptr, use_stab, dt_up ? ctx->d_scalars + SC_DT : nullptr))) return rc;
+                if ((rc = S.residuals(nullptr, use_stab, dt_up ? ctx->d_scalars + SC_DT : nullptr,
+                                      ctx->h_scalars + (odd ? SC_ERR2 : SC_ERR), cond_err, eps)))
+                    return rc;
+                SF_CUDA(cudaEventRecord(ctx->ev_check[odd], s));
             } else if (dt_up && (rc = S.compute_dt(SC_DT))) {
                 return rc;
+            }
+        }
+        return (int)SF_OK;
+    };
+    int64_t launched = 0;   // iterations
+    int cur = S.cur;        // the buffer parity after the iterations that count
+    while (err > eps && iter <= iter_max) {
+        // iterations up to and including the next check (or iter_max)
+        const int64_t last = std::min(((iter - 1) / ncheck + 1) * ncheck, iter_max);
+        if (launched < last) {
+            if ((rc = iterations(iter, last, false))) return rc;
+            launched = last;
+        }
+        cur = S.cur;
+        if (last % ncheck == 0 && last + RESIDENT_MIN_ITERS <= iter_max && resident) {
+            // Those up to the next check go behind this one if they are one resident launch: the device decides (goes_on),
+            // and does not wait for the host to read err and launch: 20 x 26 1.00 -> 0.90 us per iteration, 64^2 1.05 -> 1.03.
+            const int64_t next = std::min(last + ncheck, iter_max);
+            if (next - last <= RESIDENT_MAX_ITERS && (!use_stab || last / ndtupdate == (next - 1) / ndtupdate) &&
+                last >= itert1) {
+                if ((rc = iterations(last + 1, next, true))) return rc;
+                launched = next;
             }
         }
         niter += last - iter + 1;
         iter = last + 1;
         if (last % ncheck == 0) {
+            const int odd = (int)(last / ncheck & 1);
             ++nchecks;
-            SF_CUDA(cudaStreamSynchronize(s));
-            err = ctx->h_scalars[SC_ERR];
+            SF_CUDA(cudaEventSynchronize(ctx->ev_check[odd]));
+            err = ctx->h_scalars[odd ? SC_ERR2 : SC_ERR];
             if (!(err == err) || std::isinf(err)) break;
         }
+    }
+    if (launched >= iter) {   // what was launched behind the last check did nothing
+        S.cur = cur;
+        --fused;
     }
     SF_CUDA(cudaEventRecord(ctx->ev_b, s));
 
@@ -1479,7 +1519,7 @@ int sf_solve_stokes_decomposed(sf_domain* domains, int32_t dims_x, int32_t dims_
         if (check) {  // :69-70, compute_err with the SUM Allreduce of the local means (:103-109)
             for (Rank& k : R) {
                 SF_CUDA(cudaSetDevice(k.ctx->device));
-                if ((rc = k.S.residuals(k.ctx->d_scalars + SC_DT_CHECK, false, nullptr))) return rc;
+                if ((rc = k.S.residuals(k.ctx->d_scalars + SC_DT_CHECK, false, nullptr, k.ctx->h_scalars + SC_ERR))) return rc;
                 SF_CUDA(cudaMemcpyAsync(k.ctx->h_scalars + SC_SUM_RX, k.ctx->d_scalars + SC_SUM_RX, 3 * 8,
                                         cudaMemcpyDeviceToHost, k.s));
             }

@@ -43,6 +43,39 @@ def test_march_bitexact(sf, oracle_lib, Nx, Ny, iters, stab):
         assert np.array_equal(b[k], a[k], equal_nan=True), f"{k} differs from the oracle"
 
 
+@pytest.mark.parametrize("Nx,Ny,bad", [(20, 26, False), (150, 131, False), (20, 26, True), (150, 131, True)])
+def test_resident_stops_where_the_loop_does(sf, oracle_lib, Nx, Ny, bad):
+    """The iterations behind a check are launched before its result is known: a solve that converges there (or meets a
+    NaN) ends with that check's state, and the same holds for the solve after it in the same context."""
+    O = oracle_lib
+    dx, dy = 1.0 / (Nx - 1), 1.0 / (Ny - 1)
+    args = (9.81, dx, dy, Nx, Ny, 1e-3, 0.5, True)
+    ncheck = 5 * min(Nx, Ny)
+    a0 = O.stokes_arrays(Nx, Ny)
+    a0["rho_vy"][:], a0["mu_b"][:], a0["mu_p"][:] = random_fields(Nx, Ny, seed=5, contrast=2.0)
+    copy = lambda: {k: v.copy(order="F") for k, v in a0.items()}
+    if bad:
+        a0["rho_vy"][Nx // 2, Ny // 2] = np.nan
+        eps, stop = 1e-300, ncheck
+    else:
+        eps, stop = O.solve_stokes(copy(), *args, 1e-300, 3 * ncheck).err * (1 + 1e-9), 3 * ncheck
+    for iter_max in (10 * ncheck, 3 * ncheck + 7):
+        a = copy()
+        r = O.solve_stokes(a, *args, eps, iter_max)
+        if bad:   # reported as an error; the state is in the arrays
+            t = {k: dev(v) for k, v in copy().items()}
+            with pytest.raises(sf.StokesFlowError, match="not finite"):
+                sf.solve_stokes_info(*[t[k] for k in NAMES], *args[:7], eps=eps, iter_max=iter_max)
+            b, iters = {k: host(v) for k, v in t.items()}, stop
+        else:
+            b, info = gpu_solve(sf, copy(), *args, eps, iter_max)
+            iters = info["iters"]
+            assert info["dt"] == r.dt
+        assert iters == r.iters == stop
+        for k in NAMES:
+            assert np.array_equal(b[k], a[k], equal_nan=True), f"{k} differs from the oracle"
+
+
 def test_concurrent_solves_bitexact(sf, oracle_lib):
     """Solves of several threads at once, contexts and streams of their own, more of them than the device has room for
     resident tiles (the rest marches), some of them small enough for a cluster: each equals the oracle."""
