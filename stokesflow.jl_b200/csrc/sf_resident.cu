@@ -4,8 +4,9 @@
 // the chip for as many iterations as the reference's loop runs without an event (a residual check, a dt update):
 //
 //   * the grid is cut into at most one tile per SM; a thread owns the same points in every iteration and keeps their
-//     P, rates and parameters in registers.  Vx, Vy and the stage-1 results of a tile (P, tau_xx, tau_yy, tau_xy) are in
-//     shared memory.  An iteration is the two stages of k_pt_iter, a barrier after each, and the exchange of the
+//     P, rates and parameters in registers: up to four, one above the other, which share what they read (at 511 x 385
+//     17 accesses to shared memory per point and iteration; points of their own 25, and 2.82 us instead of 2.60).
+//     Vx, Vy and the stage-1 results of a tile (P, tau_xx, tau_yy, tau_xy) are in shared memory.  An iteration is the two stages of k_pt_iter, a barrier after each, and the exchange of the
 //     velocities on the tiles' borders, one of:
 //   * the tiles are the blocks of one cluster (up to 16): a thread stores a border point's velocities also into the
 //     neighbours' shared memory, and the second barrier is the cluster's.  The velocities are double-buffered: a
@@ -22,7 +23,7 @@
 // What bounds it: latency.  A cluster's iteration takes 0.62 us at 20 x 26 and about 0.8 at 64^2, the two stages'
 // dependent FP64 chains and the barriers; with the checks 1.1 and 1.1 us (k_pt_iter, one launch each: 4.5 and 4.4).
 // Through L2, 128^2 (110 tiles of 150 points, 8 warps) takes 1.5 us, about half of it the exchange, against 5.2; at
-// 511 x 385 (1450 points per SM) 2.8 us, there mostly issue slots, against 8.3.  Testing every point's flags and
+// 511 x 385 (1450 points per SM) 2.6 us, there mostly issue slots, against 8.3.  Testing every point's flags and
 // sending borders to L2 from the update itself took 905 instructions per warp and iteration at 511 x 385 and 4.2 us.
 #include <algorithm>
 #include <mutex>
@@ -69,6 +70,9 @@ __device__ __forceinline__ void cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
+// rows of points of a tile, its halo row included, in whole groups of K
+__host__ __device__ __forceinline__ int rows_of(int H, int K) { return (H + K) / K * K; }
+
 // what a thread's point is: one whose Vx / Vy it updates (the others' are boundary entries, zero), one of the tile (not
 // of its halo column or row), and the sides of the domain that it lies on
 enum { PT_X = 1, PT_Y = 2, PT_OWN = 4, PT_I0 = 8, PT_I1 = 16, PT_J0 = 32, PT_J1 = 64, PT_DX = 128,
@@ -82,16 +86,17 @@ __global__ void __launch_bounds__(512, 1) k_pt_resident(const __grid_constant__ 
     __shared__ unsigned long long max_v[2];
     if (p.err && !goes_on(p.err, p.eps)) return;   // (all blocks)
     const int W = p.W, H = p.H, pitch = W + 2;
-    const int comp1 = (H + 2) * pitch;                            // from an entry of Vx to that of Vy
-    double* sVx = reinterpret_cast<double*>(smem_raw);            // (H + 2) x (W + 2): entry (0, 0) is Vx(i0, j0)
+    const int rows = rows_of(H, K);                               // of points that threads have
+    const int comp1 = (rows + 1) * pitch;                         // from an entry of Vx to that of Vy
+    double* sVx = reinterpret_cast<double*>(smem_raw);            // (rows + 1) x (W + 2): entry (0, 0) is Vx(i0, j0)
     double* sVy = sVx + comp1;
     // CLUSTER: a second pair, written while the first is read (a neighbour's border may come in at any time)
     double* sVx_n = CLUSTER ? sVy + comp1 : sVx;
     double* sVy_n = sVx_n + comp1;
-    double* const sTxx = sVy_n + comp1;                           // (H + 1) rows of the same pitch
-    double* const sTyy = sTxx + (H + 1) * pitch;
-    double* const sPn = sTyy + (H + 1) * pitch;
-    double* const sTxy = sPn + (H + 1) * pitch;
+    double* const sTxx = sVy_n + comp1;                           // `rows` rows of the same pitch
+    double* const sTyy = sTxx + rows * pitch;
+    double* const sPn = sTyy + rows * pitch;
+    double* const sTxy = sPn + rows * pitch;
     const int tid = threadIdx.x, NT = blockDim.x;
     const int bx = blockIdx.x % p.ntx, by = blockIdx.x / p.ntx;
     const int i0 = bx * W, j0 = by * H;
@@ -101,7 +106,7 @@ __global__ void __launch_bounds__(512, 1) k_pt_resident(const __grid_constant__ 
     const bool has_l = bx > 0, has_r = bx + 1 < p.ntx, has_b = by > 0, has_t = by + 1 < p.nty;
 
     // ---- state and parameters onto the chip ----
-    for (int n = tid; n < (H + 2) * pitch; n += NT) {
+    for (int n = tid; n < comp1; n += NT) {
         const int b = n / pitch, a = n - b * pitch;
         // (the domain's corners are read by nothing but the last iteration's tau_xy, which finds them zero)
         const int i = i0 + a, j = j0 + b;
@@ -113,17 +118,18 @@ __global__ void __launch_bounds__(512, 1) k_pt_resident(const __grid_constant__ 
     }
     if (tid < 2) max_v[tid] = 0;   // (barriers follow)
     double P[K], dvx[K], dvy[K], tp[K], mu2[K], mb[K], tx[K], ty[K], rho[K], gx[K], gy[K];
-    int off[K];      // b * pitch + a of the thread's points (a <= W, b <= H: the tile and one more column and row)
+    // the thread's points: K of a column a <= W, from row b0 on (b <= H: the tile and one more column and row)
+    const bool live = tid < (W + 1) * (rows / K);   // (the other threads compute on the first points and store nothing)
+    const int b0 = live ? tid / (W + 1) * K : 0, a = live ? tid % (W + 1) : 0;
+    const int o0 = b0 * pitch + a;
     int kind[K];
 #pragma unroll
     for (int k = 0; k < K; ++k) {
-        const int n = tid + k * NT;
-        const int b = n / (W + 1), a = n - b * (W + 1);
+        const int b = b0 + k;
         const int i = i0 + a, j = j0 + b;
-        off[k] = b <= H ? b * pitch + a : 0;   // (points beyond the tile's compute on its first and store nothing)
         kind[k] = 0;
         P[k] = dvx[k] = dvy[k] = tp[k] = mu2[k] = mb[k] = tx[k] = ty[k] = rho[k] = gx[k] = gy[k] = 0.0;
-        if (b > H) continue;
+        if (!live || b > H) continue;
         const int64_t o = i + (int64_t)j * LD;
         const bool own = a < W && b < H && i < Nx - 1 && j < Ny - 1;
         if (own)
@@ -191,7 +197,7 @@ __global__ void __launch_bounds__(512, 1) k_pt_resident(const __grid_constant__ 
         for (int k = 0; k < K; ++k) {
             at_x[k] = at_y[k] = at_d[k] = 0;
             if (!(kind[k] & PT_OWN)) continue;
-            const int b = off[k] / pitch, a = off[k] - b * pitch, t = blockIdx.x;
+            const int b = b0 + k, t = blockIdx.x;
             if (a == 0 && has_l) at_x[k] = in_block(sVx_n + (b + 1) * pitch + W + 1, t - 1);
             if (a == W - 1 && has_r) at_x[k] = in_block(sVx_n + (b + 1) * pitch, t + 1);
             if (b == 0 && has_b) at_y[k] = in_block(sVx_n + (H + 1) * pitch + a + 1, t - p.ntx);
@@ -212,45 +218,60 @@ __global__ void __launch_bounds__(512, 1) k_pt_resident(const __grid_constant__ 
     for (int it = 0; it < p.iters; ++it) {
         // ---- stage 1: compute_P_tau! (:140-169) on the tile and one more column and row.  Evaluated at every point
         // (outside the domain on whatever is there; nothing that is kept depends on it) ----
-        double sterm[K];
+        double sterm[K], txx[K], tyy[K], txy[K];
+        {
+            // (every entry once: points of a column share theirs)
+            double vx0 = sVx[o0], vx1 = sVx[o0 + pitch], vx1r = sVx[o0 + pitch + 1], vy0r = sVy[o0 + 1];
 #pragma unroll
-        for (int k = 0; k < K; ++k) {
-            const int o = off[k];
-            const double vx00 = sVx[o], vx10 = sVx[o + pitch], vx11 = sVx[o + pitch + 1];
-            const double vy00 = sVy[o], vy01 = sVy[o + 1], vy11 = sVy[o + pitch + 1];
-            const double vx20 = sVx[o + 2 * pitch], vx21 = sVx[o + 2 * pitch + 1];
-            const double dVx_dy = (vx10 - vx00) * _dy;
-            const double dVy_dx = (vy01 - vy00) * _dx;
-            const double txy = mb[k] * (dVx_dy + dVy_dx);
-            const double dVx_dx = (vx11 - vx10) * _dx;
-            const double dVy_dy = (vy11 - vy01) * _dy;
-            const double div = dVx_dx + dVy_dy;
-            P[k] = P[k] - tp[k] * div;
-            if (p.divV && it + 1 == p.iters && (kind[k] & PT_OWN)) {
-                const int b = o / pitch;
-                p.divV[i0 + o - b * pitch + (int64_t)(j0 + b) * LD] = div;
-            }
-            const double third = 1.0 / 3.0 * div;
-            const double txx = mu2[k] * (dVx_dx - third), tyy = mu2[k] * (dVy_dy - third);
-            // the gravity term of compute_ResY (:189-202), from the old velocities
-            const double av = 0.25 * (vx10 + vx11 + vx20 + vx21);
-            sterm[k] = g_y * (rho[k] - dt * (av * gx[k] * 0.5 * _dx + vy11 * gy[k] * 0.5 * _dy));
-            if (tid + k * NT < (W + 1) * (H + 1)) {
-                sTxy[o] = txy;
-                sPn[o] = P[k];
-                sTxx[o] = txx;
-                sTyy[o] = tyy;
+            for (int k = 0; k < K; ++k) {
+                const int o = o0 + k * pitch;
+                const double vx2 = sVx[o + 2 * pitch], vx2r = sVx[o + 2 * pitch + 1];
+                const double vy0 = sVy[o], vy1r = sVy[o + pitch + 1];
+                const double dVx_dy = (vx1 - vx0) * _dy;
+                const double dVy_dx = (vy0r - vy0) * _dx;
+                txy[k] = mb[k] * (dVx_dy + dVy_dx);
+                const double dVx_dx = (vx1r - vx1) * _dx;
+                const double dVy_dy = (vy1r - vy0r) * _dy;
+                const double div = dVx_dx + dVy_dy;
+                P[k] = P[k] - tp[k] * div;
+                const double third = 1.0 / 3.0 * div;
+                txx[k] = mu2[k] * (dVx_dx - third);
+                tyy[k] = mu2[k] * (dVy_dy - third);
+                if (p.divV && it + 1 == p.iters && (kind[k] & PT_OWN)) {
+                    const int64_t q = i0 + a + (int64_t)(j0 + b0 + k) * LD;
+                    p.divV[q] = div;
+                    p.txx[q] = txx[k];
+                    p.tyy[q] = tyy[k];
+                }
+                // the gravity term of compute_ResY (:189-202), from the old velocities
+                const double av = 0.25 * (vx1 + vx1r + vx2 + vx2r);
+                sterm[k] = g_y * (rho[k] - dt * (av * gx[k] * 0.5 * _dx + vy1r * gy[k] * 0.5 * _dy));
+                if (live) {
+                    sTxy[o] = txy[k];
+                    sPn[o] = P[k];
+                    sTxx[o] = txx[k];
+                    if (k == 0) sTyy[o] = tyy[k];   // (the other rows' are read by their thread alone)
+                }
+                vx0 = vx1;
+                vx1 = vx2;
+                vx1r = vx2r;
+                vy0r = vy1r;
             }
         }
         __syncthreads();
         // ---- stage 2: compute_dV!, compute_V! (:209-234), the boundary kernels (:53-56) ----
+        double txy01 = sTxy[o0 + 1];
 #pragma unroll
         for (int k = 0; k < K; ++k) {
-            const int o = off[k];
+            const int o = o0 + k * pitch;
+            const bool top = k + 1 == K;    // the point above is another thread's
+            const int up = top ? k : k + 1;
+            const double txy10 = top ? sTxy[o + pitch] : txy[up], tyy10 = top ? sTyy[o + pitch] : tyy[up];
+            const double P10 = top ? sPn[o + pitch] : P[up];
             const double txy11 = sTxy[o + pitch + 1];
-            const double Rx = (sTxx[o + 1] - sTxx[o]) * _dx + (txy11 - sTxy[o + 1]) * _dy - (sPn[o + 1] - P[k]) * _dx;
-            const double Ry = (sTyy[o + pitch] - sTyy[o]) * _dy + (txy11 - sTxy[o + pitch]) * _dx -
-                              (sPn[o + pitch] - P[k]) * _dy + sterm[k];
+            const double Rx = (sTxx[o + 1] - txx[k]) * _dx + (txy11 - txy01) * _dy - (sPn[o + 1] - P[k]) * _dx;
+            const double Ry = (tyy10 - tyy[k]) * _dy + (txy11 - txy10) * _dx - (P10 - P[k]) * _dy + sterm[k];
+            txy01 = txy11;
             dvx[k] = dampX * dvx[k] + Rx;
             dvy[k] = dampY * dvy[k] + Ry;
             // Vx(Nx-1) and Vy(Ny-1) are the zero entries of the boundary
@@ -343,19 +364,14 @@ __global__ void __launch_bounds__(512, 1) k_pt_resident(const __grid_constant__ 
         }
     }
 
-    // ---- tau, stage 1 of the last iteration.  tau_xy: the tile's points as new velocities see them, one further in x and
-    // y, and the domain's first column and row ----
-    if (p.txx) {
+    // ---- tau_xy of the last iteration: the tile's points as new velocities see them, one further in x and y, and the
+    // domain's first column and row ----
+    if (p.txy) {
 #pragma unroll
         for (int k = 0; k < K; ++k) {
-            const int o = off[k], b = o / pitch, a = o - b * pitch;
-            const int i = i0 + a, j = j0 + b;
-            const int64_t q = i + (int64_t)j * LD;
-            if (kind[k] & PT_OWN) {
-                p.txx[q] = sTxx[o];
-                p.tyy[q] = sTyy[o];
-            }
-            if (tid + k * NT < (W + 1) * (H + 1) && i < Nx && j < Ny && (a || !has_l) && (b || !has_b)) p.txy[q] = sTxy[o];
+            const int b = b0 + k, i = i0 + a, j = j0 + b;
+            if (live && b <= H && i < Nx && j < Ny && (a || !has_l) && (b || !has_b))
+                p.txy[i + (int64_t)j * LD] = sTxy[o0 + k * pitch];
         }
     }
     if (p.max_bits) {   // max|V| over the tile; the boundary entries are copies or zero
@@ -363,7 +379,7 @@ __global__ void __launch_bounds__(512, 1) k_pt_resident(const __grid_constant__ 
 #pragma unroll
         for (int k = 0; k < K; ++k) {
             if (!(kind[k] & PT_OWN)) continue;
-            const int o = off[k] + pitch + 1;
+            const int o = o0 + (k + 1) * pitch + 1;
             mx = max(mx, (unsigned long long)__double_as_longlong(fabs(sVx[o])));
             my = max(my, (unsigned long long)__double_as_longlong(fabs(sVy[o])));
         }
@@ -383,7 +399,7 @@ __global__ void __launch_bounds__(512, 1) k_pt_resident(const __grid_constant__ 
 #pragma unroll
     for (int k = 0; k < K; ++k) {
         if (!(kind[k] & PT_OWN)) continue;
-        const int o = off[k], b = o / pitch, a = o - b * pitch;
+        const int o = o0 + k * pitch, b = b0 + k;
         const int i = i0 + a, j = j0 + b;
         const int64_t q = i + (int64_t)j * LD;
         const double xn = sVx[o + pitch + 1], yn = sVy[o + pitch + 1];
@@ -419,13 +435,14 @@ constexpr int CLUSTER_PTS = 512;     // of a tile with its halo column and row: 
 constexpr int RES_SMEM = 200 * 1024;
 
 // the last array is one row longer: stage 2 reads a row above its points, those of the halo row too
-int smem_of(int W, int H, bool cluster) { return ((cluster ? 4 : 2) * (H + 2) + 4 * (H + 1) + 1) * (W + 2) * 8; }
+int smem_of(int W, int rows, bool cluster) { return ((cluster ? 4 : 2) * (rows + 1) + 4 * rows + 1) * (W + 2) * 8; }
 
-// threads and points per thread for n points of a tile; false if they do not fit
-bool threads_for(int64_t n, ResidentPlan& p) {
+// threads and points per thread of a tile; false if they do not fit
+bool threads_for(int64_t W, int64_t H, ResidentPlan& p) {
     for (p.k = 1; p.k <= RES_MAX_K; ++p.k) {
-        p.threads = (int)round_up(ceil_div(n, p.k), 32);
-        if (p.threads <= 512) return true;
+        const int64_t n = (W + 1) * (rows_of((int)H, p.k) / p.k);
+        p.threads = (int)round_up(n, 32);
+        if (n <= 512) return true;
     }
     return false;
 }
@@ -436,7 +453,7 @@ void set_tiles(ResidentPlan& p, int64_t cols, int64_t rows, int64_t W, int64_t H
     p.nty = (int)ceil_div(rows, H);
     p.W = (int)W;
     p.H = (int)H;
-    p.smem = smem_of(p.W, p.H, p.cluster);
+    p.smem = smem_of(p.W, rows_of(p.H, p.k), p.cluster);
 }
 
 // the largest cluster that the device places at all (one in a partition of the device may have fewer SMs together)
@@ -502,26 +519,32 @@ ResidentPlan cluster_plan(int64_t Nx, int64_t Ny, int device) {
 }
 
 // The exchange through L2: which grids, and how many tiles.  Up to 512 x 4 points per SM (registers: 22 per point) the
-// state fits, and is faster than the march wherever it does (3.5 against 5.8 us per iteration at 512^2, 1.65 against 4.3
+// state fits, and is faster than the march wherever it does (3.2 against 5.8 us per iteration at 500^2, 1.4 against 4.3
 // at 128^2).  One tile per 150 points: the exchange costs the same whatever the tiles' size, and smaller ones
 // compute faster until they no longer do (128^2: 1.67 us, with 450 points 2.02, with 100 1.70); a small grid still
-// leaves SMs to solves on other streams.
+// leaves SMs to solves on other streams.  The tiles' shape, by a cost fitted to measured ones (microseconds per iteration
+// of the one taken and of others): the points, idle threads included; a warp across the end of a tile's row meets bank
+// conflicts, which wide tiles have fewer of; spills with 4 points per thread; the border.  330^2: 47 x 16 points 2.01,
+// 37 x 21 2.07, 83 x 9 2.10, 16 x 47 (the fewest points) 2.24; 511 x 385: 43 x 32 2.61, 73 x 19 with 4 points per thread
+// 2.81; 300^2: 43 x 15 1.91, 25 x 25 1.96; 128^2: 16 x 10 1.40, 10 x 16 1.46.
 ResidentPlan resident_plan(int64_t Nx, int64_t Ny, int num_sms) {
     ResidentPlan best;
     const int64_t cols = Nx - 1, rows = Ny - 1, pts = cols * rows;
-    int64_t best_pts = 0;
+    double best_cost = 0.0;
     if (pts > (int64_t)num_sms * 512 * RES_MAX_K) return best;
     const int tiles = (int)std::min<int64_t>(num_sms, ceil_div(pts, 150));
     for (int ntx = 1; ntx <= tiles && ntx <= cols; ++ntx) {
         const int nty = (int)std::min<int64_t>(tiles / ntx, rows);
-        const int64_t W = ceil_div(cols, ntx), H = ceil_div(rows, nty), n = (W + 1) * (H + 1);
+        const int64_t W = ceil_div(cols, ntx), H = ceil_div(rows, nty);
         ResidentPlan p;
-        if (W < 2 || H < 2 || (best.fits && n >= best_pts) || !threads_for(n, p)) continue;
+        if (W < 2 || H < 2 || !threads_for(W, H, p)) continue;
+        const double cost = p.threads * p.k * (1.0 + 4.0 / (W + 1) + (p.k == RES_MAX_K ? 0.1 : 0.0)) + 3.2 * (W + H);
+        if (best.fits && cost >= best_cost) continue;
         set_tiles(p, cols, rows, W, H);
         const int regs = p.threads * 128;   // the launch bound
         p.share = regs <= 65536 / 4 && p.smem <= 50 * 1024 ? 1 : regs <= 65536 / 2 && p.smem <= 100 * 1024 ? 2 : 4;
         best = p;
-        best_pts = n;
+        best_cost = cost;
     }
     return best;
 }

@@ -22,7 +22,8 @@ pytestmark = pytest.mark.gpu
     (170, 40, 403, True), (6, 900, 62, False), (70, 5, 104, True), (1000, 5, 51, True), (1400, 4, 61, True),
     (4, 4, 60, True), (5, 9, 61, True), (9, 5, 62, False), (27, 31, 300, True), (28, 31, 301, True), (59, 22, 231, True),
     (61, 4, 61, True), (114, 31, 321, True), (20, 700, 260, True), (3000, 20, 230, True), (233, 129, 700, True),
-    (300, 301, 500, False), (511, 385, 94, True), (550, 552, 61, True),
+    (300, 301, 500, False), (330, 330, 97, True), (511, 385, 94, True), (521, 520, 65, True),
+    (522, 533, 61, True), (700, 400, 63, False), (550, 552, 61, True),
     # march
     (552, 551, 62, True), (58, 5400, 63, True), (59, 5400, 64, True), (60, 5300, 65, True), (5400, 60, 66, True),
     (20000, 17, 187, True), (801, 903, 94, False), (1023, 1101, 41, True)])
