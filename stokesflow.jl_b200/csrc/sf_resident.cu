@@ -9,8 +9,9 @@
 //     Vx, Vy and the stage-1 results of a tile (P, tau_xx, tau_yy, tau_xy) are in shared memory.  An iteration is the two stages of k_pt_iter, a barrier after each, and the exchange of the
 //     velocities on the tiles' borders, one of:
 //   * the tiles are the blocks of one cluster (up to 16): a thread stores a border point's velocities also into the
-//     neighbours' shared memory, and the second barrier is the cluster's.  The velocities are double-buffered: a
-//     neighbour's border may come in while the old ones are still read;
+//     neighbours' shared memory (st.async), counted there on an mbarrier that the neighbour waits for.  Velocities and
+//     mbarriers are double-buffered: a neighbour's border may come in while the old ones are still read, but it cannot
+//     be two iterations ahead;
 //   * through L2: every value travels in a 16-byte slot as two 8-byte words {half, tag}, the tag being the iteration's
 //     number, so that a reader that sees its tag has the value: one store and one load instead of data, fence and flag.
 //     Slots are double-buffered by parity; a tile cannot be two iterations ahead of one that it exchanges with, so a
@@ -20,8 +21,8 @@
 // A tile's halo column and row of P and tau are computed by both neighbours from the same values.  Every expression
 // keeps the reference's order of operations (compiled without contraction): bit-identical to single iterations.
 //
-// What bounds it: latency.  A cluster's iteration takes 0.62 us at 20 x 26 and about 0.8 at 64^2, the two stages'
-// dependent FP64 chains and the barriers; with the checks 1.1 and 1.1 us (k_pt_iter, one launch each: 4.5 and 4.4).
+// What bounds it: latency.  A cluster's iteration takes 0.67 us at 20 x 26 and 0.74 at 64^2, checks included
+// (k_pt_iter, one launch each: 4.5 and 4.4): the two stages' dependent FP64 chains, two barriers and the neighbours.
 // Through L2, 128^2 (110 tiles of 150 points, 8 warps) takes 1.5 us, about half of it the exchange, against 5.2; at
 // 511 x 385 (1450 points per SM) 2.6 us, there mostly issue slots, against 8.3.  Testing every point's flags and
 // sending borders to L2 from the update itself took 905 instructions per warp and iteration at 511 x 385 and 4.2 us.
@@ -62,8 +63,23 @@ __device__ __forceinline__ uint32_t in_block(const void* p, uint32_t rank) {
     asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
     return a;
 }
-__device__ __forceinline__ void put_in_block(uint32_t addr, double v) {
-    asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(addr), "d"(v) : "memory");
+// v to addr in another block of the cluster, counted (8 bytes) on the barrier bar of that block
+__device__ __forceinline__ void put_in_block(uint32_t addr, double v, uint32_t bar) {
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(addr),
+                 "l"(__double_as_longlong(v)), "r"(bar)
+                 : "memory");
+}
+// whether phase `parity` of the barrier is over, and with it what other blocks put here for it is seen
+__device__ __forceinline__ bool all_in(uint64_t* bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity)
+        : "memory");
+    return ok != 0;
 }
 // every thread of the cluster: earlier shared-memory writes, remote ones too, are seen by all afterwards
 __device__ __forceinline__ void cluster_sync() {
@@ -83,6 +99,7 @@ template <int K, bool CLUSTER>
 __global__ void __launch_bounds__(512, 1) k_pt_resident(const __grid_constant__ ResidentParams p) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ int gave_up;
+    __shared__ __align__(8) uint64_t bar[2];   // CLUSTER: halo entries come in, by parity of the iteration
     __shared__ unsigned long long max_v[2];
     if (p.err && !goes_on(p.err, p.eps)) return;   // (all blocks)
     const int W = p.W, H = p.H, pitch = W + 2;
@@ -190,23 +207,37 @@ __global__ void __launch_bounds__(512, 1) k_pt_resident(const __grid_constant__ 
     int to0 = -1, from0 = -1, peer0 = 0;
     // CLUSTER: where a border point's Vx goes in the neighbour to its left or right, in the one below or above, and (a
     // corner's Vx or Vy) in the diagonal one; 0: nowhere.  Vy lies behind Vx, the other pair of buffers `other` further
-    uint32_t at_x[K], at_y[K], at_d[K];
+    uint32_t at_x[K], at_y[K], at_d[K], bar_x[K], bar_y[K], bar_d[K];
     uint32_t other = (uint32_t)(2 * comp1 * 8);
+    // bytes that come in per iteration
+    const uint32_t expected = 8u * (2 * (has_l + has_r) * hv + 2 * (has_b + has_t) * wv + (has_l && has_t) + (has_r && has_b));
+    bool lost = false;
     if (CLUSTER) {
+        if (tid == 0) {
+            mbar_init(&bar[0], 1);
+            mbar_init(&bar[1], 1);
+            fence_mbar_init();
+        }
 #pragma unroll
         for (int k = 0; k < K; ++k) {
-            at_x[k] = at_y[k] = at_d[k] = 0;
+            at_x[k] = at_y[k] = at_d[k] = bar_x[k] = bar_y[k] = bar_d[k] = 0;
             if (!(kind[k] & PT_OWN)) continue;
             const int b = b0 + k, t = blockIdx.x;
+            if ((a == 0 && has_l) || (a == W - 1 && has_r)) bar_x[k] = in_block(bar, a == 0 && has_l ? t - 1 : t + 1);
+            if ((b == 0 && has_b) || (b == H - 1 && has_t)) bar_y[k] = in_block(bar, b == 0 && has_b ? t - p.ntx : t + p.ntx);
             if (a == 0 && has_l) at_x[k] = in_block(sVx_n + (b + 1) * pitch + W + 1, t - 1);
             if (a == W - 1 && has_r) at_x[k] = in_block(sVx_n + (b + 1) * pitch, t + 1);
             if (b == 0 && has_b) at_y[k] = in_block(sVx_n + (H + 1) * pitch + a + 1, t - p.ntx);
             if (b == H - 1 && has_t) at_y[k] = in_block(sVx_n + a + 1, t + p.ntx);
             if (a == W - 1 && b == 0 && has_r && has_b) {
                 at_d[k] = in_block(sVx_n + (H + 1) * pitch, t + 1 - p.ntx);
+                bar_d[k] = in_block(bar, t + 1 - p.ntx);
                 kind[k] |= PT_DX;
             }
-            if (a == 0 && b == H - 1 && has_l && has_t) at_d[k] = in_block(sVy_n + W + 1, t - 1 + p.ntx);
+            if (a == 0 && b == H - 1 && has_l && has_t) {
+                at_d[k] = in_block(sVy_n + W + 1, t - 1 + p.ntx);
+                bar_d[k] = in_block(bar, t - 1 + p.ntx);
+            }
         }
         cluster_sync();
     } else {
@@ -218,6 +249,7 @@ __global__ void __launch_bounds__(512, 1) k_pt_resident(const __grid_constant__ 
     for (int it = 0; it < p.iters; ++it) {
         // ---- stage 1: compute_P_tau! (:140-169) on the tile and one more column and row.  Evaluated at every point
         // (outside the domain on whatever is there; nothing that is kept depends on it) ----
+        if (CLUSTER && tid == 0 && expected && it + 1 < p.iters) mbar_arrive_expect_tx(&bar[it & 1], expected);
         double sterm[K], txx[K], tyy[K], txy[K];
         {
             // (every entry once: points of a column share theirs)
@@ -294,15 +326,16 @@ __global__ void __launch_bounds__(512, 1) k_pt_resident(const __grid_constant__ 
                 if (kind[k] & PT_J1) sVx_n[o + 2 * pitch + 1] = xn;
             }
             if (CLUSTER && it + 1 < p.iters) {
+                const uint32_t q = (it & 1) * 8;
                 if (at_x[k]) {
-                    put_in_block(at_x[k], xn);
-                    put_in_block(at_x[k] + comp1 * 8, yn);
+                    put_in_block(at_x[k], xn, bar_x[k] + q);
+                    put_in_block(at_x[k] + comp1 * 8, yn, bar_x[k] + q);
                 }
                 if (at_y[k]) {
-                    put_in_block(at_y[k], xn);
-                    put_in_block(at_y[k] + comp1 * 8, yn);
+                    put_in_block(at_y[k], xn, bar_y[k] + q);
+                    put_in_block(at_y[k] + comp1 * 8, yn, bar_y[k] + q);
                 }
-                if (at_d[k]) put_in_block(at_d[k], (kind[k] & PT_DX) ? xn : yn);
+                if (at_d[k]) put_in_block(at_d[k], (kind[k] & PT_DX) ? xn : yn, bar_d[k] + q);
                 at_x[k] = at_x[k] ? at_x[k] - other : 0;
                 at_y[k] = at_y[k] ? at_y[k] - other : 0;
                 at_d[k] = at_d[k] ? at_d[k] - other : 0;
@@ -322,10 +355,17 @@ __global__ void __launch_bounds__(512, 1) k_pt_resident(const __grid_constant__ 
             t = sVy;
             sVy = sVy_n;
             sVy_n = t;
-            if (tiles == 1)
-                __syncthreads();
-            else
-                cluster_sync();
+            __syncthreads();
+            // the neighbours' entries (after a wait in vain: no more waits, and nothing of this launch is used).  Theirs of
+            // the iteration after the next cannot come before this tile has sent its own of the next.
+            if (expected && it + 1 < p.iters && !lost && !all_in(&bar[it & 1], (it >> 1) & 1)) {
+                const uint64_t t0 = global_timer_ns();
+                for (uint32_t q = 1; !all_in(&bar[it & 1], (it >> 1) & 1); ++q)
+                    if ((q & 63u) == 0u && global_timer_ns() - t0 > RES_WAIT_NS) {
+                        lost = true;
+                        break;
+                    }
+            }
             continue;
         }
         __syncthreads();
@@ -364,6 +404,10 @@ __global__ void __launch_bounds__(512, 1) k_pt_resident(const __grid_constant__ 
         }
     }
 
+    if (CLUSTER) {
+        if (lost) atomicExch(p.err_flag, 1);
+        cluster_sync();   // (no block leaves while others might still write to it)
+    }
     // ---- tau_xy of the last iteration: the tile's points as new velocities see them, one further in x and y, and the
     // domain's first column and row ----
     if (p.txy) {
@@ -427,12 +471,15 @@ __global__ void __launch_bounds__(512, 1) k_pt_resident(const __grid_constant__ 
 }
 
 typedef void (*ResKernel)(const ResidentParams);
-const ResKernel kKernels[RES_MAX_K + 1] = {k_pt_resident<1, true>, k_pt_resident<1, false>, k_pt_resident<2, false>,
-                                           k_pt_resident<3, false>, k_pt_resident<4, false>};
-const ResKernel kCluster = kKernels[0];
+const ResKernel kKernels[] = {k_pt_resident<1, false>, k_pt_resident<2, false>, k_pt_resident<3, false>,
+                              k_pt_resident<4, false>, k_pt_resident<1, true>,  k_pt_resident<2, true>};
+constexpr int RES_KERNELS = sizeof(kKernels) / sizeof(kKernels[0]);
+int kernel_of(const ResidentPlan& p) { return p.k - 1 + (p.cluster ? RES_MAX_K : 0); }
+constexpr int CLUSTER_MAX_K = 2;
 constexpr int CLUSTER_MAX = 16;
-constexpr int CLUSTER_PTS = 512;     // of a tile with its halo column and row: a thread each
+constexpr int CLUSTER_PTS = 800;     // of a tile with its halo column and row
 constexpr int RES_SMEM = 200 * 1024;
+constexpr int CLUSTER_SMEM = 72 * 1024;   // more than any tile of CLUSTER_PTS points takes
 
 // the last array is one row longer: stage 2 reads a row above its points, those of the halo row too
 int smem_of(int W, int rows, bool cluster) { return ((cluster ? 4 : 2) * (rows + 1) + 4 * rows + 1) * (W + 2) * 8; }
@@ -445,6 +492,15 @@ bool threads_for(int64_t W, int64_t H, ResidentPlan& p) {
         if (n <= 512) return true;
     }
     return false;
+}
+
+// What a tile takes, for the choice of its shape; fitted to measured ones (microseconds per iteration of the one taken and
+// of others, exchange through L2): its points, idle threads included; a warp across the end of a tile's row meets bank
+// conflicts, which wide tiles have fewer of; spills with 4 points per thread; the border.  330^2: 47 x 16 points 2.01,
+// 37 x 21 2.07, 83 x 9 2.10, 16 x 47 (the fewest points) 2.24; 511 x 385: 43 x 32 2.61, 73 x 19 with 4 points per thread
+// 2.81; 300^2: 43 x 15 1.91, 25 x 25 1.96; 128^2: 16 x 10 1.40, 10 x 16 1.46.
+double tile_cost(int64_t W, int64_t H, const ResidentPlan& p) {
+    return p.threads * p.k * (1.0 + 4.0 / (W + 1) + (p.k == RES_MAX_K ? 0.1 : 0.0)) + 3.2 * (W + H);
 }
 
 void set_tiles(ResidentPlan& p, int64_t cols, int64_t rows, int64_t W, int64_t H) {
@@ -464,10 +520,14 @@ int cluster_limit(int device) {
     int& have = limit[device & 63];
     if (have) return have;
     have = 1;
-    if (cudaFuncSetAttribute((const void*)kCluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
-        cudaGetLastError();
-        return have;
-    }
+    for (int k = 0; k < CLUSTER_MAX_K; ++k)
+        if (cudaFuncSetAttribute((const void*)kKernels[RES_MAX_K + k], cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
+                cudaSuccess ||
+            cudaFuncSetAttribute((const void*)kKernels[RES_MAX_K + k], cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 RES_SMEM) != cudaSuccess) {
+            cudaGetLastError();
+            return have;
+        }
     for (int c = CLUSTER_MAX; c > 1 && have == 1; c /= 2) {
         cudaLaunchAttribute attr[1];
         attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -475,12 +535,12 @@ int cluster_limit(int device) {
         attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3((unsigned)c);
-        cfg.blockDim = dim3(CLUSTER_PTS);
-        cfg.dynamicSmemBytes = 44 * 1024;   // more than any tile of CLUSTER_PTS points takes
+        cfg.blockDim = dim3(512);
+        cfg.dynamicSmemBytes = CLUSTER_SMEM;
         cfg.attrs = attr;
         cfg.numAttrs = 1;
         int n = 0;
-        if (cudaOccupancyMaxActiveClusters(&n, kCluster, &cfg) == cudaSuccess && n > 0)
+        if (cudaOccupancyMaxActiveClusters(&n, kKernels[RES_MAX_K + CLUSTER_MAX_K - 1], &cfg) == cudaSuccess && n > 0)
             have = c;
         else
             cudaGetLastError();
@@ -490,30 +550,34 @@ int cluster_limit(int device) {
 
 }  // namespace
 
-// The tiles as one cluster, for grids of which 16 tiles hold at most 512 points each, halo column and row included (up to
-// about 84^2).  Writing a border into the neighbour's shared memory and one cluster barrier take less than the exchange
-// through L2 and its two block barriers; beyond, 16 SMs compute for longer than that gains.  Microseconds per iteration,
-// checks included, against the exchange through L2: 20 x 26 1.12 : 1.60 (with one tile that needs no exchange 1.40),
-// 40^2 0.98 : 1.61, 64^2 1.09 : 1.52, 84^2 1.25 : 1.58, 114 x 31 1.09 : 1.65, 170 x 40 1.53 : 1.70; 100^2 with two
-// points per thread or 832 threads 1.68 : 1.63.  Tiles of 32 points (a warp or two): the barrier costs the same for 2
-// and 16 blocks, and a block's barrier less with fewer warps (20 x 26, kernel alone: 0.90 us with one block, 0.78 with
-// two, 0.70 with four, 0.64 with eight, 0.61 with sixteen).
+// The tiles as one cluster, for grids of which 16 tiles hold at most 800 points each, halo column and row included (up to
+// about 108^2).  Writing a border into the neighbour's shared memory takes less than a store to L2 and a load from it;
+// beyond, 16 SMs compute for longer than that gains.  Microseconds per iteration, checks included, against the exchange
+// through L2: 20 x 26 0.67 : 1.60 (with one tile that needs no exchange 1.40), 40^2 0.64 : 1.61, 64^2 0.74 : 1.52, 84^2
+// 1.00 : 1.46, 100^2 1.22 : 1.39, 108^2 1.35 : 1.39, 120^2 (992 points) 1.39 : 1.38, 128^2 1.79 : 1.38; 170 x 40 1.18 :
+// 1.70, 250 x 50 (850 points) 1.61 : 1.51.  With a cluster barrier per iteration instead of counted stores: 20 x 26 0.90,
+// 64^2 1.03, 84^2 1.22 (the barrier waits for every earlier write of a thread, and for all blocks instead of the
+// neighbours).  Tiles of 32 points: a block's barrier takes less with fewer warps (20 x 26, kernel alone, with cluster
+// barriers: 0.90 us with one block, 0.78 with two, 0.70 with four, 0.64 with eight, 0.61 with sixteen).
 ResidentPlan cluster_plan(int64_t Nx, int64_t Ny, int device) {
     ResidentPlan best;
     const int64_t cols = Nx - 1, rows = Ny - 1, pts = cols * rows;
     const int most = cluster_limit(device);
     int tiles = 1;
     while (tiles < most && pts > (int64_t)tiles * 32) tiles *= 2;
-    int64_t best_pts = CLUSTER_PTS + 1;
+    double best_cost = 0.0;
     for (; tiles >= 1 && !best.fits; tiles /= 2)   // (fewer only where a thin grid does not split so far)
         for (int ntx = 1; ntx <= tiles; ntx *= 2) {
-            const int64_t W = ceil_div(cols, ntx), H = ceil_div(rows, tiles / ntx), n = (W + 1) * (H + 1);
-            if (W < 2 || H < 2 || ceil_div(cols, W) != ntx || ceil_div(rows, H) != tiles / ntx || n >= best_pts) continue;
-            best.cluster = true;
-            best.k = 1;
-            best.threads = (int)round_up(n, 32);
-            set_tiles(best, cols, rows, W, H);
-            best_pts = n;
+            const int64_t W = ceil_div(cols, ntx), H = ceil_div(rows, tiles / ntx);
+            ResidentPlan p;
+            if (W < 2 || H < 2 || ceil_div(cols, W) != ntx || ceil_div(rows, H) != tiles / ntx || !threads_for(W, H, p))
+                continue;
+            const double cost = tile_cost(W, H, p);
+            if ((W + 1) * rows_of((int)H, p.k) > CLUSTER_PTS || (best.fits && cost >= best_cost)) continue;
+            p.cluster = true;
+            set_tiles(p, cols, rows, W, H);
+            best = p;
+            best_cost = cost;
         }
     return best;
 }
@@ -522,11 +586,7 @@ ResidentPlan cluster_plan(int64_t Nx, int64_t Ny, int device) {
 // state fits, and is faster than the march wherever it does (3.2 against 5.8 us per iteration at 500^2, 1.4 against 4.3
 // at 128^2).  One tile per 150 points: the exchange costs the same whatever the tiles' size, and smaller ones
 // compute faster until they no longer do (128^2: 1.67 us, with 450 points 2.02, with 100 1.70); a small grid still
-// leaves SMs to solves on other streams.  The tiles' shape, by a cost fitted to measured ones (microseconds per iteration
-// of the one taken and of others): the points, idle threads included; a warp across the end of a tile's row meets bank
-// conflicts, which wide tiles have fewer of; spills with 4 points per thread; the border.  330^2: 47 x 16 points 2.01,
-// 37 x 21 2.07, 83 x 9 2.10, 16 x 47 (the fewest points) 2.24; 511 x 385: 43 x 32 2.61, 73 x 19 with 4 points per thread
-// 2.81; 300^2: 43 x 15 1.91, 25 x 25 1.96; 128^2: 16 x 10 1.40, 10 x 16 1.46.
+// leaves SMs to solves on other streams.
 ResidentPlan resident_plan(int64_t Nx, int64_t Ny, int num_sms) {
     ResidentPlan best;
     const int64_t cols = Nx - 1, rows = Ny - 1, pts = cols * rows;
@@ -538,7 +598,7 @@ ResidentPlan resident_plan(int64_t Nx, int64_t Ny, int num_sms) {
         const int64_t W = ceil_div(cols, ntx), H = ceil_div(rows, nty);
         ResidentPlan p;
         if (W < 2 || H < 2 || !threads_for(W, H, p)) continue;
-        const double cost = p.threads * p.k * (1.0 + 4.0 / (W + 1) + (p.k == RES_MAX_K ? 0.1 : 0.0)) + 3.2 * (W + H);
+        const double cost = tile_cost(W, H, p);
         if (best.fits && cost >= best_cost) continue;
         set_tiles(p, cols, rows, W, H);
         const int regs = p.threads * 128;   // the launch bound
@@ -602,8 +662,8 @@ int resident_launch(sf_ctx* ctx, ResidentParams& p, const ResidentPlan& plan, cu
     p.nty = plan.nty;
     p.W = plan.W;
     p.H = plan.H;
-    const int which = plan.cluster ? 0 : plan.k;
-    static bool ready[64][RES_MAX_K + 1] = {};
+    const int which = kernel_of(plan);
+    static bool ready[64][RES_KERNELS] = {};
     if (!ready[ctx->device & 63][which]) {
         SF_CUDA(cudaFuncSetAttribute((const void*)kKernels[which], cudaFuncAttributeMaxDynamicSharedMemorySize, RES_SMEM));
         ready[ctx->device & 63][which] = true;

@@ -19,6 +19,7 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("Nx,Ny,iters,stab", [
     # resident
     (7, 6, 61, True), (10, 9, 93, False), (4, 61, 61, True), (18, 33, 185, True), (85, 85, 851, True), (86, 86, 861, True),
+    (100, 101, 501, True), (109, 108, 545, False), (110, 111, 551, True), (200, 50, 251, True), (9, 800, 91, True),
     (170, 40, 403, True), (6, 900, 62, False), (70, 5, 104, True), (1000, 5, 51, True), (1400, 4, 61, True),
     (4, 4, 60, True), (5, 9, 61, True), (9, 5, 62, False), (27, 31, 300, True), (28, 31, 301, True), (59, 22, 231, True),
     (61, 4, 61, True), (114, 31, 321, True), (20, 700, 260, True), (3000, 20, 230, True), (233, 129, 700, True),
