@@ -158,10 +158,11 @@ typedef struct {
     int32_t converged;       /* err <= eps                                                             */
     int32_t reserved;
     double loop_ms;          /* device time of the whole iteration loop                                */
-    double bytes_per_iter;   /* essential HBM bytes of one fused PT iteration: 8*[2*(|Vx_s|+|Vy_s|+|P|+  */
+    double bytes_per_iter;   /* essential bytes of one PT iteration by itself: 8*[2*(|Vx_s|+|Vy_s|+|P|+  */
                              /* |dVx|+|dVy|) + |rho_vy|+|mu_b|+|mu_p|], about 104*Nx*Ny                */
-    double T_eff_essential;  /* bytes_per_iter * iters / loop time, GB/s                               */
-    int64_t fused_launches;  /* launches of the fused PT iteration kernel                              */
+    double T_eff_essential;  /* bytes_per_iter * iters / loop time, GB/s; above the HBM bandwidth where  */
+                             /* several iterations share a pass over memory                             */
+    int64_t fused_launches;  /* launches of PT iteration kernels (one or several iterations each)      */
     double fused_ms;         /* device time of the fused launches alone (0 unless timing requested)    */
 } sf_solve_info;
 

@@ -642,15 +642,22 @@ void ResidentRoom::release() {
     device_ = -1;
 }
 
+int resident_scratch(sf_ctx* ctx, const ResidentPlan& plan, cudaStream_t s) {
+    if (plan.cluster) return SF_OK;
+    const size_t bytes = (size_t)2 * plan.ntx * plan.nty * slots_of(plan.W, plan.H) * sizeof(ulonglong2);
+    if (bytes <= ctx->halo.bytes) return SF_OK;
+    int rc = ensure(ctx, ctx->halo, bytes);
+    if (rc) return rc;
+    SF_CUDA(cudaMemsetAsync(ctx->halo.ptr, 0, ctx->halo.bytes, s));
+    ctx->halo_tag = 1;
+    return SF_OK;
+}
+
 int resident_launch(sf_ctx* ctx, ResidentParams& p, const ResidentPlan& plan, cudaStream_t s) {
     const int tiles = plan.ntx * plan.nty;
     if (!plan.cluster) {
-        const size_t bytes = (size_t)2 * tiles * slots_of(plan.W, plan.H) * sizeof(ulonglong2);
         // tags of earlier launches stay in the slots: new memory, and a wrap of the counter, start from zeroed slots
-        const bool fresh = bytes > ctx->halo.bytes, wrap = ctx->halo_tag > 0xffffffffu - (uint32_t)p.iters - 1u;
-        int rc = ensure(ctx, ctx->halo, bytes);
-        if (rc) return rc;
-        if (fresh || wrap) {
+        if (ctx->halo_tag > 0xffffffffu - (uint32_t)p.iters - 1u) {
             SF_CUDA(cudaMemsetAsync(ctx->halo.ptr, 0, ctx->halo.bytes, s));
             ctx->halo_tag = 1;
         }

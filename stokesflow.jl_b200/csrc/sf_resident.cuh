@@ -65,6 +65,8 @@ class ResidentRoom {
 
 ResidentPlan cluster_plan(int64_t Nx, int64_t Ny, int device);
 ResidentPlan resident_plan(int64_t Nx, int64_t Ny, int num_sms);
+// the memory that a plan's tiles exchange through; before the launches
+int resident_scratch(sf_ctx* ctx, const ResidentPlan& plan, cudaStream_t s);
 // p.iters iterations; the tiles and the exchange's slots of p are set here
 int resident_launch(sf_ctx* ctx, ResidentParams& p, const ResidentPlan& plan, cudaStream_t s);
 

@@ -67,10 +67,20 @@ enum {
 };
 static_assert(F_VXB == MARCH_Z_B && F_RHO == MARCH_Z_MAT && F_MUP == MARCH_NZ, "slab order");
 
+// The compact layout, of solves by single iterations: the rates in place (a tile's are read and written by its block
+// alone), and none of what only the march and the resident kernel read (-1).
+constexpr int COMPACT_AT[F_NUM] = {0, 1, 2, 3, 4, 5, 6, 7, 3, 4, 8, 9, -1, -1, -1, -1, 10, 11, 12, 13, 14, 15, 16};
+constexpr int COMPACT_NUM = 17;
+
 struct Layout {
     int64_t Nx, Ny, LD, rows, fstride;   // rows of a field; the slabs are two rows longer (skew)
     double* base;
-    double* f(int k) const { return base + (int64_t)k * fstride + (k < MARCH_NZ ? MARCH_SKEW[k] * LD : 0); }
+    bool compact;
+    double* f(int k) const {
+        if (compact) return COMPACT_AT[k] < 0 ? nullptr : base + COMPACT_AT[k] * fstride;
+        return base + (int64_t)k * fstride + (k < MARCH_NZ ? MARCH_SKEW[k] * LD : 0);
+    }
+    size_t bytes() const { return (size_t)fstride * 8 * (compact ? COMPACT_NUM : F_NUM); }
 };
 
 struct PTParams {
@@ -717,13 +727,14 @@ struct Solver {
             if (!rc) rc = encode_tmap_f64(&maps[c].dvy, L.f(c ? F_DVYB : F_DVYA), LD, R, BX, BY);
             if (rc) return rc;
         }
-        // all slabs as one 3-D tensor (the slab is z)
-        int rc3 = encode_tiled(&march_maps.state, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 8, L.base, LD, R + 2, MARCH_NZ,
-                               L.fstride, MARCH_CW, 1, MARCH_Z_B - MARCH_Z_A);
-        if (!rc3)
-            rc3 = encode_tiled(&march_maps.mat, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 8, L.base, LD, R + 2, MARCH_NZ,
-                               L.fstride, MARCH_CW, 1, MARCH_NZ - MARCH_Z_MAT);
-        if (rc3) return rc3;
+        if (!L.compact) {   // all slabs as one 3-D tensor (the slab is z)
+            int rc = encode_tiled(&march_maps.state, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 8, L.base, LD, R + 2, MARCH_NZ,
+                                  L.fstride, MARCH_CW, 1, MARCH_Z_B - MARCH_Z_A);
+            if (!rc)
+                rc = encode_tiled(&march_maps.mat, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 8, L.base, LD, R + 2, MARCH_NZ,
+                                  L.fstride, MARCH_CW, 1, MARCH_NZ - MARCH_Z_MAT);
+            if (rc) return rc;
+        }
         static bool attr_set = false;
         if (!attr_set) {
             SF_CUDA(cudaFuncSetAttribute(k_pt_iter<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
@@ -845,7 +856,8 @@ struct SolveArgs {
 
 // Layout, scratch, pack, compute_timesteps! and kernel parameters of one (local) grid of Nx x Ny points.
 // nx_g, ny_g are the global grid sizes the reference's constants use (nx_g(), ny_g(): :20-22): the local
-// ones on a single domain.
+// ones on a single domain.  march: for several iterations per launch, unless only the compact layout finds memory
+// (17 fields of the grid's size instead of 23).
 static int solver_prepare(Solver& S, sf_ctx* ctx, cudaStream_t s, const SolveArgs& A, int64_t Nx, int64_t Ny,
                           double g_y, double dx, double dy, double dt, double maxdisp, int use_stab, int64_t nx_g,
                           int64_t ny_g, bool march) {
@@ -857,9 +869,16 @@ static int solver_prepare(Solver& S, sf_ctx* ctx, cudaStream_t s, const SolveArg
     S.L.LD = round_up(Nx + 2, 32);
     S.L.rows = Ny + 3;
     S.L.fstride = S.L.LD * (S.L.rows + 2);
-    size_t fbytes = (size_t)S.L.fstride * 8 * F_NUM;
-    bool fresh = fbytes > ctx->fields.bytes;
-    if ((rc = ensure(ctx, ctx->fields, fbytes))) return rc;
+    S.L.compact = !march;
+    bool fresh = S.L.bytes() > ctx->fields.bytes;
+    rc = ensure(ctx, ctx->fields, S.L.bytes());
+    if (rc == SF_ERR_OOM && march) {
+        S.L.compact = true;
+        march = false;
+        fresh = true;
+        rc = ensure(ctx, ctx->fields, S.L.bytes());
+    }
+    if (rc) return rc;
     S.L.base = (double*)ctx->fields.ptr;
     if (fresh) SF_CUDA(cudaMemsetAsync(ctx->fields.ptr, 0, ctx->fields.bytes, s));
     S.res_blocks = (int)std::min<int64_t>(ceil_div((Nx - 1) * (Ny - 1), RES_THREADS), (int64_t)ctx->num_sms * 8);
@@ -1240,11 +1259,12 @@ int sf_solve_stokes(sf_ctx* ctx, double* P, double* Vx_pad, double* Vy_pad, cons
     // ---- PT loop (:43-77) ----
     ResidentRoom room;
     bool resident = false;
-    if (iter_max >= RESIDENT_MIN_ITERS) {
+    if (iter_max >= RESIDENT_MIN_ITERS && !S.L.compact) {
         S.plan = cluster_plan(Nx, Ny, ctx->device);
         if (!(resident = room.acquire(ctx->device, ctx->num_sms, S.plan, s))) {
             S.plan = resident_plan(Nx, Ny, ctx->num_sms);
-            resident = room.acquire(ctx->device, ctx->num_sms, S.plan, s);
+            resident = S.plan.fits && resident_scratch(ctx, S.plan, s) == SF_OK &&
+                       room.acquire(ctx->device, ctx->num_sms, S.plan, s);
         }
     }
     double err = 2.0 * eps;
@@ -1275,11 +1295,11 @@ int sf_solve_stokes(sf_ctx* ctx, double* P, double* Vx_pad, double* Vy_pad, cons
                 it += n - 1;
                 maxima = use_stab && it == last && it % ncheck == 0;
                 if ((rc = S.launch_resident((int)n, it == last, maxima, cond_err, eps))) return rc;
-            } else if (it < last) {
+            } else if (it < last && !S.L.compact) {
                 const int T = (int)std::min<int64_t>(march_t, std::min(stop, last - 1) - it + 1);
                 if ((rc = S.launch_march(T))) return rc;
                 it += T - 1;
-            } else if ((rc = S.launch_iter(true))) {
+            } else if ((rc = S.launch_iter(it == last))) {
                 return rc;
             }
             ++fused;

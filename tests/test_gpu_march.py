@@ -78,6 +78,37 @@ def test_resident_stops_where_the_loop_does(sf, oracle_lib, Nx, Ny, bad):
             assert np.array_equal(b[k], a[k], equal_nan=True), f"{k} differs from the oracle"
 
 
+def test_solve_where_only_the_compact_layout_fits(sf):
+    """Memory for 17 fields of the grid's size but not for 23: single iterations, the same results."""
+    import torch
+
+    Nx, Ny, iters = 1500, 1100, 25
+    dx, dy = 1.0 / (Nx - 1), 1.0 / (Ny - 1)
+    rho, mu_b, mu_p = random_fields(Nx, Ny, seed=11, contrast=5.0)
+    shape = dict(P=(Nx - 1, Ny - 1), Vx=(Nx + 2, Ny + 1), Vy=(Nx + 1, Ny + 2), dVxdt=(Nx - 2, Ny - 1),
+                 dVydt=(Nx - 1, Ny - 2), Vx_s=(Nx, Ny + 1), Vy_s=(Nx + 1, Ny))
+    par, res = [dev(rho), dev(mu_b), dev(mu_p)], []
+    held = None
+    for short in (False, True):
+        t, ctx = {k: sf.zeros(*v) for k, v in shape.items()}, sf.Context(0)
+        if short:
+            torch.cuda.synchronize()
+            torch.cuda.empty_cache()
+            field = ((Nx + 2 + 31) // 32 * 32) * (Ny + 5) * 8
+            held = torch.empty(torch.cuda.mem_get_info()[0] - 20 * field, dtype=torch.uint8, device="cuda")
+        sf.solve_stokes_info(t["P"], t["Vx"], t["Vy"], *par, *[None] * 7, t["dVxdt"], t["dVydt"], None, None, t["Vx_s"],
+                             t["Vy_s"], 9.81, dx, dy, Nx, Ny, 1e-3, 0.5, eps=1e-300, iter_max=iters, ctx=ctx)
+        scratch = ctx.scratch_bytes()
+        del held
+        held = None
+        res.append(({k: host(v) for k, v in t.items()}, scratch))
+        ctx = None
+        torch.cuda.empty_cache()
+    assert res[1][1] < 0.8 * res[0][1]
+    for k in shape:
+        assert np.array_equal(res[0][0][k], res[1][0][k]), f"{k} differs"
+
+
 def test_concurrent_solves_bitexact(sf, oracle_lib):
     """Solves of several threads at once, contexts and streams of their own, more of them than the device has room for
     resident tiles (the rest marches), some of them small enough for a cluster: each equals the oracle."""
