@@ -6,8 +6,8 @@
 //   * the grid is cut into at most one tile per SM; a thread owns the same points in every iteration and keeps their
 //     P, rates and parameters in registers: up to four, one above the other, which share what they read (at 511 x 385
 //     17 accesses to shared memory per point and iteration; points of their own 25, and 2.82 us instead of 2.60).
-//     Vx, Vy and the stage-1 results of a tile (P, tau_xx, tau_yy, tau_xy) are in shared memory.  An iteration is the two stages of k_pt_iter, a barrier after each, and the exchange of the
-//     velocities on the tiles' borders, one of:
+//     Vx, Vy and the stage-1 results of a tile (P, tau_xx, tau_yy, tau_xy) are in shared memory.  An iteration is the
+//     two stages of k_pt_iter, a barrier after each, and the exchange of the velocities on the tiles' borders, one of:
 //   * the tiles are the blocks of one cluster (up to 16): a thread stores a border point's velocities also into the
 //     neighbours' shared memory (st.async), counted there on an mbarrier that the neighbour waits for.  Velocities and
 //     mbarriers are double-buffered: a neighbour's border may come in while the old ones are still read, but it cannot
@@ -23,8 +23,8 @@
 //
 // What bounds it: latency.  A cluster's iteration takes 0.67 us at 20 x 26 and 0.74 at 64^2, checks included
 // (k_pt_iter, one launch each: 4.5 and 4.4): the two stages' dependent FP64 chains, two barriers and the neighbours.
-// Through L2, 128^2 (110 tiles of 150 points, 8 warps) takes 1.5 us, about half of it the exchange, against 5.2; at
-// 511 x 385 (1450 points per SM) 2.6 us, there mostly issue slots, against 8.3.  Testing every point's flags and
+// Through L2, 128^2 (104 tiles of 16 x 10 points, 6 warps) takes 1.4 us, about half of it the exchange, against 5.2; at
+// 511 x 385 (1450 points per SM) 2.6 us, there barriers and shared memory (16 warps, issue 40%), against 8.3.  Testing every point's flags and
 // sending borders to L2 from the update itself took 905 instructions per warp and iteration at 511 x 385 and 4.2 us.
 #include <algorithm>
 #include <mutex>
