@@ -601,8 +601,8 @@ ResidentPlan resident_plan(int64_t Nx, int64_t Ny, int num_sms) {
         const double cost = tile_cost(W, H, p);
         if (best.fits && cost >= best_cost) continue;
         set_tiles(p, cols, rows, W, H);
-        const int regs = p.threads * 128;   // the launch bound
-        p.share = regs <= 65536 / 4 && p.smem <= 50 * 1024 ? 1 : regs <= 65536 / 2 && p.smem <= 100 * 1024 ? 2 : 4;
+        // (128 registers, the launch bound)
+        p.share = (int)std::min<int64_t>(4, std::max(ceil_div(p.threads * 128, 65536 / 4), ceil_div(p.smem, 50 * 1024)));
         best = p;
         best_cost = cost;
     }
@@ -613,33 +613,51 @@ namespace {
 std::mutex g_room_mutex;
 int g_room_used[64] = {};       // quarters of SMs held by solves that exchange through L2, by device
 int g_room_clusters[64] = {};   // solves that use a cluster, by device
+int g_room_solves[64] = {};     // solves, by device
 }
 
-bool ResidentRoom::acquire(int device, int num_sms, const ResidentPlan& plan, cudaStream_t s) {
-    if (!plan.fits || device < 0 || device >= 64 || device_ >= 0) return false;
-    const int need = plan.cluster ? 0 : plan.ntx * plan.nty * plan.share;
+ResidentRoom::ResidentRoom(int device, int num_sms, cudaStream_t s)
+    : device_(device), num_sms_(num_sms), stream_(s) {
+    std::lock_guard<std::mutex> lock(g_room_mutex);
+    if (known()) ++g_room_solves[device_];
+}
+
+ResidentRoom::~ResidentRoom() {
+    release();
+    std::lock_guard<std::mutex> lock(g_room_mutex);
+    if (known()) --g_room_solves[device_];
+}
+
+bool ResidentRoom::alone() const {
+    std::lock_guard<std::mutex> lock(g_room_mutex);
+    return known() && g_room_solves[device_] == 1;
+}
+
+bool ResidentRoom::acquire(const ResidentPlan& plan) {
+    if (!plan.fits || !known() || held_ || cluster_) return false;
+    const int need = plan.ntx * plan.nty * plan.share;
     std::lock_guard<std::mutex> lock(g_room_mutex);
     if (plan.cluster) {
-        if (g_room_used[device]) return false;
-        ++g_room_clusters[device];
-    } else {
-        if (g_room_clusters[device] || g_room_used[device] + need > 4 * num_sms) return false;
-        g_room_used[device] += need;
+        if (g_room_used[device_]) return false;
+        ++g_room_clusters[device_];
+        cluster_ = true;
+        return true;
     }
-    device_ = device;
+    const int most = plan.share == 4 && g_room_solves[device_] == 1 ? 4 : 3;
+    if (g_room_clusters[device_] || plan.share > most || g_room_used[device_] + need > most * num_sms_) return false;
+    g_room_used[device_] += need;
     held_ = need;
-    cluster_ = plan.cluster;
-    stream_ = s;
     return true;
 }
 
 void ResidentRoom::release() {
-    if (device_ < 0) return;
+    if (!held_ && !cluster_) return;
     cudaStreamSynchronize(stream_);   // nothing of the solve runs any more
     std::lock_guard<std::mutex> lock(g_room_mutex);
     g_room_used[device_] -= held_;
     g_room_clusters[device_] -= cluster_;
-    device_ = -1;
+    held_ = 0;
+    cluster_ = false;
 }
 
 int resident_scratch(sf_ctx* ctx, const ResidentPlan& plan, cudaStream_t s) {

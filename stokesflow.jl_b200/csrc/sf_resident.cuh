@@ -10,7 +10,9 @@
 namespace sf {
 
 constexpr int RESIDENT_MIN_ITERS = 4;       // fewer are faster by the march
-constexpr int RESIDENT_MAX_ITERS = 20000;   // of one launch
+// iterations of one launch; of tiles that take a whole SM fewer, since kernels on other streams wait for its end (1.5 ms;
+// a launch's load and store are 0.5% of that)
+constexpr int RESIDENT_MAX_ITERS = 20000, RESIDENT_MAX_ITERS_WHOLE = 512;
 
 struct ResidentParams {
     // the state that is read, the state that is written (other buffers) and the parameters, all in the padded layout
@@ -41,26 +43,33 @@ struct ResidentPlan {
     bool fits = false;           // the grid is small enough
     bool cluster = false;        // the tiles are one thread-block cluster
     int ntx = 0, nty = 0, W = 0, H = 0, k = 0, threads = 0, smem = 0;
-    int share = 0;               // quarters of an SM that a tile takes: 1, 2 or 4
+    int share = 0;               // quarters of an SM that a tile takes: 1 to 4
+    int max_iters() const { return share == 4 ? RESIDENT_MAX_ITERS_WHOLE : RESIDENT_MAX_ITERS; }
 };
 
 // Room on a device for the tiles of a plan, held while a solve uses it.  The tiles of a launch wait for one another, so
 // all must become resident whatever else runs: concurrent solves (other threads, streams and contexts) hold at most
-// four quarters of every SM together.  Then a tile of one quarter always finds a place (an SM without one holds four
-// quarters already, and not all SMs can); its launch ends; and what is left of two and four quarters finds its place
-// in turn.  A cluster is placed whole or not at all and needs no such room, but one that waits for a free group of SMs
+// three quarters of every SM together.  Then a tile of one or two quarters always finds a place (an SM without one
+// holds two quarters or three already, and not all SMs can); its launch ends; and what is left of three quarters finds its
+// place in turn.  The last quarter stays free for kernels that are not resident: a solve that marches beside them waits
+// for no launch of theirs.  A plan of whole SMs is for a solve that is alone on the device, and gives way when another
+// one begins: a march of 64^2 would wait up to a launch of 511 x 385 at every step.
+// A cluster is placed whole or not at all and needs no such room, but one that waits for a free group of SMs
 // could stand before tiles that others wait for: clusters and tiles that exchange through L2 do not run together.
 // A solve that gets no room marches instead (same results).
 class ResidentRoom {
    public:
-    ~ResidentRoom() { release(); }
-    bool acquire(int device, int num_sms, const ResidentPlan& plan, cudaStream_t s);
+    ResidentRoom(int device, int num_sms, cudaStream_t s);   // for the duration of a solve
+    ~ResidentRoom();
+    bool acquire(const ResidentPlan& plan);
     void release();
+    bool alone() const;   // no other solve on the device
 
    private:
-    int device_ = -1, held_ = 0;
+    bool known() const { return device_ >= 0 && device_ < 64; }
+    int device_, num_sms_, held_ = 0;
     bool cluster_ = false;
-    cudaStream_t stream_ = nullptr;
+    cudaStream_t stream_;
 };
 
 ResidentPlan cluster_plan(int64_t Nx, int64_t Ny, int device);

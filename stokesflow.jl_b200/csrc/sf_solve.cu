@@ -1257,14 +1257,13 @@ int sf_solve_stokes(sf_ctx* ctx, double* P, double* Vx_pad, double* Vy_pad, cons
     const int64_t ndtupdate = 10 * mnxy;                       // :36
 
     // ---- PT loop (:43-77) ----
-    ResidentRoom room;
+    ResidentRoom room(ctx->device, ctx->num_sms, s);
     bool resident = false;
     if (iter_max >= RESIDENT_MIN_ITERS && !S.L.compact) {
         S.plan = cluster_plan(Nx, Ny, ctx->device);
-        if (!(resident = room.acquire(ctx->device, ctx->num_sms, S.plan, s))) {
+        if (!(resident = room.acquire(S.plan))) {
             S.plan = resident_plan(Nx, Ny, ctx->num_sms);
-            resident = S.plan.fits && resident_scratch(ctx, S.plan, s) == SF_OK &&
-                       room.acquire(ctx->device, ctx->num_sms, S.plan, s);
+            resident = S.plan.fits && resident_scratch(ctx, S.plan, s) == SF_OK && room.acquire(S.plan);
         }
     }
     double err = 2.0 * eps;
@@ -1291,7 +1290,7 @@ int sf_solve_stokes(sf_ctx* ctx, double* P, double* Vx_pad, double* Vy_pad, cons
             if (use_stab) stop = std::min(stop, ((it - 1) / ndtupdate + 1) * ndtupdate);
             if (it < itert1) stop = std::min(stop, itert1 - 1);
             if (resident && stop - it + 1 >= RESIDENT_MIN_ITERS) {
-                const int64_t n = std::min<int64_t>(stop - it + 1, RESIDENT_MAX_ITERS);
+                const int64_t n = std::min<int64_t>(stop - it + 1, S.plan.max_iters());
                 it += n - 1;
                 maxima = use_stab && it == last && it % ncheck == 0;
                 if ((rc = S.launch_resident((int)n, it == last, maxima, cond_err, eps))) return rc;
@@ -1322,6 +1321,10 @@ int sf_solve_stokes(sf_ctx* ctx, double* P, double* Vx_pad, double* Vy_pad, cons
     while (err > eps && iter <= iter_max) {
         // iterations up to and including the next check (or iter_max)
         const int64_t last = std::min(((iter - 1) / ncheck + 1) * ncheck, iter_max);
+        if (resident && S.plan.share == 4 && !room.alone()) {
+            room.release();
+            resident = false;
+        }
         if (launched < last) {
             if ((rc = iterations(iter, last, false))) return rc;
             launched = last;
@@ -1331,7 +1334,7 @@ int sf_solve_stokes(sf_ctx* ctx, double* P, double* Vx_pad, double* Vy_pad, cons
             // Those up to the next check go behind this one if they are one resident launch: the device decides (goes_on),
             // and does not wait for the host to read err and launch: 20 x 26 1.00 -> 0.90 us per iteration, 64^2 1.05 -> 1.03.
             const int64_t next = std::min(last + ncheck, iter_max);
-            if (next - last <= RESIDENT_MAX_ITERS && (!use_stab || last / ndtupdate == (next - 1) / ndtupdate) &&
+            if (next - last <= S.plan.max_iters() && (!use_stab || last / ndtupdate == (next - 1) / ndtupdate) &&
                 last >= itert1) {
                 if ((rc = iterations(last + 1, next, true))) return rc;
                 launched = next;
