@@ -77,6 +77,12 @@ int sf_get_warnings(sf_ctx* ctx, sf_warnings* out, int reset);
  * and the context stays usable.  Synchronises the context's work stream. */
 int sf_selftest_bounded_wait(sf_ctx* ctx, int arrive, int64_t budget_ns, int32_t* timed_out);
 
+/* Self-test of the waits of resident tiles for one another (sf_solve_stokes on small grids): in the next solve of ctx
+ * that launches such tiles, the first launch goes without its last tile, whose neighbours give up after budget_ns
+ * (1 .. 2e9; tiles of a cluster: the launch counts as given up).  That solve begins again without resident tiles: the
+ * same results, SF_OK. */
+int sf_selftest_tile_wait(sf_ctx* ctx, int64_t budget_ns);
+
 /* ---------------------------------------------------------------------- */
 /* marker->grid deposit                                                     */
 /* ---------------------------------------------------------------------- */

@@ -262,7 +262,7 @@ int sf_ctx_create(int device, sf_ctx** out) {
     if (cudaGetDeviceProperties(&prop, device) == cudaSuccess) c->num_sms = prop.multiProcessorCount;
     if (cudaMalloc(&c->d_counters, sizeof(unsigned long long) * CNT_N) != cudaSuccess ||
         cudaMalloc(&c->d_scalars, sizeof(double) * SC_N) != cudaSuccess ||
-        cudaMalloc(&c->d_flags, sizeof(int) * 4) != cudaSuccess ||
+        cudaMalloc(&c->d_flags, sizeof(int) * FL_N) != cudaSuccess ||
         cudaMallocHost(&c->h_scalars, sizeof(double) * SC_N) != cudaSuccess ||
         cudaEventCreate(&c->ev_a) != cudaSuccess || cudaEventCreate(&c->ev_b) != cudaSuccess ||
         cudaEventCreate(&c->ev_c) != cudaSuccess ||
@@ -339,12 +339,20 @@ int sf_selftest_bounded_wait(sf_ctx* c, int arrive, int64_t budget_ns, int32_t* 
         return fail(SF_ERR_INVALID_ARG, "sf_selftest_bounded_wait: budget_ns must be in 1 .. 2e9");
     int rc = set_device(c);
     if (rc) return rc;
-    int* d = c->d_flags + 1;   // the second flag word: the solvers' copy-timeout flag stays untouched
+    int* d = c->d_flags + FL_SELFTEST;   // (the solvers' flags stay untouched)
     SF_CUDA(cudaMemsetAsync(d, 0, sizeof(int), c->work));
     k_wait_selftest<<<1, 128, 0, c->work>>>(arrive, (uint64_t)budget_ns, d);
     SF_LAUNCHED(c);
     SF_CUDA(cudaMemcpyAsync(timed_out, d, sizeof(int), cudaMemcpyDeviceToHost, c->work));
     SF_CUDA(cudaStreamSynchronize(c->work));
+    return SF_OK;
+}
+
+int sf_selftest_tile_wait(sf_ctx* c, int64_t budget_ns) {
+    if (!c) return fail(SF_ERR_INVALID_ARG, "sf_selftest_tile_wait: ctx is NULL");
+    if (budget_ns < 1 || budget_ns > 2000000000LL)
+        return fail(SF_ERR_INVALID_ARG, "sf_selftest_tile_wait: budget_ns must be in 1 .. 2e9");
+    c->tiles_fail_ns = budget_ns;
     return SF_OK;
 }
 

@@ -60,7 +60,14 @@ enum { CNT_BAD_MARKERS = 0, CNT_EMPTY_NODES = 1, CNT_INTERP_FAILSAFE = 2, CNT_OU
 // SC_TICKET: blocks of k_residuals that are done, zero between launches.
 enum { SC_DT = 0, SC_DT_CHECK = 1, SC_ERR = 2, SC_SUM_RX = 3, SC_SUM_RY = 4, SC_SUM_DIV = 5,
        SC_MAX_VX = 6, SC_MAX_VY = 7, SC_SCALE = 8, SC_DT_OUT = 9,
-       SC_ERR2 = 10 /* host: every other check's err */, SC_MAXBITS = 12, SC_TICKET = 14, SC_N = 16 };
+       SC_ERR2 = 10 /* host: every other check's err */, SC_WAITS = 11 /* host: WAIT_* bits */, SC_MAXBITS = 12, SC_TICKET = 14, SC_N = 16 };
+
+// d_flags: waits that gave up.  FL_COPY: for a tile copy; FL_SELFTEST; FL_TILES: of resident tiles for one another
+enum { FL_COPY = 0, FL_SELFTEST = 1, FL_TILES = 2, FL_N = 4 };
+enum { WAIT_COPY = 1, WAIT_TILES = 2 };   // the same as bits
+__host__ __device__ __forceinline__ int wait_bits(const volatile int* flags) {
+    return (flags[FL_COPY] ? WAIT_COPY : 0) | (flags[FL_TILES] ? WAIT_TILES : 0);
+}
 
 }  // namespace sf
 
@@ -82,7 +89,8 @@ struct sf_ctx {
     unsigned long long* d_counters = nullptr;
     double* d_scalars = nullptr;
     double* h_scalars = nullptr;  // pinned mirror
-    int* d_flags = nullptr;       // device error flags (int[4]); [0]: a bounded wait timed out
+    int* d_flags = nullptr;       // device error flags, int[FL_N]
+    int64_t tiles_fail_ns = 0;    // self-test: the next resident launch fails, its waits giving up after this (0: no)
     cudaEvent_t ev_a = nullptr, ev_b = nullptr, ev_c = nullptr;
     cudaEvent_t ev_check[2] = {};  // the PT loop's residual checks
     int64_t launches = 0;         // kernels launched through this context

@@ -101,7 +101,10 @@ __global__ void __launch_bounds__(512, 1) k_pt_resident(const __grid_constant__ 
     __shared__ int gave_up;
     __shared__ __align__(8) uint64_t bar[2];   // CLUSTER: halo entries come in, by parity of the iteration
     __shared__ unsigned long long max_v[2];
+    // An earlier launch's tiles were lost (a block that starts after one of this launch gave up may leave, too)
+    const int lost_before = *(const volatile int*)p.err_flag;
     if (p.err && !goes_on(p.err, p.eps)) return;   // (all blocks)
+    if (lost_before) return;
     const int W = p.W, H = p.H, pitch = W + 2;
     const int rows = rows_of(H, K);                               // of points that threads have
     const int comp1 = (rows + 1) * pitch;                         // from an entry of Vx to that of Vy
@@ -361,7 +364,7 @@ __global__ void __launch_bounds__(512, 1) k_pt_resident(const __grid_constant__ 
             if (expected && it + 1 < p.iters && !lost && !all_in(&bar[it & 1], (it >> 1) & 1)) {
                 const uint64_t t0 = global_timer_ns();
                 for (uint32_t q = 1; !all_in(&bar[it & 1], (it >> 1) & 1); ++q)
-                    if ((q & 63u) == 0u && global_timer_ns() - t0 > RES_WAIT_NS) {
+                    if ((q & 63u) == 0u && global_timer_ns() - t0 > p.wait_ns) {
                         lost = true;
                         break;
                     }
@@ -385,7 +388,7 @@ __global__ void __launch_bounds__(512, 1) k_pt_resident(const __grid_constant__ 
             if (!get(mine + n, tag, &v)) {
                 const uint64_t t0 = global_timer_ns();
                 for (uint32_t q = 1; !get(mine + n, tag, &v); ++q)
-                    if ((q & 63u) == 0u && global_timer_ns() - t0 > RES_WAIT_NS) {
+                    if ((q & 63u) == 0u && global_timer_ns() - t0 > p.wait_ns) {
                         gave_up = 1;
                         break;
                     }
@@ -693,9 +696,19 @@ int resident_launch(sf_ctx* ctx, ResidentParams& p, const ResidentPlan& plan, cu
         SF_CUDA(cudaFuncSetAttribute((const void*)kKernels[which], cudaFuncAttributeMaxDynamicSharedMemorySize, RES_SMEM));
         ready[ctx->device & 63][which] = true;
     }
+    p.wait_ns = RES_WAIT_NS;
+    int blocks = tiles;
+    if (ctx->tiles_fail_ns) {   // sf_selftest_tile_wait
+        p.wait_ns = (uint64_t)ctx->tiles_fail_ns;
+        ctx->tiles_fail_ns = 0;
+        if (plan.cluster)       // (a block is not sent to one that is not there)
+            SF_CUDA(cudaMemsetAsync(p.err_flag, 1, sizeof(int), s));
+        else
+            --blocks;           // nothing fills the neighbours' slots
+    }
     cudaLaunchAttribute attr[1];
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)tiles);
+    cfg.gridDim = dim3((unsigned)blocks);
     cfg.blockDim = dim3((unsigned)plan.threads);
     cfg.dynamicSmemBytes = (size_t)plan.smem;
     cfg.stream = s;
@@ -709,7 +722,13 @@ int resident_launch(sf_ctx* ctx, ResidentParams& p, const ResidentPlan& plan, cu
         attr[0].id = cudaLaunchAttributeCooperative;
         attr[0].val.cooperative = 1;
     }
-    SF_CUDA(cudaLaunchKernelEx(&cfg, kKernels[which], (const ResidentParams)p));
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kKernels[which], (const ResidentParams)p);
+    if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorLaunchOutOfResources || e == cudaErrorInvalidClusterSize ||
+        e == cudaErrorInvalidConfiguration) {
+        (void)cudaGetLastError();
+        return RESIDENT_LOST;
+    }
+    SF_CUDA(e);
     SF_LAUNCHED(ctx);
     return SF_OK;
 }

@@ -9,6 +9,7 @@
 
 namespace sf {
 
+constexpr int RESIDENT_LOST = -1;           // (no sf_status) the tiles could not run: march
 constexpr int RESIDENT_MIN_ITERS = 4;       // fewer are faster by the march
 // iterations of one launch; of tiles that take a whole SM fewer, since kernels on other streams wait for its end (1.5 ms;
 // a launch's load and store are 0.5% of that)
@@ -27,7 +28,8 @@ struct ResidentParams {
     int iters;
     uint32_t tag0;               // iteration k (0-based) publishes with tag tag0 + k
     ulonglong2* comm;            // received halo entries, [parity][tile][slot]
-    int* err_flag;
+    int* err_flag;               // set where a wait for another tile gave up; nothing is done where it is set already
+    uint64_t wait_ns;            // (set by resident_launch)
     // of the last iteration, where wanted: tau and divV (NULL: not), and max|Vx|, max|Vy| as bit patterns, accumulated
     // onto what is there (NULL: not)
     double *txx, *tyy, *txy, *divV;
@@ -56,7 +58,9 @@ struct ResidentPlan {
 // one begins: a march of 64^2 would wait up to a launch of 511 x 385 at every step.
 // A cluster is placed whole or not at all and needs no such room, but one that waits for a free group of SMs
 // could stand before tiles that others wait for: clusters and tiles that exchange through L2 do not run together.
-// A solve that gets no room marches instead (same results).
+// A solve that gets no room marches instead (same results).  The ledger is this process's: tiles of other processes
+// on the device (MPS) or a partition of it with fewer SMs are not in it.  There a launch may be refused, or a tile's wait
+// for another may run out (RESIDENT_LOST): the solve begins again and marches.
 class ResidentRoom {
    public:
     ResidentRoom(int device, int num_sms, cudaStream_t s);   // for the duration of a solve
@@ -76,7 +80,7 @@ ResidentPlan cluster_plan(int64_t Nx, int64_t Ny, int device);
 ResidentPlan resident_plan(int64_t Nx, int64_t Ny, int num_sms);
 // the memory that a plan's tiles exchange through; before the launches
 int resident_scratch(sf_ctx* ctx, const ResidentPlan& plan, cudaStream_t s);
-// p.iters iterations; the tiles and the exchange's slots of p are set here
+// p.iters iterations; the tiles and the exchange's slots of p are set here.  RESIDENT_LOST: the device did not take them
 int resident_launch(sf_ctx* ctx, ResidentParams& p, const ResidentPlan& plan, cudaStream_t s);
 
 }  // namespace sf

@@ -397,6 +397,8 @@ struct ResParams {
     double _dx, _dy, g_y;
     double* scalars;
     double* host_err;  // pinned host memory
+    const int* flags;  // where given, their wait_bits go to *host_waits (pinned) with err
+    double* host_waits;
     const double* err; // where given, nothing is done unless eps < *err < infinity
     double eps;
 };
@@ -462,6 +464,7 @@ __global__ void __launch_bounds__(RES_THREADS) k_residuals(const ResParams p) {
     __syncthreads();
     if (!last) return;
     __threadfence();
+    const int waits = (threadIdx.x == 0 && p.flags) ? wait_bits(p.flags) : 0;
     // the partials in 1024 strided sums, their warps' trees, and the tree of those 32
     double t[3];
 #pragma unroll
@@ -492,6 +495,7 @@ __global__ void __launch_bounds__(RES_THREADS) k_residuals(const ResParams p) {
         p.scalars[SC_SUM_DIV] = t[2];
         p.scalars[SC_ERR] = m;
         *p.host_err = m;
+        if (p.flags) *p.host_waits = (double)waits;
         if (p.max_bits) p.max_bits[0] = p.max_bits[1] = 0;
     }
 }
@@ -864,6 +868,7 @@ static int solver_prepare(Solver& S, sf_ctx* ctx, cudaStream_t s, const SolveArg
     int rc;
     S.ctx = ctx;
     S.s = s;
+    S.cur = 0;
     S.L.Nx = Nx;
     S.L.Ny = Ny;
     S.L.LD = round_up(Nx + 2, 32);
@@ -954,8 +959,9 @@ static int solver_prepare(Solver& S, sf_ctx* ctx, cudaStream_t s, const SolveArg
         pt.pow2 = (fr == 0.5) ? 1 : 0;
         pt.inv_max_nxy = pt.pow2 ? std::ldexp(1.0, 1 - e) : 0.0;
     }
-    pt.err_flag = ctx->d_flags;
-    SF_CUDA(cudaMemsetAsync(ctx->d_flags, 0, sizeof(int), s));
+    pt.err_flag = ctx->d_flags + FL_COPY;
+    SF_CUDA(cudaMemsetAsync(ctx->d_flags + FL_COPY, 0, sizeof(int), s));
+    SF_CUDA(cudaMemsetAsync(ctx->d_flags + FL_TILES, 0, sizeof(int), s));
     if ((rc = S.setup_maps())) return rc;
     for (int T = 1; march && T <= MARCH_MAX_T; ++T) {
         MarchParams& m = S.mp[T];
@@ -990,7 +996,7 @@ static int solver_prepare(Solver& S, sf_ctx* ctx, cudaStream_t s, const SolveArg
         r.g_y = g_y;
         r.dampX = dampX;
         r.dampY = dampY;
-        r.err_flag = pt.err_flag;
+        r.err_flag = ctx->d_flags + FL_TILES;
     }
     ResParams& rp = S.rp;
     rp.txx = S.L.f(F_TXX);
@@ -1002,6 +1008,8 @@ static int solver_prepare(Solver& S, sf_ctx* ctx, cudaStream_t s, const SolveArg
     rp.dx = dx;
     rp.dy = dy;
     rp.scalars = ctx->d_scalars;
+    rp.flags = nullptr;
+    rp.host_waits = nullptr;
     rp.Rx = S.L.f(F_RX);
     rp.Ry = S.L.f(F_RY);
     rp.partials = (double*)ctx->partials.ptr;
@@ -1206,72 +1214,50 @@ static int set_scalar_all(std::vector<Rank>& R, int slot, double v) {
     return SF_OK;
 }
 
-}  // namespace sf
+// what a solve's iterations end with
+struct PTLoop {
+    double err = 0.0;
+    int64_t niter = 0, nchecks = 0, fused = 0;   // iterations, checks, launches of iterations
+    bool have_t1 = false;                        // ev_a was recorded, at iteration `itert1`
+    static constexpr int64_t itert1 = 11;
+};
 
-using namespace sf;
-
-extern "C" {
-
-int sf_stokes_residual_scale(sf_ctx* ctx, const double* rho_vy, int64_t Nx, int64_t Ny, double g_y, void* stream,
-                             double* scale) {
-    SF_REQUIRE(ctx && rho_vy && scale, "sf_stokes_residual_scale: NULL argument");
-    SF_REQUIRE(Nx >= 3 && Ny >= 3, "sf_stokes_residual_scale: grid too small");
-    int rc = set_device(ctx);
-    if (rc) return rc;
-    cudaStream_t s = as_stream(stream);
-    int nb = (int)std::min<int64_t>(ceil_div((Nx - 1) * (Ny - 2), 256), 1024);
-    if ((rc = ensure(ctx, ctx->partials, (size_t)nb * 8))) return rc;
-    k_rho_scale<<<nb, 256, 0, s>>>(rho_vy, (int)Nx, (int)Ny, g_y, (double*)ctx->partials.ptr);
-    SF_LAUNCHED(ctx);
-    k_sum_partials<<<1, 1024, 0, s>>>((double*)ctx->partials.ptr, nb, (double)((Nx - 1) * (Ny - 2)),
-                                      ctx->d_scalars + SC_SCALE);
-    SF_LAUNCHED(ctx);
-    SF_CUDA(cudaMemcpyAsync(ctx->h_scalars + SC_SCALE, ctx->d_scalars + SC_SCALE, 8, cudaMemcpyDeviceToHost, s));
-    SF_CUDA(cudaStreamSynchronize(s));
-    *scale = ctx->h_scalars[SC_SCALE];
-    return SF_OK;
+// a wait of the loop's kernels gave up: for another tile (the solve can begin again without tiles), or for a tile copy
+static int waits_failed(int bits) {
+    if (bits & WAIT_COPY) return fail(SF_ERR_CUDA, "sf_solve_stokes: a tile copy into shared memory did not complete in time");
+    return RESIDENT_LOST;
 }
 
-int sf_solve_stokes(sf_ctx* ctx, double* P, double* Vx_pad, double* Vy_pad, const double* rho_vy, const double* mu_b,
-                    const double* mu_p, double* txx, double* tyy, double* txy, double* divV, double* dtPt, double* Rx,
-                    double* Ry, double* dVxdt, double* dVydt, double* dtVx, double* dtVy, double* Vx_s, double* Vy_s,
-                    double g_y, double dx, double dy, int64_t Nx, int64_t Ny, double dt, double maxdisp,
-                    int use_stab, double eps, int print_info, int64_t iter_max, void* stream, sf_solve_info* info) {
-    SF_REQUIRE(ctx, "sf_solve_stokes: ctx is NULL");
-    SF_REQUIRE(Nx >= 4 && Ny >= 4, "sf_solve_stokes: Nx, Ny must be >= 4");
-    SF_REQUIRE(Nx < (1 << 20) && Ny < (1 << 20), "sf_solve_stokes: Nx, Ny too large");
-    SF_REQUIRE(P && Vx_pad && Vy_pad && rho_vy && mu_b && mu_p && dVxdt && dVydt && Vx_s && Vy_s,
-               "sf_solve_stokes: a state / parameter array is NULL");
-    SF_REQUIRE(dx > 0.0 && dy > 0.0, "sf_solve_stokes: dx, dy must be positive");
-    int rc = set_device(ctx);
-    if (rc) return rc;
-    cudaStream_t s = as_stream(stream);
-
-    Solver S;
-    const SolveArgs A{P, Vx_pad, Vy_pad, rho_vy, mu_b, mu_p, txx, tyy, txy, divV, dtPt, Rx, Ry, dVxdt, dVydt,
-                      dtVx, dtVy, Vx_s, Vy_s};
-    if ((rc = solver_prepare(S, ctx, s, A, Nx, Ny, g_y, dx, dy, dt, maxdisp, use_stab, Nx, Ny, true)))
-        return rc;
+// The PT loop (:43-77).  tiles: small grids may stay on the chip.  RESIDENT_LOST: they could not; the state in the
+// solver's buffers is of no use, the caller's arrays are as they were.
+static int pt_loop(Solver& S, ResidentRoom& room, bool tiles, int64_t Nx, int64_t Ny, bool use_stab, double eps,
+                   int64_t iter_max, PTLoop& out) {
+    sf_ctx* const ctx = S.ctx;
+    cudaStream_t const s = S.s;
+    int rc;
+    out = PTLoop{};
+    double& err = out.err;
+    int64_t &niter = out.niter, &nchecks = out.nchecks, &fused = out.fused;
+    bool& have_t1 = out.have_t1;
+    constexpr int64_t itert1 = PTLoop::itert1;
+    S.rp.flags = ctx->d_flags;
+    S.rp.host_waits = ctx->h_scalars + SC_WAITS;
+    ctx->h_scalars[SC_WAITS] = 0.0;   // (nothing of an earlier solve runs any more)
     const int64_t mnxy = std::min(Nx, Ny);
     const int64_t ncheck = std::min<int64_t>(5 * mnxy, 2000);  // :35
     const int64_t ndtupdate = 10 * mnxy;                       // :36
 
-    // ---- PT loop (:43-77) ----
-    ResidentRoom room(ctx->device, ctx->num_sms, s);
     bool resident = false;
-    if (iter_max >= RESIDENT_MIN_ITERS && !S.L.compact) {
+    if (tiles && iter_max >= RESIDENT_MIN_ITERS && !S.L.compact) {
         S.plan = cluster_plan(Nx, Ny, ctx->device);
         if (!(resident = room.acquire(S.plan))) {
             S.plan = resident_plan(Nx, Ny, ctx->num_sms);
             resident = S.plan.fits && resident_scratch(ctx, S.plan, s) == SF_OK && room.acquire(S.plan);
         }
     }
-    double err = 2.0 * eps;
-    int64_t iter = 1, niter = 0, nchecks = 0;
-    const int64_t itert1 = 11;
+    err = 2.0 * eps;
+    int64_t iter = 1;
     const int march_t = march_iterations(Nx, Ny);
-    bool have_t1 = false;
-    int64_t fused = 0;
     SF_CUDA(cudaEventRecord(ctx->ev_c, s));
     // launches the iterations from `it` to `last`, the next check or iter_max, and the check; all of it on the condition
     // that the loop goes on after the check before, if cond
@@ -1317,6 +1303,7 @@ int sf_solve_stokes(sf_ctx* ctx, double* P, double* Vx_pad, double* Vy_pad, cons
         return (int)SF_OK;
     };
     int64_t launched = 0;   // iterations
+    bool seen = true;       // the waits of all launches
     int cur = S.cur;        // the buffer parity after the iterations that count
     while (err > eps && iter <= iter_max) {
         // iterations up to and including the next check (or iter_max)
@@ -1342,10 +1329,12 @@ int sf_solve_stokes(sf_ctx* ctx, double* P, double* Vx_pad, double* Vy_pad, cons
         }
         niter += last - iter + 1;
         iter = last + 1;
+        seen = last % ncheck == 0;
         if (last % ncheck == 0) {
             const int odd = (int)(last / ncheck & 1);
             ++nchecks;
             SF_CUDA(cudaEventSynchronize(ctx->ev_check[odd]));
+            if (ctx->h_scalars[SC_WAITS] != 0.0) return waits_failed((int)ctx->h_scalars[SC_WAITS]);
             err = ctx->h_scalars[odd ? SC_ERR2 : SC_ERR];
             if (!(err == err) || std::isinf(err)) break;
         }
@@ -1355,6 +1344,72 @@ int sf_solve_stokes(sf_ctx* ctx, double* P, double* Vx_pad, double* Vy_pad, cons
         --fused;
     }
     SF_CUDA(cudaEventRecord(ctx->ev_b, s));
+    if (!seen) {   // iterations after the last check
+        int flags[FL_N];
+        SF_CUDA(cudaMemcpyAsync(flags, ctx->d_flags, sizeof(flags), cudaMemcpyDeviceToHost, s));
+        SF_CUDA(cudaStreamSynchronize(s));
+        if (wait_bits(flags)) return waits_failed(wait_bits(flags));
+    }
+    return SF_OK;
+}
+
+}  // namespace sf
+
+using namespace sf;
+
+extern "C" {
+
+int sf_stokes_residual_scale(sf_ctx* ctx, const double* rho_vy, int64_t Nx, int64_t Ny, double g_y, void* stream,
+                             double* scale) {
+    SF_REQUIRE(ctx && rho_vy && scale, "sf_stokes_residual_scale: NULL argument");
+    SF_REQUIRE(Nx >= 3 && Ny >= 3, "sf_stokes_residual_scale: grid too small");
+    int rc = set_device(ctx);
+    if (rc) return rc;
+    cudaStream_t s = as_stream(stream);
+    int nb = (int)std::min<int64_t>(ceil_div((Nx - 1) * (Ny - 2), 256), 1024);
+    if ((rc = ensure(ctx, ctx->partials, (size_t)nb * 8))) return rc;
+    k_rho_scale<<<nb, 256, 0, s>>>(rho_vy, (int)Nx, (int)Ny, g_y, (double*)ctx->partials.ptr);
+    SF_LAUNCHED(ctx);
+    k_sum_partials<<<1, 1024, 0, s>>>((double*)ctx->partials.ptr, nb, (double)((Nx - 1) * (Ny - 2)),
+                                      ctx->d_scalars + SC_SCALE);
+    SF_LAUNCHED(ctx);
+    SF_CUDA(cudaMemcpyAsync(ctx->h_scalars + SC_SCALE, ctx->d_scalars + SC_SCALE, 8, cudaMemcpyDeviceToHost, s));
+    SF_CUDA(cudaStreamSynchronize(s));
+    *scale = ctx->h_scalars[SC_SCALE];
+    return SF_OK;
+}
+
+int sf_solve_stokes(sf_ctx* ctx, double* P, double* Vx_pad, double* Vy_pad, const double* rho_vy, const double* mu_b,
+                    const double* mu_p, double* txx, double* tyy, double* txy, double* divV, double* dtPt, double* Rx,
+                    double* Ry, double* dVxdt, double* dVydt, double* dtVx, double* dtVy, double* Vx_s, double* Vy_s,
+                    double g_y, double dx, double dy, int64_t Nx, int64_t Ny, double dt, double maxdisp,
+                    int use_stab, double eps, int print_info, int64_t iter_max, void* stream, sf_solve_info* info) {
+    SF_REQUIRE(ctx, "sf_solve_stokes: ctx is NULL");
+    SF_REQUIRE(Nx >= 4 && Ny >= 4, "sf_solve_stokes: Nx, Ny must be >= 4");
+    SF_REQUIRE(Nx < (1 << 20) && Ny < (1 << 20), "sf_solve_stokes: Nx, Ny too large");
+    SF_REQUIRE(P && Vx_pad && Vy_pad && rho_vy && mu_b && mu_p && dVxdt && dVydt && Vx_s && Vy_s,
+               "sf_solve_stokes: a state / parameter array is NULL");
+    SF_REQUIRE(dx > 0.0 && dy > 0.0, "sf_solve_stokes: dx, dy must be positive");
+    int rc = set_device(ctx);
+    if (rc) return rc;
+    cudaStream_t s = as_stream(stream);
+
+    Solver S;
+    const SolveArgs A{P, Vx_pad, Vy_pad, rho_vy, mu_b, mu_p, txx, tyy, txy, divV, dtPt, Rx, Ry, dVxdt, dVydt,
+                      dtVx, dtVy, Vx_s, Vy_s};
+    ResidentRoom room(ctx->device, ctx->num_sms, s);
+    PTLoop loop;
+    // Where tiles that wait for one another could not all run, once more without them, from the caller's arrays.
+    for (bool tiles = true;; tiles = false) {
+        if ((rc = solver_prepare(S, ctx, s, A, Nx, Ny, g_y, dx, dy, dt, maxdisp, use_stab, Nx, Ny, true))) return rc;
+        rc = pt_loop(S, room, tiles, Nx, Ny, use_stab != 0, eps, iter_max, loop);
+        if (rc != RESIDENT_LOST) break;
+        SF_CUDA(cudaStreamSynchronize(s));
+        room.release();
+    }
+    if (rc) return rc;
+    const double err = loop.err;
+    const int64_t niter = loop.niter, nchecks = loop.nchecks;
 
     // ---- unpack (:89-95) ----
     if ((rc = solver_unpack(S, A, niter, nchecks))) return rc;
@@ -1365,9 +1420,9 @@ int sf_solve_stokes(sf_ctx* ctx, double* P, double* Vx_pad, double* Vy_pad, cons
 
     float ms_loop = 0.f, ms_t1 = 0.f;
     SF_CUDA(cudaEventElapsedTime(&ms_loop, ctx->ev_c, ctx->ev_b));
-    if (have_t1) SF_CUDA(cudaEventElapsedTime(&ms_t1, ctx->ev_a, ctx->ev_b));
-    double runtime = have_t1 ? ms_t1 * 1e-3 : 0.0;
-    double t_it = (niter - itert1 + 1) > 0 ? runtime / (double)(niter - itert1 + 1) : 0.0;
+    if (loop.have_t1) SF_CUDA(cudaEventElapsedTime(&ms_t1, ctx->ev_a, ctx->ev_b));
+    double runtime = loop.have_t1 ? ms_t1 * 1e-3 : 0.0;
+    double t_it = (niter - PTLoop::itert1 + 1) > 0 ? runtime / (double)(niter - PTLoop::itert1 + 1) : 0.0;
     double A_eff = (3.0 * 2.0) / 1e9 * (double)Nx * (double)Ny * 8.0;
     double T_eff = t_it > 0 ? A_eff / t_it : 0.0;
     // essential bytes: read+write Vx_s, Vy_s, P, dVx, dVy; read rho, mu_b, mu_p
@@ -1389,12 +1444,9 @@ int sf_solve_stokes(sf_ctx* ctx, double* P, double* Vx_pad, double* Vy_pad, cons
         info->loop_ms = ms_loop;
         info->bytes_per_iter = bpi;
         info->T_eff_essential = ms_loop > 0 ? bpi * (double)niter / (ms_loop * 1e-3) / 1e9 : 0.0;
-        info->fused_launches = fused;
+        info->fused_launches = loop.fused;
         info->fused_ms = 0.0;
     }
-    int hflag = 0;
-    SF_CUDA(cudaMemcpy(&hflag, ctx->d_flags, sizeof(int), cudaMemcpyDeviceToHost));
-    if (hflag) return fail(SF_ERR_CUDA, "sf_solve_stokes: a tile copy into shared memory did not complete in time");
     if (!(err == err) || std::isinf(err)) return fail(SF_ERR_NONFINITE, "sf_solve_stokes: residual is not finite");
     return SF_OK;
 }

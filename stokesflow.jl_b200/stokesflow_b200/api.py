@@ -153,6 +153,12 @@ def selftest_bounded_wait(arrive: bool, budget_ns: int, *, ctx: Context | None =
     return bool(out.value)
 
 
+def selftest_tile_wait(budget_ns: int, *, ctx: Context | None = None) -> None:
+    """The next solve of ctx that launches resident tiles does so without the last one, and its neighbours' waits give
+    up after budget_ns: the solve begins again without resident tiles, with the same results."""
+    check(lib().sf_selftest_tile_wait(_ctx(ctx).handle, int(budget_ns)), "selftest_tile_wait")
+
+
 def bilinear_marker_to_grid(x_grid_min, y_grid_min, val_grid, x_m, y_m, val_m, dx, dy, val_wt_sum=None,
                             wt_sum=None, grid=None, *, ctx: Context | None = None, stream=None):
     """bilinearMarkerToGrid! (MarkerToGrid.jl:18-38): deposit val_m onto val_grid in place."""
