@@ -210,6 +210,7 @@ int sf_move_markers_rk4(sf_ctx* ctx, double* x_m, double* y_m, int64_t nm, const
     if (nm == 0) return SF_OK;
     int rc = set_device(ctx);
     if (rc) return rc;
+    markers_launched(ctx, ctx->device, nm);
     AdvectArgs a{Vx, Vy, vx_nx, vx_ny, vy_nx, vy_ny, x_vx_min, y_vx_min, x_vy_min, y_vy_min, dx, dy, 1.0 / dx, 1.0 / dy, 0};
     a.fast = div_const_takes(dx) && div_const_takes(dy) && vx_nx < INT32_MAX / 4 / vx_ny && vy_nx < INT32_MAX / 4 / vy_ny;
     unsigned blocks = (unsigned)std::min<int64_t>(ceil_div(nm, 256), (int64_t)ctx->num_sms * 16);

@@ -275,14 +275,16 @@ int sf_ctx_create(int device, sf_ctx** out) {
     }
     cudaMemset(c->d_counters, 0, sizeof(unsigned long long) * CNT_N);
     cudaMemset(c->d_scalars, 0, sizeof(double) * SC_N);
-    cudaMemset(c->d_flags, 0, sizeof(int) * 4);
+    cudaMemset(c->d_flags, 0, sizeof(int) * FL_N);
     SF_CUDA(cudaDeviceSynchronize());
+    room_add_context(c);
     *out = c;
     return SF_OK;
 }
 
 int sf_ctx_destroy(sf_ctx* c) {
     if (!c) return SF_OK;
+    room_remove_context(c);
     cudaSetDevice(c->device);
     cudaDeviceSynchronize();
     mixed_engine_release(c);

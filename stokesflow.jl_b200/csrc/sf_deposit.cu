@@ -799,6 +799,7 @@ int sf_bilinear_marker_to_grid(sf_ctx* ctx, double x_grid_min, double y_grid_min
     if (wt_sum) SF_REQUIRE(ld_sum >= nx && n_sum >= ld_sum * (ny - 1) + nx, "sf_bilinear_marker_to_grid: sum arrays too small");
     int rc = set_device(ctx);
     if (rc) return rc;
+    markers_launched(ctx, ctx->device, nm);
     cudaStream_t s = as_stream(stream);
     SortGrids sg{};
     sg.n = 1;
@@ -838,6 +839,7 @@ int sf_bilinear_marker_to_grids(sf_ctx* ctx, const sf_deposit_grid* grids, int n
     }
     int rc = set_device(ctx);
     if (rc) return rc;
+    markers_launched(ctx, ctx->device, nm);
     cudaStream_t s = as_stream(stream);
     SortGrids sg{};
     sg.n = n_grids;
@@ -868,6 +870,7 @@ int sf_rebin_markers(sf_ctx* ctx, const double* x_m, const double* y_m, int64_t 
     SF_REQUIRE(nm < (int64_t)INT32_MAX && (nx + 1) * (ny + 1) < (int64_t)INT32_MAX, "sf_rebin_markers: too large");
     int rc = set_device(ctx);
     if (rc) return rc;
+    markers_launched(ctx, ctx->device, nm);
     cudaStream_t s = as_stream(stream);
     SortGrids sg{};
     sg.n = 1;
@@ -933,7 +936,7 @@ static std::mutex g_noalloc_mutex;
 // is looked up once per device (with that device current) and cached, with
 // the SM count that sizes the marker kernels' grids.  A device reset
 // invalidates the cache (documented at the declaration).
-static int noalloc_scratch(unsigned char** out, int* num_sms) {
+static int noalloc_scratch(unsigned char** out, int* num_sms, int* device) {
     int dev = 0;
     SF_CUDA(cudaGetDevice(&dev));
     if (dev < 0 || dev >= NA_MAX_DEVICES) return fail(SF_ERR_NO_DEVICE, "noalloc deposit: device index too large");
@@ -951,6 +954,7 @@ static int noalloc_scratch(unsigned char** out, int* num_sms) {
         g_noalloc_ptr[dev] = (unsigned char*)p;
     }
     *out = g_noalloc_ptr[dev];
+    *device = dev;
     *num_sms = g_noalloc_sms[dev];
     return SF_OK;
 }
@@ -972,9 +976,10 @@ extern "C" int sf_bilinear_marker_to_grid_noalloc(double x_grid_min, double y_gr
                                           std::to_string(ny) + " grid exceeds the fixed scratch (at most " +
                                           std::to_string(NA_MAX_CELLS) + " cells (nx+1)*(ny+1))");
     unsigned char* base = nullptr;
-    int num_sms = 0;
-    int rc = noalloc_scratch(&base, &num_sms);
+    int num_sms = 0, device = 0;
+    int rc = noalloc_scratch(&base, &num_sms, &device);
     if (rc) return rc;
+    markers_launched(nullptr, device, nm);
     cudaStream_t s = as_stream(stream);
     unsigned long long* counters = (unsigned long long*)(base + NA_OFF_COUNTERS);
     const int64_t ncells = (nx + 1) * (ny + 1);

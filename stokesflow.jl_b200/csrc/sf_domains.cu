@@ -343,6 +343,7 @@ int sf_exchange_markers(sf_marker_rank* ranks, int32_t dims_x, int32_t dims_y, d
         sf_ctx* c = k.ctx;
         if ((rc = set_device(c))) break;
         SF_CUDA(cudaDeviceSynchronize());   // the caller's markers are complete
+        markers_launched(c, c->device, k.n);
         SF_CUDA(cudaEventCreateWithFlags(&w.ev, cudaEventDisableTiming));
         w.nblk = ceil_div(std::max<int64_t>(k.n, 1), (int64_t)XT * XITEMS);
         const size_t o_dir = 0, o_cnt = round_up(o_dir + (size_t)k.n + 1, 256);

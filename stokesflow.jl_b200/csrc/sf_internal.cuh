@@ -6,6 +6,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
 #include <cmath>
 #include <map>
 #include <utility>
@@ -94,6 +95,8 @@ struct sf_ctx {
     cudaEvent_t ev_a = nullptr, ev_b = nullptr, ev_c = nullptr;
     cudaEvent_t ev_check[2] = {};  // the PT loop's residual checks
     int64_t launches = 0;         // kernels launched through this context
+    // until when (steady clock, ns) marker kernels of this context are taken to run; other contexts' solves read it
+    std::atomic<int64_t> markers_until{0};
     sf_engine* batch_engine = nullptr;  // the engine sf_solve_stokes_batch_mixed reuses across calls
     // sweep shapes the engines' autotuner measured best, by workload class (sf_mixed.cu)
     std::map<int, int> sweep_shapes;
@@ -144,6 +147,12 @@ cudaError_t launch_overlapped(bool overlap, void (*kern)(Params...), dim3 grid, 
     cfg.numAttrs = overlap ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...);
 }
+
+// for the ledger of resident tiles (sf_resident.cuh): the contexts, and marker kernels over nm markers launched on a device
+// (ctx NULL: without a context)
+void room_add_context(const sf_ctx* ctx);
+void room_remove_context(const sf_ctx* ctx);
+void markers_launched(sf_ctx* ctx, int device, int64_t nm);
 
 inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 inline int64_t round_up(int64_t a, int64_t b) { return ceil_div(a, b) * b; }

@@ -40,11 +40,13 @@
 #include <deque>
 #include <iterator>
 #include <map>
+#include <memory>
 #include <string>
 #include <type_traits>
 #include <vector>
 
 #include "sf_internal.cuh"
+#include "sf_resident.cuh"
 #include "sf_tma.cuh"
 
 namespace sf {
@@ -979,6 +981,7 @@ struct sf_engine {
     cudaGraphExec_t march_gexec = nullptr;
     int march_graph_k = 0;
     cudaEvent_t ev_in = nullptr, ev_out = nullptr;
+    std::unique_ptr<OtherWork> at_work;  // while instances are admitted
     // the sweep candidate in use (shape, schedule, launch mode) and its tuner: the first round of a workload
     // class the context has not seen starts with short timed pieces of every candidate on the engine stream; the
     // candidate with the fewest ns per point-sweep is then used and recorded in the context for that class
@@ -1608,6 +1611,7 @@ int engine_submit(sf_engine* e, sf_batch_instance* u, cudaStream_t caller, int64
         return rc;
     }
     h.active = true;
+    if (!e->at_work) e->at_work.reset(new OtherWork(e->ctx->device));
     h.ticket = e->next_ticket++;
     ++e->submitted;
     if (ticket) *ticket = h.ticket;
@@ -1723,7 +1727,10 @@ int engine_round(sf_engine* e, cudaStream_t caller) {
         SF_CUDA(cudaEventRecord(e->ev_out, s));
         SF_CUDA(cudaStreamWaitEvent(caller, e->ev_out, 0));
     }
-    if (sweep.empty()) return SF_OK;
+    if (sweep.empty()) {
+        e->at_work.reset();
+        return SF_OK;
+    }
     // budgets: up to the next event of each instance, at most fold_every.  Events are counted from the start
     // of the current attempt (a restarted instance runs the schedule of a fresh solve); max_sweeps counts the
     // sweeps of every attempt.

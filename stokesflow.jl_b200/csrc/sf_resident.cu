@@ -27,7 +27,12 @@
 // 511 x 385 (1450 points per SM) 2.6 us, there barriers and shared memory (16 warps, issue 40%), against 8.3.  Testing every point's flags and
 // sending borders to L2 from the update itself took 905 instructions per warp and iteration at 511 x 385 and 4.2 us.
 #include <algorithm>
+#include <atomic>
+#include <chrono>
+#include <functional>
 #include <mutex>
+#include <thread>
+#include <vector>
 
 #include "sf_resident.cuh"
 #include "sf_tma.cuh"
@@ -613,14 +618,66 @@ ResidentPlan resident_plan(int64_t Nx, int64_t Ny, int num_sms) {
 }
 
 namespace {
+constexpr int ROOM_DEVICES = 64;
 std::mutex g_room_mutex;
-int g_room_used[64] = {};       // quarters of SMs held by solves that exchange through L2, by device
-int g_room_clusters[64] = {};   // solves that use a cluster, by device
-int g_room_solves[64] = {};     // solves, by device
+int g_room_used[ROOM_DEVICES] = {};       // quarters of SMs held by solves that exchange through L2, by device
+int g_room_clusters[ROOM_DEVICES] = {};   // solves that use a cluster
+int g_room_solves[ROOM_DEVICES] = {};     // plain solves
+int g_room_others[ROOM_DEVICES] = {};     // OtherWork
+std::vector<const sf_ctx*> g_room_contexts;
+// marker kernels without a context: until when, and the thread that launched them
+std::atomic<int64_t> g_noalloc_until[ROOM_DEVICES];
+std::atomic<size_t> g_noalloc_thread[ROOM_DEVICES];
+
+size_t this_thread() { return std::hash<std::thread::id>()(std::this_thread::get_id()); }
+
+int64_t now_ns() {
+    return std::chrono::duration_cast<std::chrono::nanoseconds>(std::chrono::steady_clock::now().time_since_epoch()).count();
 }
 
-ResidentRoom::ResidentRoom(int device, int num_sms, cudaStream_t s)
-    : device_(device), num_sms_(num_sms), stream_(s) {
+// (with the mutex) whether another context's marker kernels are under way
+bool markers_at_work(const sf_ctx* ctx, int device) {
+    const int64_t now = now_ns();
+    if (g_noalloc_until[device].load(std::memory_order_relaxed) > now &&
+        g_noalloc_thread[device].load(std::memory_order_relaxed) != this_thread())
+        return true;
+    for (const sf_ctx* c : g_room_contexts)
+        if (c != ctx && c->device == device && c->markers_until.load(std::memory_order_relaxed) > now) return true;
+    return false;
+}
+}  // namespace
+
+void room_add_context(const sf_ctx* ctx) {
+    std::lock_guard<std::mutex> lock(g_room_mutex);
+    g_room_contexts.push_back(ctx);
+}
+
+void room_remove_context(const sf_ctx* ctx) {
+    std::lock_guard<std::mutex> lock(g_room_mutex);
+    g_room_contexts.erase(std::remove(g_room_contexts.begin(), g_room_contexts.end(), ctx), g_room_contexts.end());
+}
+
+// Taken to last 10 ms and 0.2 ns per marker (three deposits 0.11, rebin and advection 0.06) from the call on: beside
+// whole-SM tiles they wait for the solve's next check first (up to 7 ms).
+void markers_launched(sf_ctx* ctx, int device, int64_t nm) {
+    if (device < 0 || device >= ROOM_DEVICES) return;
+    if (!ctx) g_noalloc_thread[device].store(this_thread(), std::memory_order_relaxed);
+    (ctx ? ctx->markers_until : g_noalloc_until[device]).store(now_ns() + 10000000 + nm / 5, std::memory_order_relaxed);
+}
+
+OtherWork::OtherWork(int device) : device_(device) {
+    std::lock_guard<std::mutex> lock(g_room_mutex);
+    if (device_ >= 0 && device_ < ROOM_DEVICES) ++g_room_others[device_];
+}
+
+OtherWork::~OtherWork() {
+    std::lock_guard<std::mutex> lock(g_room_mutex);
+    if (device_ >= 0 && device_ < ROOM_DEVICES) --g_room_others[device_];
+}
+
+bool ResidentRoom::known() const { return device_ >= 0 && device_ < ROOM_DEVICES; }
+
+ResidentRoom::ResidentRoom(const sf_ctx* ctx, cudaStream_t s) : ctx_(ctx), device_(ctx->device), stream_(s) {
     std::lock_guard<std::mutex> lock(g_room_mutex);
     if (known()) ++g_room_solves[device_];
 }
@@ -631,10 +688,13 @@ ResidentRoom::~ResidentRoom() {
     if (known()) --g_room_solves[device_];
 }
 
-bool ResidentRoom::alone() const {
+bool ResidentRoom::keeps(const ResidentPlan& plan) const {
+    if (plan.cluster) return true;
     std::lock_guard<std::mutex> lock(g_room_mutex);
-    return known() && g_room_solves[device_] == 1;
+    return g_room_others[device_] == 0 && (plan.share < 4 || whole_sms());
 }
+
+bool ResidentRoom::whole_sms() const { return g_room_solves[device_] == 1 && !markers_at_work(ctx_, device_); }
 
 bool ResidentRoom::acquire(const ResidentPlan& plan) {
     if (!plan.fits || !known() || held_ || cluster_) return false;
@@ -646,8 +706,10 @@ bool ResidentRoom::acquire(const ResidentPlan& plan) {
         cluster_ = true;
         return true;
     }
-    const int most = plan.share == 4 && g_room_solves[device_] == 1 ? 4 : 3;
-    if (g_room_clusters[device_] || plan.share > most || g_room_used[device_] + need > most * num_sms_) return false;
+    const int most = plan.share == 4 && whole_sms() ? 4 : 3;
+    if (g_room_clusters[device_] || g_room_others[device_] || plan.share > most ||
+        g_room_used[device_] + need > most * ctx_->num_sms)
+        return false;
     g_room_used[device_] += need;
     held_ = need;
     return true;

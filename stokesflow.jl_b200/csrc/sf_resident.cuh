@@ -53,9 +53,17 @@ struct ResidentPlan {
 // all must become resident whatever else runs: concurrent solves (other threads, streams and contexts) hold at most
 // three quarters of every SM together.  Then a tile of one or two quarters always finds a place (an SM without one
 // holds two quarters or three already, and not all SMs can); its launch ends; and what is left of three quarters finds its
-// place in turn.  The last quarter stays free for kernels that are not resident: a solve that marches beside them waits
-// for no launch of theirs.  A plan of whole SMs is for a solve that is alone on the device, and gives way when another
-// one begins: a march of 64^2 would wait up to a launch of 511 x 385 at every step.
+// place in turn.  The last quarter stays free for solves that march beside them and wait for no launch of theirs.  A plan
+// of whole SMs (222^2 - 257^2, 317^2 - 373^2, 387^2 - 529^2) is for a solve that is alone on the device: a march of 64^2
+// would wait up to a launch of 511 x 385 at every step.
+// Other work of this library comes first where it is known.  Beside an engine or batched solve under way, or a decomposed
+// one, no tiles are placed that exchange through L2: their sweeps fill the device, and a quarter of every SM is too little
+// (an engine's sweep takes 11.2 us beside 256^2 by single iterations, beside its tiles 67.7, beside its march 12.0; beside
+// 450^2 12.7, 103 and 13.0; beside 300^2, which takes three quarters, 11.4, 22.9 and 12.3).  Beside marker kernels that
+// another context has just launched no tiles of whole SMs are (three deposits of 128^2 beside 450^2: 331, 546 and 129 us; a
+// rebin of 0.6 M markers 137, 453 and 104): other tiles gain more than such short kernels lose.  A solve gives its tiles up,
+// or takes some, at a check.  A cluster has 16 SMs and leaves the others.  Kernels of other libraries are not known here;
+// they wait for a launch's end (1.5 ms for whole SMs).
 // A cluster is placed whole or not at all and needs no such room, but one that waits for a free group of SMs
 // could stand before tiles that others wait for: clusters and tiles that exchange through L2 do not run together.
 // A solve that gets no room marches instead (same results).  The ledger is this process's: tiles of other processes
@@ -63,17 +71,31 @@ struct ResidentPlan {
 // for another may run out (RESIDENT_LOST): the solve begins again and marches.
 class ResidentRoom {
    public:
-    ResidentRoom(int device, int num_sms, cudaStream_t s);   // for the duration of a solve
+    ResidentRoom(const sf_ctx* ctx, cudaStream_t s);   // for the duration of a solve
     ~ResidentRoom();
     bool acquire(const ResidentPlan& plan);
     void release();
-    bool alone() const;   // no other solve on the device
+    bool keeps(const ResidentPlan& plan) const;   // whether a solve that has room for the plan may go on using it
 
    private:
-    bool known() const { return device_ >= 0 && device_ < 64; }
-    int device_, num_sms_, held_ = 0;
+    bool known() const;
+    bool whole_sms() const;   // (with the ledger's lock) no other solve, no marker kernels
+    const sf_ctx* ctx_;
+    int device_, held_ = 0;
     bool cluster_ = false;
     cudaStream_t stream_;
+};
+
+// Announces work on a device that is neither a plain solve nor marker kernels, for as long as it lives.
+class OtherWork {
+   public:
+    explicit OtherWork(int device);
+    ~OtherWork();
+    OtherWork(const OtherWork&) = delete;
+    OtherWork& operator=(const OtherWork&) = delete;
+
+   private:
+    int device_;
 };
 
 ResidentPlan cluster_plan(int64_t Nx, int64_t Ny, int device);

@@ -50,6 +50,7 @@
 #include <cstdio>
 #include <cstring>
 #include <functional>
+#include <memory>
 #include <vector>
 
 #include "sf_internal.cuh"
@@ -1247,14 +1248,25 @@ static int pt_loop(Solver& S, ResidentRoom& room, bool tiles, int64_t Nx, int64_
     const int64_t ncheck = std::min<int64_t>(5 * mnxy, 2000);  // :35
     const int64_t ndtupdate = 10 * mnxy;                       // :36
 
-    bool resident = false;
+    // room for tiles: those of one cluster, or those that exchange through L2
+    ResidentPlan plans[2];
     if (tiles && iter_max >= RESIDENT_MIN_ITERS && !S.L.compact) {
-        S.plan = cluster_plan(Nx, Ny, ctx->device);
-        if (!(resident = room.acquire(S.plan))) {
-            S.plan = resident_plan(Nx, Ny, ctx->num_sms);
-            resident = S.plan.fits && resident_scratch(ctx, S.plan, s) == SF_OK && room.acquire(S.plan);
-        }
+        plans[0] = cluster_plan(Nx, Ny, ctx->device);
+        plans[1] = resident_plan(Nx, Ny, ctx->num_sms);
     }
+    auto take_room = [&]() {
+        for (ResidentPlan& p : plans) {
+            if (!room.acquire(p)) continue;
+            if (resident_scratch(ctx, p, s) == SF_OK) {
+                S.plan = p;
+                return true;
+            }
+            room.release();
+            p.fits = false;
+        }
+        return false;
+    };
+    bool resident = false;
     err = 2.0 * eps;
     int64_t iter = 1;
     const int march_t = march_iterations(Nx, Ny);
@@ -1308,9 +1320,11 @@ static int pt_loop(Solver& S, ResidentRoom& room, bool tiles, int64_t Nx, int64_
     while (err > eps && iter <= iter_max) {
         // iterations up to and including the next check (or iter_max)
         const int64_t last = std::min(((iter - 1) / ncheck + 1) * ncheck, iter_max);
-        if (resident && S.plan.share == 4 && !room.alone()) {
+        if (resident && !room.keeps(S.plan)) {
             room.release();
             resident = false;
+        } else if (!resident) {
+            resident = take_room();
         }
         if (launched < last) {
             if ((rc = iterations(iter, last, false))) return rc;
@@ -1397,7 +1411,7 @@ int sf_solve_stokes(sf_ctx* ctx, double* P, double* Vx_pad, double* Vy_pad, cons
     Solver S;
     const SolveArgs A{P, Vx_pad, Vy_pad, rho_vy, mu_b, mu_p, txx, tyy, txy, divV, dtPt, Rx, Ry, dVxdt, dVydt,
                       dtVx, dtVy, Vx_s, Vy_s};
-    ResidentRoom room(ctx->device, ctx->num_sms, s);
+    ResidentRoom room(ctx, s);
     PTLoop loop;
     // Where tiles that wait for one another could not all run, once more without them, from the caller's arrays.
     for (bool tiles = true;; tiles = false) {
@@ -1478,6 +1492,8 @@ int sf_solve_stokes_decomposed(sf_domain* domains, int32_t dims_x, int32_t dims_
     const int64_t ndtupdate = 10 * mnxy;                       // :36
     if (!use_stab) dt = 0.0;
 
+    std::vector<std::unique_ptr<OtherWork>> at_work;
+    for (int r = 0; r < nr; ++r) at_work.emplace_back(new OtherWork(domains[r].ctx->device));
     std::vector<Rank> R((size_t)nr);
     int rc;
     for (int r = 0; r < nr; ++r) {
