@@ -164,8 +164,11 @@ __global__ void k_cell_runs(const double* __restrict__ x, const double* __restri
 
 // 2. exclusive scan of the counts -> offsets, in tiles of SCAN_TILE cells: the tiles' sums, then every tile with the sum
 // of the tiles before it, which a block adds up itself (or, of more than SCAN_DIRECT tiles, finds scanned already).
-// The second pass also lists the long cells.
-constexpr int SCAN_THREADS = 1024, SCAN_ITEMS = 8, SCAN_TILE = SCAN_THREADS * SCAN_ITEMS, SCAN_DIRECT = 2048;
+// The second pass also lists the long cells.  Blocks of 256 threads find a place beside the resident tiles of a solve on
+// another stream, which leave a quarter of an SM; 1024 threads waited for a launch of those to end.  A rebin of 0.6 M
+// markers beside 180^2: 203 -> 137 - 164 us, beside 300^2 245 -> 193; by itself, with more blocks, 82 -> 75, three deposits of
+// 128^2 with the host's time 102 -> 95.
+constexpr int SCAN_THREADS = 256, SCAN_ITEMS = 8, SCAN_TILE = SCAN_THREADS * SCAN_ITEMS, SCAN_DIRECT = 4096;
 
 __device__ __forceinline__ int32_t block_exclusive_scan(int32_t v, int32_t* warp_sums, int32_t* total) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -912,7 +915,7 @@ namespace sf {
 
 constexpr int64_t NA_MAX_MARKERS = SF_NOALLOC_MAX_MARKERS;
 constexpr int64_t NA_MAX_CELLS = SF_NOALLOC_MAX_CELLS;          // (nx + 1) * (ny + 1)
-constexpr int64_t NA_SCAN_TILES = (NA_MAX_CELLS + 1 + 8191) / 8192;
+constexpr int64_t NA_SCAN_TILES = (NA_MAX_CELLS + SCAN_TILE - 1) / SCAN_TILE;
 // layout (bytes): keys | perm | offsets | counts | cursors | scan tiles | long cells | counters
 constexpr size_t NA_OFF_KEYS = 0;
 constexpr size_t NA_OFF_PERM = NA_OFF_KEYS + 4 * NA_MAX_MARKERS;
