@@ -98,6 +98,18 @@ int copy_block(sf_ctx* ctx, cudaStream_t s, double* dst, int64_t ld_dst, const d
     return SF_OK;
 }
 
+static size_t scratch_size(size_t bytes) { return (size_t)round_up((int64_t)bytes, 1 << 20); }
+
+bool may_have(const Scratch& s, size_t bytes) {
+    if (bytes <= s.bytes) return true;
+    size_t free_bytes = 0, total = 0;
+    if (cudaMemGetInfo(&free_bytes, &total) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return true;   // (the allocation will tell)
+    }
+    return scratch_size(bytes) <= free_bytes + s.bytes;
+}
+
 int ensure(sf_ctx* ctx, Scratch& s, size_t bytes) {
     if (bytes <= s.bytes) return SF_OK;
     (void)ctx;
@@ -106,7 +118,7 @@ int ensure(sf_ctx* ctx, Scratch& s, size_t bytes) {
         s.ptr = nullptr;
         s.bytes = 0;
     }
-    size_t want = (size_t)round_up((int64_t)bytes, 1 << 20);
+    size_t want = scratch_size(bytes);
     cudaError_t e = cudaMalloc(&s.ptr, want);
     if (e != cudaSuccess) {
         s.ptr = nullptr;

@@ -104,6 +104,8 @@ struct sf_ctx {
 
 namespace sf {
 
+// Whether the device has the memory for `s` to hold `bytes`, what `s` holds now among it.
+bool may_have(const Scratch& s, size_t bytes);
 // Ensures `s` holds at least `bytes`; contents are not preserved.
 int ensure(sf_ctx* ctx, Scratch& s, size_t bytes);
 int set_device(sf_ctx* ctx);

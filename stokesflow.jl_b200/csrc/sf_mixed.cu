@@ -1891,7 +1891,8 @@ extern "C" int sf_solve_stokes_batch_mixed(sf_ctx* ctx, sf_batch_instance* inst,
     e->opt = normalized(o);
     if ((rc = configure_tuner(e))) return rc;
     // where the device has no room for the rates' second buffers, the sweeps do without (one per launch)
-    e->rates_b = e->opt.tile_rows == 0 && ensure(ctx, ctx->mixed, (size_t)total[1]) == SF_OK;
+    e->rates_b = e->opt.tile_rows == 0 && may_have(ctx->mixed, (size_t)total[1]) &&
+                 ensure(ctx, ctx->mixed, (size_t)total[1]) == SF_OK;
     if (!e->rates_b && (rc = ensure(ctx, ctx->mixed, (size_t)total[0]))) return rc;
     e->arena = (unsigned char*)ctx->mixed.ptr;
     e->alloc.reset(total[e->rates_b ? 1 : 0]);

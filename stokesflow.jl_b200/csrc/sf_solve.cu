@@ -862,7 +862,8 @@ struct SolveArgs {
 // Layout, scratch, pack, compute_timesteps! and kernel parameters of one (local) grid of Nx x Ny points.
 // nx_g, ny_g are the global grid sizes the reference's constants use (nx_g(), ny_g(): :20-22): the local
 // ones on a single domain.  march: for several iterations per launch, unless only the compact layout finds memory
-// (17 fields of the grid's size instead of 23).
+// (17 fields of the grid's size instead of 23).  That is looked up first: freeing the fields of an earlier solve to find
+// that 23 do not fit stalls the device and leaves the 17 to whoever allocates in between.
 static int solver_prepare(Solver& S, sf_ctx* ctx, cudaStream_t s, const SolveArgs& A, int64_t Nx, int64_t Ny,
                           double g_y, double dx, double dy, double dt, double maxdisp, int use_stab, int64_t nx_g,
                           int64_t ny_g, bool march) {
@@ -876,6 +877,10 @@ static int solver_prepare(Solver& S, sf_ctx* ctx, cudaStream_t s, const SolveArg
     S.L.rows = Ny + 3;
     S.L.fstride = S.L.LD * (S.L.rows + 2);
     S.L.compact = !march;
+    if (march && !may_have(ctx->fields, S.L.bytes())) {
+        S.L.compact = true;
+        march = false;
+    }
     bool fresh = S.L.bytes() > ctx->fields.bytes;
     rc = ensure(ctx, ctx->fields, S.L.bytes());
     if (rc == SF_ERR_OOM && march) {
