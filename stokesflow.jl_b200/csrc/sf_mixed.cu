@@ -981,7 +981,7 @@ struct sf_engine {
     cudaGraphExec_t march_gexec = nullptr;
     int march_graph_k = 0;
     cudaEvent_t ev_in = nullptr, ev_out = nullptr;
-    std::unique_ptr<OtherWork> at_work;  // while instances are admitted
+    std::unique_ptr<OtherWork> at_work;  // from an instance's admission until there is none
     // the sweep candidate in use (shape, schedule, launch mode) and its tuner: the first round of a workload
     // class the context has not seen starts with short timed pieces of every candidate on the engine stream; the
     // candidate with the fewest ns per point-sweep is then used and recorded in the context for that class
@@ -1583,6 +1583,12 @@ int validate(const sf_batch_instance& u, const char* who) {
     return SF_OK;
 }
 
+int active_count(const sf_engine* e) {
+    int n = 0;
+    for (const Slot& h : e->slots) n += h.active ? 1 : 0;
+    return n;
+}
+
 int engine_submit(sf_engine* e, sf_batch_instance* u, cudaStream_t caller, int64_t* ticket) {
     int rc = validate(*u, "sf_engine_submit");
     if (rc) return rc;
@@ -1595,6 +1601,7 @@ int engine_submit(sf_engine* e, sf_batch_instance* u, cudaStream_t caller, int64
     if (off < 0) return fail(SF_ERR_BUSY, "sf_engine_submit: arena full");
     const int q = e->free_slots.back();
     e->free_slots.pop_back();
+    if (!e->at_work) e->at_work.reset(new OtherWork(e->ctx->device));   // (its packing waits for a device that is full, too)
     Slot& h = e->slots[q];
     h = Slot{};
     h.user = u;
@@ -1608,10 +1615,10 @@ int engine_submit(sf_engine* e, sf_batch_instance* u, cudaStream_t caller, int64
     if ((rc = admit(e, q, *u, e->opt.dtau_local_max ? 1 : 0))) {
         e->alloc.release(off, bytes);
         e->free_slots.push_back(q);
+        if (active_count(e) == 0) e->at_work.reset();
         return rc;
     }
     h.active = true;
-    if (!e->at_work) e->at_work.reset(new OtherWork(e->ctx->device));
     h.ticket = e->next_ticket++;
     ++e->submitted;
     if (ticket) *ticket = h.ticket;
@@ -1756,12 +1763,6 @@ int engine_round(sf_engine* e, cudaStream_t caller) {
     return SF_OK;
 }
 
-int active_count(const sf_engine* e) {
-    int n = 0;
-    for (const Slot& h : e->slots) n += h.active ? 1 : 0;
-    return n;
-}
-
 }  // namespace
 
 void sf::mixed_engine_release(sf_ctx* ctx) {
@@ -1868,6 +1869,7 @@ extern "C" int sf_solve_stokes_batch_mixed(sf_ctx* ctx, sf_batch_instance* inst,
     SF_REQUIRE(ctx && inst && n >= 1, "sf_solve_stokes_batch_mixed: bad arguments");
     int rc = set_device(ctx);
     if (rc) return rc;
+    const OtherWork at_work(ctx->device);
     int64_t total[2] = {0, 0};   // without and with second rate buffers
     for (int b = 0; b < n; ++b) {
         if ((rc = validate(inst[b], "sf_solve_stokes_batch_mixed"))) return rc;
