@@ -1,7 +1,5 @@
 """Solves for which only the smaller of two layouts finds memory: a second one keeps the first one's memory, instead of
 freeing it to find out again (another allocator could take it in between)."""
-import threading
-
 import numpy as np
 import pytest
 import torch
@@ -14,22 +12,17 @@ pytestmark = pytest.mark.gpu
 STATE = {"P": (-1, -1), "Vx": (2, 1), "Vy": (1, 2), "dVxdt": (-2, -1), "dVydt": (-1, -2), "Vx_s": (0, 1), "Vy_s": (1, 0)}
 
 
-def most_free_during(call):
-    """The device's free memory, at most, while call() runs."""
-    seen, stop = [0], threading.Event()
-
-    def watch():
-        while not stop.is_set():
-            seen[0] = max(seen[0], torch.cuda.mem_get_info()[0])
-
-    th = threading.Thread(target=watch)
-    th.start()
-    try:
-        call()
-    finally:
-        stop.set()
-        th.join()
-    return seen[0]
+def waits_for_the_device(call):
+    """Whether call() waits for a kernel of another stream, as freeing device memory does."""
+    torch.cuda.synchronize()
+    with torch.cuda.stream(torch.cuda.Stream()):
+        torch.cuda._sleep(1_000_000_000)    # half a second, one thread
+        done = torch.cuda.Event()
+        done.record()
+    call()
+    waited = done.query()
+    done.synchronize()
+    return waited
 
 
 @pytest.mark.parametrize("form", ["plain", "mixed"])
@@ -56,15 +49,16 @@ def test_second_solve_keeps_its_memory(sf, form):
         # the engine and its tables, before memory is short
         mixed({k: sf.zeros(20 + a, 20 + b) for k, (a, b) in STATE.items()}, [dev(a) for a in random_fields(20, 20, seed=1)], 20, 20)
         call = lambda: mixed(z, par, Nx, Ny)  # noqa: E731
+    torch.cuda._sleep(1)   # (its module, too, before memory is short)
     torch.cuda.synchronize()
     torch.cuda.empty_cache()
     held = torch.empty(torch.cuda.mem_get_info()[0] - (small + large) // 2, dtype=torch.uint8, device="cuda")
     try:
-        call()
-        left = torch.cuda.mem_get_info()[0]
-        assert left < large - small
+        for _ in range(3):   # (the batched solve's sweeps are timed and captured first)
+            call()
+        assert torch.cuda.mem_get_info()[0] < large - small
         scratch = ctx.scratch_bytes()
-        assert most_free_during(call) < left + small // 4, "the scratch was freed"
+        assert not waits_for_the_device(call), "the scratch was freed"
         assert ctx.scratch_bytes() == scratch
     finally:
         del held
