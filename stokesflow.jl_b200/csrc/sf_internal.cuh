@@ -156,6 +156,23 @@ void room_add_context(const sf_ctx* ctx);
 void room_remove_context(const sf_ctx* ctx);
 void markers_launched(sf_ctx* ctx, int device, int64_t nm);
 
+// What is done or looked up once per device; threads that come at the same time each do it, with the same outcome.
+constexpr int MAX_DEVICES = 64;
+struct PerDevice {
+    std::atomic<int> value[MAX_DEVICES] = {};   // 0: not yet
+    int get(int device) const { return device >= 0 && device < MAX_DEVICES ? value[device].load(std::memory_order_acquire) : 0; }
+    void set(int device, int v) {
+        if (device >= 0 && device < MAX_DEVICES) value[device].store(v, std::memory_order_release);
+    }
+};
+// lets launches of `kern` on the current device, `device`, have `bytes` of dynamic shared memory
+inline int allow_smem(PerDevice& done, int device, const void* kern, int bytes) {
+    if (done.get(device)) return SF_OK;
+    SF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+    done.set(device, 1);
+    return SF_OK;
+}
+
 inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 inline int64_t round_up(int64_t a, int64_t b) { return ceil_div(a, b) * b; }
 

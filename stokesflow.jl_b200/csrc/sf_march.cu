@@ -347,11 +347,9 @@ __global__ void __launch_bounds__(32, WPS) k_pt_march(const __grid_constant__ Ma
 template <int T, int NSS, int WPS>
 int launch(sf_ctx* ctx, const MarchMaps& maps, const MarchParams& p, cudaStream_t s) {
     using R = Ring<T, NSS>;
-    static bool ready[64] = {};
-    if (!ready[ctx->device & 63]) {
-        SF_CUDA(cudaFuncSetAttribute(k_pt_march<T, NSS, WPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, R::BYTES));
-        ready[ctx->device & 63] = true;
-    }
+    static PerDevice ready;
+    const int rc = allow_smem(ready, ctx->device, (const void*)k_pt_march<T, NSS, WPS>, R::BYTES);
+    if (rc) return rc;
     k_pt_march<T, NSS, WPS><<<(unsigned)(p.ns * p.nseg), 32, R::BYTES, s>>>(maps, p);
     SF_LAUNCHED(ctx);
     return SF_OK;

@@ -814,17 +814,17 @@ static int shape_of_rows(int rows) {
 
 // resident CTAs per SM of each shape on a device (0: not yet queried); the attribute is set per device
 static int shape_per_sm(int device, int k, int* out) {
-    static int cache[64][NSHAPES] = {};
-    if (device < 0 || device >= 64) return fail(SF_ERR_INVALID_ARG, "sf_engine: device index");
-    if (!cache[device][k]) {
+    static PerDevice cache[NSHAPES];
+    if (device < 0 || device >= MAX_DEVICES) return fail(SF_ERR_INVALID_ARG, "sf_engine: device index");
+    if (!cache[k].get(device)) {
         const SweepShape& sh = kShapes[k];
         SF_CUDA(cudaFuncSetAttribute((const void*)sh.kern, cudaFuncAttributeMaxDynamicSharedMemorySize, sh.smem));
         int n = 0;
         SF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, (const void*)sh.kern, NT, sh.smem));
         if (n < 1) return fail(SF_ERR_CUDA, "k_pt32 does not fit on an SM");
-        cache[device][k] = n;
+        cache[k].set(device, n);
     }
-    *out = cache[device][k];
+    *out = cache[k].get(device);
     return SF_OK;
 }
 
@@ -1354,11 +1354,8 @@ int launch_march32(sf_engine* e, const std::vector<int>& ids) {
     const auto kern = k_march32<MARCH_T, MARCH_WARPS>;
     int rc = upload_march_list(e, ids);
     if (rc) return rc;
-    static bool ready[64] = {};
-    if (!ready[e->ctx->device & 63]) {
-        SF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        ready[e->ctx->device & 63] = true;
-    }
+    static PerDevice ready;
+    if ((rc = allow_smem(ready, e->ctx->device, (const void*)kern, smem))) return rc;
     for (int q : ids) {
         Slot& h = e->slots[q];
         h.flips = march_launches(T, h.budget, (e->h_ctl[q].flags & CTL_CHECK) != 0);

@@ -523,9 +523,10 @@ void set_tiles(ResidentPlan& p, int64_t cols, int64_t rows, int64_t W, int64_t H
 // the largest cluster that the device places at all (one in a partition of the device may have fewer SMs together)
 int cluster_limit(int device) {
     static std::mutex m;
-    static int limit[64] = {};
+    static int limit[MAX_DEVICES] = {};
+    if (device < 0 || device >= MAX_DEVICES) return 1;
     std::lock_guard<std::mutex> lock(m);
-    int& have = limit[device & 63];
+    int& have = limit[device];
     if (have) return have;
     have = 1;
     for (int k = 0; k < CLUSTER_MAX_K; ++k)
@@ -618,7 +619,7 @@ ResidentPlan resident_plan(int64_t Nx, int64_t Ny, int num_sms) {
 }
 
 namespace {
-constexpr int ROOM_DEVICES = 64;
+constexpr int ROOM_DEVICES = MAX_DEVICES;
 std::mutex g_room_mutex;
 int g_room_used[ROOM_DEVICES] = {};       // quarters of SMs held by solves that exchange through L2, by device
 int g_room_clusters[ROOM_DEVICES] = {};   // solves that use a cluster
@@ -753,11 +754,9 @@ int resident_launch(sf_ctx* ctx, ResidentParams& p, const ResidentPlan& plan, cu
     p.W = plan.W;
     p.H = plan.H;
     const int which = kernel_of(plan);
-    static bool ready[64][RES_KERNELS] = {};
-    if (!ready[ctx->device & 63][which]) {
-        SF_CUDA(cudaFuncSetAttribute((const void*)kKernels[which], cudaFuncAttributeMaxDynamicSharedMemorySize, RES_SMEM));
-        ready[ctx->device & 63][which] = true;
-    }
+    static PerDevice ready[RES_KERNELS];
+    const int rc = allow_smem(ready[which], ctx->device, (const void*)kKernels[which], RES_SMEM);
+    if (rc) return rc;
     p.wait_ns = RES_WAIT_NS;
     int blocks = tiles;
     if (ctx->tiles_fail_ns) {   // sf_selftest_tile_wait

@@ -662,16 +662,16 @@ int encode_tmap_f32(CUtensorMap* map, const float* base, int64_t ld, int64_t row
 }
 
 static int get_encoder(PFN_encodeTiled* out) {
-    static PFN_encodeTiled fn = nullptr;
-    if (!fn) {
+    static std::atomic<PFN_encodeTiled> found{nullptr};
+    if (!found.load(std::memory_order_acquire)) {
         void* p = nullptr;
         cudaDriverEntryPointQueryResult q;
         SF_CUDA(cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q));
         if (q != cudaDriverEntryPointSuccess || !p)
             return fail(SF_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
-        fn = (PFN_encodeTiled)p;
+        found.store((PFN_encodeTiled)p, std::memory_order_release);
     }
-    *out = fn;
+    *out = found.load(std::memory_order_acquire);
     return SF_OK;
 }
 
@@ -740,16 +740,15 @@ struct Solver {
                                   L.fstride, MARCH_CW, 1, MARCH_NZ - MARCH_Z_MAT);
             if (rc) return rc;
         }
-        static bool attr_set = false;
-        if (!attr_set) {
-            SF_CUDA(cudaFuncSetAttribute(k_pt_iter<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
-            SF_CUDA(cudaFuncSetAttribute(k_pt_iter<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
-            attr_set = true;
-        }
-        static int per_sm = 0;
+        static PerDevice ready[2], blocks_per_sm;
+        int rc = allow_smem(ready[0], ctx->device, (const void*)k_pt_iter<true>, SMEM_BYTES);
+        if (!rc) rc = allow_smem(ready[1], ctx->device, (const void*)k_pt_iter<false>, SMEM_BYTES);
+        if (rc) return rc;
+        int per_sm = blocks_per_sm.get(ctx->device);
         if (!per_sm) {
             SF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pt_iter<false>, PT_THREADS, SMEM_BYTES));
             if (per_sm < 1) return fail(SF_ERR_CUDA, "k_pt_iter does not fit on an SM");
+            blocks_per_sm.set(ctx->device, per_sm);
         }
         pt.ntx = (int)ceil_div(L.Nx - 1, BX);
         pt.nty = (int)ceil_div(L.Ny - 1, BY);

@@ -52,8 +52,9 @@ def test_tiles_give_way_to_other_work(sf, beside):
     from test_gpu_parity import dev
 
     main = Solve(sf, 250, 240)               # tiles of whole SMs
-    want, alone = main(4800)
-    assert alone < 4800 / 100
+    n = 20 * 1200                            # twenty checks
+    want, alone = main(n)
+    assert alone < n / 100
     stop, begun = threading.Event(), threading.Event()
     ctx = sf.Context(0)
 
@@ -70,14 +71,14 @@ def test_tiles_give_way_to_other_work(sf, beside):
                         sf.bilinear_marker_to_grid_noalloc(0.0, 0.0, out, x, x, x, 0.01, 0.01)
                     torch.cuda.current_stream().synchronize()
             elif beside == "decomposed":
-                n = domains.local_size(2, 128)
+                nloc = domains.local_size(2, 128)
                 glob = {k: sf.zeros(128 + a, 100 + b) for k, (a, b) in domains.ARRAYS.items()}
                 for k, a in zip(("rho_vy", "mu_b", "mu_p"), random_fields(128, 100, seed=1, contrast=5.0)):
                     glob[k] = dev(a)
-                ranks = domains.split(glob, (2, 1), n, 100)
+                ranks = domains.split(glob, (2, 1), nloc, 100)
                 ctxs = {c: sf.Context(0) for c in ranks}
                 call = lambda: domains.solve_stokes_decomposed(  # noqa: E731
-                    ranks, (2, 1), n, 100, 9.81, 1 / 127, 1 / 99, 1e-4, 0.5, eps=1e-300, iter_max=600, contexts=ctxs)
+                    ranks, (2, 1), nloc, 100, 9.81, 1 / 127, 1 / 99, 1e-4, 0.5, eps=1e-300, iter_max=600, contexts=ctxs)
             else:
                 p, opt = mixed(sf, 200, 3000)
                 if beside == "batch":
@@ -98,13 +99,14 @@ def test_tiles_give_way_to_other_work(sf, beside):
     th.start()
     try:
         assert begun.wait(60)
-        got, shared = main(4800)
+        got, shared = main(n)
     finally:
         stop.set()
         th.join()
-    assert shared > 4800 / 6, "the tiles did not give way"
+    # two iterations per launch; at some checks the other thread may be between two calls
+    assert shared > n / 4, "the tiles did not give way"
     time.sleep(0.02)
-    again, after = main(4800)
+    again, after = main(n)
     assert after == alone, "the tiles did not come back"
     for k in want:
         assert np.array_equal(got[k], want[k]) and np.array_equal(again[k], want[k]), k
