@@ -49,7 +49,7 @@ def test_second_solve_keeps_its_memory(sf, form):
         # the engine and its tables, before memory is short
         mixed({k: sf.zeros(20 + a, 20 + b) for k, (a, b) in STATE.items()}, [dev(a) for a in random_fields(20, 20, seed=1)], 20, 20)
         call = lambda: mixed(z, par, Nx, Ny)  # noqa: E731
-    torch.cuda._sleep(1)   # (its module, too, before memory is short)
+    waits_for_the_device(lambda: None)   # (its streams and module, too, before memory is short)
     torch.cuda.synchronize()
     torch.cuda.empty_cache()
     held = torch.empty(torch.cuda.mem_get_info()[0] - (small + large) // 2, dtype=torch.uint8, device="cuda")
