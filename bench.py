@@ -589,8 +589,8 @@ def run_precision_form(a, *, n=None, cases=None, steps=None, contrast=None):
         out_cases.append({"contrast": C, "mu_plume": model.mu_plume, "fp64_solve_ms_total": round(fs, 1),
                           "mixed_solve_ms_total": round(ms, 1), "solve_speedup": round(fs / ms, 3),
                           "same_iterations": all(r["fp64_iters"] == r["mixed_sweeps"] for r in rows),
-                          "sweeps": {k: eng.get(k) for k in ("tile_rows", "tile_schedule", "overlap_launches",
-                                                             "tune_state")},
+                          "sweeps": {k: eng.get(k) for k in ("sweeps_per_launch", "tile_rows", "tile_schedule",
+                                                             "overlap_launches", "tune_state")},
                           "steps": rows})
         del states
         mctx.close()

@@ -395,8 +395,9 @@ enum {
  * Ny), 2000) on the same quantities as the reference's, and the solve stops at
  * the first check with err <= eps or after max_sweeps iterations -- so it stops
  * at the same iteration as sf_solve_stokes on the same inputs, apart from a
- * check whose err lies within FP32 rounding of eps.  One sweep of every
- * instance still iterating is a single kernel launch over a shared tile list.
+ * check whose err lies within FP32 rounding of eps.  A kernel launch covers
+ * every instance still iterating: one sweep over a shared list of tiles, or
+ * three over a shared list of strips.
  * opt may be NULL (defaults above).  Synchronises the stream.  The results are
  * FP32-accurate corrections of an FP64 solution, not bit-identical to
  * sf_solve_stokes. */
@@ -435,15 +436,18 @@ typedef struct {
     int64_t arena_used;        /* bytes held by admitted instances              */
     int64_t arena_peak;
     int64_t submitted, finished, rounds;
-    int64_t sweeps;            /* FP32 sweep launches (one covers all instances) */
+    int64_t sweeps;            /* FP32 sweeps (one covers all instances)         */
     int32_t active;            /* admitted, not finished                         */
     int32_t pending_results;   /* finished, not yet reported by sf_engine_step   */
-    int32_t tile_rows;         /* rows of the sweep tiles in use                 */
-    int32_t tile_schedule;     /* 1 strided, 2 chunked                           */
-    int32_t overlap_launches;  /* 1: sweeps launched overlapped                  */
+    int32_t tile_rows;         /* rows of the sweep tiles, of launches of one sweep: given by the options,
+                                  or the tuner's choice.  A batched solve with tile_rows 0 takes the choice
+                                  while it measures a class, and after that only where its launches do one
+                                  sweep each (sweeps_per_launch)                          */
+    int32_t tile_schedule;     /* 1 strided, 2 chunked (likewise)                */
+    int32_t overlap_launches;  /* 1: sweeps launched overlapped (likewise)       */
     int32_t tune_state;        /* SF_TUNE_* for the current workload class       */
     int32_t tune_classes;      /* workload classes with a recorded choice in the context */
-    int32_t reserved;
+    int32_t sweeps_per_launch; /* of the last round's launches: 1 (tiles), 3 (a batched solve's march), 0: none yet */
     int64_t tune_rounds;       /* rounds whose sweeps began with timed trial pieces */
     int64_t tune_hits;         /* workload-class changes answered from the context's record */
     double tune_ns[12];        /* the last completed measurement: ns per point-sweep of each candidate,

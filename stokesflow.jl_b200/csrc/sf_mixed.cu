@@ -971,6 +971,7 @@ struct sf_engine {
     int blocks = 0;                      // persistent CTAs of the current shape
     // the march: what the batched solve's sweeps run once their workload class is measured
     bool rates_b = false;                // instances have second rate buffers
+    int per_launch = 0;                  // sweeps of the last round's launches
     CUtensorMap* d_march_maps = nullptr; // [slot][M_NUM_MARCH]
     MItem* d_items = nullptr;
     int64_t item_cap = 0;
@@ -1350,6 +1351,7 @@ int launch_trials(sf_engine* e, const std::vector<int>& ids, double points) {
 // one fold's worth of sweeps over the sweep set `ids`, marching
 int launch_march32(sf_engine* e, const std::vector<int>& ids) {
     const int K = e->opt.fold_every, T = MARCH_T;
+    e->per_launch = T;
     constexpr int smem = MRing::BYTES;
     const auto kern = k_march32<MARCH_T, MARCH_WARPS>;
     int rc = upload_march_list(e, ids);
@@ -1394,6 +1396,7 @@ int launch_march32(sf_engine* e, const std::vector<int>& ids) {
 int launch_sweeps(sf_engine* e, const std::vector<int>& ids) {
     const int K = e->opt.fold_every;
     int rc;
+    e->per_launch = 1;
     for (int q : ids) {   // k_pt32: the buffers change with every sweep, the rates stay where they are
         e->slots[q].flips = e->slots[q].budget;
         e->slots[q].rflips = 0;
@@ -1849,6 +1852,7 @@ extern "C" int sf_engine_get_stats(sf_engine* e, sf_engine_stats* st) {
     st->overlap_launches = e->overlap;
     st->tune_state = e->tune_state;
     st->tune_classes = (int32_t)e->ctx->sweep_shapes.size();
+    st->sweeps_per_launch = e->per_launch;
     st->tune_rounds = e->tune_rounds;
     st->tune_hits = e->tune_hits;
     for (int k = 0; k < NCAND; ++k) st->tune_ns[k] = e->tune_ns[k];

@@ -327,8 +327,9 @@ def mixed_options(max_sweeps=4_000_000, fold_every=400, use_graphs=True, dtau_lo
 
 
 def batch_stats(ctx: Context | None = None) -> dict:
-    """Stats of the engine behind the context's last batched / mixed solve (sf_ctx_batch_stats): the sweep
-    tile rows and schedule in use, the tuner's state and its measured ns per point-sweep of each candidate
+    """Stats of the engine behind the context's last batched / mixed solve (sf_ctx_batch_stats): the sweeps per
+    launch of its last round (3 once a class is measured and the second rate buffers fit), the tile rows and
+    schedule of its single sweeps, the tuner's state and its measured ns per point-sweep of each candidate
     ((rows, schedule) -> ns)."""
     s = _lib.EngineStats()
     check(lib().sf_ctx_batch_stats(_ctx(ctx).handle, C.byref(s)), "sf_ctx_batch_stats")
