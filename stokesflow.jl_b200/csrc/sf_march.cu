@@ -21,7 +21,7 @@
 // reference's order of operations (and the file is compiled without contraction): bit-identical to T single
 // iterations.
 //
-// What bounds it: at 2048^2 a launch of three iterations moves 558 MB (128 B per point and the halos) in 100 us, 5.5 TB/s,
+// What bounds it: at 2048^2 a launch of three iterations moves 549 MB (128 B per point and the halos) in 100 us, 5.4 TB/s,
 // with the FP64 pipe some 60% busy; on smaller grids the halo rows of short segments.  85 -> 33.5 us per iteration at
 // 2048^2, 241 -> 97 at 4001 x 3003, 24.6 -> 11.9 at 1024^2; in runs of seconds, which draw the 1000 W limit and settle at
 // 1.69 GHz, 89.9 -> 37.5, 258 -> 105 and (1.86 GHz) 24.6 -> 12.4.  One warp per block, 234 registers, 8 blocks per SM (two warps
@@ -359,11 +359,16 @@ constexpr int WARPS_PER_SM = 8;
 
 }  // namespace
 
-// A warp of a grid of some 600 points per side or less has few rows of its own, and the rows above and below that it
-// computes for T = 3 outweigh what a third iteration saves: 5.5 us per iteration with T = 2 against 6.4 at 511 x 385
-// points (where no resident tiles are to be had), but 13.9 against 12.7 at 1024^2 and 54.4 against 37.3 at 2048^2 (T = 1:
-// 8.4, 24.7, 101.5), timed before the items' code was made one.
-int march_iterations(int64_t Nx, int64_t Ny) { return Nx * Ny < 600 * 600 ? 2 : 3; }
+// The rows above and below that a warp computes for a third iteration outweigh what it saves where segments are short but
+// the launch is not all latency.  Microseconds per iteration with T = 2 : T = 3: 100^2 3.80 : 3.67, 150^2 3.77 : 3.64, 200^2
+// 4.28 : 3.63, 225^2 4.28 : 3.65, 600 x 100 4.31 : 3.62; 250^2 4.26 : 4.33, 300^2 4.26 : 4.61, 350^2 5.29 : 5.63, 375^2 5.32 :
+// 5.67, 900 x 150 5.33 : 5.67; 400^2 5.72 : 5.64, 425^2 5.81 : 5.64, 450^2 5.31 : 5.64, 475^2 5.77 : 5.64, 500^2 5.89 : 5.68, 600^2
+// 6.72 : 6.39, 700^2 7.94 : 7.49, 800^2 9.68 : 9.32, 1024^2 13.95 : 12.21, 2048^2 54.4 : 37.3 (T = 1: 101.5).
+// (Below 530^2 solves march only where no resident tiles are to be had.)
+int march_iterations(int64_t Nx, int64_t Ny) {
+    const int64_t points = Nx * Ny;
+    return points >= 240 * 240 && points < 400 * 400 ? 2 : 3;
+}
 
 void march_plan(MarchParams& p, int T, int num_sms) {
     const int te = left_halo(T);

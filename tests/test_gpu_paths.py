@@ -50,10 +50,21 @@ def expected(n, per_launch, ncheck, ndt, resident):
     (4, 4, "cluster", 20000), (20, 26, "cluster", 20000), (85, 85, "cluster", 20000), (108, 108, "cluster", 20000),
     (170, 40, "cluster", 20000), (120, 120, "L2", 20000), (200, 150, "L2", 20000), (300, 301, "L2", 20000),
     (240, 240, "L2", 512), (511, 385, "L2", 512), (529, 529, "L2", 512),
-    (601, 605, "march", 3), (58, 6400, "march", 3), (1023, 1101, "march", 3), (20000, 18, "march", 3)])
+    (601, 605, "march", 3), (58, 6400, "march", 3), (58, 5400, "march", 3), (551, 551, "march", 3), (1023, 1101, "march", 3), (20000, 18, "march", 3)])
 def test_path_of_a_solve(sf, Nx, Ny, kind, per_launch):
     ncheck, ndt = min(5 * min(Nx, Ny), 2000), 10 * min(Nx, Ny)
     n = min(2 * ncheck + 17, 1200)
     got, extra = launches(sf, Nx, Ny, n)
     assert got == expected(n, per_launch, ncheck, ndt, kind != "march")
     assert (extra > 0) == (kind == "L2")
+
+
+@pytest.mark.parametrize("Nx,Ny,per_launch", [(235, 230, 3), (250, 240, 2), (395, 400, 2), (402, 400, 3)])
+def test_iterations_per_launch_where_tiles_are_lost(sf, Nx, Ny, per_launch):
+    """The march of grids that have tiles: two iterations per launch between 240^2 and 400^2 points."""
+    sf.selftest_tile_wait(1_000_000, ctx=sf.default_context())
+    z = {k: sf.zeros(Nx + a, Ny + b) for k, (a, b) in STATE.items()}
+    par = [dev(a) for a in random_fields(Nx, Ny, seed=1, contrast=5.0)]
+    info = sf.solve_stokes_info(z["P"], z["Vx"], z["Vy"], *par, *[None] * 7, z["dVxdt"], z["dVydt"], None, None, z["Vx_s"],
+                                z["Vy_s"], 9.81, 1 / (Nx - 1), 1 / (Ny - 1), Nx, Ny, 1e-3, 0.5, eps=1e-300, iter_max=200)
+    assert info["fused_launches"] == expected(200, per_launch, 2000, 10 * min(Nx, Ny), False)
