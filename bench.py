@@ -44,9 +44,36 @@ METRIC = "PT T_eff (essential HBM bytes of the PT iterations / time), FP64, rela
 UNIT = "GB/s"
 MEASURED_PEAKS = os.path.join(ROOT, "MEASURED_PEAKS.json")
 FALLBACK_HBM_GBS = 6650.0
-MARCH_ITERS = 3                       # iterations per launch of k_pt_march at the benchmark's size
+MARCH_MAX_ITERS = 3                   # iterations per launch of k_pt_march at most
 MARCH_BYTES_PER_POINT = 16 * 8        # of a launch: 5 state fields read and written, 6 parameter fields read
+ITER_BYTES_PER_POINT = 13 * 8         # of k_pt_iter: 5 state fields read and written, rho_vy, mu_b, mu_p read
+L2_BYTES = 126e6
 TRAFFIC_PER_LAUNCH_2048 = 549.1e6     # dram__bytes_read.sum + dram__bytes_write.sum, k_pt_march<3>, 2047^2 points
+
+
+def roofline(n, iters, launches, loop_ms, peak, peak_source):
+    """The PT loop against the measured copy rate.  iters iterations of an n x n grid in `launches` launches say which
+    kernel ran them: k_pt_march does two or three per launch, one pass over memory each; k_pt_iter one (where memory is short);
+    k_pt_resident hundreds, with the state on the chip, where HBM bounds nothing."""
+    per_launch = round(iters / max(launches, 1))
+    if per_launch > MARCH_MAX_ITERS:
+        return {"bound": "latency", "kernel": "k_pt_resident (state on the chip)", "achieved": None, "peak": peak,
+                "peak_source": peak_source, "unit": "GB/s", "frac": None, "traffic": None,
+                "note": "no pass over memory per iteration; see us_per_iter"}
+    bytes_launch = (MARCH_BYTES_PER_POINT if per_launch > 1 else ITER_BYTES_PER_POINT) * (n - 1) ** 2
+    achieved = bytes_launch / per_launch * iters / (loop_ms * 1e-3) / 1e9
+    # DRAM bytes (read + write) of one launch, measured by ncu at 2047^2 points with three iterations, scaled by the point
+    # count (the kernel streams each field once per launch); given for that form, where the fields exceed the L2
+    traffic = TRAFFIC_PER_LAUNCH_2048 * ((n - 1) / 2047.0) ** 2 if per_launch == 3 and bytes_launch > 2 * L2_BYTES else None
+    return {"bound": "hbm",
+            "kernel": f"k_pt_march ({per_launch} PT iterations per launch)" if per_launch > 1 else "k_pt_iter",
+            "achieved": round(achieved, 1), "peak": peak, "peak_source": peak_source, "unit": "GB/s",
+            "frac": round(achieved / peak, 4), "traffic": None if traffic is None else round(traffic),
+            "algorithmic_bytes_per_launch": bytes_launch,
+            "note": "achieved = algorithmic bytes of a launch x launches / PT-loop device time (CUDA events; "
+                    "checks and dt updates included, pack/unpack excluded); traffic from ncu per launch.  The "
+                    "metric's T_eff counts bytes_per_iter for every iteration and may exceed the peak: a "
+                    "launch does several iterations in one pass over memory"}
 
 
 # ---------------------------------------------------------------------------
@@ -405,19 +432,7 @@ def run_ours(a, rank, world, local_rank):
         "bytes_per_iter": bpi, "us_per_iter": round(loop_ms * 1e3 / max(iters, 1), 3)}
     out["ms_per_timestep"] = {k: round(sum(getattr(r["times"], k) for r in recs) / len(recs), 3)
                               for k in ("deposit_ms", "solve_ms", "advect_ms", "rebin_ms")}
-    bytes_launch = MARCH_BYTES_PER_POINT * (a.n - 1) ** 2
-    achieved = bytes_launch / MARCH_ITERS * iters / (loop_ms * 1e-3) / 1e9
-    # DRAM bytes (read + write) of one k_pt_march launch, measured by ncu at 2047^2 points, scaled by the
-    # point count (the kernel streams each field once per launch, so its traffic grows with the points)
-    traffic = TRAFFIC_PER_LAUNCH_2048 * ((a.n - 1) / 2047.0) ** 2
-    out["roofline"] = {"bound": "hbm", "kernel": f"k_pt_march ({MARCH_ITERS} PT iterations per launch)",
-                       "achieved": round(achieved, 1),
-                       "peak": peak, "peak_source": peak_src, "unit": "GB/s", "frac": round(achieved / peak, 4),
-                       "traffic": round(traffic), "algorithmic_bytes_per_launch": bytes_launch,
-                       "note": "achieved = algorithmic bytes of a launch x launches / PT-loop device time (CUDA events; "
-                               "checks and dt updates included, pack/unpack excluded); traffic from ncu per launch.  The "
-                               "metric's T_eff counts bytes_per_iter for every iteration and may exceed the peak: a "
-                               "launch does several iterations in one pass over memory"}
+    out["roofline"] = roofline(a.n, iters, sum(r["info"]["fused_launches"] for r in recs), loop_ms, peak, peak_src)
     out["clocks"] = clk
     out["gpu_launches"] = launches
     # ---- end to end through the public API with host buffers ----
