@@ -829,7 +829,6 @@ int sf_bilinear_marker_to_grids(sf_ctx* ctx, const sf_deposit_grid* grids, int n
     SF_REQUIRE(nm < (int64_t)INT32_MAX, "sf_bilinear_marker_to_grids: more than 2^31-1 markers");
     SF_REQUIRE(dx > 0.0 && dy > 0.0, "sf_bilinear_marker_to_grids: dx, dy must be positive");
     SF_REQUIRE((val_wt_sum == nullptr) == (wt_sum == nullptr), "sf_bilinear_marker_to_grids: give both sum arrays or neither");
-    int64_t total_cells = 0;
     for (int g = 0; g < n_grids; ++g) {
         const sf_deposit_grid& d = grids[g];
         SF_REQUIRE(d.val_grid && d.nx >= 1 && d.ny >= 1, "sf_bilinear_marker_to_grids: bad grid");
@@ -838,7 +837,6 @@ int sf_bilinear_marker_to_grids(sf_ctx* ctx, const sf_deposit_grid* grids, int n
         if (wt_sum)
             SF_REQUIRE(ld_sum >= d.nx && n_sum >= ld_sum * (d.ny - 1) + d.nx,
                        "sf_bilinear_marker_to_grids: sum arrays too small");
-        total_cells += (d.nx + 1) * (d.ny + 1) + 1;
     }
     int rc = set_device(ctx);
     if (rc) return rc;

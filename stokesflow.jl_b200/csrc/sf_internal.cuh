@@ -82,7 +82,7 @@ struct sf_ctx {
     sf::Scratch fields, partials, mixed;
     // decomposed timestep: marker-exchange and overlap-sum staging
     sf::Scratch exch;
-    // resident iterations: the tiles' halo slots, and the tag of the next iteration (0: none yet)
+    // resident iterations: the tiles' halo slots, and the tag of the next iteration (1 at first: slots start zeroed)
     sf::Scratch halo;
     uint32_t halo_tag = 1;
     cudaStream_t work = nullptr;  // private non-blocking stream (graph capture needs a non-legacy stream)
